@@ -554,6 +554,7 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
     FamDev& d = Lo.F[k];
     StatsArgs& A = d.sa;
     memset(&A, 0, sizeof(A));
+    A.negzero2 = NEGZERO2;
     A.cnt = T.need_w ? d.cnt : nullptr;
     A.ucnt = T.need_u ? d.ucnt : nullptr;
     A.pm = d.pm; A.pmdf = d.pmdf; A.lpi = d.lpi; A.logtab = b->d_logtab; A.meanp = d.meanp;
@@ -653,6 +654,7 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
   const FamDev* dF = reinterpret_cast<const FamDev*>(S.tab + oF);
   auto P = [&](size_t o) { return reinterpret_cast<const int*>(S.tab + o); };
   if (pup.total() && !grp_weights_gsc_prepare()) return bfail(b, 90, "GSC kernel attributes");
+  if (!stats_grid()) return bfail(b, 90, "statistics kernel attributes");
 
   // the key of this chunk's device passes: the descriptor tables (they hold
   // every pointer and size the launches read) and the launch parameters

@@ -682,6 +682,7 @@ static int score_async(covgpu_ctx* ctx, int first, int nslots, int ntypes, const
   unsigned mask = 0;
   StatsArgs A;
   memset(&A, 0, sizeof(A));
+  A.negzero2 = NEGZERO2;
   CorrTypes ct;
   ct.nout = ntypes;
   int rafs_q[MAXOUT], nrafs = 0;

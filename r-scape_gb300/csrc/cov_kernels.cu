@@ -20,11 +20,12 @@
 // FP64 is kept for the row/column means, a bin next to a bin boundary, and
 // the E-value tables.
 #include "cov_dev.cuh"
-#include "cov_df.cuh"
+#include "cov_df2.cuh"
 #include "cov_kernels.h"
 #include "cov_batch.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -516,8 +517,67 @@ __device__ __forceinline__ bool above_h(df H) {   // H > 1e-2 as the FP64 value 
   return (H.hi > 0.0100001f) || (H.hi > 0.0099999f && df_to_d(H) > 1e-2);
 }
 
-template <unsigned CF>
-__device__ __forceinline__ void pair_stats(const StatsArgs& A, const df (&c)[16], const float (&uc)[16],
+// RAF of a pair from the sums of its unit counts over the allowed cells:
+// c_ij = nA^2 - (sum r_x^2 + sum c_y^2)/2 in 64-bit integers (the counts are
+// integers below 2^24, c_ij below 2^48), then split exactly into a
+// double-float (sum r_x^2 + sum c_y^2 is even: each sum has the parity of nA)
+__device__ __forceinline__ df raf_of(const StatsArgs& A, float nAf, const float (&r)[4], const float (&cc)[4]) {
+  int64_t sq = 0;
+#pragma unroll
+  for (int x = 0; x < 4; x++) {
+    const int a = (int)r[x], b = (int)cc[x];
+    sq += (int64_t)a * a + (int64_t)b * b;
+  }
+  const int nA = (int)nAf;
+  const int64_t ci = (int64_t)nA * nA - sq / 2;
+  const float ci_hi = (float)ci;
+  const df cnum = {ci_hi, (float)(ci - (int64_t)ci_hi)};   // exact: the rest is an integer below 2^24
+  const df q1 = df_mul(cnum, {A.invD.x, A.invD.y});
+  const df q2 = df_mul({(float)A.N - nAf, 0.f}, {A.invN.x, A.invN.y});
+  return df_add({2.f * q1.hi, 2.f * q1.lo}, df_neg(q2));
+}
+
+// CCF (src/correlators.c:1038-1053), FP64: the sum over the cells of
+// ((nseff pm_i(x) - mean(x)) (nseff pm_j(y) - mean(y)))^2 is the product of the
+// two columns' sums of squares (FP64 runs at 1/64 of the FP32 rate here: 24
+// operations a pair instead of 80)
+__device__ __forceinline__ df ccf_of(double ned, const double* pmid, const double* pmjd, const double* meanp) {
+  double si = 0.0, sj = 0.0;
+#pragma unroll
+  for (int x = 0; x < 4; x++) {
+    const double a = ned * pmid[x] - meanp[x], b = ned * pmjd[x] - meanp[x];
+    si += a * a;
+    sj += b * b;
+  }
+  return df_of(sqrt(si * sj));
+}
+
+// a pair without a sequence with both residues canonical: pp = 1/16 (prior
+// only), FP64; CHI, GT and OMES are 0 and MIg = MI
+struct PriorStats { df mi, mir; };
+__device__ __noinline__ PriorStats prior_stats(const float* allow, int cls, const double* pmid, const double* pmjd) {
+  double mi = 0.0, hh = 0.0;
+  if (cls != 1) {
+    for (int x = 0; x < 4; x++)
+      for (int y = 0; y < 4; y++) {
+        const double p = 0.0625;
+        if (pmid[x] > 0.0 && pmjd[y] > 0.0) mi += p * (log(p) - log(pmid[x]) - log(pmjd[y]));
+        hh -= p * log(p);
+      }
+  } else {
+    double pw = 0, pn = 0, qw = 0, qn = 0;
+    for (int x = 0; x < 4; x++)
+      for (int y = 0; y < 4; y++) {
+        if (allow[x * 4 + y] > 0.f) { pw += 0.0625; qw += pmid[x] * pmjd[y]; }
+        else                          { pn += 0.0625; qn += pmid[x] * pmjd[y]; }
+      }
+    if (pw > 0.0) { mi += pw * (log(pw) - log(qw)); hh -= pw * log(pw); }
+    if (pn > 0.0) { mi += pn * (log(pn) - log(qn)); hh -= pn * log(pn); }
+  }
+  return {df_of(mi), df_of((hh > 1e-2) ? mi / hh : 0.0)};
+}
+
+__device__ __forceinline__ void merged_stats(const StatsArgs& A, const df (&c)[16], const float (&uc)[16],
                                            bool have_uc, const float2* pmi, const float2* pmj, const float4* lpi,
                                            const float4* lpj, const double* pmid, const double* pmjd,
                                            const double* meanp, const float4* tab, PairOut& out) {
@@ -536,23 +596,7 @@ __device__ __forceinline__ void pair_stats(const StatsArgs& A, const df (&c)[16]
           const float n = uc[x * 4 + y];
           nAf += n; r[x] += n; cc[y] += n;
         }
-    // c_ij = nA^2 - (sum r_x^2 + sum c_y^2)/2 in 64-bit integers (the
-    // counts are integers below 2^24, c_ij below 2^48), then split exactly
-    // into a double-float
-    // (sum r_x^2 + sum c_y^2 is even: each sum has the parity of nA)
-    int64_t sq = 0;
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-      const int a = (int)r[x], b = (int)cc[x];
-      sq += (int64_t)a * a + (int64_t)b * b;
-    }
-    const int nA = (int)nAf;
-    const int64_t ci = (int64_t)nA * nA - sq / 2;
-    const float ci_hi = (float)ci;
-    const df cnum = {ci_hi, (float)(ci - (int64_t)ci_hi)};   // exact: the rest is an integer below 2^24
-    const df q1 = df_mul(cnum, {A.invD.x, A.invD.y});
-    const df q2 = df_mul({(float)A.N - nAf, 0.f}, {A.invN.x, A.invN.y});
-    out.raf = df_add({2.f * q1.hi, 2.f * q1.lo}, df_neg(q2));
+    out.raf = raf_of(A, nAf, r, cc);
   }
   // ---- CCF (src/correlators.c:1038-1053), FP64 ----
   df ne;
@@ -564,106 +608,23 @@ __device__ __forceinline__ void pair_stats(const StatsArgs& A, const df (&c)[16]
   }
   if (S & S_CCF) {
     const double ned = df_to_d(ne);
-    double ccf = 0.0;
-#pragma unroll
-    for (int x = 0; x < 4; x++)
-#pragma unroll
-      for (int y = 0; y < 4; y++) {
-        const double cc = (ned * pmid[x] - meanp[x]) * (ned * pmjd[y] - meanp[y]);
-        ccf += cc * cc;
-      }
-    out.ccf = df_of(sqrt(ccf));
+    out.ccf = ccf_of(ned, pmid, pmjd, meanp);
   }
   const unsigned SP = S & (S_CHI | S_GT | S_MI | S_MIr | S_MIg | S_OMES);
   if (!SP) return;
 
   if (ne.hi <= 0.f) {
-    // no sequence with both residues canonical: pp = 1/16 (prior only)
-    double mi = 0.0, hh = 0.0;
-    if (A.cls != 1) {
-      for (int x = 0; x < 4; x++)
-        for (int y = 0; y < 4; y++) {
-          const double p = 0.0625;
-          if (pmid[x] > 0.0 && pmjd[y] > 0.0) mi += p * (log(p) - log(pmid[x]) - log(pmjd[y]));
-          hh -= p * log(p);
-        }
-    } else {
-      double pw = 0, pn = 0, qw = 0, qn = 0;
-      for (int x = 0; x < 4; x++)
-        for (int y = 0; y < 4; y++) {
-          if (A.allow[x * 4 + y] > 0.f) { pw += 0.0625; qw += pmid[x] * pmjd[y]; }
-          else                          { pn += 0.0625; qn += pmid[x] * pmjd[y]; }
-        }
-      if (pw > 0.0) { mi += pw * (log(pw) - log(qw)); hh -= pw * log(pw); }
-      if (pn > 0.0) { mi += pn * (log(pn) - log(qn)); hh -= pn * log(pn); }
-    }
+    const PriorStats z = prior_stats(A.allow, A.cls, pmid, pmjd);
     out.chi = out.gt = out.omes = df{0.f, 0.f};
-    out.mi = df_of(mi); out.mir = df_of((hh > 1e-2) ? mi / hh : 0.0); out.mig = df_of(mi);
+    out.mi = out.mig = z.mi;
+    out.mir = z.mir;
     return;
   }
 
   const df Z = df_add_f(ne, 16.f * 1e-10f);
   const df iZ = df_recip(Z);
   const df wt = {A.wtot.x, A.wtot.y};
-  if (A.cls == 0) {
-    // ---- C16: one pass over the cells ----
-    df R[4], K[4], T[4], V[4], Sx = {0.f, 0.f}, W = {0.f, 0.f};
-#pragma unroll
-    for (int x = 0; x < 4; x++) R[x] = K[x] = T[x] = V[x] = df{0.f, 0.f};
-#pragma unroll
-    for (int x = 0; x < 4; x++)
-#pragma unroll
-      for (int y = 0; y < 4; y++) {
-        const df cp = df_add_f(c[x * 4 + y], 1e-10f);
-        df_acc(R[x], cp);
-        df_acc(K[y], cp);
-        if (CF & CF_G) df_acc(Sx, df_mul_u(cp, df_log(cp, tab)));
-        if (CF & (CF_CHI | CF_OMES)) {
-          const df sq = df_sqr_u(cp);
-          if (CF & CF_CHI) df_acc(T[x], df_mul_u(sq, {lpj[y].z, lpj[y].w}));
-          if (CF & CF_OMES) { df_acc(W, sq); df_acc(V[x], df_mul_u(cp, {pmj[y].x, pmj[y].y})); }
-        }
-      }
-    if (CF & CF_G) {
-      const df Sn = df_norm(Sx);
-      const df lnZ = df_log(Z, tab);
-      df P = {0.f, 0.f};
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        df_acc(P, df_mul_u(df_norm(R[x]), {lpi[x].x, lpi[x].y}));
-        df_acc(P, df_mul_u(df_norm(K[x]), {lpj[x].x, lpj[x].y}));
-      }
-      const df Mn = df_sub(df_sub(Sn, df_mul(Z, lnZ)), df_norm(P));
-      const df mi = df_mul(Mn, iZ);
-      out.mi = mi;
-      out.gt = df_scale(df_mul(ne, mi), 2.f);
-      // the mask is the same for every thread: no divergence
-      if (S & S_MIr) {
-        const df H = df_sub(lnZ, df_mul(Sn, iZ));
-        out.mir = above_h(H) ? df_div(mi, H) : df{0.f, 0.f};
-      }
-      if (S & S_MIg) out.mig = df_sub(mi, df_div(df_sub(wt, ne), ne));
-    }
-    if (CF & CF_CHI) {
-      df Q = {0.f, 0.f};
-#pragma unroll
-      for (int x = 0; x < 4; x++) df_acc(Q, df_mul_u(df_norm(T[x]), {lpi[x].z, lpi[x].w}));
-      out.chi = df_sub(df_mul(df_mul(ne, df_mul(iZ, iZ)), df_norm(Q)), ne);
-    }
-    if (CF & CF_OMES) {
-      df U = {0.f, 0.f}, Ai = {0.f, 0.f}, Aj = {0.f, 0.f};
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        df_acc(U, df_mul_u({pmi[x].x, pmi[x].y}, df_norm(V[x])));
-        df_acc(Ai, df_sqr_u({pmi[x].x, pmi[x].y}));
-        df_acc(Aj, df_sqr_u({pmj[x].x, pmj[x].y}));
-      }
-      const df t1 = df_mul(df_norm(W), df_mul(iZ, iZ));
-      const df t2 = df_scale(df_mul(df_norm(U), iZ), 2.f);
-      const df t3 = df_mul(df_norm(Ai), df_norm(Aj));
-      out.omes = df_mul(ne, df_add(df_sub(t1, t2), t3));
-    }
-  } else if (A.cls == 2) {
+  if (A.cls == 2) {
     // ---- GT, CWC: the allowed cells only ----
     df SA = {0.f, 0.f}, CA = {0.f, 0.f}, PA = {0.f, 0.f};
 #pragma unroll
@@ -726,16 +687,339 @@ __device__ __forceinline__ void pair_stats(const StatsArgs& A, const df (&c)[16]
   }
 }
 
-// One CTA per (tile, alignment), 256 threads, thread tid owns the pairs
-// p = tid + 256k (row a = warp + 8k, column b = lane).  Each pair's scores
-// go straight to the score planes and into a shared-memory copy of the
-// tile; after the tile, one thread per (row, output) adds its row and one
-// per (column, output) its column in double-float, in a fixed order, for the
-// APC/ASC partials.
+// Persistent CTAs of 256 threads work through (tile, alignment) tasks.  Each
+// pair's scores go straight to the score planes and into a shared-memory copy
+// of the tile; after the tile, one thread per (row, output) adds its row and
+// one per (column, output) its column in double-float, in a fixed order, for
+// the APC/ASC partials.
+//
+// C16 pairs (c16_tile) go two at a time, the adjacent columns (b, b + 1) of
+// one row as the halves of packed FP32 instructions (cov_df2.cuh): a count
+// plane's two values are one 8-byte access.  Thread tid owns rows (tid >> 4) and
+// (tid >> 4) + 16, columns 2 (tid & 15) + {0, 1}.  Every operation rounds as
+// the scalar one would.
+//
+// The counts come through a ring of three rows of cells (8 planes x 8 bytes of
+// each thread) that the thread fills for itself with cp.async two rows ahead,
+// across tiles: no barrier, and no load latency in the chain.  The columns'
+// tables are staged the same way one tile ahead (double-buffered; one load
+// gives the values of both columns j, and of i to both halves).
+//
+// Bound: the FMA pipe and the latency of its chains (58-63% of the pipe busy,
+// 16 warps of 122-128 registers per SM); HBM at 0.27 of its rate.  Against the
+// form before (one pair per thread and scalar operations, counts loaded where
+// they are used, one CTA per tile): 138 for 206 warp instructions per 32
+// pairs of GT, MI, CHI and RAF; 8.53 for 9.53 ms on 21 alignments of
+// 2,000 x 3,000; GT alone 1.16 for 1.44 ms on 201 alignments of 500 x 400.
+constexpr int STATS_UC = 6;   // allowed cells staged; with more, RAF reads its counts directly
+struct StatsSmem {
+  float2 ring[3][8][256];             // [row of cells][cell and word][thread]: a plane's two values
+  float2 vs[MAXOUT][TP][TP + 1];      // the tile's scores, [q][a][b]
+  float4 tab[LOGTAB_TOT];
+  float2 uc[STATS_UC][256];           // unit counts of the allowed cells (RAF), the next half tile's
+  float col[2][2][6][4][TP];          // [buffer][j, i][{ln pm, 1/pm, pm} x {hi, lo}][state][column]
+};
+static_assert(LOGTAB_TOT <= 256, "one table entry per thread");
+// two CTAs on an SM: (228 KB - 2 KB reserved) / 2
+static_assert(sizeof(StatsSmem) <= 113 * 1024, "two CTAs per SM");
+
+// a (tile, alignment) task: its pass arguments and place
+struct StatsTask { const StatsArgs* A; int t, slot; };
+
+__device__ __forceinline__ void cpa8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cpa4z(void* dst, const void* src, bool ok) {   // zero fill when !ok
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(ok ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cpa_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cpa_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+__device__ __forceinline__ bool stats_c16(const StatsTask& T) { return T.A->cls == 0 && T.A->cnt; }
+
+// the column tables of a task into buffer buf: threads 0-127 the columns j,
+// the others i; columns past L are 0 (their pairs are not valid)
 template <unsigned CF>
-__device__ __forceinline__ void stats_body(
-    const GridIdx g, StatsArgs A) {
-  const int t = g.x, slot = g.y, tid = threadIdx.x;
+__device__ __forceinline__ void stats_tables(const StatsTask& T, StatsSmem& sm, int buf) {
+  const StatsArgs& A = *T.A;
+  const TileRC tr = A.tiles[T.t];
+  const int tid = threadIdx.x, side = tid >> 7, c = (tid & 127) >> 2, x = tid & 3;
+  const int col = (side ? tr.I : tr.J) * TP + c;
+  const bool ok = col < A.L;
+  const int64_t o = ((int64_t)T.slot * A.Lp + (ok ? col : 0)) * 4 + x;
+  const float* l = reinterpret_cast<const float*>(A.lpi + o);
+#pragma unroll
+  for (int k = 0; k < 4; k++) cpa4z(&sm.col[buf][side][k][x][c], l + k, ok);
+  if (CF & CF_OMES) {
+    const float* p = reinterpret_cast<const float*>(A.pmdf + o);
+#pragma unroll
+    for (int k = 0; k < 2; k++) cpa4z(&sm.col[buf][side][4 + k][x][c], p + k, ok);
+  }
+}
+
+// the number of allowed cells when RAF's counts are staged, else 0
+__device__ __forceinline__ int stats_uc(const StatsTask& T) {
+  if (!T.A->ucnt || !(T.A->stats & (S_RAF | S_RAFS))) return 0;
+  int n = 0;
+#pragma unroll
+  for (int q = 0; q < 16; q++) n += (T.A->allow[q] > 0.f);
+  return n <= STATS_UC ? n : 0;
+}
+// the unit counts of this thread's pairs of half k of a task's tile
+__device__ __forceinline__ const float* stats_uptr(const StatsTask& T, int k) {
+  return T.A->ucnt + ((int64_t)T.slot * T.A->ntiles + T.t) * 16 * TPP + ((threadIdx.x >> 4) + 16 * k) * TP +
+         2 * (threadIdx.x & 15);
+}
+__device__ __forceinline__ void stats_fetch_uc(const StatsTask& T, int k, StatsSmem& sm) {
+  const float* U = stats_uptr(T, k);
+  int n = 0;
+#pragma unroll
+  for (int q = 0; q < 16; q++)
+    if (T.A->allow[q] > 0.f) cpa8(&sm.uc[n++][threadIdx.x], U + q * TPP);
+}
+
+// the count ring of one thread: rows of cells in the order they are used
+// (tasks, then the two halves of a tile, then x)
+template <class GET>
+struct StatsRing {
+  const GET& get;
+  StatsSmem& sm;
+  int vb, G, ntask, row, slot;     // the next row to fetch, and its place
+  const float* src;
+  __device__ __forceinline__ StatsRing(const GET& g, StatsSmem& s, int vb0, int G_, int n)
+      : get(g), sm(s), vb(vb0 - G_), G(G_), ntask(n), row(8), slot(0), src(nullptr) {}
+  __device__ __forceinline__ void fetch() {
+    if (row == 8) {   // the next task with a count ring
+      do {
+        vb += G;
+        if (vb >= ntask) { vb = ntask - 1; cpa_commit(); return; }   // none left: an empty group, and again next time
+        const StatsTask T = get(vb);
+        if (!stats_c16(T)) continue;
+        src = T.A->cnt + ((int64_t)T.slot * T.A->ntiles + T.t) * 32 * TPP + (threadIdx.x >> 4) * TP +
+              2 * (threadIdx.x & 15);
+        row = 0;
+      } while (row == 8);
+    }
+    const float* s = src + (row & 3) * 8 * TPP + (row >> 2) * 16 * TP;
+#pragma unroll
+    for (int k = 0; k < 8; k++) cpa8(&sm.ring[slot][k][threadIdx.x], s + k * TPP);
+    cpa_commit();
+    row++;
+    slot = slot == 2 ? 0 : slot + 1;
+  }
+};
+
+enum { CT_LN = 0, CT_INV = 2, CT_PM = 4 };
+__device__ __forceinline__ df2 col_j(const StatsSmem& sm, int buf, int tbl, int y, int b) {   // columns b, b + 1
+  return {*reinterpret_cast<const f2*>(&sm.col[buf][0][tbl][y][b]),
+          *reinterpret_cast<const f2*>(&sm.col[buf][0][tbl + 1][y][b])};
+}
+__device__ __forceinline__ df2 col_i(const StatsSmem& sm, int buf, int tbl, int x, int a) {
+  return {dup2(sm.col[buf][1][tbl][x][a]), dup2(sm.col[buf][1][tbl + 1][x][a])};
+}
+
+// next: the task whose tables are staged meanwhile (buffer buf ^ 1), or null
+template <unsigned CF, class GET>
+__device__ __forceinline__ void c16_tile(const StatsTask& task, const StatsTask* next, int buf, StatsSmem& sm,
+                                         StatsRing<GET>& ring, int& rslot) {
+  const StatsArgs& A = *task.A;
+  const int t = task.t, slot = task.slot, tid = threadIdx.x;
+  const TileRC tr = A.tiles[t];
+  const double* pm = A.pm + (int64_t)slot * A.Lp * 4;
+  const double* meanp = A.meanp + slot * 4;
+  const int nuc = stats_uc(task);
+  const unsigned S = A.stats;
+  const f2 nz = A.negzero2;
+#pragma unroll 1
+  for (int k = 0; k < 2; k++) {
+    const int a = (tid >> 4) + 16 * k, b = 2 * (tid & 15), p = a * TP + b;
+    const int i = tr.I * TP + a, j = tr.J * TP + b;
+    const bool ok0 = (i < j) && (j < A.L), ok1 = (i < j + 1) && (j + 1 < A.L);
+    df2 chi = dfz2(), gt = dfz2(), mi = dfz2(), mir = dfz2(), mig = dfz2(), omes = dfz2(), raf = dfz2(), ccf = dfz2();
+    {
+      if ((S & (S_RAF | S_RAFS)) && A.ucnt) {
+        const float* U = stats_uptr(task, k);
+        f2 nA = 0ull, r[4] = {0ull, 0ull, 0ull, 0ull}, cc[4] = {0ull, 0ull, 0ull, 0ull};
+        if (nuc) cpa_wait<1>();   // fetched two rows or more ago
+        int m = 0;
+#pragma unroll
+        for (int x = 0; x < 4; x++)
+#pragma unroll
+          for (int y = 0; y < 4; y++)
+            if (A.allow[x * 4 + y] > 0.f) {   // RAF reads the allowed cells only
+              const f2 n = *reinterpret_cast<const f2*>(nuc ? (const float*)&sm.uc[m++][tid] : U + (x * 4 + y) * TPP);
+              nA = add2(nA, n); r[x] = add2(r[x], n); cc[y] = add2(cc[y], n);
+            }
+        df o[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          auto half = [h](f2 v) { const float2 w = un2(v); return h ? w.y : w.x; };
+          const float rr[4] = {half(r[0]), half(r[1]), half(r[2]), half(r[3])};
+          const float cr[4] = {half(cc[0]), half(cc[1]), half(cc[2]), half(cc[3])};
+          o[h] = raf_of(A, half(nA), rr, cr);
+        }
+        raf = {pk2(o[0].hi, o[1].hi), pk2(o[0].lo, o[1].lo)};
+      }
+      {
+        df2 R[4], K[4], T[4], V[4], Sx = dfz2(), W = dfz2(), ne = dfz2();
+#pragma unroll
+        for (int x = 0; x < 4; x++) K[x] = dfz2();
+        // one row of cells at a time, the loop kept rolled: unrolled fully the
+        // body outgrows the instruction cache and the warps wait for it
+#pragma unroll 1
+        for (int x = 0; x < 4; x++) {
+          df2 cur[4], Rx, Tx, Vx;
+          cpa_wait<1>();   // this row has landed (the next one may be in flight)
+#pragma unroll
+          for (int y = 0; y < 4; y++)
+            cur[y] = {*reinterpret_cast<const f2*>(&sm.ring[rslot][2 * y][tid]),
+                      *reinterpret_cast<const f2*>(&sm.ring[rslot][2 * y + 1][tid])};
+          if (x == 0) {   // with this row's fetch: the next tile's tables, the next half tile's unit counts
+            if (k == 0) {
+              if (next) stats_tables<CF>(*next, sm, buf ^ 1);
+              if (nuc) stats_fetch_uc(task, 1, sm);
+            } else if (next && stats_uc(*next)) {
+              stats_fetch_uc(*next, 0, sm);
+            }
+          }
+          ring.fetch();
+          rslot = rslot == 2 ? 0 : rslot + 1;
+#pragma unroll
+          for (int y = 0; y < 4; y++) {
+            const df2 c = cur[y];
+            df2_acc(ne, c);
+            // counts are 0 or at least a weight's quantum, above the prior
+            // for weights that sum to N
+            const df2 cp = df2_add_f_fast(c, dup2(1e-10f));
+            const f2 ncp = neg2(cp.hi);
+            if (y == 0) Rx = cp; else df2_acc(Rx, cp);
+            df2_acc(K[y], cp);
+            if (CF & CF_G) df2_acc_mul(Sx, cp, ncp, df2_log(cp, sm.tab, nz), nz);
+            if (CF & (CF_CHI | CF_OMES)) {
+              const df2 sq = df2_sqr_u(cp, ncp, nz);
+              if (CF & CF_CHI) {
+                const df2 inv = col_j(sm, buf, CT_INV, y, b);
+                if (y == 0) Tx = df2_mul_un(sq, neg2(sq.hi), inv, nz);
+                else        df2_acc_mul(Tx, sq, neg2(sq.hi), inv, nz);
+              }
+              if (CF & CF_OMES) {
+                const df2 pj = col_j(sm, buf, CT_PM, y, b);
+                df2_acc(W, sq);
+                if (y == 0) Vx = df2_mul_un(cp, ncp, pj, nz);
+                else        df2_acc_mul(Vx, cp, ncp, pj, nz);
+              }
+            }
+          }
+          R[x] = df2_norm(Rx);   // R, T, V: indexed by the loop, in local memory
+          if (CF & CF_CHI) T[x] = df2_norm(Tx);
+          if (CF & CF_OMES) V[x] = df2_norm(Vx);
+        }
+#pragma unroll
+        for (int y = 0; y < 4; y++) K[y] = df2_norm(K[y]);
+        ne = df2_norm(ne);
+        const df2 Z = df2_add_f(ne, dup2(16.f * 1e-10f));
+        const df2 iZ = df2_recip(Z, nz);
+        if (CF & CF_G) {
+          const df2 Sn = df2_norm(Sx), lnZ = df2_log(Z, sm.tab, nz);
+          df2 P = dfz2();
+#pragma unroll
+          for (int x = 0; x < 4; x++) {
+            df2_acc_mul(P, R[x], neg2(R[x].hi), col_i(sm, buf, CT_LN, x, a), nz);
+            df2_acc_mul(P, K[x], neg2(K[x].hi), col_j(sm, buf, CT_LN, x, b), nz);
+          }
+          mi = df2_mul(df2_sub(df2_sub(Sn, df2_mul(Z, lnZ, nz)), df2_norm(P)), iZ, nz);
+          gt = df2_scale(df2_mul(ne, mi, nz), 2.f);
+          // the mask is the same for every thread: no divergence
+          if (S & S_MIr) {
+            const df2 H = df2_sub(lnZ, df2_mul(Sn, iZ, nz)), q = df2_div(mi, H, nz);
+            const bool h0 = above_h(half_df(H, 0)), h1 = above_h(half_df(H, 1));
+            const float2 qh = un2(q.hi), ql = un2(q.lo);
+            mir = {pk2(h0 ? qh.x : 0.f, h1 ? qh.y : 0.f), pk2(h0 ? ql.x : 0.f, h1 ? ql.y : 0.f)};
+          }
+          if (S & S_MIg) mig = df2_sub(mi, df2_div(df2_sub(dup_df({A.wtot.x, A.wtot.y}), ne), ne, nz));
+        }
+        if (CF & CF_CHI) {
+          df2 Q = dfz2();
+#pragma unroll
+          for (int x = 0; x < 4; x++) {
+            df2_acc_mul(Q, T[x], neg2(T[x].hi), col_i(sm, buf, CT_INV, x, a), nz);
+          }
+          chi = df2_sub(df2_mul(df2_mul(ne, df2_mul(iZ, iZ, nz), nz), df2_norm(Q), nz), ne);
+        }
+        if (CF & CF_OMES) {
+          df2 Uo = dfz2(), Ai = dfz2(), Aj = dfz2();
+#pragma unroll
+          for (int x = 0; x < 4; x++) {
+            const df2 pi = col_i(sm, buf, CT_PM, x, a), pj = col_j(sm, buf, CT_PM, x, b);
+            df2_acc_mul(Uo, pi, neg2(pi.hi), V[x], nz);
+            df2_acc(Ai, df2_sqr_u(pi, neg2(pi.hi), nz));
+            df2_acc(Aj, df2_sqr_u(pj, neg2(pj.hi), nz));
+          }
+          const df2 t1 = df2_mul(df2_norm(W), df2_mul(iZ, iZ, nz), nz);
+          const df2 t2 = df2_scale(df2_mul(df2_norm(Uo), iZ, nz), 2.f);
+          const df2 t3 = df2_mul(df2_norm(Ai), df2_norm(Aj), nz);
+          omes = df2_mul(ne, df2_add(df2_sub(t1, t2), t3), nz);
+        }
+        const float2 neh = un2(ne.hi);
+        const bool none0 = ok0 && neh.x <= 0.f, none1 = ok1 && neh.y <= 0.f;   // no sequence with both residues
+        if (S & S_CCF) {
+          df o[2] = {{0.f, 0.f}, {0.f, 0.f}};
+          if (ok0) o[0] = ccf_of(df_to_d(half_df(ne, 0)), pm + i * 4, pm + j * 4, meanp);
+          if (ok1) o[1] = ccf_of(df_to_d(half_df(ne, 1)), pm + i * 4, pm + j * 4 + 4, meanp);
+          ccf = {pk2(o[0].hi, o[1].hi), pk2(o[0].lo, o[1].lo)};
+        }
+        if (none0 || none1) {
+#pragma unroll 1
+          for (int h = 0; h < 2; h++) {
+            if (!(h ? none1 : none0)) continue;
+            const PriorStats z = prior_stats(A.allow, 0, pm + i * 4, pm + (j + h) * 4);
+            const f2 keep = h ? 0x00000000FFFFFFFFull : 0xFFFFFFFF00000000ull;
+            auto put = [keep](df2& d, df v) {
+              d.hi = (d.hi & keep) | (dup2(v.hi) & ~keep);
+              d.lo = (d.lo & keep) | (dup2(v.lo) & ~keep);
+            };
+            put(chi, {0.f, 0.f}); put(gt, {0.f, 0.f}); put(omes, {0.f, 0.f});
+            put(mi, z.mi); put(mig, z.mi); put(mir, z.mir);
+          }
+        }
+      }
+    }
+    if (k == 0) __syncthreads();   // the previous tile's sums have read vs
+#pragma unroll
+    for (int q = 0; q < MAXOUT; q++) {
+      if (q < A.nout) {
+        df2 v;
+        switch (A.outstat[q]) {
+          case 0: v = chi; break;
+          case 1: v = gt; break;
+          case 2: v = mi; break;
+          case 3: v = mir; break;
+          case 4: v = mig; break;
+          case 5: v = omes; break;
+          case 6: v = raf; break;
+          default: v = ccf; break;
+        }
+        const float2 h = un2(v.hi), l = un2(v.lo);
+        const float4 o = make_float4(ok0 ? h.x : 0.f, ok0 ? l.x : 0.f, ok1 ? h.y : 0.f, ok1 ? l.y : 0.f);
+        *reinterpret_cast<float4*>(A.cov + (((int64_t)slot * A.nout + q) * A.ntiles + t) * TPP + p) = o;
+        sm.vs[q][a][b] = make_float2(o.x, o.y);
+        sm.vs[q][a][b + 1] = make_float2(o.z, o.w);
+      }
+    }
+  }
+}
+
+// every other task: the merged classes, and RAF alone (no weighted counts)
+__device__ __forceinline__ void merged_tile(const StatsTask& T, StatsSmem& sm) {
+  const StatsArgs& A = *T.A;
+  const int t = T.t, slot = T.slot, tid = threadIdx.x;
   const TileRC tr = A.tiles[t];
   const float* C = A.cnt ? A.cnt + ((int64_t)slot * A.ntiles + t) * 32 * TPP : nullptr;
   const float* U = A.ucnt ? A.ucnt + ((int64_t)slot * A.ntiles + t) * 16 * TPP : nullptr;
@@ -743,11 +1027,6 @@ __device__ __forceinline__ void stats_body(
   const float2* pmdf = A.pmdf + (int64_t)slot * A.Lp * 4;
   const float4* lpi = A.lpi + (int64_t)slot * A.Lp * 4;
   const double* meanp = A.meanp + slot * 4;
-  __shared__ float2 vs[MAXOUT][TP][TP + 1];   // the tile's scores, [q][a][b]
-  __shared__ float4 tab[LOGTAB_TOT];
-  static_assert(LOGTAB_TOT <= 256, "one table entry per thread");
-  if (tid < LOGTAB_TOT) tab[tid] = A.logtab[tid];
-  __syncthreads();
 #pragma unroll 1
   for (int k = 0; k < 4; k++) {
     const int p = tid + 256 * k, a = p >> 5, b = p & 31;
@@ -762,23 +1041,27 @@ __device__ __forceinline__ void stats_body(
     }
     PairOut o;
     o.chi = o.gt = o.mi = o.mir = o.mig = o.omes = o.raf = o.ccf = df{0.f, 0.f};
-    if (valid) {
-      const int ii = i < A.L ? i : 0, jj = j < A.L ? j : 0;
-      pair_stats<CF>(A, c, uc, U != nullptr, pmdf + ii * 4, pmdf + jj * 4, lpi + ii * 4, lpi + jj * 4, pm + ii * 4,
-                     pm + jj * 4, meanp, tab, o);
-    }
+    if (valid)
+      merged_stats(A, c, uc, U != nullptr, pmdf + i * 4, pmdf + j * 4, lpi + i * 4, lpi + j * 4, pm + i * 4,
+                   pm + j * 4, meanp, sm.tab, o);
 #pragma unroll
     for (int q = 0; q < MAXOUT; q++) {
       if (q < A.nout) {
         const df v = valid ? pick_df(o, A.outstat[q]) : df{0.f, 0.f};
         st_df(A.cov + (((int64_t)slot * A.nout + q) * A.ntiles + t) * TPP + p, v);
-        vs[q][a][b] = make_float2(v.hi, v.lo);
+        sm.vs[q][a][b] = make_float2(v.hi, v.lo);
       }
     }
   }
-  __syncthreads();
+}
+
+// the rows' and columns' sums of a task's tile from sm.vs
+__device__ __forceinline__ void stats_sums(const StatsTask& T, const StatsSmem& sm) {
+  const StatsArgs& A = *T.A;
+  const int t = T.t, slot = T.slot, tid = threadIdx.x;
   // rows of tile (I,J) at part[I][J], columns at part[J][I]; a diagonal tile
   // adds both roles into part[I][I]
+  const TileRC tr = A.tiles[t];
   double* base = A.part1 + (int64_t)slot * A.nout * A.nT * A.nT * TP;
   const int64_t qstride = (int64_t)A.nT * A.nT * TP;
   if (tr.I != tr.J) {
@@ -786,23 +1069,76 @@ __device__ __forceinline__ void stats_body(
       const int role = tid / (TP * A.nout), rem = tid % (TP * A.nout);
       const int line = rem / A.nout, q = rem % A.nout;
       df sum = {0.f, 0.f};
-      if (role == 0) { for (int b = 0; b < TP; b++) sum = df_add(sum, {vs[q][line][b].x, vs[q][line][b].y}); }
-      else           { for (int a = 0; a < TP; a++) sum = df_add(sum, {vs[q][a][line].x, vs[q][a][line].y}); }
+      if (role == 0) { for (int b = 0; b < TP; b++) sum = df_add(sum, {sm.vs[q][line][b].x, sm.vs[q][line][b].y}); }
+      else           { for (int a = 0; a < TP; a++) sum = df_add(sum, {sm.vs[q][a][line].x, sm.vs[q][a][line].y}); }
       const int64_t cell = (role == 0) ? ((int64_t)tr.I * A.nT + tr.J) : ((int64_t)tr.J * A.nT + tr.I);
       base[q * qstride + cell * TP + line] = df_to_d(sum);
     }
   } else if (tid < TP * A.nout) {
     const int line = tid / A.nout, q = tid % A.nout;
     df r = {0.f, 0.f}, c = {0.f, 0.f};
-    for (int b = 0; b < TP; b++) r = df_add(r, {vs[q][line][b].x, vs[q][line][b].y});
-    for (int a = 0; a < TP; a++) c = df_add(c, {vs[q][a][line].x, vs[q][a][line].y});
+    for (int b = 0; b < TP; b++) r = df_add(r, {sm.vs[q][line][b].x, sm.vs[q][line][b].y});
+    for (int a = 0; a < TP; a++) c = df_add(c, {sm.vs[q][a][line].x, sm.vs[q][a][line].y});
     base[q * qstride + ((int64_t)tr.I * A.nT + tr.I) * TP + line] = df_to_d(df_add(r, c));
   }
 }
+// tasks bid, bid + G, ... of ntask; get(vb): the task
+template <unsigned CF, class GET>
+__device__ __forceinline__ void stats_body(const GET& get, const float4* logtab, int ntask) {
+  extern __shared__ __align__(16) unsigned char stats_smem[];
+  StatsSmem& sm = *reinterpret_cast<StatsSmem*>(stats_smem);
+  const int tid = threadIdx.x, G = gridDim.x;
+  int vb = blockIdx.x;
+  if (vb >= ntask) return;
+  StatsTask T = get(vb), N = T;
+  if (tid < LOGTAB_TOT) sm.tab[tid] = logtab[tid];
+  StatsRing<GET> ring(get, sm, vb, G, ntask);
+  int buf = 0, rslot = 0;
+  if (stats_c16(T)) {
+    stats_tables<CF>(T, sm, 0);
+    if (stats_uc(T)) stats_fetch_uc(T, 0, sm);
+  }
+  cpa_commit();
+  cpa_wait<0>();
+  ring.fetch();
+  ring.fetch();
+  __syncthreads();
+  for (;;) {
+    const int nvb = vb + G;
+    const bool more = nvb < ntask;
+    if (more) N = get(nvb);
+    const bool tables = more && stats_c16(N);
+    if (stats_c16(T)) {
+      // N's tables land with the row fetched at the tile's start, long before its end
+      c16_tile<CF>(T, tables ? &N : nullptr, buf, sm, ring, rslot);
+    } else {
+      __syncthreads();   // the previous tile's sums have read vs
+      merged_tile(T, sm);
+      if (tables) {
+        stats_tables<CF>(N, sm, buf ^ 1);
+        if (stats_uc(N)) stats_fetch_uc(N, 0, sm);
+        cpa_wait_all();
+      }
+    }
+    __syncthreads();     // vs and N's tables
+    stats_sums(T, sm);
+    if (!more) break;
+    T = N;
+    vb = nvb;
+    buf ^= 1;
+  }
+  cpa_wait_all();
+}
+
+struct StatsGet {
+  const StatsArgs* A;
+  __device__ __forceinline__ StatsTask operator()(int vb) const { return {A, vb % A->ntiles, vb / A->ntiles}; }
+};
 template <unsigned CF>
 __global__ void __launch_bounds__(256, 2)
-k_stats(StatsArgs A) {
-  stats_body<CF>(native_grid(), A);
+k_stats(const __grid_constant__ StatsArgs A, int ntask) {
+  const StatsGet get{&A};
+  stats_body<CF>(get, A.logtab, ntask);
 }
 
 // power_SPAIR_AddMI (src/power.c:201-218) for every pair i < j of one
@@ -1341,11 +1677,15 @@ cudaError_t launch_stats(const StatsArgs& A, int nslots, cudaStream_t st) {
   if (A.stats & (S_GT | S_MI | S_MIr | S_MIg)) cf |= CF_G;
   if (A.stats & S_CHI) cf |= CF_CHI;
   if (A.stats & S_OMES) cf |= CF_OMES;
-  const dim3 grid(A.ntiles, nslots);
-  if (cf == 0 || cf == CF_G)          k_stats<CF_G><<<grid, 256, 0, st>>>(A);
-  else if (cf == CF_CHI)              k_stats<CF_CHI><<<grid, 256, 0, st>>>(A);
-  else if (cf == (CF_G | CF_CHI))     k_stats<CF_G | CF_CHI><<<grid, 256, 0, st>>>(A);
-  else                                k_stats<CF_ALL><<<grid, 256, 0, st>>>(A);
+  const int64_t ntask = (int64_t)A.ntiles * nslots;
+  if (ntask >= ((int64_t)1 << 30)) return cudaErrorInvalidValue;   // tasks are indexed in 32 bits
+  const int grid = (int)std::min<int64_t>(ntask, stats_grid());
+  if (grid < 1) return cudaErrorInvalidValue;
+  const size_t sm = sizeof(StatsSmem);
+  if (cf == 0 || cf == CF_G)          k_stats<CF_G><<<grid, 256, sm, st>>>(A, (int)ntask);
+  else if (cf == CF_CHI)              k_stats<CF_CHI><<<grid, 256, sm, st>>>(A, (int)ntask);
+  else if (cf == (CF_G | CF_CHI))     k_stats<CF_G | CF_CHI><<<grid, 256, sm, st>>>(A, (int)ntask);
+  else                                k_stats<CF_ALL><<<grid, 256, sm, st>>>(A, (int)ntask);
   return cudaGetLastError();
 }
 
@@ -1579,11 +1919,41 @@ __global__ void k_meanp_grp(const FamDev* __restrict__ F, const int* __restrict_
   meanp_body(GridIdx{l.g.y, 0, 1}, d.mpc, d.L, d.Lp, d.meanp);
 }
 
+struct StatsGetGrp {
+  const FamDev* F;
+  const int* pre;
+  int nf;
+  __device__ __forceinline__ StatsTask operator()(int vb) const {
+    const int f = grp_find(pre, nf, vb);
+    const StatsArgs* A = &F[f].sa;
+    const int loc = vb - __ldg(pre + f);
+    return {A, loc % A->ntiles, loc / A->ntiles};
+  }
+};
 template <unsigned CF>
 __global__ void __launch_bounds__(256, 2)
-k_stats_grp(const FamDev* __restrict__ F, const int* __restrict__ pre, int nf) {
-  const GrpLoc l = grp_loc(pre, nf, gx_tiles, F);
-  stats_body<CF>(l.g, F[l.f].sa);
+k_stats_grp(const FamDev* __restrict__ F, const int* __restrict__ pre, int nf, int ntask) {
+  const StatsGetGrp get{F, pre, nf};
+  stats_body<CF>(get, F[0].sa.logtab, ntask);
+}
+
+// CTAs resident on the current device, two per SM (0 when the kernels' shared
+// memory cannot be had); the launch limits are raised once per device
+int stats_grid() {
+  constexpr int MAXDEV = 64;
+  static std::atomic<int> known[MAXDEV];
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev < MAXDEV && (nsm = known[dev].load()) > 0) return 2 * nsm;
+  const void* k[] = {(const void*)k_stats<CF_G>, (const void*)k_stats<CF_CHI>, (const void*)k_stats<CF_G | CF_CHI>,
+                     (const void*)k_stats<CF_ALL>, (const void*)k_stats_grp<CF_G>, (const void*)k_stats_grp<CF_CHI>,
+                     (const void*)k_stats_grp<CF_G | CF_CHI>, (const void*)k_stats_grp<CF_ALL>};
+  for (const void* f : k)
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StatsSmem)) != cudaSuccess)
+      return 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (dev < MAXDEV) known[dev].store(nsm);
+  return 2 * nsm;
 }
 
 __global__ void __launch_bounds__(256)
@@ -1674,10 +2044,13 @@ cudaError_t grp_marginals(const FamDev* F, int nf, const int* pre_marg, int nb_m
 
 cudaError_t grp_stats(const FamDev* F, int nf, const int* pre, int nb, unsigned cf, cudaStream_t st) {
   if (nb <= 0) return cudaSuccess;
-  if (cf == 0 || cf == CF_G)          k_stats_grp<CF_G><<<nb, 256, 0, st>>>(F, pre, nf);
-  else if (cf == CF_CHI)              k_stats_grp<CF_CHI><<<nb, 256, 0, st>>>(F, pre, nf);
-  else if (cf == (CF_G | CF_CHI))     k_stats_grp<CF_G | CF_CHI><<<nb, 256, 0, st>>>(F, pre, nf);
-  else                                k_stats_grp<CF_ALL><<<nb, 256, 0, st>>>(F, pre, nf);
+  const int grid = std::min(nb, stats_grid());
+  if (grid < 1) return cudaErrorInvalidValue;
+  const size_t sm = sizeof(StatsSmem);
+  if (cf == 0 || cf == CF_G)          k_stats_grp<CF_G><<<grid, 256, sm, st>>>(F, pre, nf, nb);
+  else if (cf == CF_CHI)              k_stats_grp<CF_CHI><<<grid, 256, sm, st>>>(F, pre, nf, nb);
+  else if (cf == (CF_G | CF_CHI))     k_stats_grp<CF_G | CF_CHI><<<grid, 256, sm, st>>>(F, pre, nf, nb);
+  else                                k_stats_grp<CF_ALL><<<grid, 256, sm, st>>>(F, pre, nf, nb);
   return cudaGetLastError();
 }
 

@@ -8,6 +8,7 @@
 namespace covgpu {
 
 constexpr int MAXOUT = 4;   // score matrices produced by one k_stats launch
+constexpr unsigned long long NEGZERO2 = 0x8000000080000000ull;   // two FP32 -0
 
 struct StatsArgs {
   const float*  cnt;        // weighted counts [slot][tile][16][2][TPP] (double-float planes)
@@ -28,6 +29,7 @@ struct StatsArgs {
   int           nout;       // number of output matrices (<= MAXOUT)
   int           outstat[MAXOUT];  // index into PairOut.v for output q
   float         allow[16];
+  unsigned long long negzero2;  // NEGZERO2, for the rounded products of cov_df2.cuh
 };
 
 // constants of the histogram's bin function, split on the host
@@ -88,6 +90,9 @@ cudaError_t launch_pm_final(const double* part4, const double* partR, int L, int
                             float2* pmdf, float4* lpi, double* mpc, double* meanp, int* status, cudaStream_t st);
 cudaError_t launch_ps(const uint8_t* ax, int64_t slot_stride, const double* w, int N, int L, int Lp, int nslots,
                       double* ps, cudaStream_t st);
+// CTAs of the statistics kernels on the current device; the first call on a
+// device raises their shared-memory limit (make it before a stream capture)
+int         stats_grid();
 cudaError_t launch_stats(const StatsArgs& A, int nslots, cudaStream_t st);
 // power_SPAIR_AddMI's pair classes of one alignment's double-float counts:
 // [L(L-1)/2] each, row-major over i < j
