@@ -80,10 +80,11 @@ struct Layout {
   double* w = nullptr;                       // weights region start (w, limbf, limbs)
   size_t wreg_bytes = 0;
   std::vector<size_t> w_off, lf_off, lb_off; // byte offsets inside the weights region
-  int* tree = nullptr; size_t tree_n = 0;    // left, right, lnodes of every family
+  int* tree = nullptr; size_t tree_n = 0;    // left, right, lnodes (nodes, depth offsets) of every family
   uint8_t* tiles = nullptr; size_t tiles_bytes = 0;
   uint16_t* ops = nullptr; int pitch = 0; int64_t op_rows = 0;
   float* cnt = nullptr; int64_t cnt_floats = 0;
+  int* ns = nullptr; size_t ns_bytes = 0;    // the nulls' substitution counts
   double* pm = nullptr; size_t pm_bytes = 0; // pm, pmdf, lpi regions (RAF only: zeroed)
   double* mm = nullptr; size_t mm_n = 0;
   int* status = nullptr;
@@ -292,7 +293,7 @@ size_t fam_bytes_hint(const FamHost& f, int nout, bool need_u, bool rafs, int pi
   const size_t S = f.nslots, nT2 = (size_t)f.nT * f.nT, ntl = f.ntiles;
   size_t b = S * f.N * f.Lp + 3 * (size_t)f.N * 16 + ntl * 16 + nT2 * 4;
   b += (f.gsc ? (size_t)f.N * f.N * 8 + 2 * (size_t)f.N * f.Lw * 4 : 0) + (f.pb ? (size_t)f.L * 32 : 0);
-  b += 2 * (size_t)f.ns * std::max(f.N - 1, 0) * f.Lp;
+  b += (size_t)f.ns * ((size_t)f.N * f.Lp + (size_t)f.N * 200 + 2 * kAlign);
   b += (size_t)4 * S * 4 * f.Lp * pitch * 2;           // tensor operands
   b += S * ntl * 32 * TPP * 4 + (need_u ? S * ntl * 16 * TPP * 4 : 0);
   b += S * nT2 * TP * 40 + S * f.Lp * 4 * 40;
@@ -322,10 +323,10 @@ void place(Layout& Lo, std::vector<FamHost>& fams, const Types& T, int counter, 
   }
   Lo.w = base ? reinterpret_cast<double*>(base + w0) : nullptr;
   Lo.wreg_bytes = m.off - w0;
-  // tree: left, right, lnodes per family, one int array
+  // tree: left, right, lnodes (the nodes by depth, then the depths' offsets) per family, one int array
   const size_t t0 = m.off;
   size_t tn = 0;
-  for (int k = 0; k < nf; k++) tn += 3 * (size_t)std::max(fams[k].N - 1, 1);
+  for (int k = 0; k < nf; k++) tn += 3 * (size_t)std::max(fams[k].N - 1, 1) + fams[k].loff.size();
   int* tree = m.take<int>(tn);
   Lo.tree = tree; Lo.tree_n = tn;
   {
@@ -335,7 +336,7 @@ void place(Layout& Lo, std::vector<FamHost>& fams, const Types& T, int counter, 
       Lo.F[k].left = tree ? tree + o : nullptr;
       Lo.F[k].right = tree ? tree + o + n : nullptr;
       Lo.F[k].lnodes = tree ? tree + o + 2 * n : nullptr;
-      o += 3 * n;
+      o += 3 * n + fams[k].loff.size();
     }
   }
   (void)t0;
@@ -364,9 +365,17 @@ void place(Layout& Lo, std::vector<FamHost>& fams, const Types& T, int counter, 
   for (int k = 0; k < nf; k++) {
     const FamHost& f = fams[k];
     const size_t rows = (size_t)f.ns * std::max(f.N - 1, 0) * f.Lp;
-    Lo.F[k].fitch = rows ? m.take<uint8_t>(rows) : nullptr;
+    Lo.F[k].fitch = rows ? m.take<uint8_t>((size_t)f.ns * f.Lp) : nullptr;
     Lo.F[k].scratch = rows ? m.take<uint8_t>(rows) : nullptr;
+    Lo.F[k].nlevels = f.depth();
   }
+  const size_t ns0 = m.off;
+  for (int k = 0; k < nf; k++) {
+    const FamHost& f = fams[k];
+    Lo.F[k].ns = (f.ns > 0 && f.N > 1) ? m.take<int>((size_t)f.ns * 2 * f.N * 25) : nullptr;
+  }
+  Lo.ns = base ? reinterpret_cast<int*>(base + ns0) : nullptr;
+  Lo.ns_bytes = m.off - ns0;
   // tensor operands of the families counted on the tensor cores:
   // [family][4 buffers][nslots][4 Lp] rows of pitch
   Lo.pitch = 64;
@@ -494,8 +503,9 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
         memcpy(&tree_h[o], fam_in[f.idx].left, (f.N - 1) * sizeof(int));
         memcpy(&tree_h[o + n], fam_in[f.idx].right, (f.N - 1) * sizeof(int));
         memcpy(&tree_h[o + 2 * n], f.order.data(), (f.N - 1) * sizeof(int));
+        memcpy(&tree_h[o + 3 * n], f.loff.data(), f.loff.size() * sizeof(int));
       }
-      o += 3 * n;
+      o += 3 * n + f.loff.size();
     }
   }
   for (int k = 0; k < nf; k++) {
@@ -580,7 +590,7 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
   int maxdepth = 0, maxLp = 32;
   for (auto& f : fams) { maxdepth = std::max(maxdepth, f.depth()); maxLp = std::max(maxLp, f.Lp); }
   const bool srow_cta = maxLp <= replay_smem_max(), srow_warp = 8 * maxLp <= replay_smem_max();
-  struct Lvl { size_t lv, up, cta, warp; int nup, ncta, nwarp; };
+  struct Lvl { size_t lv, cta, warp; int ncta, nwarp; };
   std::vector<Lvl> lvl(maxdepth);
   for (int dd = 0; dd < maxdepth; dd++) {
     std::vector<int2> lv(nf);
@@ -589,15 +599,12 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
       const bool has = f.ns > 0 && dd < f.depth();
       lv[k] = has ? make_int2(f.loff[dd], f.loff[dd + 1] - f.loff[dd]) : make_int2(0, 0);
     }
-    Pre pu = prefix(nf, [&](int k) { return lv[k].y ? (lv[k].y * (fams[k].Lp >> 4) + 255) / 256 * fams[k].ns : 0; });
-    Pre pc = prefix(nf, [&](int k) {
-      return (lv[k].y && replay_uses_cta(lv[k].y, fams[k].ns)) ? 2 * lv[k].y * fams[k].ns : 0;
-    });
-    Pre pw = prefix(nf, [&](int k) {
-      return (lv[k].y && !replay_uses_cta(lv[k].y, fams[k].ns)) ? (2 * lv[k].y + 7) / 8 * fams[k].ns : 0;
-    });
+    int64_t items = 0;   // of all families: they fill the device together
+    for (int k = 0; k < nf; k++) items += (int64_t)2 * lv[k].y * fams[k].ns;
+    const bool cta = replay_uses_cta(items);
+    Pre pc = prefix(nf, [&](int k) { return cta ? 2 * lv[k].y * fams[k].ns : 0; });
+    Pre pw = prefix(nf, [&](int k) { return cta ? 0 : (2 * lv[k].y + 7) / 8 * fams[k].ns; });
     lvl[dd].lv = tb.put(lv.data(), nf * sizeof(int2));
-    lvl[dd].up = tb.put(pu.v.data(), pu.v.size() * 4); lvl[dd].nup = pu.total();
     lvl[dd].cta = tb.put(pc.v.data(), pc.v.size() * 4); lvl[dd].ncta = pc.total();
     lvl[dd].warp = tb.put(pw.v.data(), pw.v.size() * 4); lvl[dd].nwarp = pw.total();
   }
@@ -612,7 +619,9 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
   const size_t o_col = tb.put(pcol.v.data(), pcol.v.size() * 4), o_row = tb.put(prow.v.data(), prow.v.size() * 4);
   const size_t o_cod = tb.put(pcod.v.data(), pcod.v.size() * 4), o_id = tb.put(pid.v.data(), pid.v.size() * 4);
   const size_t o_up = tb.put(pup.v.data(), pup.v.size() * 4), o_lb = tb.put(plb.v.data(), plb.v.size() * 4);
-  Pre prs = prefix(nf, [&](int k) { return fams[k].ns > 0 ? (fams[k].L + 255) / 256 * fams[k].ns : 0; });
+  Pre prs = prefix(nf, [&](int k) { return fams[k].ns > 0 ? fitch_blocks(fams[k].Lp) * fams[k].ns : 0; });
+  int maxNnull = 1;
+  for (auto& f : fams) if (f.ns > 0) maxNnull = std::max(maxNnull, f.N);
   Pre prr = prefix(nf, [&](int k) { return fams[k].ns > 0 ? (fams[k].Lp + 255) / 256 * fams[k].ns : 0; });
   Pre pprep = prefix(nf, [&](int k) {
     return fams[k].tens ? fams[k].Npad / 64 * (fams[k].Lp / 32) * fams[k].nslots : 0;
@@ -654,6 +663,7 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
   const FamDev* dF = reinterpret_cast<const FamDev*>(S.tab + oF);
   auto P = [&](size_t o) { return reinterpret_cast<const int*>(S.tab + o); };
   if (pup.total() && !grp_weights_gsc_prepare()) return bfail(b, 90, "GSC kernel attributes");
+  if (prs.total() && !grp_null_prepare()) return bfail(b, 90, "null kernel attributes");
   if (!stats_grid()) return bfail(b, 90, "statistics kernel attributes");
 
   // the key of this chunk's device passes: the descriptor tables (they hold
@@ -681,15 +691,10 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
       BK(cudaEventRecord(S.join, S.st2));
       launches += (pcol.total() ? 2 : 0) + (pup.total() ? 3 : 0) + 1;
     }
-    // nulls: Fitch up the tree, the roots, the replay down it
-    for (int dd = maxdepth - 1; dd >= 0; dd--)
-      if (lvl[dd].nup) {
-        BK(grp_fitch_up(dF, nf, reinterpret_cast<const int2*>(S.tab + lvl[dd].lv), P(lvl[dd].up), lvl[dd].nup,
-                        p->seed, S.st));
-        launches++;
-      }
+    // nulls: the reconstructions, the roots' rows, the replay down the tree
     if (prs.total()) {
-      BK(grp_root(dF, nf, P(o_rs), prs.total(), P(o_rr), prr.total(), p->seed, S.st));
+      BK(cudaMemsetAsync(Lo.ns, 0, Lo.ns_bytes, S.st));
+      BK(grp_fitch(dF, nf, P(o_rs), prs.total(), maxNnull, P(o_rr), prr.total(), p->seed, S.st));
       launches += 2;
     }
     for (int dd = 0; dd < maxdepth; dd++) {

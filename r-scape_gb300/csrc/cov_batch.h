@@ -36,9 +36,11 @@ struct FamDev {
   int* glen;                   // [N] residues per sequence
   const int* left;             // [N-1] tree (Easel convention)
   const int* right;            // [N-1]
-  const int* lnodes;           // [N-1] internal nodes by depth
-  uint8_t* fitch;              // [ns][N-1][Lp]
-  uint8_t* scratch;            // [ns][N-1][Lp]
+  const int* lnodes;           // [N-1] internal nodes by depth, then the depths' offsets [nlevels + 1]
+  int nlevels;
+  uint8_t* fitch;              // [ns][Lp] the root's states
+  uint8_t* scratch;            // [ns][N-1][Lp] the nulls' internal rows
+  int* ns;                     // [ns][2N][25] substitutions per branch
   float* cnt;                  // [nslots][ntiles][32][TPP] weighted counts (double-float planes)
   float* ucnt;                 // [nslots][ntiles][16][TPP] unit counts (RAF) or nullptr
   double* part4;               // [nslots][nT][nT][TP][4]
@@ -102,15 +104,17 @@ cudaError_t grp_weights_gsc(const FamDev* F, int nf, const int* pre_codes, int n
 // normalisation and limbs of the device weights (one block per family of pre)
 cudaError_t grp_weights_limbs(FamDev* F, int nf, const int* pre, int nb, UmmaFam* U, cudaStream_t st);
 int         grp_weights_gsc_prepare();
-// nulls (cov_null.cu): one depth d of every family; lv[f] = {offset of depth d
-// in lnodes, nodes at depth d} (nn = 0: nothing at this depth)
-cudaError_t grp_fitch_up(const FamDev* F, int nf, const int2* lv, const int* pre, int nb, uint64_t seed,
-                         cudaStream_t st);
-cudaError_t grp_root(const FamDev* F, int nf, const int* pre_state, int nb_state, const int* pre_row, int nb_row,
-                     uint64_t seed, cudaStream_t st);
+// nulls (cov_null.cu): the reconstructions' substitution counts (zeroed
+// before) and the roots' rows; then one depth d of every family: lv[f] =
+// {offset of depth d in lnodes, nodes at depth d} (nn = 0: nothing at this
+// depth).  maxN: the largest N of the families with nulls.
+cudaError_t grp_fitch(const FamDev* F, int nf, const int* pre_cols, int nb_cols, int maxN, const int* pre_row,
+                      int nb_row, uint64_t seed, cudaStream_t st);
+int         fitch_blocks(int Lp);
+int         grp_null_prepare();
 cudaError_t grp_replay(const FamDev* F, int nf, const int2* lv, const int* pre, int nb, bool cta, bool srow,
                        int maxLp, uint64_t seed, cudaStream_t st);
-bool        replay_uses_cta(int nn, int nnull);
+bool        replay_uses_cta(int64_t items);
 int         replay_smem_max();
 // counting (cov_kernels.cu SIMT, cov_umma.cu tensor)
 cudaError_t grp_count_simt(const FamDev* F, int nf, const int* pre, int nb, bool unit, bool limbs,

@@ -69,6 +69,7 @@ struct covgpu_ctx {
   std::vector<int> loff;
   bool have_tree = false;
   uint8_t *d_fitch = nullptr, *d_scratch = nullptr;
+  int* d_bsub = nullptr;            // the nulls' substitutions per branch [maxnull][2N][25]
   unsigned long long* d_obs = nullptr;
   int nbcap = 0;
   double *d_sf = nullptr, *d_tail = nullptr;
@@ -212,6 +213,7 @@ extern "C" int covgpu_create(covgpu_ctx** ret, int device, int N, int L, int max
   if (maxnull > 0 && N > 1) {
     CK(dalloc(&ctx->d_fitch, (size_t)maxnull * (N - 1) * ctx->Lp));
     CK(dalloc(&ctx->d_scratch, (size_t)maxnull * (N - 1) * ctx->Lp));
+    CK(dalloc(&ctx->d_bsub, (size_t)maxnull * 2 * N * 25));
   }
   ctx->err[0] = 0;
   return 0;
@@ -224,7 +226,7 @@ extern "C" void covgpu_destroy(covgpu_ctx* ctx) {
   void* ptrs[] = {ctx->d_tiles, ctx->d_tile_index, ctx->d_ax, ctx->d_limbf, ctx->d_logtab, ctx->d_lpi, ctx->d_wd, ctx->d_cnt, ctx->d_ucnt,
                   ctx->d_part4, ctx->d_partR, ctx->d_pm, ctx->d_meanp, ctx->d_ps, ctx->d_cov, ctx->d_cov2,
                   ctx->d_part1, ctx->d_colx, ctx->d_avg, ctx->d_tmin, ctx->d_tmax, ctx->d_mm, ctx->d_status,
-                  ctx->d_left, ctx->d_right, ctx->d_lnodes, ctx->d_fitch, ctx->d_scratch, ctx->d_obs, ctx->d_sf,
+                  ctx->d_left, ctx->d_right, ctx->d_lnodes, ctx->d_fitch, ctx->d_scratch, ctx->d_bsub, ctx->d_obs, ctx->d_sf,
                   ctx->d_tail, ctx->d_nhits, ctx->d_hi, ctx->d_hj, ctx->d_hsc, ctx->d_hE, ctx->d_hp, ctx->d_full,
                   ctx->d_flush, ctx->d_pmdf, ctx->d_colxf, ctx->d_apcf, ctx->d_evt, ctx->d_pcls,
                   ctx->d_bpmask, ctx->d_pphost, ctx->d_ci, ctx->d_cj, ctx->d_cd};
@@ -370,11 +372,12 @@ extern "C" int covgpu_set_tree(covgpu_ctx* ctx, const int* parent, const int* le
   if (!ctx->d_left) {
     CK(dalloc(&ctx->d_left, ctx->capN - 1));
     CK(dalloc(&ctx->d_right, ctx->capN - 1));
-    CK(dalloc(&ctx->d_lnodes, ctx->capN - 1));
+    CK(dalloc(&ctx->d_lnodes, 2 * (size_t)ctx->capN));   // the nodes by depth, then the depths' offsets
   }
   CK(cudaMemcpy(ctx->d_left, left, (N - 1) * sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ctx->d_right, right, (N - 1) * sizeof(int), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->d_lnodes, order.data(), (N - 1) * sizeof(int), cudaMemcpyHostToDevice));
+  order.insert(order.end(), ctx->loff.begin(), ctx->loff.end());   // at most N offsets
+  CK(cudaMemcpy(ctx->d_lnodes, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
   ctx->have_tree = true;
   return 0;
 }
@@ -390,8 +393,7 @@ static int make_nulls_async(covgpu_ctx* ctx, uint64_t seed, int first_null, int 
   const int64_t sstride = (int64_t)ctx->N * ctx->Lp;
   CK(launch_nullgen(ctx->d_ax, ctx->N, ctx->L, ctx->Lp, T, ctx->d_lnodes, ctx->loff.data(),
                     (int)ctx->loff.size() - 1, seed, (uint32_t)first_null, nnull, ctx->d_fitch, ctx->d_scratch,
-                    ctx->d_ax + first_slot * sstride, sstride, ctx->st));
-  ctx->nlaunch += 2 + 2 * ((int)ctx->loff.size() - 1);
+                    ctx->d_bsub, ctx->d_ax + first_slot * sstride, sstride, ctx->st, &ctx->nlaunch));
   return 0;
 }
 
@@ -478,7 +480,7 @@ extern "C" int covgpu_substitutions(covgpu_ctx* ctx, int slot, uint64_t seed, in
   const uint8_t* ax = ctx->d_ax + (size_t)slot * N * Lp;
   NullTree T{N, ctx->d_left, ctx->d_right};
   if (e == cudaSuccess)
-    e = launch_fitch_recon(ax, N, L, Lp, T, ctx->d_lnodes, ctx->loff.data(), (int)ctx->loff.size() - 1, seed,
+    e = launch_fitch_recon(ax, N, L, Lp, T, ctx->d_lnodes, (int)ctx->loff.size() - 1, seed,
                            kReconStream, F, S, ctx->st);
   if (e == cudaSuccess)
     e = launch_substitutions(ax, F, ctx->d_left, ctx->d_right, N, L, Lp, includegaps ? 1 : 0, bits,
@@ -492,7 +494,7 @@ extern "C" int covgpu_substitutions(covgpu_ctx* ctx, int slot, uint64_t seed, in
   if (bits) cudaFree(bits);
   if (tmp) cudaFree(tmp);
   if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
-  ctx->nlaunch += 4 + 2 * ((int)ctx->loff.size() - 1);
+  ctx->nlaunch += 4;
   return 0;
 }
 

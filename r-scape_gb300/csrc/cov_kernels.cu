@@ -707,9 +707,9 @@ __device__ __forceinline__ void merged_stats(const StatsArgs& A, const df (&c)[1
 //
 // Bound: the FMA pipe and the latency of its chains (58-63% of the pipe busy,
 // 16 warps of 122-128 registers per SM); HBM at 0.27 of its rate.  Against the
-// form before (one pair per thread and scalar operations, counts loaded where
-// they are used, one CTA per tile): 138 for 206 warp instructions per 32
-// pairs of GT, MI, CHI and RAF; 8.53 for 9.53 ms on 21 alignments of
+// form before (one pair per thread, scalar operations, counts loaded where
+// they are used, one CTA per tile): 69 for 103 warp instructions per pair
+// for GT, MI, CHI and RAF; 8.53 for 9.53 ms on 21 alignments of
 // 2,000 x 3,000; GT alone 1.16 for 1.44 ms on 201 alignments of 500 x 400.
 constexpr int STATS_UC = 6;   // allowed cells staged; with more, RAF reads its counts directly
 struct StatsSmem {

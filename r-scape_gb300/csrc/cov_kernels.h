@@ -135,16 +135,18 @@ struct NullTree {
   const int* left;    // [N-1] device, Easel convention (<= 0: leaf -value)
   const int* right;   // [N-1] device
 };
-// level_nodes: device list of internal nodes ordered by depth; level_off:
-// host offsets of each depth in that list (nlevels + 1 entries)
+// level_nodes: device list of the N - 1 internal nodes ordered by depth, then
+// the nlevels + 1 offsets of each depth in it; level_off: the offsets on the
+// host
 // the Fitch reconstruction of one alignment (random tie-breaks from stream
 // nid): F [N-1][Lp] states of the internal nodes, S [N-1][Lp] scratch sets
 cudaError_t launch_fitch_recon(const uint8_t* ax, int N, int L, int Lp, const NullTree& T, const int* level_nodes,
-                               const int* level_off, int nlevels, uint64_t seed, uint32_t nid, uint8_t* F, uint8_t* S,
-                               cudaStream_t st);
+                               int nlevels, uint64_t seed, uint32_t nid, uint8_t* F, uint8_t* S, cudaStream_t st);
+// nulls first_null .. of the alignment ax into out_ax; fitch, rows
+// [nnull][N-1][Lp] and ns [nnull][2N][25] scratch; *nlaunch gains the launches
 cudaError_t launch_nullgen(const uint8_t* ax, int N, int L, int Lp, const NullTree& T, const int* level_nodes,
                            const int* level_off, int nlevels, uint64_t seed, uint32_t first_null, int nnull,
-                           uint8_t* fitch, uint8_t* scratch, uint8_t* out_ax, int64_t out_slot_stride,
-                           cudaStream_t st);
+                           uint8_t* fitch, uint8_t* rows, int* ns, uint8_t* out_ax, int64_t out_slot_stride,
+                           cudaStream_t st, int* nlaunch);
 
 }  // namespace covgpu

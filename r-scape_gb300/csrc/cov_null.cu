@@ -1,38 +1,43 @@
 // cov_null.cu -- null alignments on the GPU: Fitch ancestral states and the
 // shuffled-substitution replay of R-scape's default null (--nullphylo).
 //
-// The work goes by tree depth (nodes of one depth are independent):
-//   k_fitch_up   deepest depth first, one thread per (internal node, 16
-//                columns, null): the up pass of Tree_FitchAlgorithmAncenstral
-//                / tree_fitch_column (src/msatree.c:173-227, 1700-1838):
-//                intersection of the children's sets over the five states,
-//                else the union of residues only (tree_fitch_upwards
-//                :1877-1908), as byte-SIMD on 16-column vectors.
-//   k_root       the root's state per column, then its row with the columns
-//                shuffled (msamanip_ShuffleColumns, src/msamanip.c:1164-1233).
-//                Only the root's shuffled row is ever read: every other row
-//                is replaced by its parent's row before use.
-//   k_replay     top depth first, one CTA per (branch, null):
-//                shuffle_tree_substitutions + shuffle_tree_substitute_all
-//                (src/msamanip.c:1597-1747).  The CTA finishes the child's
-//                Fitch state (down pass: keep the parent's state when the
-//                child's set holds it), counts the branch's substitutions on
-//                the unshuffled reconstruction, copies the parent's current
-//                row and replays the substitutions on positions of that row
-//                holding the old state, visited in a random order (a Feistel
-//                permutation), 256 slots at a time; each class's positions
-//                are ranked with warp ballots and a prefix over the warps,
-//                and the pass stops once every substitution is placed.
+// The reconstruction depends on the columns only one by one, the replay only
+// on the branches' substitution counts and the parent's current row, so the
+// work goes in two parts:
+//   k_fitch_cols   a CTA per (16 columns, null), the whole tree in its shared
+//                  memory: the up pass of Tree_FitchAlgorithmAncenstral /
+//                  tree_fitch_column (src/msatree.c:173-227, 1700-1838):
+//                  intersection of the children's sets over the five states,
+//                  else the union of residues only (tree_fitch_upwards
+//                  :1877-1908), as byte-SIMD; the root's state; the down pass
+//                  (keep the parent's state when the child's set holds it);
+//                  and the substitutions of each kind on each branch, added
+//                  over the columns into the branch's 25 counters.
+//   the replay     the root's row with the columns shuffled
+//                  (msamanip_ShuffleColumns, src/msamanip.c:1164-1233; only
+//                  the root's shuffled row is ever read, every other row is
+//                  replaced by its parent's row before use), then top depth
+//                  first shuffle_tree_substitutions + shuffle_tree_substitute_all
+//                  (src/msamanip.c:1597-1747): a branch copies the parent's
+//                  current row and replays its substitutions on positions of
+//                  that row holding the old state, visited in a random order (a
+//                  Feistel permutation); each class's positions are ranked with
+//                  warp ballots and the pass stops once every substitution is
+//                  placed.  Small alignments: one launch, a cluster of CTAs per
+//                  null (k_null_replay); larger ones a launch per depth.
 //
 // Random draws are counter-based (Philox keyed by the seed, the null index,
 // the node and the column), so the result does not depend on scheduling.
 //
-// Buffers (per null q): F[q][v][Lp] the Fitch states of internal node v;
-// SR[q][v][Lp] first its Fitch set, then (once the set is used) its row of
+// Buffers (per null q): F[q] the root's states (row 0); ns[q][2N][25] the
+// substitutions from state a to state b on the branch above leaf s (entry s)
+// or internal node v (entry N + v), at 5 a + b; SR[q][v][Lp] node v's row of
 // the null alignment; leaf rows go straight to the output alignment slot.
 #include "cov_dev.cuh"
 #include "cov_kernels.h"
 #include "cov_batch.h"
+#include <algorithm>
+#include <atomic>
 
 namespace covgpu {
 
@@ -46,26 +51,43 @@ __device__ __forceinline__ int choose_member(unsigned S, uint64_t seed, uint32_t
 }
 
 
-// set of a leaf residue: one state, a random one for ambiguity codes
-__device__ __forceinline__ uint32_t leaf_byte(uint32_t x, int n, int c, uint64_t seed, uint32_t nid) {
-  if (x <= 4) return 1u << x;
-  return 1u << (int)(((uint64_t)rng_u32(seed, TAG_FLEAF, nid, (uint32_t)n, (uint32_t)c) * 5u) >> 32);
-}
-
-// the sets of 16 consecutive columns of child ch (internal row or leaf)
-__device__ __forceinline__ uint4 child_sets(int ch, const uint8_t* ax, const uint8_t* S, int Lp, int c0, uint64_t seed,
-                                           uint32_t nid) {
-  if (ch > 0) return *reinterpret_cast<const uint4*>(S + (int64_t)ch * Lp + c0);
-  const uint4 a = *reinterpret_cast<const uint4*>(ax + (int64_t)(-ch) * Lp + c0);
-  uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
+// States are kept as one bit per byte (1 << state), four columns to a word,
+// so the passes work on whole words; only random draws go byte by byte.
+//
+// word of four leaf codes: the states of codes 0-4; an ambiguity code gets a
+// random state, marked with bit 7
+constexpr uint32_t AMBIG = 0x80u;
+__device__ __forceinline__ uint32_t leaf_word(uint32_t w, int n, int c0, uint64_t seed, uint32_t nid) {
+  if ((w + 0x7B7B7B7Bu) & 0x80808080u) {   // a code above 4 (codes are below 18)
     uint32_t o = 0;
-#pragma unroll
-    for (int b = 0; b < 4; b++) o |= leaf_byte((w[k] >> (8 * b)) & 0xFFu, -ch, c0 + 4 * k + b, seed, nid) << (8 * b);
-    w[k] = o;
+    for (int b = 0; b < 4; b++) {
+      const uint32_t x = (w >> (8 * b)) & 0xFFu;
+      const uint32_t s =
+          x <= 4 ? 1u << x
+                 : AMBIG | (1u << (int)(((uint64_t)rng_u32(seed, TAG_FLEAF, nid, (uint32_t)n, (uint32_t)(c0 + b)) * 5u) >> 32));
+      o |= s << (8 * b);
+    }
+    return o;
   }
-  return make_uint4(w[0], w[1], w[2], w[3]);
+  const uint32_t sel = (w | (w >> 4)) & 0x00FF00FFu;   // codes to nibbles
+  return __byte_perm(0x08040201u, 0x00000010u, (sel | (sel >> 8)) & 0xFFFFu);
+}
+// the state numbers of a word of states
+__device__ __forceinline__ uint32_t state_codes(uint32_t w) {
+  return ((w >> 1) & 0x0F0F0F0Fu) - ((w >> 3) & 0x01010101u) - ((w >> 2) & 0x04040404u);
+}
+// one state of every set of a word: the only member, or a random one; the
+// bytes of pick are considered, the others kept
+__device__ __forceinline__ uint32_t choose_word(uint32_t s, uint32_t pick, int L, uint64_t seed, uint32_t nid,
+                                                uint32_t node, int c0) {
+  uint32_t multi = (s & (s - 0x01010101u)) & pick;   // sets are not empty: no borrow between bytes
+  if (multi == 0u) return s;
+  for (int b = 0; b < 4; b++)
+    if ((multi >> (8 * b)) & 0xFFu) {
+      const uint32_t st = (uint32_t)choose_member((s >> (8 * b)) & 0xFFu, seed, nid, node, (uint32_t)(c0 + b));
+      s = (s & ~(0xFFu << (8 * b))) | (1u << (8 * b + st));
+    }
+  return s;
 }
 
 // per byte: I = a & b if nonzero, else (a | b) without the gap bit
@@ -75,143 +97,179 @@ __device__ __forceinline__ uint32_t fitch_word(uint32_t a, uint32_t b) {
   return (I & ~z) | (U & z);
 }
 
-// up pass for the internal nodes of one depth
-__device__ __forceinline__ void fitch_up_body(
-    const GridIdx g, const uint8_t* __restrict__ ax, int N, int Lp, const int* __restrict__ left,
-    const int* __restrict__ right, const int* __restrict__ nodes, int nn, uint64_t seed, uint32_t first_null,
-    uint8_t* __restrict__ SR) {
-  const int chunks = Lp >> 4;
-  const int idx = g.x * blockDim.x + threadIdx.x;
-  if (idx >= nn * chunks) return;
-  const int q = g.y, v = nodes[idx / chunks], c0 = (idx % chunks) << 4;
-  const uint32_t nid = first_null + q;
-  uint8_t* S = SR + (int64_t)q * (N - 1) * Lp;
-  const uint4 a = child_sets(left[v], ax, S, Lp, c0, seed, nid);
-  const uint4 b = child_sets(right[v], ax, S, Lp, c0, seed, nid);
-  *reinterpret_cast<uint4*>(S + (int64_t)v * Lp + c0) =
-      make_uint4(fitch_word(a.x, b.x), fitch_word(a.y, b.y), fitch_word(a.z, b.z), fitch_word(a.w, b.w));
-}
-__global__ void __launch_bounds__(256)
-k_fitch_up(const uint8_t* __restrict__ ax, int N, int Lp, const int* __restrict__ left, const int* __restrict__ right,
-           const int* __restrict__ nodes, int nn, uint64_t seed, uint32_t first_null, uint8_t* __restrict__ SR) {
-  fitch_up_body(native_grid(), ax, N, Lp, left, right, nodes, nn, seed, first_null, SR);
-}
+// The reconstruction of FW words of four columns by one CTA.  With SM the
+// leaves, the nodes' sets (then states) and the tree lie in shared memory, 38
+// bytes per sequence for 16 columns, so a depth costs a barrier and a few
+// shared accesses; alignments too deep for that take the rows from global
+// memory (the null's row buffer SR, each CTA its own columns).  Bound by
+// instructions on large alignments (64% of the issue slots; 457 us for 20
+// nulls of 2,000 x 3,000), by the barriers on small ones (13 us for 30 x 61).
+// With the reconstruction inside the replay, depth by depth, the null
+// generation took (now): 30 x 61, 20 nulls 134 us (50); 400 x 300, 20 nulls
+// 572 (236); 500 x 400, 200 nulls 895 (762); 2,000 x 3,000, 20 nulls 1,266
+// (1,076); the reconstruction alone, 701 x 650, 300 us in 42 launches (20).
+constexpr int FW = 4;
+struct FitchCols {
+  const uint8_t* ax;
+  int N, L, Lp;
+  const int *left, *right, *lnodes, *loff;
+  int nlevels;
+  uint64_t seed;
+  uint32_t nid;
+  uint8_t* SR;     // [N-1][Lp] (not SM: scratch)
+  uint8_t* F;      // state numbers: the root's row, or every node's with all_rows
+  bool all_rows;
+  int* ns;         // [2N][25] branch counters, or nullptr
+};
+static size_t fitch_smem(int N) { return (size_t)N * (2 * FW * 4 + 3 * 2) + 16; }
+constexpr size_t FITCH_SMEM_MAX = 200 * 1024;
+static_assert(FITCH_SMEM_MAX / (2 * FW * 4 + 3 * 2) < 32768, "the tree's node numbers fit 16 bits");
 
-// the root's states F[q][0][c] from its sets
-__device__ __forceinline__ void root_state_body(
-    const GridIdx g, int N, int L, int Lp, uint64_t seed, uint32_t first_null, const uint8_t* __restrict__ SR,
-             uint8_t* __restrict__ F) {
-  const int c = g.x * blockDim.x + threadIdx.x, q = g.y;
-  if (c >= L) return;
-  const int64_t off = (int64_t)q * (N - 1) * Lp;
-  F[off + c] = (uint8_t)choose_member(SR[off + c], seed, first_null + q, 0u, (uint32_t)c);
+template <bool SM>
+__device__ __forceinline__ void fitch_cols(const FitchCols& a, int grp) {
+  extern __shared__ __align__(16) uint32_t fsm[];
+  const int N = a.N, tid = threadIdx.x, nthr = blockDim.x, c0 = grp * FW * 4;
+  uint32_t* leaf = fsm;
+  uint32_t* node = SM ? fsm + (size_t)N * FW : reinterpret_cast<uint32_t*>(a.SR + c0);
+  const int stride = SM ? FW : a.Lp / 4;
+  int16_t* lr = reinterpret_cast<int16_t*>(fsm + (size_t)2 * N * FW);   // SM: left, right, lnodes
+  if (SM) {
+    for (int i = tid; i < N * FW; i += nthr) {
+      const int s = i / FW, c = c0 + 4 * (i % FW);
+      leaf[i] = leaf_word(*reinterpret_cast<const uint32_t*>(a.ax + (int64_t)s * a.Lp + c), s, c, a.seed, a.nid);
+    }
+    for (int v = tid; v < N - 1; v += nthr) {
+      lr[v] = (int16_t)a.left[v]; lr[N + v] = (int16_t)a.right[v]; lr[2 * N + v] = (int16_t)a.lnodes[v];
+    }
+    __syncthreads();
+  }
+  auto left = [&](int v) { return SM ? (int)lr[v] : a.left[v]; };
+  auto right = [&](int v) { return SM ? (int)lr[N + v] : a.right[v]; };
+  auto order = [&](int k) { return SM ? (int)lr[2 * N + k] : a.lnodes[k]; };
+  auto leafw = [&](int s, int w) -> uint32_t {
+    if (SM) return leaf[s * FW + w];
+    const int c = c0 + 4 * w;
+    return leaf_word(*reinterpret_cast<const uint32_t*>(a.ax + (int64_t)s * a.Lp + c), s, c, a.seed, a.nid);
+  };
+  auto sets = [&](int ch, int w) -> uint32_t {
+    return ch > 0 ? node[(int64_t)ch * stride + w] : leafw(-ch, w) & ~(AMBIG * 0x01010101u);
+  };
+  for (int d = a.nlevels - 1; d >= 0; d--) {
+    const int o = a.loff[d], n = (a.loff[d + 1] - o) * FW;
+    for (int i = tid; i < n; i += nthr) {
+      const int v = order(o + i / FW), w = i % FW;
+      node[(int64_t)v * stride + w] = fitch_word(sets(left(v), w), sets(right(v), w));
+    }
+    __syncthreads();
+  }
+  for (int w = tid; w < FW; w += nthr) {   // the root's state
+    const uint32_t s = choose_word(node[w], 0xFFFFFFFFu, a.L, a.seed, a.nid, 0u, c0 + 4 * w);
+    node[w] = s;
+    *reinterpret_cast<uint32_t*>(a.F + c0 + 4 * w) = state_codes(s);
+  }
+  __syncthreads();
+  for (int d = 0; d < a.nlevels; d++) {
+    const int o = a.loff[d], n = 2 * (a.loff[d + 1] - o) * FW;
+    for (int i = tid; i < n; i += nthr) {
+      const int k = i / FW, w = i % FW, v = order(o + (k >> 1)), ch = (k & 1) ? right(v) : left(v);
+      const uint32_t p = node[(int64_t)v * stride + w];
+      uint32_t q;
+      if (ch > 0) {
+        // the parent's state where the child's set holds it, else one of the set
+        const uint32_t s = node[(int64_t)ch * stride + w], z = __vcmpeq4(s & p, 0u);
+        q = choose_word((p & ~z) | (s & z), z, a.L, a.seed, a.nid, (uint32_t)ch, c0 + 4 * w);
+        node[(int64_t)ch * stride + w] = q;
+        if (a.all_rows) *reinterpret_cast<uint32_t*>(a.F + (int64_t)ch * a.Lp + c0 + 4 * w) = state_codes(q);
+      } else {
+        q = leafw(-ch, w);
+      }
+      // bytes that differ, not ambiguous (a leaf's bit 7); columns past L hold
+      // gaps in every row and never differ
+      uint32_t diff = __vcmpne4(p, q) & ~__vcmpne4(q & (AMBIG * 0x01010101u), 0u);
+      if (!a.ns || diff == 0u) continue;
+      int* ns = a.ns + (int64_t)(ch > 0 ? N + ch : -ch) * 25;
+      do {
+        const int sh = (__ffs(diff) - 1) & ~7;
+        diff &= ~(0xFFu << sh);
+        const int x = __ffs((p >> sh) & 0xFFu) - 1, y = __ffs((q >> sh) & 0xFFu) - 1;
+        atomicAdd(ns + x * 5 + y, 1);
+      } while (diff);
+    }
+    __syncthreads();
+  }
 }
-__global__ void __launch_bounds__(256)
-k_root_state(int N, int L, int Lp, uint64_t seed, uint32_t first_null, const uint8_t* __restrict__ SR,
-             uint8_t* __restrict__ F) {
-  root_state_body(native_grid(), N, L, Lp, seed, first_null, SR, F);
+__device__ __forceinline__ int fitch_groups(int Lp) { return Lp / (FW * 4); }   // Lp is a multiple of 32
+
+template <bool SM>
+__global__ void __launch_bounds__(512)
+k_fitch_cols(FitchCols a, int64_t nstride, int64_t sstride) {
+  a.nid += blockIdx.y;
+  a.SR += blockIdx.y * sstride;
+  a.F += blockIdx.y * sstride;
+  if (a.ns) a.ns += blockIdx.y * nstride;
+  fitch_cols<SM>(a, blockIdx.x);
 }
 
 // the root's row of the null: its states with the columns shuffled
 __device__ __forceinline__ void root_row_body(
-    const GridIdx g, int N, int L, int Lp, uint64_t seed, uint32_t first_null, const uint8_t* __restrict__ F,
-           uint8_t* __restrict__ SR) {
+    const GridIdx g, int L, int Lp, uint64_t seed, uint32_t first_null, int64_t stride, const uint8_t* __restrict__ F,
+    int64_t fstride, uint8_t* __restrict__ SR) {
   const int c = g.x * blockDim.x + threadIdx.x, q = g.y;
   if (c >= Lp) return;
   uint32_t rk[6];
   round_keys(seed, TAG_COLPERM, first_null + q, 0, rk);
-  const int64_t off = (int64_t)q * (N - 1) * Lp;
-  SR[off + c] = (c < L) ? F[off + feistel_perm((uint32_t)c, feistel_hbits((uint32_t)L), (uint32_t)L, rk)] : (uint8_t)4;
+  SR[q * stride + c] = (c < L) ? F[q * fstride + feistel_perm((uint32_t)c, feistel_hbits((uint32_t)L), (uint32_t)L, rk)]
+                               : (uint8_t)4;
 }
 __global__ void __launch_bounds__(256)
-k_root_row(int N, int L, int Lp, uint64_t seed, uint32_t first_null, const uint8_t* __restrict__ F,
+k_root_row(int L, int Lp, uint64_t seed, uint32_t first_null, int64_t stride, const uint8_t* __restrict__ F,
            uint8_t* __restrict__ SR) {
-  root_row_body(native_grid(), N, L, Lp, seed, first_null, F, SR);
+  root_row_body(native_grid(), L, Lp, seed, first_null, stride, F, stride, SR);
 }
 
-// The replay of one (branch, null) item: phase 1, the child's Fitch states
-// (down pass) and the branch's substitution counts, 16 columns per thread;
-// phase 2, the child's row starts as a copy of the parent's row (staged in
-// shared memory too when srow is given, for the random reads of phase 3);
-// phase 3 walks the slots t in order, maps each to position perm(t) of the
-// parent's row and, for the state o there, ranks the slot among the slots of
-// class o so far: the r-th takes substitution r of class o while r <
-// need[o].  Once every class has its substitutions the walk stops (later
-// slots would place nothing).  Two kernels run phase 3: one warp per item,
-// 32 slots a step (levels with many items), and one CTA per item, 256 slots
-// a step with a prefix over the warps (levels with few, long items).
+// The replay of one (branch, null) item: the child's row starts as a copy of
+// the parent's row (staged in shared memory too when srow is given, for the
+// random reads that follow); then the walk goes through the slots t in order,
+// maps each to position perm(t) of the parent's row and, for the state o
+// there, ranks the slot among the slots of class o so far: the r-th takes
+// substitution r of class o while r < need[o].  Once every class has its
+// substitutions the walk stops (later slots would place nothing).  One warp
+// per item walks 32 slots a step, one CTA per item as many as it has threads,
+// with a prefix over the warps.
 struct ReplayItem {
-  int ch, cidx;
+  int cidx;            // leaf s: s; internal node v: N + v
   uint32_t nid;
-  const uint8_t *Fp, *Rp, *Sc, *Lc;
-  uint8_t *Fc, *Cc;
+  const uint8_t* Rp;   // parent's current row
+  uint8_t* Cc;         // child's row
+  const int* ns;       // the branch's 25 counters
 };
 
-__device__ __forceinline__ ReplayItem replay_item(const uint8_t* ax, int N, int Lp, const int* left, const int* right,
-                                                  const int* nodes, int item, int q, uint32_t first_null,
-                                                  uint8_t* F, uint8_t* SR, uint8_t* out_ax, int64_t out_slot_stride) {
+// this null's rows SR [N-1][Lp], alignment out [N][Lp] and counters ns [2N][25]
+__device__ __forceinline__ ReplayItem replay_item(int N, int Lp, const int* left, const int* right, const int* nodes,
+                                                  int item, uint32_t nid, uint8_t* SR, uint8_t* out, const int* ns) {
   ReplayItem it;
   const int v = nodes[item >> 1];
-  it.ch = (item & 1) ? right[v] : left[v];
-  it.cidx = (it.ch <= 0) ? -it.ch : N + it.ch;
-  it.nid = first_null + q;
-  const int64_t qoff = (int64_t)q * (N - 1) * Lp;
-  it.Fp = F + qoff + (int64_t)v * Lp;
-  it.Rp = SR + qoff + (int64_t)v * Lp;                            // parent's current row
-  it.Fc = F + qoff + (int64_t)(it.ch > 0 ? it.ch : 0) * Lp;       // written for an internal child only
-  it.Sc = SR + qoff + (int64_t)(it.ch > 0 ? it.ch : 0) * Lp;
-  it.Lc = ax + (int64_t)(it.ch <= 0 ? -it.ch : 0) * Lp;
-  it.Cc = (it.ch <= 0) ? out_ax + (int64_t)q * out_slot_stride + (int64_t)(-it.ch) * Lp
-                       : SR + qoff + (int64_t)it.ch * Lp;
+  const int ch = (item & 1) ? right[v] : left[v];
+  it.cidx = (ch <= 0) ? -ch : N + ch;
+  it.nid = nid;
+  it.Rp = SR + (int64_t)v * Lp;
+  it.Cc = (ch <= 0) ? out + (int64_t)(-ch) * Lp : SR + (int64_t)ch * Lp;
+  it.ns = ns + (int64_t)it.cidx * 25;
   return it;
 }
 
-// phases 1 and 2 by nthr threads (this one: tid); nsub (25 counters, zeroed)
-// and srow (nullptr or Lp bytes) in shared memory
-__device__ __forceinline__ void replay_prepare(const ReplayItem& it, int L, int Lp, uint64_t seed, int tid, int nthr,
-                                               int* nsub, uint8_t* srow) {
-  for (int c0 = tid * 16; c0 < Lp; c0 += nthr * 16) {
-    const uint4 pv = *reinterpret_cast<const uint4*>(it.Fp + c0);
-    uint4 cv;
-    if (it.ch > 0) {
-      const uint4 sv = *reinterpret_cast<const uint4*>(it.Sc + c0);
-      uint32_t pw[4] = {pv.x, pv.y, pv.z, pv.w}, sw[4] = {sv.x, sv.y, sv.z, sv.w}, ow[4];
+// the row copy by nthr threads (this one: tid), and cum [5][6], the running
+// sums of each class's counters (rows that other SMs wrote: past L1)
+__device__ __forceinline__ void replay_prepare(const ReplayItem& it, int Lp, int tid, int nthr, int (*cum)[6],
+                                               uint8_t* srow) {
+  if (tid < 5) {
+    int s = 0;
+    cum[tid][0] = 0;
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        uint32_t o = 0;
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-          const int c = c0 + 4 * k + b;
-          uint32_t st = 4;
-          if (c < L) {
-            const uint32_t a = (pw[k] >> (8 * b)) & 0xFFu;
-            unsigned set = (sw[k] >> (8 * b)) & 0xFFu;
-            if (set & (1u << a)) set = 1u << a;
-            st = (uint32_t)choose_member(set, seed, it.nid, (uint32_t)it.ch, (uint32_t)c);
-          }
-          o |= st << (8 * b);
-        }
-        ow[k] = o;
-      }
-      cv = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-      *reinterpret_cast<uint4*>(it.Fc + c0) = cv;
-    } else {
-      cv = *reinterpret_cast<const uint4*>(it.Lc + c0);
-    }
-    const uint32_t pw[4] = {pv.x, pv.y, pv.z, pv.w}, cw[4] = {cv.x, cv.y, cv.z, cv.w};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (pw[k] == cw[k]) continue;
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const int c = c0 + 4 * k + b;
-        const uint32_t a = (pw[k] >> (8 * b)) & 0xFFu, d = (cw[k] >> (8 * b)) & 0xFFu;
-        if (c < L && a != d && a <= 4 && d <= 4) atomicAdd(&nsub[a * 5 + d], 1);
-      }
-    }
+    for (int d = 0; d < 5; d++) { s += it.ns[tid * 5 + d]; cum[tid][d + 1] = s; }
   }
   for (int c0 = tid * 16; c0 < Lp; c0 += nthr * 16) {   // Lp is a multiple of 32
-    const uint4 v4 = *reinterpret_cast<const uint4*>(it.Rp + c0);
+    const uint4 v4 = __ldcg(reinterpret_cast<const uint4*>(it.Rp + c0));
     *reinterpret_cast<uint4*>(it.Cc + c0) = v4;
     if (srow) *reinterpret_cast<uint4*>(srow + c0) = v4;
   }
@@ -221,49 +279,29 @@ __device__ __forceinline__ unsigned pick5(const unsigned (&m)[5], int k) {
   return k == 0 ? m[0] : k == 1 ? m[1] : k == 2 ? m[2] : k == 3 ? m[3] : m[4];
 }
 
-// one warp per item, eight items per CTA (SROW: Lp bytes of row per warp)
-template <bool SROW>
-__device__ __forceinline__ void replay_warp_body(
-    const GridIdx g, const uint8_t* __restrict__ ax, int N, int L, int Lp, const int* __restrict__ left,
-              const int* __restrict__ right, const int* __restrict__ nodes, int nn, uint64_t seed,
-              uint32_t first_null, uint8_t* __restrict__ F, uint8_t* __restrict__ SR, uint8_t* __restrict__ out_ax,
-              int64_t out_slot_stride) {
-  extern __shared__ __align__(16) uint8_t rowbuf[];
-  __shared__ int nsub_s[8][25];
-  __shared__ int cum_s[8][5][6];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int item = g.x * 8 + warp;
-  if (item >= 2 * nn) return;
-  const ReplayItem it = replay_item(ax, N, Lp, left, right, nodes, item, g.y, first_null, F, SR, out_ax,
-                                    out_slot_stride);
-  int* nsub = nsub_s[warp];
-  if (lane < 25) nsub[lane] = 0;
+// one item by one warp; srow (nullptr or Lp bytes) and cum [5][6] in shared
+// memory, the warp's own
+__device__ __forceinline__ void replay_item_warp(const ReplayItem& it, int L, int Lp, uint64_t seed, int lane,
+                                                 int (*cum)[6], uint8_t* srow) {
+  replay_prepare(it, Lp, lane, 32, cum, srow);
   __syncwarp();
-  uint8_t* srow = SROW ? rowbuf + (size_t)warp * Lp : nullptr;
-  replay_prepare(it, L, Lp, seed, lane, 32, nsub, srow);
-  __syncwarp();
-  int (*cum)[6] = cum_s[warp];
-  if (lane < 5) {
-    cum[lane][0] = 0;
-    for (int d = 0; d < 5; d++) cum[lane][d + 1] = cum[lane][d] + nsub[lane * 5 + d];
-  }
-  __syncwarp();
-  int need[5], run[5] = {0, 0, 0, 0, 0}, total = 0;
+  int need[5], total = 0;
 #pragma unroll
   for (int o = 0; o < 5; o++) { need[o] = cum[o][5]; total += need[o]; }
   if (total == 0) return;
   uint32_t rk[6];
   round_keys(seed, TAG_SUBST, it.nid, (uint32_t)it.cidx, rk);
+  const uint8_t* R = srow ? srow : it.Rp;
   const uint32_t hb = feistel_hbits((uint32_t)L);
   const unsigned lt = (1u << lane) - 1u;
-  const uint8_t* R = SROW ? srow : it.Rp;
+  int run[5] = {0, 0, 0, 0, 0};
   for (int t0 = 0; t0 < L; t0 += 32) {
     const int t = t0 + lane;
     uint32_t p = 0;
     int o = 5;
     if (t < L) {
       p = feistel_perm((uint32_t)t, hb, (uint32_t)L, rk);
-      o = R[p];
+      o = srow ? R[p] : __ldcg(R + p);
     }
     bool done = true;
 #pragma unroll
@@ -283,42 +321,41 @@ __device__ __forceinline__ void replay_warp_body(
     if (done) break;
   }
 }
+
+// one warp per item, eight items per CTA (SROW: Lp bytes of row per warp)
+template <bool SROW>
+__device__ __forceinline__ void replay_warp_body(
+    const GridIdx g, int N, int L, int Lp, const int* __restrict__ left, const int* __restrict__ right,
+    const int* __restrict__ nodes, int nn, uint64_t seed, uint32_t first_null, const int* __restrict__ ns, uint8_t* SR,
+    uint8_t* out_ax, int64_t out_slot_stride) {
+  extern __shared__ __align__(16) uint8_t rowbuf[];
+  __shared__ int cum_s[8][5][6];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int item = g.x * 8 + warp;
+  if (item >= 2 * nn) return;
+  const ReplayItem it = replay_item(N, Lp, left, right, nodes, item, first_null + g.y,
+                                    SR + (int64_t)g.y * (N - 1) * Lp, out_ax + g.y * out_slot_stride,
+                                    ns + (int64_t)g.y * 2 * N * 25);
+  replay_item_warp(it, L, Lp, seed, lane, cum_s[warp], SROW ? rowbuf + (size_t)warp * Lp : nullptr);
+}
 template <bool SROW>
 __global__ void __launch_bounds__(256)
-k_replay_warp(const uint8_t* __restrict__ ax, int N, int L, int Lp, const int* __restrict__ left,
-              const int* __restrict__ right, const int* __restrict__ nodes, int nn, uint64_t seed,
-              uint32_t first_null, uint8_t* __restrict__ F, uint8_t* __restrict__ SR, uint8_t* __restrict__ out_ax,
-              int64_t out_slot_stride) {
-  replay_warp_body<SROW>(native_grid(), ax, N, L, Lp, left, right, nodes, nn, seed, first_null, F, SR, out_ax,
-                                        out_slot_stride);
+k_replay_warp(int N, int L, int Lp, const int* __restrict__ left, const int* __restrict__ right,
+              const int* __restrict__ nodes, int nn, uint64_t seed, uint32_t first_null, const int* __restrict__ ns,
+              uint8_t* SR, uint8_t* out_ax, int64_t out_slot_stride) {
+  replay_warp_body<SROW>(native_grid(), N, L, Lp, left, right, nodes, nn, seed, first_null, ns, SR, out_ax,
+                         out_slot_stride);
 }
 
-// one CTA per item (SROW: Lp bytes of row)
-template <bool SROW>
-__device__ __forceinline__ void replay_cta_body(
-    const GridIdx g, const uint8_t* __restrict__ ax, int N, int L, int Lp, const int* __restrict__ left,
-             const int* __restrict__ right, const int* __restrict__ nodes, int nn, uint64_t seed,
-             uint32_t first_null, uint8_t* __restrict__ F, uint8_t* __restrict__ SR, uint8_t* __restrict__ out_ax,
-             int64_t out_slot_stride) {
-  extern __shared__ __align__(16) uint8_t rowbuf[];
-  __shared__ int nsub[25];
-  __shared__ int cum[5][6];
-  __shared__ int gcnt[8][5];   // slots per class in each warp's group of the chunk
-  __shared__ int base[5];      // slots per class before the chunk
+// one item by a CTA of NW warps; srow as above; cum [5][6], gcnt [NW][5]
+// (slots per class in each warp's group of the chunk) and base [5] (slots per
+// class before it) in shared memory
+template <int NW>
+__device__ __forceinline__ void replay_item_cta(const ReplayItem& it, int L, int Lp, uint64_t seed, int (*cum)[6],
+                                                int (*gcnt)[5], int* base, uint8_t* srow) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int item = g.x;
-  if (item >= 2 * nn) return;
-  const ReplayItem it = replay_item(ax, N, Lp, left, right, nodes, item, g.y, first_null, F, SR, out_ax,
-                                    out_slot_stride);
-  if (tid < 25) nsub[tid] = 0;
-  __syncthreads();
-  replay_prepare(it, L, Lp, seed, tid, 256, nsub, SROW ? rowbuf : nullptr);
-  __syncthreads();
-  if (tid < 5) {
-    cum[tid][0] = 0;
-    for (int d = 0; d < 5; d++) cum[tid][d + 1] = cum[tid][d] + nsub[tid * 5 + d];
-    base[tid] = 0;
-  }
+  if (tid < 5) base[tid] = 0;
+  replay_prepare(it, Lp, tid, NW * 32, cum, srow);
   __syncthreads();
   int need[5], total = 0;
 #pragma unroll
@@ -328,14 +365,14 @@ __device__ __forceinline__ void replay_cta_body(
   round_keys(seed, TAG_SUBST, it.nid, (uint32_t)it.cidx, rk);
   const uint32_t hb = feistel_hbits((uint32_t)L);
   const unsigned lt = (1u << lane) - 1u;
-  const uint8_t* R = SROW ? rowbuf : it.Rp;
-  for (int t0 = 0; t0 < L; t0 += 256) {
+  const uint8_t* R = srow ? srow : it.Rp;
+  for (int t0 = 0; t0 < L; t0 += NW * 32) {
     const int t = t0 + tid;
     uint32_t p = 0;
     int o = 5;
     if (t < L) {
       p = feistel_perm((uint32_t)t, hb, (uint32_t)L, rk);
-      o = R[p];
+      o = srow ? R[p] : __ldcg(R + p);
     }
     unsigned m[5];
 #pragma unroll
@@ -354,7 +391,7 @@ __device__ __forceinline__ void replay_cta_body(
     __syncthreads();   // base and gcnt read
     if (tid < 5) {
       int s2 = base[tid];
-      for (int w = 0; w < 8; w++) s2 += gcnt[w][tid];
+      for (int w = 0; w < NW; w++) s2 += gcnt[w][tid];
       base[tid] = s2;
     }
     __syncthreads();
@@ -364,20 +401,125 @@ __device__ __forceinline__ void replay_cta_body(
     if (all) break;   // the same in every thread
   }
 }
+
+// one CTA per item (SROW: Lp bytes of row)
+template <bool SROW>
+__device__ __forceinline__ void replay_cta_body(
+    const GridIdx g, int N, int L, int Lp, const int* __restrict__ left, const int* __restrict__ right,
+    const int* __restrict__ nodes, int nn, uint64_t seed, uint32_t first_null, const int* __restrict__ ns, uint8_t* SR,
+    uint8_t* out_ax, int64_t out_slot_stride) {
+  extern __shared__ __align__(16) uint8_t rowbuf[];
+  __shared__ int cum[5][6], gcnt[8][5], base[5];
+  if (g.x >= 2 * nn) return;
+  const ReplayItem it = replay_item(N, Lp, left, right, nodes, g.x, first_null + g.y,
+                                    SR + (int64_t)g.y * (N - 1) * Lp, out_ax + g.y * out_slot_stride,
+                                    ns + (int64_t)g.y * 2 * N * 25);
+  replay_item_cta<8>(it, L, Lp, seed, cum, gcnt, base, SROW ? rowbuf : nullptr);
+}
 template <bool SROW>
 __global__ void __launch_bounds__(256)
-k_replay_cta(const uint8_t* __restrict__ ax, int N, int L, int Lp, const int* __restrict__ left,
-             const int* __restrict__ right, const int* __restrict__ nodes, int nn, uint64_t seed,
-             uint32_t first_null, uint8_t* __restrict__ F, uint8_t* __restrict__ SR, uint8_t* __restrict__ out_ax,
-             int64_t out_slot_stride) {
-  replay_cta_body<SROW>(native_grid(), ax, N, L, Lp, left, right, nodes, nn, seed, first_null, F, SR, out_ax,
-                                       out_slot_stride);
+k_replay_cta(int N, int L, int Lp, const int* __restrict__ left, const int* __restrict__ right,
+             const int* __restrict__ nodes, int nn, uint64_t seed, uint32_t first_null, const int* __restrict__ ns,
+             uint8_t* SR, uint8_t* out_ax, int64_t out_slot_stride) {
+  replay_cta_body<SROW>(native_grid(), N, L, Lp, left, right, nodes, nn, seed, first_null, ns, SR, out_ax,
+                        out_slot_stride);
 }
 
-// items per level up to which the replay goes one CTA per item: measured on
+// The replay of one null by one cluster of CTAs, every depth in one launch: a
+// cluster barrier between depths (the levels of one null depend on each
+// other, the nulls do not).  A depth with at most one item per CTA takes a CTA
+// per item, the others a warp per item.
+struct NullOne {
+  int N, L, Lp;
+  const int *left, *right, *lnodes, *loff;   // loff [nlevels + 1]: depth offsets in lnodes
+  int nlevels;
+  const uint8_t* F;                          // the root's states
+  const int* ns;
+  uint8_t *SR, *out;                         // this null's rows and alignment
+  uint64_t seed;
+  uint32_t nid;
+};
+
+constexpr int NULL_WARPS = 16;
+
+__device__ __forceinline__ void null_sync(int csize) {
+  if (csize == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  }
+}
+
+__device__ __forceinline__ void null_replay(const NullOne& a, int crank, int csize, bool srow) {
+  extern __shared__ __align__(16) uint8_t rowbuf[];
+  __shared__ int cum_s[NULL_WARPS][5][6];
+  __shared__ int gcnt[NULL_WARPS][5], base[5];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  {
+    uint32_t rk[6];
+    round_keys(a.seed, TAG_COLPERM, a.nid, 0, rk);
+    const uint32_t hb = feistel_hbits((uint32_t)a.L);
+    for (int c = crank * (NULL_WARPS * 32) + tid; c < a.Lp; c += csize * (NULL_WARPS * 32))
+      a.SR[c] = (c < a.L) ? a.F[feistel_perm((uint32_t)c, hb, (uint32_t)a.L, rk)] : (uint8_t)4;
+  }
+  null_sync(csize);
+  for (int d = 0; d < a.nlevels; d++) {
+    const int o = a.loff[d], n = 2 * (a.loff[d + 1] - o);
+    if (n <= csize) {
+      if (crank < n) {
+        const ReplayItem it = replay_item(a.N, a.Lp, a.left, a.right, a.lnodes + o, crank, a.nid, a.SR, a.out, a.ns);
+        replay_item_cta<NULL_WARPS>(it, a.L, a.Lp, a.seed, cum_s[0], gcnt, base, srow ? rowbuf : nullptr);
+      }
+    } else {
+      for (int item = warp * csize + crank; item < n; item += NULL_WARPS * csize) {
+        const ReplayItem it = replay_item(a.N, a.Lp, a.left, a.right, a.lnodes + o, item, a.nid, a.SR, a.out, a.ns);
+        replay_item_warp(it, a.L, a.Lp, a.seed, lane, cum_s[warp], srow ? rowbuf + (size_t)warp * a.Lp : nullptr);
+        __syncwarp();
+      }
+    }
+    if (d + 1 < a.nlevels) null_sync(csize);
+  }
+}
+
+__global__ void __launch_bounds__(NULL_WARPS * 32, 2)
+k_null_replay(int N, int L, int Lp, const int* left, const int* right, const int* lnodes, const int* loff,
+              int nlevels, uint64_t seed, uint32_t first_null, const uint8_t* F, const int* ns, uint8_t* SR,
+              uint8_t* out, int64_t out_stride, int csize, bool srow) {
+  const int q = blockIdx.x / csize;
+  const int64_t off = (int64_t)q * (N - 1) * Lp;
+  const NullOne a{N, L, Lp, left, right, lnodes, loff, nlevels, F + off, ns + (int64_t)q * 2 * N * 25, SR + off,
+                  out + q * out_stride, seed, first_null + q};
+  null_replay(a, blockIdx.x % csize, csize, srow);
+}
+
+// items of a launch up to which the replay goes one CTA per item: measured on
 // N=2000 x L=3000 with 20 nulls, one CTA per item is faster up to about 3,000
-// items (long branches near the root), one warp per item beyond
+// items (long branches near the root), one warp per item beyond.  In a family
+// batch the items of all families count: 64 ragged families 84 ms a call, 96
+// with the rule taken family by family.
 constexpr int64_t kReplayCtaItems = 3000;
+
+bool replay_uses_cta(int64_t items) { return items <= kReplayCtaItems; }
+
+constexpr size_t NULL_SMEM_MAX = 100 * 1024;   // two CTAs per SM
+// CTAs of the cluster that replays one null in one launch, 0: a launch per
+// depth.  One launch wins where the depths are short: up to 13M columns x
+// sequences x nulls in all and rows of 1,024 columns (a warp's walk along a
+// longer row takes longer than the launches).  Measured against the launches
+// (us, the whole null generation): N=30 x L=61, 20 nulls 50 / 77 (C = 1);
+// 100 x 120 112 / 151; 400 x 300 236 / 375; 301 x 773 193 / 218; 2,000 x 300
+// 521 / 544; but 500 x 400 with 200 nulls 803 / 762, 100 x 3,000 263 / 205,
+// 2,000 x 3,000 1,338 / 1,076.
+static int null_cluster(int N, int L, int nnull) {
+  if (L > 1024 || (double)N * L * nnull > 13e6) return 0;
+  if ((int64_t)N * L < 8192) return 1;
+  int dev = 0, nsm = 152, C = 8;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  while (C > 1 && (int64_t)C * nnull > 2 * nsm) C >>= 1;
+  return C;
+}
 
 // the replay's shared-memory row buffers: the launch limit of both kernels
 // is raised once to the device's opt-in maximum; rows that do not fit are
@@ -398,68 +540,95 @@ static int replay_smem_limit() {
   return lim;
 }
 
-// down pass of the Fitch reconstruction for the internal children of one
-// depth: one thread per (branch, 16 columns); a child keeps its parent's
-// state when its set holds it, else a random member of its set
-__global__ void __launch_bounds__(256)
-k_fitch_down(int N, int L, int Lp, const int* __restrict__ left, const int* __restrict__ right,
-             const int* __restrict__ nodes, int nn, uint64_t seed, uint32_t nid, const uint8_t* __restrict__ S,
-             uint8_t* __restrict__ F) {
-  const int chunks = Lp >> 4;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 2 * nn * chunks) return;
-  const int kb = idx / chunks, c0 = (idx % chunks) << 4;
-  const int v = nodes[kb >> 1];
-  const int ch = (kb & 1) ? right[v] : left[v];
-  if (ch <= 0) return;
-  for (int k = 0; k < 16; k++) {
-    const int c = c0 + k;
-    uint8_t st = 4;
-    if (c < L) {
-      const int a = F[(int64_t)v * Lp + c];
-      unsigned set = S[(int64_t)ch * Lp + c];
-      if (set & (1u << a)) set = 1u << a;
-      st = (uint8_t)choose_member(set, seed, nid, (uint32_t)ch, (uint32_t)c);
-    }
-    F[(int64_t)ch * Lp + c] = st;
-  }
+template <bool SM>
+__global__ void __launch_bounds__(512)
+k_fitch_cols_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre, uint64_t seed) {
+  const int f = grp_find(pre, nf, (int)blockIdx.x);
+  const FamDev& d = F[f];
+  const int gx = fitch_groups(d.Lp), loc = (int)blockIdx.x - __ldg(pre + f), q = loc / gx;
+  const FitchCols a{d.ax, d.N, d.L, d.Lp, d.left, d.right, d.lnodes, d.lnodes + (d.N - 1), d.nlevels, seed,
+                    (uint32_t)q, d.scratch + (int64_t)q * (d.N - 1) * d.Lp, d.fitch + (int64_t)q * d.Lp, false,
+                    d.ns + (int64_t)q * 2 * d.N * 25};
+  fitch_cols<SM>(a, loc % gx);
+}
+
+// raises the shared-memory limits of this file's kernels on the current
+// device, once (before any stream capture)
+static cudaError_t null_attrs() {
+  constexpr int MAXDEV = 64;
+  static std::atomic<int> done[MAXDEV];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < MAXDEV && done[dev].load()) return cudaSuccess;
+  const void* fit[] = {(const void*)k_fitch_cols<true>, (const void*)k_fitch_cols_grp<true>};
+  for (const void* f : fit)
+    if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FITCH_SMEM_MAX)) != cudaSuccess)
+      return e;
+  if ((e = cudaFuncSetAttribute(k_null_replay, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NULL_SMEM_MAX)) !=
+      cudaSuccess)
+    return e;
+  if (dev < MAXDEV) done[dev].store(1);
+  return cudaSuccess;
+}
+
+// the widest depth of a tree of N leaves is about N / 10 nodes (coalescent): 4
+// words of each
+static int fitch_threads(int N) { return N >= 512 ? 512 : (N >= 128 ? 256 : 128); }
+
+static cudaError_t launch_fitch_cols(const FitchCols& a, int nnull, int64_t nstride, int64_t sstride,
+                                     cudaStream_t st) {
+  const size_t sm = fitch_smem(a.N);
+  const dim3 g(a.Lp / (FW * 4), nnull);
+  const int thr = fitch_threads(a.N);
+  if (sm <= FITCH_SMEM_MAX) k_fitch_cols<true><<<g, thr, sm, st>>>(a, nstride, sstride);
+  else                      k_fitch_cols<false><<<g, thr, 0, st>>>(a, nstride, sstride);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_fitch_recon(const uint8_t* ax, int N, int L, int Lp, const NullTree& T, const int* level_nodes,
-                               const int* level_off, int nlevels, uint64_t seed, uint32_t nid, uint8_t* F, uint8_t* S,
-                               cudaStream_t st) {
-  const int chunks = Lp / 16;
-  for (int d = nlevels - 1; d >= 0; d--) {
-    const int nn = level_off[d + 1] - level_off[d];
-    if (nn <= 0) continue;
-    k_fitch_up<<<dim3((nn * chunks + 255) / 256, 1), 256, 0, st>>>(ax, N, Lp, T.left, T.right,
-                                                                    level_nodes + level_off[d], nn, seed, nid, S);
-  }
-  k_root_state<<<dim3((L + 255) / 256, 1), 256, 0, st>>>(N, L, Lp, seed, nid, S, F);
-  for (int d = 0; d < nlevels; d++) {
-    const int nn = level_off[d + 1] - level_off[d];
-    if (nn <= 0) continue;
-    k_fitch_down<<<(2 * nn * chunks + 255) / 256, 256, 0, st>>>(N, L, Lp, T.left, T.right, level_nodes + level_off[d],
-                                                                 nn, seed, nid, S, F);
-  }
-  return cudaGetLastError();
+                               int nlevels, uint64_t seed, uint32_t nid, uint8_t* F, uint8_t* S, cudaStream_t st) {
+  cudaError_t e = null_attrs();
+  if (e != cudaSuccess) return e;
+  const FitchCols a{ax, N, L, Lp, T.left, T.right, level_nodes, level_nodes + (N - 1), nlevels, seed, nid, S, F, true,
+                    nullptr};
+  return launch_fitch_cols(a, 1, 0, 0, st);
 }
 
 cudaError_t launch_nullgen(const uint8_t* ax, int N, int L, int Lp, const NullTree& T, const int* level_nodes,
                            const int* level_off, int nlevels, uint64_t seed, uint32_t first_null, int nnull,
-                           uint8_t* fitch, uint8_t* scratch, uint8_t* out_ax, int64_t out_slot_stride,
-                           cudaStream_t st) {
-  // scratch holds the Fitch sets, each row replaced by the null's row once used
-  const int chunks = Lp / 16;
-  for (int d = nlevels - 1; d >= 0; d--) {
-    const int nn = level_off[d + 1] - level_off[d];
-    if (nn <= 0) continue;
-    k_fitch_up<<<dim3((nn * chunks + 255) / 256, nnull), 256, 0, st>>>(ax, N, Lp, T.left, T.right,
-                                                                       level_nodes + level_off[d], nn, seed,
-                                                                       first_null, scratch);
+                           uint8_t* fitch, uint8_t* rows, int* ns, uint8_t* out_ax, int64_t out_slot_stride,
+                           cudaStream_t st, int* nlaunch) {
+  cudaError_t e = null_attrs();
+  if (e != cudaSuccess) return e;
+  const int64_t stride = (int64_t)(N - 1) * Lp, nstride = (int64_t)2 * N * 25;
+  const int* d_off = level_nodes + (N - 1);
+  if ((e = cudaMemsetAsync(ns, 0, (size_t)nstride * nnull * sizeof(int), st)) != cudaSuccess) return e;
+  const FitchCols a{ax, N, L, Lp, T.left, T.right, level_nodes, d_off, nlevels, seed, first_null, rows, fitch, false,
+                    ns};
+  if ((e = launch_fitch_cols(a, nnull, nstride, stride, st)) != cudaSuccess) return e;
+  const int C = null_cluster(N, L, nnull);
+  if (C) {
+    const size_t sm = (size_t)NULL_WARPS * Lp;
+    const bool srow = sm <= NULL_SMEM_MAX;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C * nnull);
+    cfg.blockDim = dim3(NULL_WARPS * 32);
+    cfg.dynamicSmemBytes = srow ? sm : 0;
+    cfg.stream = st;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeClusterDimension;
+    la[0].val.clusterDim.x = C;
+    la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    *nlaunch += 2;
+    return cudaLaunchKernelEx(&cfg, k_null_replay, N, L, Lp, T.left, T.right, level_nodes, d_off, nlevels, seed,
+                              first_null, (const uint8_t*)fitch, (const int*)ns, rows, out_ax, out_slot_stride, C,
+                              srow);
   }
-  k_root_state<<<dim3((L + 255) / 256, nnull), 256, 0, st>>>(N, L, Lp, seed, first_null, scratch, fitch);
-  k_root_row<<<dim3((Lp + 255) / 256, nnull), 256, 0, st>>>(N, L, Lp, seed, first_null, fitch, scratch);
+  k_root_row<<<dim3((Lp + 255) / 256, nnull), 256, 0, st>>>(L, Lp, seed, first_null, stride, fitch, rows);
+  *nlaunch += 2;
   // levels with few items (near the root and the leaves) go one CTA per
   // item; the others one warp per item
   const int lim = replay_smem_limit();
@@ -468,22 +637,23 @@ cudaError_t launch_nullgen(const uint8_t* ax, int N, int L, int Lp, const NullTr
     const int nn = level_off[d + 1] - level_off[d];
     if (nn <= 0) continue;
     const int* lv = level_nodes + level_off[d];
-    if ((int64_t)2 * nn * nnull <= kReplayCtaItems) {
+    *nlaunch += 1;
+    if (replay_uses_cta((int64_t)2 * nn * nnull)) {
       const dim3 g(2 * nn, nnull);
       if (srow_cta)
-        k_replay_cta<true><<<g, 256, (size_t)Lp, st>>>(ax, N, L, Lp, T.left, T.right, lv, nn, seed, first_null, fitch,
-                                                      scratch, out_ax, out_slot_stride);
+        k_replay_cta<true><<<g, 256, (size_t)Lp, st>>>(N, L, Lp, T.left, T.right, lv, nn, seed, first_null, ns, rows,
+                                                      out_ax, out_slot_stride);
       else
-        k_replay_cta<false><<<g, 256, 0, st>>>(ax, N, L, Lp, T.left, T.right, lv, nn, seed, first_null, fitch,
-                                               scratch, out_ax, out_slot_stride);
+        k_replay_cta<false><<<g, 256, 0, st>>>(N, L, Lp, T.left, T.right, lv, nn, seed, first_null, ns, rows, out_ax,
+                                               out_slot_stride);
     } else {
       const dim3 g((2 * nn + 7) / 8, nnull);
       if (srow_warp)
-        k_replay_warp<true><<<g, 256, (size_t)8 * Lp, st>>>(ax, N, L, Lp, T.left, T.right, lv, nn, seed, first_null,
-                                                            fitch, scratch, out_ax, out_slot_stride);
+        k_replay_warp<true><<<g, 256, (size_t)8 * Lp, st>>>(N, L, Lp, T.left, T.right, lv, nn, seed, first_null, ns,
+                                                            rows, out_ax, out_slot_stride);
       else
-        k_replay_warp<false><<<g, 256, 0, st>>>(ax, N, L, Lp, T.left, T.right, lv, nn, seed, first_null, fitch,
-                                                scratch, out_ax, out_slot_stride);
+        k_replay_warp<false><<<g, 256, 0, st>>>(N, L, Lp, T.left, T.right, lv, nn, seed, first_null, ns, rows, out_ax,
+                                                out_slot_stride);
     }
   }
   return cudaGetLastError();
@@ -495,30 +665,12 @@ cudaError_t launch_nullgen(const uint8_t* ax, int N, int L, int Lp, const NullTr
 // every family's nulls use the single-family streams (null ids 0..ns-1)
 // ------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-k_fitch_up_grp(const FamDev* __restrict__ F, int nf, const int2* __restrict__ lv, const int* __restrict__ pre,
-               uint64_t seed) {
-  const int f = grp_find(pre, nf, (int)blockIdx.x);
-  const FamDev& d = F[f];
-  const int2 v = lv[f];
-  const int gx = (v.y * (d.Lp >> 4) + 255) / 256, loc = (int)blockIdx.x - __ldg(pre + f);
-  fitch_up_body(GridIdx{loc % gx, loc / gx, gx}, d.ax, d.N, d.Lp, d.left, d.right, d.lnodes + v.x, v.y, seed, 0u,
-                d.scratch);
-}
-
-__global__ void __launch_bounds__(256)
-k_root_state_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre, uint64_t seed) {
-  const int f = grp_find(pre, nf, (int)blockIdx.x);
-  const FamDev& d = F[f];
-  const int gx = (d.L + 255) / 256, loc = (int)blockIdx.x - __ldg(pre + f);
-  root_state_body(GridIdx{loc % gx, loc / gx, gx}, d.N, d.L, d.Lp, seed, 0u, d.scratch, d.fitch);
-}
-
-__global__ void __launch_bounds__(256)
 k_root_row_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre, uint64_t seed) {
   const int f = grp_find(pre, nf, (int)blockIdx.x);
   const FamDev& d = F[f];
   const int gx = (d.Lp + 255) / 256, loc = (int)blockIdx.x - __ldg(pre + f);
-  root_row_body(GridIdx{loc % gx, loc / gx, gx}, d.N, d.L, d.Lp, seed, 0u, d.fitch, d.scratch);
+  root_row_body(GridIdx{loc % gx, loc / gx, gx}, d.L, d.Lp, seed, 0u, (int64_t)(d.N - 1) * d.Lp, d.fitch, d.Lp,
+                d.scratch);
 }
 
 template <bool SROW>
@@ -530,8 +682,8 @@ k_replay_warp_grp(const FamDev* __restrict__ F, int nf, const int2* __restrict__
   const int2 v = lv[f];
   const int gx = (2 * v.y + 7) / 8, loc = (int)blockIdx.x - __ldg(pre + f);
   const int64_t ss = (int64_t)d.N * d.Lp;
-  replay_warp_body<SROW>(GridIdx{loc % gx, loc / gx, gx}, d.ax, d.N, d.L, d.Lp, d.left, d.right, d.lnodes + v.x, v.y,
-                         seed, 0u, d.fitch, d.scratch, d.ax + ss, ss);
+  replay_warp_body<SROW>(GridIdx{loc % gx, loc / gx, gx}, d.N, d.L, d.Lp, d.left, d.right, d.lnodes + v.x, v.y, seed,
+                         0u, d.ns, d.scratch, d.ax + ss, ss);
 }
 
 template <bool SROW>
@@ -543,11 +695,10 @@ k_replay_cta_grp(const FamDev* __restrict__ F, int nf, const int2* __restrict__ 
   const int2 v = lv[f];
   const int gx = 2 * v.y, loc = (int)blockIdx.x - __ldg(pre + f);
   const int64_t ss = (int64_t)d.N * d.Lp;
-  replay_cta_body<SROW>(GridIdx{loc % gx, loc / gx, gx}, d.ax, d.N, d.L, d.Lp, d.left, d.right, d.lnodes + v.x, v.y,
-                        seed, 0u, d.fitch, d.scratch, d.ax + ss, ss);
+  replay_cta_body<SROW>(GridIdx{loc % gx, loc / gx, gx}, d.N, d.L, d.Lp, d.left, d.right, d.lnodes + v.x, v.y, seed,
+                        0u, d.ns, d.scratch, d.ax + ss, ss);
 }
 
-bool replay_uses_cta(int nn, int nnull) { return (int64_t)2 * nn * nnull <= kReplayCtaItems; }
 int replay_smem_max() {
   static const int lim = [] {
     const int l = replay_smem_limit();
@@ -560,18 +711,18 @@ int replay_smem_max() {
   return lim;
 }
 
-cudaError_t grp_fitch_up(const FamDev* F, int nf, const int2* lv, const int* pre, int nb, uint64_t seed,
-                         cudaStream_t st) {
-  if (nb > 0) k_fitch_up_grp<<<nb, 256, 0, st>>>(F, nf, lv, pre, seed);
-  return cudaGetLastError();
-}
-
-cudaError_t grp_root(const FamDev* F, int nf, const int* pre_state, int nb_state, const int* pre_row, int nb_row,
-                     uint64_t seed, cudaStream_t st) {
-  if (nb_state > 0) k_root_state_grp<<<nb_state, 256, 0, st>>>(F, nf, pre_state, seed);
+cudaError_t grp_fitch(const FamDev* F, int nf, const int* pre_cols, int nb_cols, int maxN, const int* pre_row,
+                      int nb_row, uint64_t seed, cudaStream_t st) {
+  const size_t sm = fitch_smem(maxN);
+  if (nb_cols > 0) {
+    if (sm <= FITCH_SMEM_MAX) k_fitch_cols_grp<true><<<nb_cols, fitch_threads(maxN), sm, st>>>(F, nf, pre_cols, seed);
+    else                      k_fitch_cols_grp<false><<<nb_cols, 512, 0, st>>>(F, nf, pre_cols, seed);
+  }
   if (nb_row > 0) k_root_row_grp<<<nb_row, 256, 0, st>>>(F, nf, pre_row, seed);
   return cudaGetLastError();
 }
+int fitch_blocks(int Lp) { return Lp / (FW * 4); }
+int grp_null_prepare() { return null_attrs() == cudaSuccess ? 1 : 0; }
 
 // srow: every family of the launch has its rows staged in shared memory
 // (maxLp bytes per item)

@@ -33,3 +33,38 @@ def test_statistics_at_tile_edges(covgpu, oracle, N, L, cells):
             assert ok, "%s rel %g small %g" % (t, rel, small)
             assert mm[0, q, 0] == got[iu].min() and mm[0, q, 1] == got[iu].max()
     e.close()
+
+
+@pytest.mark.parametrize("N,L,ns", [(2, 33, 2), (3, 17, 1), (300, 64, 40), (40, 1100, 2), (5600, 33, 1)])
+def test_nulls_on_every_route(covgpu, oracle, N, L, ns):
+    """Null alignments byte for byte on each route: one launch per null
+    cluster (1 CTA, 4 CTAs), a launch per depth (more than 1,024 columns), and
+    the reconstruction of a tree too deep for shared memory; with ambiguity
+    codes and a root of two leaves."""
+    s = covgpu.Synth(N, L, 1.5, 4, 1, 4, 4, 0.15, seed=N + L)
+    rng = np.random.default_rng(N)
+    for code in (5, 15, 17):
+        s.ax[rng.integers(0, N, 4 + N // 50), rng.integers(0, L, 4 + N // 50)] = code
+    e = covgpu.Engine(N, L, maxslots=ns + 1, maxnull=ns)
+    e.set_alignment(0, s.ax)
+    e.set_tree(s.parent, s.left, s.right)
+    e.make_nulls(7, 5, ns, 1)
+    T = oracle.TreeArrays(s.parent, s.left, s.right, s.ld, s.rd)
+    for q in sorted({0, ns // 2, ns - 1}):
+        assert np.array_equal(e.get_alignment(1 + q), oracle.null_msa(s.ax, T, 7, 5 + q)), q
+    e.close()
+
+
+@pytest.mark.parametrize("N,L", [(2, 20), (129, 31), (5600, 33)])
+def test_reconstruction_with_ambiguity_codes(covgpu, oracle, N, L):
+    """Substitutions per column and pair on the Fitch reconstruction, in shared
+    memory and (the deepest tree) in global rows."""
+    s = covgpu.Synth(N, L, 1.5, 4, 1, 4, 4, 0.15, seed=N)
+    s.ax[0, : L // 2] = 15
+    e = covgpu.Engine(N, L)
+    e.set_alignment(0, s.ax)
+    e.set_tree(s.parent, s.left, s.right)
+    T = oracle.TreeArrays(s.parent, s.left, s.right, s.ld, s.rd)
+    for got, ref in zip(e.substitutions(0, seed=9), oracle.substitutions(s.ax, T, 9, 0xFFFFFFFF)):
+        assert np.array_equal(got, ref)
+    e.close()
