@@ -608,7 +608,7 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
     lvl[dd].cta = tb.put(pc.v.data(), pc.v.size() * 4); lvl[dd].ncta = pc.total();
     lvl[dd].warp = tb.put(pw.v.data(), pw.v.size() * 4); lvl[dd].nwarp = pw.total();
   }
-  Pre pcol = prefix(nf, [&](int k) { return fams[k].pb ? (fams[k].L + 255) / 256 : 0; });
+  Pre pcol = prefix(nf, [&](int k) { return fams[k].pb ? pb_blocks(fams[k].L) : 0; });
   Pre prow = prefix(nf, [&](int k) { return fams[k].pb ? fams[k].N : 0; });
   Pre pcod = prefix(nf, [&](int k) { return fams[k].gsc ? fams[k].N : 0; });
   Pre pid = prefix(nf, [&](int k) { const int nt = (fams[k].N + 31) / 32; return fams[k].gsc ? nt * nt : 0; });

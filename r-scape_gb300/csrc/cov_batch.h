@@ -99,6 +99,7 @@ struct UmmaFam {
 // weights (cov_prep.cu)
 cudaError_t grp_weights_pb(const FamDev* F, int nf, const int* pre_col, int nb_col, const int* pre_row, int nb_row,
                            cudaStream_t st);
+int         pb_blocks(int L);   // blocks of a family in pre_col
 cudaError_t grp_weights_gsc(const FamDev* F, int nf, const int* pre_codes, int nb_codes, const int* pre_ident,
                             int nb_ident, const int* pre_upgma, int nb_upgma, int maxN, cudaStream_t st);
 // normalisation and limbs of the device weights (one block per family of pre)

@@ -444,7 +444,6 @@ extern "C" int covgpu_weights_gsc_dev(covgpu_ctx* ctx, int slot, int set, double
   if (e == cudaSuccess) e = cudaMemcpyAsync(wgt, d_w, N * sizeof(double), cudaMemcpyDeviceToHost, ctx->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
   if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
-  if (gsc_error(scratch, ctx->st)) return fail(ctx, 24, "GSC weights: a grid barrier timed out");
   double sum = 0.0;
   for (int s = 0; s < N; s++) sum += wgt[s];
   for (int s = 0; s < N; s++) wgt[s] = (sum > 0.0) ? wgt[s] * (double)N / sum : 1.0;

@@ -1,14 +1,14 @@
 // cov_prep.cu -- alignment preparation on the device: sequence weights and
 // the gap-column filter of an alignment already resident in a context slot.
 //
-//   k_pb_colinv   one thread per column: counts of the canonical residues
-//                 and of the residue types; inv[c][x] = 1/(types * count_x)
+//   k_pb_colinv   per column the counts of the canonical residues and of the
+//                 residue types; inv[c][x] = 1/(types * count_x)
 //   k_pb_rows     one CTA per sequence: w_s = sum_c inv[c][a_sc] over its
 //                 canonical residues (fixed-order block reduction)
 //                 -- position-based weights, Henikoff & Henikoff 1994
 //                 (esl_msaweight_PB, called at src/R-scape.c:1556 for
 //                 nseq > 1000), renormalised to sum to N on the host
-//   k_gapfilter   one thread per column: the weighted fraction of residues
+//   k_gapfilter   per column the weighted fraction of residues
 //                 (ACGU and degenerate codes) among residues and gaps ('-',
 //                 '*'; '~' is skipped) against 1 - gapthresh
 //                 (msamanip_RemoveGapColumns, src/msamanip.c:461-501)
@@ -20,23 +20,19 @@
 //     k_gsc_ident  32 x 32 tiles of sequence pairs: identities counted four
 //                  columns at a time (__vcmpeq4) from shared-memory tiles;
 //                  D = 1 - identities / min(len_a, len_b)
-//     k_gsc_scan   UPGMA step 1: the closest pair of live clusters, ties to
-//                  the first pair in row-major order (a < b), per block
-//     k_gsc_merge  UPGMA step 2 (one CTA): the pair; each side's new branch
-//                  shared among its leaves in proportion to their weights
-//                  (equally while those are 0); size-weighted average
-//                  distances of the merged cluster (FP64 without
-//                  contraction, the operations of the definition)
-//     k_gsc_upgma_grid  all merges in one cooperative launch over the SMs,
-//                  one grid barrier per merge (bounded wait), cached row
-//                  minima, FP64 work spread over every SM
-//     k_gsc_upgma  all merges in one CTA with cached row minima (where a
-//                  cooperative launch is not available); the two kernels
-//                  above for sizes beyond shared memory
+//     k_gsc_upgma  UPGMA, all merges in one launch of one cluster of CTAs:
+//                  the closest pair of live clusters, ties to the first pair
+//                  in row-major order (a < b); each side's new branch shared
+//                  among its leaves in proportion to their weights (equally
+//                  while those are 0); size-weighted average distances of the
+//                  merged cluster (FP64 without contraction, the operations
+//                  of the definition)
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "cov_dev.cuh"
 #include "cov_prep.h"
@@ -44,19 +40,43 @@
 
 namespace covgpu {
 
+// 32 columns by a CTA of 8 words x 32 slices of the sequences: a thread counts
+// its word's four columns in packed bytes, emptied into the columns' counters
+// before they can overflow.  One thread per column and all N rows in turn took
+// 1.5 ms on 64 ragged families (N up to 2,000), 0.1 ms now.
+constexpr int PB_COLS = 32;
+__host__ __device__ __forceinline__ int pb_blocks_of(int L) { return (L + PB_COLS - 1) / PB_COLS; }
 __device__ __forceinline__ void pb_colinv_body(
     const GridIdx g, const uint8_t* __restrict__ ax, int N, int L, int Lp, double* __restrict__ inv) {
-  const int c = g.x * blockDim.x + threadIdx.x;
-  if (c >= L) return;
-  int cnt[4] = {0, 0, 0, 0};
-  for (int s = 0; s < N; s++) {
-    const int x = ax[(int64_t)s * Lp + c];
-    if (x < 4) cnt[x]++;
-  }
-  const int types = (cnt[0] > 0) + (cnt[1] > 0) + (cnt[2] > 0) + (cnt[3] > 0);
+  __shared__ int cnt[PB_COLS][4];
+  const int tid = threadIdx.x, word = tid & 7, slice = tid >> 3, c0 = g.x * PB_COLS;
+  if (tid < PB_COLS * 4) (&cnt[0][0])[tid] = 0;
+  __syncthreads();
+  const uint8_t* col = ax + c0 + 4 * word;   // Lp is a multiple of 32
+  for (int s0 = slice; s0 < N; s0 += 32 * 255) {
+    const int s1 = min(N, s0 + 32 * 255);
+    uint32_t k[4] = {0, 0, 0, 0};
+    for (int s = s0; s < s1; s += 32) {
+      const uint32_t v = *reinterpret_cast<const uint32_t*>(col + (int64_t)s * Lp);
 #pragma unroll
-  for (int x = 0; x < 4; x++)
-    inv[(int64_t)c * 4 + x] = (types > 0 && cnt[x] > 0) ? 1.0 / ((double)types * (double)cnt[x]) : 0.0;
+      for (int x = 0; x < 4; x++) k[x] = __vsub4(k[x], __vcmpeq4(v, 0x01010101u * x));
+    }
+#pragma unroll
+    for (int x = 0; x < 4; x++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        const int n = (k[x] >> (8 * b)) & 0xFF;
+        if (n) atomicAdd(&cnt[4 * word + b][x], n);
+      }
+  }
+  __syncthreads();
+  if (tid < PB_COLS && c0 + tid < L) {
+    const int* n = cnt[tid];
+    const int types = (n[0] > 0) + (n[1] > 0) + (n[2] > 0) + (n[3] > 0);
+#pragma unroll
+    for (int x = 0; x < 4; x++)
+      inv[(int64_t)(c0 + tid) * 4 + x] = (types > 0 && n[x] > 0) ? 1.0 / ((double)types * (double)n[x]) : 0.0;
+  }
 }
 __global__ void __launch_bounds__(256)
 k_pb_colinv(const uint8_t* __restrict__ ax, int N, int L, int Lp, double* __restrict__ inv) {
@@ -88,19 +108,31 @@ k_pb_rows(const uint8_t* __restrict__ ax, int L, int Lp, const double* __restric
   pb_rows_body(native_grid(), ax, L, Lp, inv, w);
 }
 
-__global__ void __launch_bounds__(256)
+// 32 columns by a CTA of 32 slices of the sequences, each summed in order, the
+// slices then in order.  One thread per column and all rows in turn: 286 us at
+// N=900 x L=700, 13 us now.
+__global__ void __launch_bounds__(1024)
 k_gapfilter(const uint8_t* __restrict__ ax, const double* __restrict__ wgt, int N, int L, int Lp, double idthresh,
             int* __restrict__ useme) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= L) return;
+  __shared__ double sr[32][33], st[32][33];
+  const int x0 = threadIdx.x & 31, slice = threadIdx.x >> 5, c = blockIdx.x * 32 + x0;
+  const int per = (N + 31) / 32, s1 = min(N, (slice + 1) * per);
   double r = 0.0, tot = 0.0;
-  for (int s = 0; s < N; s++) {
-    const int x = ax[(int64_t)s * Lp + c];
+#pragma unroll 4
+  for (int s = slice * per; s < s1; s++) {
+    const int x = ax[(int64_t)s * Lp + c];   // columns up to Lp, a multiple of 32, exist
     const double w = wgt ? wgt[s] : 1.0;
     if (x < 4 || (x > 4 && x <= 15)) { r += w; tot += w; }
     else if (x == 4 || x == 16) tot += w;
   }
-  useme[c] = (r > 0.0 && r / tot >= idthresh) ? 1 : 0;
+  sr[slice][x0] = r;
+  st[slice][x0] = tot;
+  __syncthreads();
+  if (slice == 0 && c < L) {
+    r = tot = 0.0;
+    for (int k = 0; k < 32; k++) { r += sr[k][x0]; tot += st[k][x0]; }
+    useme[c] = (r > 0.0 && r / tot >= idthresh) ? 1 : 0;
+  }
 }
 
 __device__ __forceinline__ void gsc_codes_body(
@@ -180,106 +212,6 @@ k_gsc_ident(const uint32_t* __restrict__ ra, const uint32_t* __restrict__ rb, co
   gsc_ident_body(native_grid(), ra, rb, len, N, Lw, D);
 }
 
-struct GscBest { double d; int a, b; };
-
-__device__ __forceinline__ bool gsc_better(double d, int a, int b, double d2, int a2, int b2) {
-  return d < d2 || (d == d2 && (a < a2 || (a == a2 && b < b2)));
-}
-
-// per block: the best live pair (a < b) among rows a = warp id, strided
-__global__ void __launch_bounds__(256)
-k_gsc_scan(const double* __restrict__ D, const int* __restrict__ alive, int N, GscBest* __restrict__ part) {
-  __shared__ GscBest wb[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gw = blockIdx.x * 8 + warp, nw = gridDim.x * 8;
-  double bd = INFINITY;
-  int ba = N, bb = N;
-  for (int a = gw; a < N; a += nw) {
-    if (!alive[a]) continue;
-    for (int b = a + 1 + lane; b < N; b += 32) {
-      if (!alive[b]) continue;
-      const double d = D[(int64_t)a * N + b];
-      if (gsc_better(d, a, b, bd, ba, bb)) { bd = d; ba = a; bb = b; }
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double d2 = __shfl_xor_sync(0xffffffffu, bd, o);
-    const int a2 = __shfl_xor_sync(0xffffffffu, ba, o), b2 = __shfl_xor_sync(0xffffffffu, bb, o);
-    if (gsc_better(d2, a2, b2, bd, ba, bb)) { bd = d2; ba = a2; bb = b2; }
-  }
-  if (lane == 0) wb[warp] = GscBest{bd, ba, bb};
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    GscBest r = wb[0];
-    for (int w = 1; w < 8; w++)
-      if (gsc_better(wb[w].d, wb[w].a, wb[w].b, r.d, r.a, r.b)) r = wb[w];
-    part[blockIdx.x] = r;
-  }
-}
-
-// one CTA of 1024 threads: the merge of the closest pair
-__global__ void __launch_bounds__(1024)
-k_gsc_merge(double* __restrict__ D, int* __restrict__ alive, int* __restrict__ size, double* __restrict__ height,
-            int* __restrict__ cl, double* __restrict__ w, int N, const GscBest* __restrict__ part, int nparts) {
-  __shared__ GscBest best;
-  __shared__ double rtot[2][32];
-  __shared__ int rcnt[2][32];
-  __shared__ double tot[2];
-  __shared__ int cnt[2];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    GscBest r = part[0];
-    for (int i = 1; i < nparts; i++)
-      if (gsc_better(part[i].d, part[i].a, part[i].b, r.d, r.a, r.b)) r = part[i];
-    best = r;
-  }
-  __syncthreads();
-  const int ba = best.a, bb = best.b;
-  if (ba >= N || bb >= N) return;   // one cluster left
-  const double h = best.d / 2.0;
-  // the leaves of each side: their weight sums and counts
-  double ta = 0.0, tb = 0.0;
-  int ca = 0, cb = 0;
-  for (int l = tid; l < N; l += blockDim.x) {
-    if (cl[l] == ba) { ta += w[l]; ca++; }
-    else if (cl[l] == bb) { tb += w[l]; cb++; }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ta += __shfl_xor_sync(0xffffffffu, ta, o); tb += __shfl_xor_sync(0xffffffffu, tb, o);
-    ca += __shfl_xor_sync(0xffffffffu, ca, o); cb += __shfl_xor_sync(0xffffffffu, cb, o);
-  }
-  if (lane == 0) { rtot[0][warp] = ta; rtot[1][warp] = tb; rcnt[0][warp] = ca; rcnt[1][warp] = cb; }
-  __syncthreads();
-  if (tid == 0) {
-    double x = 0.0, y = 0.0;
-    int m = 0, n = 0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) { x += rtot[0][i]; y += rtot[1][i]; m += rcnt[0][i]; n += rcnt[1][i]; }
-    tot[0] = x; tot[1] = y; cnt[0] = m; cnt[1] = n;
-  }
-  __syncthreads();
-  double bla = h - height[ba], blb = h - height[bb];
-  if (bla < 0.0) bla = 0.0;
-  if (blb < 0.0) blb = 0.0;
-  const int sa = size[ba], sb = size[bb];
-  for (int l = tid; l < N; l += blockDim.x) {
-    if (cl[l] == ba) w[l] += (tot[0] > 0.0) ? __ddiv_rn(__dmul_rn(bla, w[l]), tot[0]) : bla / (double)cnt[0];
-    else if (cl[l] == bb) w[l] += (tot[1] > 0.0) ? __ddiv_rn(__dmul_rn(blb, w[l]), tot[1]) : blb / (double)cnt[1];
-  }
-  for (int c = tid; c < N; c += blockDim.x) {
-    if (alive[c] && c != ba && c != bb) {
-      const double d = __ddiv_rn(__dadd_rn(__dmul_rn(D[(int64_t)ba * N + c], (double)sa),
-                                           __dmul_rn(D[(int64_t)bb * N + c], (double)sb)),
-                                 (double)(sa + sb));
-      D[(int64_t)ba * N + c] = d;
-      D[(int64_t)c * N + ba] = d;
-    }
-  }
-  __syncthreads();
-  for (int l = tid; l < N; l += blockDim.x)
-    if (cl[l] == bb) cl[l] = ba;
-  if (tid == 0) { size[ba] = sa + sb; height[ba] = h; alive[bb] = 0; }
-}
-
 // Order key of a distance: distances lie in [0, 1] (or +inf), and for
 // non-negative doubles the IEEE bit patterns order as the values, so the
 // searches compare 64-bit integers (GB300's FP64 pipe is 1/64 of FP32, its
@@ -288,465 +220,479 @@ __device__ __forceinline__ unsigned long long dkey(double d) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(d);
   return (u <= 0x7FF0000000000000ull) ? u : ~0ull;
 }
-struct GscKey { unsigned long long k; int a, b; };
-__device__ __forceinline__ bool key_better(unsigned long long k, int a, int b, unsigned long long k2, int a2,
-                                           int b2) {
-  return k < k2 || (k == k2 && (a < a2 || (a == a2 && b < b2)));
+// x / b correctly rounded from y = 1 / b correctly rounded: a quotient within
+// two ulps and two residual steps with exact FMA residuals (Markstein, IBM J.
+// Res. Dev. 34, 1990: a faithful quotient plus one such step is the correctly
+// rounded one).  Five FP64 operations where the reciprocal is shared by a whole
+// merge, against the general division's several dozen: this part issues two
+// FP64 operations per cycle and SM.  Finite x and b well inside the exponent
+// range.
+__device__ __forceinline__ double div_by(double x, double b, double y) {
+  double q = __dmul_rn(x, y);
+  q = __fma_rn(__fma_rn(-q, b, x), y, q);
+  return __fma_rn(__fma_rn(-q, b, x), y, q);
 }
 
-// all N-1 UPGMA merges in one CTA of 1024 threads.  The clusters' state
-// (liveness, sizes, heights, weight sums, leaf labels, weights) sits in
-// shared memory,
-// the distances in global memory (L2-resident).  Each live row a keeps its
-// closest live column b > a (ties to the smaller b), so the closest pair is
-// the best row minimum in (d, a, b) order -- the same pair as a full scan.
-// A merge of (ba, bb) changes row ba, column ba of the rows above it and
-// kills column bb; only rows whose cached minimum pointed at ba or bb, and
-// row ba, are rescanned (one warp per row).  The weight split and the
-// distance update are the FP64 operations of k_gsc_upgma_grid, and each
-// cluster's weight sum is kept as that kernel keeps it ((ta + bla) + (tb +
-// blb) at a merge), so both kernels give the same weights.
-__device__ __forceinline__ void gsc_upgma_body(double* __restrict__ D, int N, double* __restrict__ w_out) {
+// ------------------------------------------------------------------------
+// UPGMA by one cluster of G CTAs, one cluster barrier per merge.
+// Index i (row, column, leaf) belongs to CTA i % G.  Every CTA keeps a private
+// copy of the clusters' state (size, height, weight sum) and updates it
+// identically; each caches the minima of its own rows (the closest live
+// column b > a, ties to the smaller b, so the best row minimum in (d, a, b)
+// order is the pair a full scan finds) and rescans the ones a merge
+// invalidated (their entries were written by the CTA itself or before the last
+// barrier).  The merged row's new minimum is not rescanned: every CTA offers
+// its best new entry of that row with its next partial, and the reduction
+// after the barrier yields both the row's minimum and the next closest pair.
+// The partials go straight into the other CTAs' shared memory.
+//
+// Each row keeps its two closest columns while they are known: a merge that
+// removes the first leaves the second, and the merged cluster's distance
+// (mostly between the two it replaces) takes its place where it is known to
+// come before every other column, so rows are rescanned about a third as
+// often.  A lane owns NR rows, columns and leaves, all their state in its
+// registers.
+//
+// Bound by the chain of one merge: the barrier with its release of the stores,
+// one round trip to L2 for the two rows (another where a row is rescanned), the
+// reductions and eight dependent FP64 operations.  The first warp carries the
+// merges alone: one block barrier in the chain, and FP64 work is issued once (a
+// warp instruction holds the SM's FP64 pipe for 16 cycles).  The last warp
+// follows it with the branch lengths and the leaves' weights; three more take
+// part in rescans, whose two round trips and compares held up the whole cluster
+// (3.6 ms without them at N=900).
+// N=900, the 899 merges: 2.5 ms; one cooperative launch with a barrier in global
+// memory per merge took 10.0 ms, 128 equal threads per CTA in a cluster 5.7.
+// In a family batch each family has its own cluster: 3.0 ms for 64 ragged
+// families; one CTA per family, whose FP64 pipe did every distance of a merge
+// with general divisions, took 19.5.
+// ------------------------------------------------------------------------
+constexpr int GSC_MAXG = 16;
+struct __align__(16) GscPart { unsigned long long k, ck; unsigned ab, cb; };
+
+// lexicographic minimum over the warp of (key, tag), in every lane
+__device__ __forceinline__ void gsc_warp_min(unsigned long long& k, unsigned& tag) {
+  const unsigned full = 0xffffffffu;
+  const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
+  const unsigned mh = __reduce_min_sync(full, hi);
+  const unsigned ml = __reduce_min_sync(full, hi == mh ? lo : full);
+  tag = __reduce_min_sync(full, (hi == mh && lo == ml) ? tag : full);
+  k = ((unsigned long long)mh << 32) | ml;
+}
+
+constexpr size_t GSC_SMEM_MAX = 216 * 1024;   // beside 7 KB of static arrays
+// the clusters' sizes as doubles, and the weights warp's state (heights, weight
+// sums and sizes, GSC_STATE bytes a sequence), which lies in global memory for
+// alignments too deep to hold both (the weights are off the merges' chain)
+constexpr size_t GSC_STATE = 2 * sizeof(double) + sizeof(int);
+__host__ __device__ __forceinline__ size_t gsc_state_stride(int N) { return (size_t)3 * N; }   // doubles per CTA
+static bool gsc_state_global(int N) { return (size_t)N * (sizeof(double) + GSC_STATE) > GSC_SMEM_MAX; }
+static size_t gsc_cluster_smem(int N) {
+  return (size_t)N * sizeof(double) + (gsc_state_global(N) ? 0 : (size_t)N * GSC_STATE);
+}
+
+// the last warp of a CTA: the leaves' weights.  Per merge each side's new
+// branch is shared among its leaves in proportion to their weights (equally
+// while those are 0); st: heights, weight sums and sizes of the clusters
+template <int NR>
+__device__ __forceinline__ void gsc_weights(int N, double* __restrict__ w_out, int G, int rank, double* st,
+                                            const GscPart (*part)[GSC_MAXG]) {
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu;
+  const int nown = (N - rank + G - 1) / G;
+  double *height = st, *cw = height + N;
+  int* size = reinterpret_cast<int*>(cw + N);
+  for (int s = lane; s < N; s += 32) { height[s] = 0.0; cw[s] = 0.0; size[s] = 1; }
+  int cl[NR];
+  double w[NR];
+#pragma unroll
+  for (int j = 0; j < NR; j++) { cl[j] = rank + (lane + 32 * j) * G; w[j] = 0.0; }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  for (int m = 0; m < N - 1; m++) {
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    unsigned long long k = lane < G ? part[m & 1][lane].k : ~0ull;
+    unsigned ab = lane < G ? part[m & 1][lane].ab : full;
+    gsc_warp_min(k, ab);
+    if (k == ~0ull) break;   // uniform over the cluster, as in the first warp
+    const int ba = (int)(ab >> 16), bb = (int)(ab & 0xFFFFu);
+    const double h = __longlong_as_double((long long)k) / 2.0;
+    const double ta = cw[ba], tb = cw[bb];
+    double bla = h - height[ba], blb = h - height[bb];
+    if (bla < 0.0) bla = 0.0;
+    if (blb < 0.0) blb = 0.0;
+    const int sa = size[ba], sb = size[bb];
+    double rec = lane == 0 ? ta : tb;     // both reciprocals at once
+    rec = rec > 0.0 ? __drcp_rn(rec) : 0.0;
+    const double ra = __shfl_sync(full, rec, 0), rb = __shfl_sync(full, rec, 1);
+#pragma unroll
+    for (int j = 0; j < NR; j++) {
+      if (lane + 32 * j >= nown || (cl[j] != ba && cl[j] != bb)) continue;
+      const bool A = cl[j] == ba;
+      const double t = A ? ta : tb, bl = A ? bla : blb;
+      if (t > 0.0) w[j] += div_by(__dmul_rn(bl, w[j]), t, A ? ra : rb);
+      else         w[j] += bl / (double)(A ? sa : sb);
+      cl[j] = ba;
+    }
+    __syncwarp();
+    if (lane == 0) { height[ba] = h; cw[ba] = (ta + bla) + (tb + blb); size[ba] = sa + sb; }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int j = 0; j < NR; j++)
+    if (lane + 32 * j < nown) w_out[rank + (lane + 32 * j) * G] = w[j];
+}
+
+// Rescans: the CTA's first warp and three helpers take a quarter of the row
+// each.  The two smallest of a lane's columns, then of the warp's, in
+// (key, column) order.
+constexpr int SCAN_WARPS = 4, SCAN_ROWS = 8;
+struct __align__(16) GscTwo { unsigned long long p, q; unsigned pa, qa, pad0, pad1; };
+struct GscScan {
+  int n;                                   // rows to rescan, -1: the merges are over
+  int rows[32 * 32];
+  GscTwo res[2][SCAN_ROWS][SCAN_WARPS];
+};
+__device__ __forceinline__ bool gsc_less(unsigned long long k, unsigned a, unsigned long long k2, unsigned a2) {
+  return k < k2 || (k == k2 && a < a2);
+}
+// the two smallest of two such pairs
+__device__ __forceinline__ GscTwo gsc_merge2(const GscTwo& x, const GscTwo& y) {
+  const bool f = gsc_less(x.p, x.pa, y.p, y.pa);
+  GscTwo r;
+  r.p = f ? x.p : y.p; r.pa = f ? x.pa : y.pa;
+  const unsigned long long a = f ? x.q : y.q, b = f ? y.p : x.p;
+  const unsigned aa = f ? x.qa : y.qa, ba = f ? y.pa : x.pa;
+  const bool g = gsc_less(a, aa, b, ba);
+  r.q = g ? a : b; r.qa = g ? aa : ba;
+  r.pad0 = r.pad1 = 0;
+  return r;
+}
+__device__ __forceinline__ bool gsc_alive(const double* dsz, int s) {
+  return reinterpret_cast<const int*>(dsz + s)[1] != 0;
+}
+// row a's live columns past it by warp k of SCAN_WARPS
+__device__ __forceinline__ GscTwo gsc_scan_part(const double* __restrict__ D, int N, int a, const double* dsz, int k,
+                                                int lane) {
+  const unsigned long long NONE = ~0ull;
+  GscTwo r{NONE, NONE, 0xFFFFu, 0xFFFFu, 0, 0};
+  const double* row = D + (int64_t)a * N;
+  for (int b0 = a + 1 + k * 32 + lane; b0 - lane < N; b0 += 32 * SCAN_WARPS * 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      v[u] = (b0 + 32 * SCAN_WARPS * u < N) ? __ldcg(row + b0 + 32 * SCAN_WARPS * u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int b = b0 + 32 * SCAN_WARPS * u;
+      const unsigned long long d = dkey(v[u]), key = (b < N && gsc_alive(dsz, b)) ? d : NONE;
+      const bool l1 = key < r.p, l2 = key < r.q;   // b ascends: ties keep the smaller first
+      r.q = l1 ? r.p : (l2 ? key : r.q);
+      r.qa = l1 ? r.pa : (l2 ? (unsigned)b : r.qa);
+      r.p = l1 ? key : r.p;
+      r.pa = l1 ? (unsigned)b : r.pa;
+    }
+  }
+  unsigned long long m1 = r.p, m2;
+  unsigned b1 = r.pa, b2;
+  gsc_warp_min(m1, b1);
+  const bool won = r.p == m1 && r.pa == b1;
+  m2 = won ? r.q : r.p;
+  b2 = won ? r.qa : r.pa;
+  gsc_warp_min(m2, b2);
+  return GscTwo{m1, m2, b1, b2, 0, 0};
+}
+__device__ __forceinline__ void gsc_scan_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * SCAN_WARPS) : "memory"); }
+// one round of up to SCAN_ROWS rows by warp k
+__device__ __forceinline__ void gsc_scan_round(const double* D, int N, int G, int rank, const double* dsz, GscScan& sc,
+                                               int base, int k, int lane) {
+  const int n = min(sc.n - base, SCAN_ROWS);
+  for (int i = 0; i < n; i++) {
+    const GscTwo r = gsc_scan_part(D, N, rank + sc.rows[base + i] * G, dsz, k, lane);
+    if (lane == 0) sc.res[(base / SCAN_ROWS) & 1][i][k] = r;
+  }
+}
+
+template <int NR>
+__device__ __forceinline__ void gsc_cluster_body(double* __restrict__ D, int N, double* __restrict__ w_out, int G,
+                                                 int rank, double* state) {
   extern __shared__ __align__(16) unsigned char gsm[];
-  unsigned long long* rkey = reinterpret_cast<unsigned long long*>(gsm);
-  double* height = reinterpret_cast<double*>(rkey + N);
-  double* w = height + N;
-  double* cw = w + N;
-  int* rarg = reinterpret_cast<int*>(cw + N);
-  int* size = rarg + N;
-  int* cl = size + N;
-  int* resc = cl + N;
-  unsigned char* alive = reinterpret_cast<unsigned char*>(resc + N);
-  __shared__ GscKey wb[32];
-  __shared__ GscKey best;
-  __shared__ int nresc;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu;
+  const int nown = (N - rank + G - 1) / G;           // rows/columns/leaves rank, rank + G, ...
+  double* dsz = reinterpret_cast<double*>(gsm);      // cluster sizes, 0: dead
+  __shared__ GscPart part[2][GSC_MAXG];              // every CTA's partial, by the parity of the merge
   const unsigned long long NONE = ~0ull;
-  for (int s = tid; s < N; s += blockDim.x) {
-    alive[s] = 1; size[s] = 1; height[s] = 0.0; cl[s] = s; w[s] = 0.0; cw[s] = 0.0;
+  const unsigned NO = 0xFFFFu, UNK = 0xFFFEu;        // no column; not known
+  __shared__ GscScan sc;
+  const int warp = threadIdx.x >> 5;
+  if (warp == SCAN_WARPS) {   // the weights
+    gsc_weights<NR>(N, w_out, G, rank, state ? state + (size_t)rank * gsc_state_stride(N) : dsz + N, part);
+    return;
   }
-  __syncthreads();
-  // the best live column b > a of row a (warp-wide; 8 loads in flight per
-  // lane, the row comes from L2), into rkey/rarg
-  auto scan_row = [&](int a) {
-    unsigned long long bk = NONE;
-    int bb2 = N;
-    const double* row = D + (int64_t)a * N;
-    for (int b0 = a + 1 + lane; b0 < N; b0 += 32 * 8) {
-      unsigned long long v[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int b = b0 + 32 * u;
-        v[u] = (b < N && alive[b]) ? dkey(row[b]) : NONE;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int b = b0 + 32 * u;
-        if (v[u] < bk || (v[u] == bk && v[u] != NONE && b < bb2)) { bk = v[u]; bb2 = b; }
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, bk, o);
-      const int b2 = __shfl_xor_sync(0xffffffffu, bb2, o);
-      if (k2 < bk || (k2 == bk && b2 < bb2)) { bk = k2; bb2 = b2; }
-    }
-    if (lane == 0) { rkey[a] = bk; rarg[a] = (bk == NONE) ? N : bb2; }
-  };
-  for (int a = warp; a < N; a += nwarps) scan_row(a);
-  __syncthreads();
-  for (int m = 0; m < N - 1; m++) {
-    // the closest pair
-    GscKey r{NONE, N, N};
-    for (int a = tid; a < N; a += blockDim.x)
-      if (alive[a] && rkey[a] != NONE && key_better(rkey[a], a, rarg[a], r.k, r.a, r.b)) r = GscKey{rkey[a], a, rarg[a]};
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, r.k, o);
-      const int a2 = __shfl_xor_sync(0xffffffffu, r.a, o), b2 = __shfl_xor_sync(0xffffffffu, r.b, o);
-      if (key_better(k2, a2, b2, r.k, r.a, r.b)) { r.k = k2; r.a = a2; r.b = b2; }
-    }
-    if (lane == 0) wb[warp] = r;
-    __syncthreads();
-    if (tid == 0) {
-      GscKey q = wb[0];
-      for (int i = 1; i < nwarps; i++)
-        if (key_better(wb[i].k, wb[i].a, wb[i].b, q.k, q.a, q.b)) q = wb[i];
-      best = q;
-      nresc = 0;
-    }
-    __syncthreads();
-    const int ba = best.a, bb = best.b;
-    if (best.k == NONE || ba >= N || bb >= N) break;   // no pair left with a distance
-    const double h = __longlong_as_double((long long)best.k) / 2.0;
-    // the leaves of each side share the side's new branch in proportion to
-    // their weights (equally while the side's weight sum is 0)
-    const double ta = cw[ba], tb = cw[bb];
-    double bla = h - height[ba], blb = h - height[bb];
-    if (bla < 0.0) bla = 0.0;
-    if (blb < 0.0) blb = 0.0;
-    const int sa = size[ba], sb = size[bb];
-    for (int l = tid; l < N; l += blockDim.x) {
-      if (cl[l] == ba) w[l] += (ta > 0.0) ? __ddiv_rn(__dmul_rn(bla, w[l]), ta) : bla / (double)sa;
-      else if (cl[l] == bb) w[l] += (tb > 0.0) ? __ddiv_rn(__dmul_rn(blb, w[l]), tb) : blb / (double)sb;
-    }
-    for (int c = tid; c < N; c += blockDim.x) {
-      if (alive[c] && c != ba && c != bb) {
-        const double d = __ddiv_rn(__dadd_rn(__dmul_rn(D[(int64_t)ba * N + c], (double)sa),
-                                             __dmul_rn(D[(int64_t)bb * N + c], (double)sb)),
-                                   (double)(sa + sb));
-        D[(int64_t)ba * N + c] = d;
-        D[(int64_t)c * N + ba] = d;
-        if (c < ba) {            // column ba of row c changed, column bb dies
-          const unsigned long long kd = dkey(d);
-          if (kd != NONE && (kd < rkey[c] || (kd == rkey[c] && ba < rarg[c]))) { rkey[c] = kd; rarg[c] = ba; }
-          else if (rarg[c] == ba || rarg[c] == bb) resc[atomicAdd(&nresc, 1)] = c;
-        } else if (c < bb && rarg[c] == bb) {
-          resc[atomicAdd(&nresc, 1)] = c;
-        }
-      }
-    }
-    __syncthreads();
-    for (int l = tid; l < N; l += blockDim.x)
-      if (cl[l] == bb) cl[l] = ba;
-    if (tid == 0) {
-      size[ba] = sa + sb; height[ba] = h; cw[ba] = (ta + bla) + (tb + blb); alive[bb] = 0;
-      resc[atomicAdd(&nresc, 1)] = ba;
-    }
-    __syncthreads();
-    for (int k = warp; k < nresc; k += nwarps) scan_row(resc[k]);
-    __syncthreads();
+  if (warp == 0) {            // the first scan takes every row
+    for (int s = lane; s < N; s += 32) dsz[s] = 1.0;
+    for (int r = lane; r < nown; r += 32) sc.rows[r] = r;
+    if (lane == 0) sc.n = nown;
   }
-  for (int s = tid; s < N; s += blockDim.x) w_out[s] = w[s];
-}
-__global__ void __launch_bounds__(1024)
-k_gsc_upgma(double* __restrict__ D, int N, double* __restrict__ w_out) {
-  gsc_upgma_body(D, N, w_out);
-}
-
-// ------------------------------------------------------------------------
-// UPGMA across the grid: one cooperative launch, one grid barrier per merge.
-// Index i (row, column, leaf) belongs to block i % G.  Every block keeps a
-// private copy of the clusters' state (liveness, size, height, weight sum)
-// and updates it identically; each block caches the minima of its own rows
-// and rescans the ones a merge invalidated (their entries were written by the
-// block itself or before the last barrier).  The merged row's new minimum is
-// not rescanned: every block offers its best new entry of that row with its
-// next partial, and the reduction after the barrier yields both the row's
-// minimum and the next closest pair.  FP64 work (the size-weighted distances
-// and the weight split) is spread over every SM.
-// ------------------------------------------------------------------------
-struct __align__(16) GscPart { unsigned long long k; int a, b; unsigned long long ck; int cb, pad; };
-
-__device__ __forceinline__ unsigned gsc_ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint64_t gsc_clock() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-constexpr uint64_t kGscWaitNs = 2000000000ull;   // a grid barrier gives up after 2 s
-
-__global__ void __launch_bounds__(256)
-k_gsc_upgma_grid(double* __restrict__ D, int N, double* __restrict__ w, int* __restrict__ cl,
-                 GscPart* __restrict__ part, unsigned* __restrict__ bar, int* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char gsm2[];
-  const int G = gridDim.x, bid = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = blockDim.x >> 5;
-  const int nown = (N - bid + G - 1) / G;           // rows/columns/leaves bid, bid + G, ...
-  double* height = reinterpret_cast<double*>(gsm2);
-  double* cw = height + N;
-  unsigned long long* rkey = reinterpret_cast<unsigned long long*>(cw + N);   // own rows
-  int* size = reinterpret_cast<int*>(rkey + nown);
-  int* rarg = size + N;                              // own rows
-  int* resc = rarg + nown;                           // own rows to rescan
-  unsigned char* alive = reinterpret_cast<unsigned char*>(resc + nown);
-  __shared__ GscPart wpart[8];
-  __shared__ unsigned long long sk[2];
-  __shared__ int si[4];
-  __shared__ int nresc, ok;
-  const unsigned long long NONE = ~0ull;
-  for (int s = tid; s < N; s += blockDim.x) { alive[s] = 1; size[s] = 1; height[s] = 0.0; cw[s] = 0.0; }
-  for (int r = tid; r < nown; r += blockDim.x) { const int l = bid + r * G; cl[l] = l; w[l] = 0.0; }
-  __syncthreads();
-  // the best live column b > a of row a, warp-wide
-  auto scan_row = [&](int a, int r) {
-    unsigned long long bk = NONE;
-    int bb2 = N;
-    const double* row = D + (int64_t)a * N;
-    for (int b0 = a + 1 + lane; b0 < N; b0 += 32 * 8) {
-      unsigned long long v[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int b = b0 + 32 * u;
-        v[u] = (b < N && alive[b]) ? dkey(__ldcg(row + b)) : NONE;
+  gsc_scan_sync();
+  if (warp > 0) {             // the scan helpers
+    for (int m = -1; m < N - 1; m++) {
+      if (m >= 0) {
+        asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        gsc_scan_sync();      // the rows to rescan
       }
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int b = b0 + 32 * u;
-        if (v[u] < bk || (v[u] == bk && v[u] != NONE && b < bb2)) { bk = v[u]; bb2 = b; }
+      const int n = sc.n;
+      if (n < 0) break;
+      for (int base = 0; base < n; base += SCAN_ROWS) {
+        gsc_scan_round(D, N, G, rank, dsz, sc, base, warp, lane);
+        gsc_scan_sync();
+      }
+      if (m < 0) {
+        asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, bk, o);
-      const int b2 = __shfl_xor_sync(0xffffffffu, bb2, o);
-      if (k2 < bk || (k2 == bk && b2 < bb2)) { bk = k2; bb2 = b2; }
+    return;
+  }
+  // own rows: the closest column (k1, a1), the second (k2, a2) or a2 = UNK
+  unsigned long long k1[NR], k2[NR];
+  unsigned a1[NR], a2[NR];
+  bool own[NR];                                      // live rows of this lane
+#pragma unroll
+  for (int j = 0; j < NR; j++) {
+    own[j] = lane + 32 * j < nown;
+    k1[j] = k2[j] = NONE;
+    a1[j] = a2[j] = NO;
+  }
+  // the scan of the n rows in sc.rows (helpers released already), into the
+  // rows' lanes
+  auto scan_rows = [&](int n) {
+    for (int base = 0; base < n; base += SCAN_ROWS) {
+      gsc_scan_round(D, N, G, rank, dsz, sc, base, 0, lane);
+      gsc_scan_sync();
+      // lane 4 i + k: warp k's part of row i
+      GscTwo r = sc.res[(base / SCAN_ROWS) & 1][lane >> 2][lane & 3];
+#pragma unroll
+      for (int o = 1; o < SCAN_WARPS; o <<= 1) {
+        GscTwo y;
+        y.p = __shfl_xor_sync(full, r.p, o); y.q = __shfl_xor_sync(full, r.q, o);
+        y.pa = __shfl_xor_sync(full, r.pa, o); y.qa = __shfl_xor_sync(full, r.qa, o);
+        r = gsc_merge2(r, y);
+      }
+      const int cnt = min(n - base, SCAN_ROWS);
+      for (int i = 0; i < cnt; i++) {
+        const unsigned long long p = __shfl_sync(full, r.p, 4 * i), q2 = __shfl_sync(full, r.q, 4 * i);
+        const unsigned pa = __shfl_sync(full, r.pa, 4 * i), qa = __shfl_sync(full, r.qa, 4 * i);
+        const int row = sc.rows[base + i];
+#pragma unroll
+        for (int j = 0; j < NR; j++)
+          if (lane + 32 * j == row) {
+            k1[j] = p; a1[j] = p == NONE ? NO : pa;
+            k2[j] = q2; a2[j] = q2 == NONE ? NO : qa;
+          }
+      }
     }
-    if (lane == 0) { rkey[r] = bk; rarg[r] = (bk == NONE) ? N : bb2; }
   };
-  for (int r = warp; r < nown; r += nwarps) scan_row(bid + r * G, r);
-  __syncthreads();
-  int prev = -1;                          // merged row whose minimum comes from the partials
-  unsigned long long ck = NONE;           // this block's best new entry of row prev
-  int cb = N;
+  scan_rows(nown);
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");   // every CTA has started: its shared memory
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");     // can be written
+  int prev = -1;                          // the last merge's row
+  unsigned long long ck = NONE;           // this lane's best new entry of row prev
+  unsigned cb = NO;
   for (int m = 0; m < N - 1; m++) {
-    // phase 1: the best cached minimum over own live rows (row prev excluded)
-    GscPart q{NONE, N, N, ck, cb, 0};
-    for (int r = tid; r < nown; r += blockDim.x) {
-      const int a = bid + r * G;
-      if (a != prev && alive[a] && rkey[r] != NONE && key_better(rkey[r], a, rarg[r], q.k, q.a, q.b)) {
-        q.k = rkey[r]; q.a = a; q.b = rarg[r];
-      }
+    // the best cached minimum over own live rows, row prev's by the new entries
+    unsigned long long qk = ck;
+    unsigned qab = ((unsigned)prev << 16) | cb;
+#pragma unroll
+    for (int j = 0; j < NR; j++) {
+      const int a = rank + (lane + 32 * j) * G;
+      const unsigned ab = ((unsigned)a << 16) | a1[j];
+      if (own[j] && a != prev && (k1[j] < qk || (k1[j] == qk && qk != NONE && ab < qab))) { qk = k1[j]; qab = ab; }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, q.k, o);
-      const int a2 = __shfl_xor_sync(0xffffffffu, q.a, o), b2 = __shfl_xor_sync(0xffffffffu, q.b, o);
-      if (key_better(k2, a2, b2, q.k, q.a, q.b)) { q.k = k2; q.a = a2; q.b = b2; }
+    gsc_warp_min(qk, qab);
+    gsc_warp_min(ck, cb);
+    if (lane < G) {   // into CTA `lane`'s copy
+      uint32_t dst;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
+                   : "r"((uint32_t)__cvta_generic_to_shared(&part[m & 1][rank])), "r"(lane));
+      asm volatile("st.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(dst), "l"(qk), "l"(ck) : "memory");
+      asm volatile("st.shared::cluster.v2.u32 [%0 + 16], {%1, %2};" ::"r"(dst), "r"(qab), "r"(cb) : "memory");
     }
-    if (lane == 0) wpart[warp] = q;
-    __syncthreads();
-    GscPart* pp = part + (size_t)(m & 1) * G;
-    if (tid == 0) {
-      GscPart r0 = wpart[0];
-      for (int i = 1; i < nwarps; i++)
-        if (key_better(wpart[i].k, wpart[i].a, wpart[i].b, r0.k, r0.a, r0.b)) {
-          r0.k = wpart[i].k; r0.a = wpart[i].a; r0.b = wpart[i].b;
-        }
-      r0.ck = ck; r0.cb = cb;
-      pp[bid] = r0;
-      __threadfence();
-      atomicAdd(bar, 1u);
-      const unsigned target = (unsigned)(m + 1) * (unsigned)G;
-      uint64_t t0 = 0;
-      int good = 1;
-      while (gsc_ld_acquire(bar) < target) {
-        const uint64_t now = gsc_clock();
-        if (t0 == 0) t0 = now;
-        else if (now - t0 > kGscWaitNs) { good = 0; break; }
-      }
-      ok = good;
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    GscPart q = lane < G ? part[m & 1][lane] : GscPart{NONE, NONE, full, NO};
+    gsc_warp_min(q.k, q.ab);
+    if (q.k == NONE) {         // uniform over the cluster: no pair left
+      if (lane == 0) sc.n = -1;
+      gsc_scan_sync();
+      break;
     }
-    __syncthreads();
-    if (!ok) { if (tid == 0) atomicExch(err, 1); return; }
-    // phase 2: every block reduces all partials in block order
-    if (warp == 0) {
-      unsigned long long bk = NONE, pk = NONE;
-      int ba = N, bb = N, pb = N;
-      for (int i = lane; i < G; i += 32) {   // written by other SMs: read past L1, 32 bytes in two loads
-        const int4 x = __ldcg(reinterpret_cast<const int4*>(pp + i));
-        const int4 y = __ldcg(reinterpret_cast<const int4*>(pp + i) + 1);
-        const unsigned long long vk = ((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x;
-        const unsigned long long vck = ((unsigned long long)(unsigned)y.y << 32) | (unsigned)y.x;
-        const int va = x.z, vb = x.w, vcb = y.z;
-        if (key_better(vk, va, vb, bk, ba, bb)) { bk = vk; ba = va; bb = vb; }
-        if (vck < pk || (vck == pk && vck != NONE && vcb < pb)) { pk = vck; pb = vcb; }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, bk, o);
-        const int a2 = __shfl_xor_sync(0xffffffffu, ba, o), b2 = __shfl_xor_sync(0xffffffffu, bb, o);
-        if (key_better(k2, a2, b2, bk, ba, bb)) { bk = k2; ba = a2; bb = b2; }
-        const unsigned long long p2 = __shfl_xor_sync(0xffffffffu, pk, o);
-        const int c2 = __shfl_xor_sync(0xffffffffu, pb, o);
-        if (p2 < pk || (p2 == pk && c2 < pb)) { pk = p2; pb = c2; }
-      }
-      if (lane == 0) {
-        if (prev >= 0 && pk != NONE && key_better(pk, prev, pb, bk, ba, bb)) { bk = pk; ba = prev; bb = pb; }
-        sk[0] = bk; sk[1] = pk; si[0] = ba; si[1] = bb; si[2] = pb;
-      }
+    const int ba = (int)(q.ab >> 16), bb = (int)(q.ab & 0xFFFFu);
+    // the rows of the pair at own columns
+    double x[NR], y[NR];
+#pragma unroll
+    for (int j = 0; j < NR; j++) {
+      const int c = rank + (lane + 32 * j) * G;
+      x[j] = own[j] ? __ldcg(D + (int64_t)ba * N + c) : 0.0;
+      y[j] = own[j] ? __ldcg(D + (int64_t)bb * N + c) : 0.0;
     }
-    __syncthreads();
-    if (prev >= 0 && prev % G == bid && tid == 0) {
+    if (prev >= 0 && prev % G == rank) {   // row prev's minimum, for its owner
+      gsc_warp_min(q.ck, q.cb);
       const int r = prev / G;
-      rkey[r] = sk[1]; rarg[r] = (sk[1] == NONE) ? N : si[2];
+#pragma unroll
+      for (int j = 0; j < NR; j++)
+        if (lane + 32 * j == r) { k1[j] = q.ck; a1[j] = q.ck == NONE ? NO : q.cb; a2[j] = UNK; }
     }
-    const unsigned long long bk = sk[0];
-    const int ba = si[0], bb = si[1];
-    if (bk == NONE || ba >= N || bb >= N) break;   // uniform: no pair left
-    const double h = __longlong_as_double((long long)bk) / 2.0;
-    const int sa = size[ba], sb = size[bb];
-    const double ta = cw[ba], tb = cw[bb];
-    double bla = h - height[ba], blb = h - height[bb];
-    if (bla < 0.0) bla = 0.0;
-    if (blb < 0.0) blb = 0.0;
-    if (tid == 0) nresc = 0;
-    __syncthreads();
-    // own leaves: the branch shares, then the new label
-    for (int r = tid; r < nown; r += blockDim.x) {
-      const int l = bid + r * G;
-      const int c = cl[l];
-      if (c == ba) {
-        w[l] += (ta > 0.0) ? __ddiv_rn(__dmul_rn(bla, w[l]), ta) : bla / (double)sa;
-      } else if (c == bb) {
-        w[l] += (tb > 0.0) ? __ddiv_rn(__dmul_rn(blb, w[l]), tb) : blb / (double)sb;
-        cl[l] = ba;
+    const double sa = dsz[ba], sb = dsz[bb], n = sa + sb, rn = __drcp_rn(n);
+    // own columns: the merged cluster's distances, the two closest of own
+    // rows, and this lane's best new entry of row ba
+    ck = NONE; cb = NO;
+    unsigned lost = 0u;
+#pragma unroll
+    for (int j = 0; j < NR; j++)   // the lane's chains together; 0 for columns it does not own
+      x[j] = div_by(__dadd_rn(__dmul_rn(x[j], sa), __dmul_rn(y[j], sb)), n, rn);
+#pragma unroll
+    for (int j = 0; j < NR; j++) {
+      const int c = rank + (lane + 32 * j) * G;
+      if (c == bb) own[j] = false;
+      if (own[j] && c != ba) {
+        __stcg(D + (int64_t)ba * N + c, x[j]);
+        __stcg(D + (int64_t)c * N + ba, x[j]);
       }
     }
-    // own columns: the merged cluster's distances, the cached minima of own
-    // rows, and this block's best new entry of row ba
-    unsigned long long myk = NONE;
-    int myb = N;
-    for (int r = tid; r < nown; r += blockDim.x) {
-      const int c = bid + r * G;
-      if (!alive[c] || c == ba || c == bb) continue;
-      const double d = __ddiv_rn(__dadd_rn(__dmul_rn(__ldcg(D + (int64_t)ba * N + c), (double)sa),
-                                           __dmul_rn(__ldcg(D + (int64_t)bb * N + c), (double)sb)),
-                                 (double)(sa + sb));
-      D[(int64_t)ba * N + c] = d;
-      D[(int64_t)c * N + ba] = d;
-      const unsigned long long kd = dkey(d);
-      if (c > ba) {
-        if (kd < myk || (kd == myk && kd != NONE && c < myb)) { myk = kd; myb = c; }
-      } else {            // row c, column ba changed, column bb dies
-        if (kd != NONE && (kd < rkey[r] || (kd == rkey[r] && ba < rarg[r]))) { rkey[r] = kd; rarg[r] = ba; }
-        else if (rarg[r] == ba || rarg[r] == bb) resc[atomicAdd(&nresc, 1)] = r;
+#pragma unroll
+    for (int j = 0; j < NR; j++) {
+      const int c = rank + (lane + 32 * j) * G;
+      if (!own[j] || c == ba) continue;
+      const unsigned long long kd = dkey(x[j]);
+      if (c > ba && kd < ck) { ck = kd; cb = (unsigned)c; }
+      if (c > bb || k1[j] == NONE) continue;          // the row holds neither column
+      const bool low = c < ba;                        // column ba changes as well as bb going
+      const bool rem1 = a1[j] == (unsigned)bb || (low && a1[j] == (unsigned)ba);
+      const bool known2 = a2[j] != UNK;
+      const bool rem2 = a2[j] == (unsigned)bb || (low && a2[j] == (unsigned)ba);
+      // every column not listed comes after (kb, ab)
+      const unsigned long long kb = known2 ? k2[j] : k1[j];
+      const unsigned ab = known2 ? a2[j] : a1[j];
+      if (rem1) {
+        if (known2 && !rem2) { k1[j] = k2[j]; a1[j] = a2[j]; }
+        else a1[j] = UNK;
+        a2[j] = UNK;
+      } else if (rem2) {
+        a2[j] = UNK;
       }
-      if (c > ba && c < bb && rarg[r] == bb) resc[atomicAdd(&nresc, 1)] = r;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, myk, o);
-      const int b2 = __shfl_xor_sync(0xffffffffu, myb, o);
-      if (k2 < myk || (k2 == myk && b2 < myb)) { myk = k2; myb = b2; }
-    }
-    if (lane == 0) { wpart[warp].ck = myk; wpart[warp].cb = myb; }
-    __syncthreads();
-    // the private cluster state, identical in every block
-    if (tid == 0) {
-      size[ba] = sa + sb; height[ba] = h; cw[ba] = (ta + bla) + (tb + blb); alive[bb] = 0;
-      ck = NONE; cb = N;
-      for (int i = 0; i < nwarps; i++)
-        if (wpart[i].ck < ck || (wpart[i].ck == ck && wpart[i].ck != NONE && wpart[i].cb < cb)) {
-          ck = wpart[i].ck; cb = wpart[i].cb;
+      if (low && (kd < kb || (kd == kb && (unsigned)ba < ab) || ab == NO)) {   // in its place among the listed
+        if (a1[j] == UNK) { k1[j] = kd; a1[j] = (unsigned)ba; }
+        else if (kd < k1[j] || (kd == k1[j] && (unsigned)ba < a1[j])) {
+          k2[j] = k1[j]; a2[j] = a1[j]; k1[j] = kd; a1[j] = (unsigned)ba;
+        } else if (a2[j] == UNK || kd < k2[j] || (kd == k2[j] && (unsigned)ba < a2[j])) {
+          k2[j] = kd; a2[j] = (unsigned)ba;
         }
-      si[3] = cb; sk[1] = ck;
+      }
+      if (a1[j] == UNK) lost |= 1u << j;
     }
-    __syncthreads();
-    ck = sk[1]; cb = si[3];
-    // rescans of own rows whose minimum was lost (their entries are this
-    // block's own writes or older than the last barrier)
-    for (int k = warp; k < nresc; k += nwarps) { const int r = resc[k]; scan_row(bid + r * G, r); }
+    __syncwarp();
+    if (lane == 0) { dsz[ba] = n; dsz[bb] = 0.0; }
+    __syncwarp();
+    // rescans of own rows whose minimum was lost (their entries are this CTA's
+    // own writes or older than the last barrier)
+    int nl = 0;
+#pragma unroll
+    for (int j = 0; j < NR; j++) {
+      const unsigned lm = __ballot_sync(full, (lost >> j) & 1u);
+      if ((lost >> j) & 1u) sc.rows[nl + __popc(lm & ((1u << lane) - 1u))] = lane + 32 * j;
+      nl += __popc(lm);
+    }
+    if (lane == 0) sc.n = nl;
+    gsc_scan_sync();
+    scan_rows(nl);
     prev = ba;
-    __syncthreads();
   }
 }
 
-static size_t gsc_grid_smem(int N, int G) {
-  const int nown = (N + G - 1) / G;
-  return (size_t)N * (2 * sizeof(double) + sizeof(int) + 1) + (size_t)nown * (sizeof(unsigned long long) +
-         2 * sizeof(int)) + 16;
+template <int NR>
+__global__ void __launch_bounds__(32 * (SCAN_WARPS + 1))
+k_gsc_upgma(double* __restrict__ D, int N, double* __restrict__ w, int G, double* state) {
+  gsc_cluster_body<NR>(D, N, w, G, blockIdx.x % G, state);
 }
 
-// shared memory of k_gsc_upgma for N sequences
-static size_t gsc_upgma_smem(int N) { return (size_t)N * (4 * sizeof(double) + 4 * sizeof(int) + 1) + 16; }
-
-__global__ void k_gsc_init(int N, int* __restrict__ alive, int* __restrict__ size, double* __restrict__ height,
-                           int* __restrict__ cl, double* __restrict__ w) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < N; s += gridDim.x * blockDim.x) {
-    alive[s] = 1; size[s] = 1; height[s] = 0.0; cl[s] = s; w[s] = 0.0;
-  }
+// CTAs of the merges' cluster (N <= 16384)
+static int gsc_cluster(int N) { return N <= 256 ? 8 : 16; }
+// rows per lane: the smallest kernel that holds N
+template <class F>
+static cudaError_t gsc_with_nr(int N, int G, F f) {
+  const int nr = (N + 32 * G - 1) / (32 * G);
+  if (nr <= 1) return f(std::integral_constant<int, 1>());
+  if (nr <= 2) return f(std::integral_constant<int, 2>());
+  if (nr <= 4) return f(std::integral_constant<int, 4>());
+  if (nr <= 16) return f(std::integral_constant<int, 16>());
+  if (nr <= 32) return f(std::integral_constant<int, 32>());
+  return cudaErrorInvalidValue;
 }
 
-constexpr int kGscMaxGrid = 256;
-constexpr size_t kGscHead = 16 + 2 * kGscMaxGrid * sizeof(GscPart);   // barrier, error flag, partials
+template <class... A>
+static cudaError_t gsc_cluster_launch(const void* k, int grid, int G, size_t sm, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(32 * (SCAN_WARPS + 1));
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = st;
+  cudaLaunchAttribute la[1];
+  la[0].id = cudaLaunchAttributeClusterDimension;
+  la[0].val.clusterDim.x = G;
+  la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+  cfg.attrs = la;
+  cfg.numAttrs = 1;
+  void* args[] = {(void*)&a...};
+  return cudaLaunchKernelExC(&cfg, k, args);
+}
+
+// the merge kernels' limits (shared memory, clusters of 16) on the current
+// device, raised once (before any stream capture)
+static cudaError_t gsc_attrs();
 
 size_t gsc_scratch_bytes(int N, int L) {
   const size_t Lw = ((size_t)L + 3) / 4;
-  return kGscHead + (size_t)N * N * sizeof(double) + 2 * (size_t)N * Lw * sizeof(uint32_t) +
-         (size_t)N * (4 * sizeof(int) + 2 * sizeof(double)) + 64 * sizeof(GscBest) + 256;
+  return (size_t)N * N * sizeof(double) + 2 * (size_t)N * Lw * sizeof(uint32_t) + (size_t)N * sizeof(int) + 512 +
+         (gsc_state_global(N) ? GSC_MAXG * gsc_state_stride(N) * sizeof(double) : 0);
 }
 
 cudaError_t launch_weights_gsc(const uint8_t* ax, int N, int L, int Lp, void* scratch, double* w, cudaStream_t st) {
   const int Lw = (L + 3) / 4;
   uint8_t* p = (uint8_t*)scratch;
-  unsigned* bar = (unsigned*)p;
-  int* err = (int*)(p + 4);
-  GscPart* gpart = (GscPart*)(p + 16);
-  p += kGscHead;
   double* D = (double*)p;                 p += (size_t)N * N * sizeof(double);
-  double* height = (double*)p;            p += (size_t)N * sizeof(double);
+  double* state = nullptr;
+  if (gsc_state_global(N)) { state = (double*)p; p += GSC_MAXG * gsc_state_stride(N) * sizeof(double); }
   uint32_t* ra = (uint32_t*)p;            p += (size_t)N * Lw * sizeof(uint32_t);
   uint32_t* rb = (uint32_t*)p;            p += (size_t)N * Lw * sizeof(uint32_t);
-  int* len = (int*)p;                     p += (size_t)N * sizeof(int);
-  int* alive = (int*)p;                   p += (size_t)N * sizeof(int);
-  int* size = (int*)p;                    p += (size_t)N * sizeof(int);
-  int* cl = (int*)p;                      p += (size_t)N * sizeof(int);
-  p = (uint8_t*)(((uintptr_t)p + 15) & ~(uintptr_t)15);
-  GscBest* part = (GscBest*)p;
-  cudaError_t e = cudaMemsetAsync(scratch, 0, 16, st);
+  int* len = (int*)p;
+  if (N < 2) return cudaErrorInvalidValue;
+  const cudaError_t e = gsc_attrs();
   if (e != cudaSuccess) return e;
   k_gsc_codes<<<N, 256, 0, st>>>(ax, N, L, Lp, Lw, ra, rb, len);
   const int nt = (N + 31) / 32;
   k_gsc_ident<<<dim3(nt, nt), 256, 0, st>>>(ra, rb, len, N, Lw, D);
-  // all merges in one cooperative launch over the SMs (FP64 work spread out)
-  int dev = 0, nsm = 1, coop = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  // about 64 rows per block: the FP64 work of a merge stays small per SM and
-  // the barrier and the reduction of the partials stay short
-  const int G = std::max(1, std::min(std::min(nsm, 32), (N + 63) / 64));
-  const size_t smg = gsc_grid_smem(N, G);
-  // the launch limit of both merge kernels is raised once, to the 200 KB
-  // that either may take: a limit set per call to that call's size would
-  // race with other host threads' calls for other N (a launch above the
-  // limit another thread just set fails with an invalid argument)
-  static const cudaError_t attr = [] {
-    cudaError_t r = cudaFuncSetAttribute(k_gsc_upgma_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (r == cudaSuccess) r = cudaFuncSetAttribute(k_gsc_upgma, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return r;
-  }();
-  if (attr != cudaSuccess) return attr;
-  if (coop && N >= 2 && smg <= 200 * 1024) {
-    int occ = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_gsc_upgma_grid, 256, smg)) != cudaSuccess) return e;
-    if (occ >= 1 && G <= occ * nsm) {
-      int n = N;
-      void* args[] = {(void*)&D, (void*)&n, (void*)&w, (void*)&cl, (void*)&gpart, (void*)&bar, (void*)&err};
-      return cudaLaunchCooperativeKernel((const void*)k_gsc_upgma_grid, dim3(G), dim3(256), args, smg, st);
-    }
-  }
-  // one CTA while the cluster state fits in its shared memory
-  const size_t sm = gsc_upgma_smem(N);
-  if (sm <= 200 * 1024) {
-    k_gsc_upgma<<<1, 1024, sm, st>>>(D, N, w);
-    return cudaGetLastError();
-  }
-  k_gsc_init<<<(N + 255) / 256, 256, 0, st>>>(N, alive, size, height, cl, w);
-  const int Gs = std::min(48, std::max(1, (N + 7) / 8));
-  for (int m = 0; m < N - 1; m++) {
-    k_gsc_scan<<<Gs, 256, 0, st>>>(D, alive, N, part);
-    k_gsc_merge<<<1, 1024, 0, st>>>(D, alive, size, height, cl, w, N, part, Gs);
-  }
-  return cudaGetLastError();
-}
-
-int gsc_error(const void* scratch, cudaStream_t st) {
-  int err = 0;
-  if (cudaMemcpyAsync(&err, (const uint8_t*)scratch + 4, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return 90;
-  return err;
+  // all merges in one launch of one cluster
+  const int G = gsc_cluster(N);
+  return gsc_with_nr(N, G, [&](auto nr) {
+    return gsc_cluster_launch((const void*)k_gsc_upgma<decltype(nr)::value>, G, G, gsc_cluster_smem(N), st, D, N, w, G,
+                              state);
+  });
 }
 
 cudaError_t launch_weights_pb(const uint8_t* ax, int N, int L, int Lp, double* inv, double* w, cudaStream_t st) {
-  k_pb_colinv<<<(L + 255) / 256, 256, 0, st>>>(ax, N, L, Lp, inv);
+  k_pb_colinv<<<pb_blocks_of(L), 256, 0, st>>>(ax, N, L, Lp, inv);
   k_pb_rows<<<N, 256, 0, st>>>(ax, L, Lp, inv, w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gapfilter(const uint8_t* ax, const double* wgt, int N, int L, int Lp, double gapthresh, int* useme,
                              cudaStream_t st) {
-  k_gapfilter<<<(L + 255) / 256, 256, 0, st>>>(ax, wgt, N, L, Lp, 1.0 - gapthresh, useme);
+  k_gapfilter<<<(L + 31) / 32, 1024, 0, st>>>(ax, wgt, N, L, Lp, 1.0 - gapthresh, useme);
   return cudaGetLastError();
 }
 
@@ -759,7 +705,7 @@ __global__ void __launch_bounds__(256)
 k_pb_colinv_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre) {
   const int f = grp_find(pre, nf, (int)blockIdx.x);
   const FamDev& d = F[f];
-  pb_colinv_body(GridIdx{(int)blockIdx.x - __ldg(pre + f), 0, (d.L + 255) / 256}, d.ax, d.N, d.L, d.Lp, d.pbinv);
+  pb_colinv_body(GridIdx{(int)blockIdx.x - __ldg(pre + f), 0, pb_blocks_of(d.L)}, d.ax, d.N, d.L, d.Lp, d.pbinv);
 }
 
 __global__ void __launch_bounds__(256)
@@ -784,12 +730,35 @@ k_gsc_ident_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pr
   gsc_ident_body(GridIdx{loc % nt, loc / nt, nt}, d.gra, d.grb, d.glen, d.N, d.Lw, d.gD);
 }
 
-__global__ void __launch_bounds__(1024)
-k_gsc_upgma_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre) {
-  const int f = grp_find(pre, nf, (int)blockIdx.x);
+template <int NR>
+__global__ void __launch_bounds__(32 * (SCAN_WARPS + 1))
+k_gsc_upgma_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre, int G) {
+  const int f = grp_find(pre, nf, (int)blockIdx.x / G);
   const FamDev& d = F[f];
-  gsc_upgma_body(d.gD, d.N, d.w);
+  gsc_cluster_body<NR>(d.gD, d.N, d.w, G, (int)blockIdx.x % G, nullptr);
 }
+
+static cudaError_t gsc_attrs() {
+  constexpr int MAXDEV = 64;
+  static std::atomic<int> done[MAXDEV];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < MAXDEV && done[dev].load()) return cudaSuccess;
+  const void* k[] = {(const void*)k_gsc_upgma<1>, (const void*)k_gsc_upgma<2>, (const void*)k_gsc_upgma<4>,
+                     (const void*)k_gsc_upgma<16>, (const void*)k_gsc_upgma<32>, (const void*)k_gsc_upgma_grp<1>, (const void*)k_gsc_upgma_grp<2>,
+                     (const void*)k_gsc_upgma_grp<4>, (const void*)k_gsc_upgma_grp<16>,
+                     (const void*)k_gsc_upgma_grp<32>};
+  for (const void* f : k) {
+    if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GSC_SMEM_MAX)) != cudaSuccess)
+      return e;
+    if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+  }
+  if (dev < MAXDEV) done[dev].store(1);
+  return cudaSuccess;
+}
+
+int pb_blocks(int L) { return pb_blocks_of(L); }
 
 cudaError_t grp_weights_pb(const FamDev* F, int nf, const int* pre_col, int nb_col, const int* pre_row, int nb_row,
                            cudaStream_t st) {
@@ -802,12 +771,14 @@ cudaError_t grp_weights_pb(const FamDev* F, int nf, const int* pre_col, int nb_c
 cudaError_t grp_weights_gsc(const FamDev* F, int nf, const int* pre_codes, int nb_codes, const int* pre_ident,
                             int nb_ident, const int* pre_upgma, int nb_upgma, int maxN, cudaStream_t st) {
   if (nb_upgma <= 0) return cudaSuccess;
-  const size_t sm = gsc_upgma_smem(maxN);
-  if (sm > 200 * 1024 || !grp_weights_gsc_prepare()) return cudaErrorInvalidValue;
+  const int G = gsc_cluster(maxN);
+  if (gsc_state_global(maxN) || !grp_weights_gsc_prepare()) return cudaErrorInvalidValue;
   if (nb_codes > 0) k_gsc_codes_grp<<<nb_codes, 256, 0, st>>>(F, nf, pre_codes);
   if (nb_ident > 0) k_gsc_ident_grp<<<nb_ident, 256, 0, st>>>(F, nf, pre_ident);
-  k_gsc_upgma_grp<<<nb_upgma, 1024, sm, st>>>(F, nf, pre_upgma);
-  return cudaGetLastError();
+  return gsc_with_nr(maxN, G, [&](auto nr) {
+    return gsc_cluster_launch((const void*)k_gsc_upgma_grp<decltype(nr)::value>, nb_upgma * G, G,
+                              gsc_cluster_smem(maxN), st, F, nf, pre_upgma, G);
+  });
 }
 
 // the device weights of each family of pre (one block each), made as the
@@ -893,13 +864,7 @@ cudaError_t grp_weights_limbs(FamDev* F, int nf, const int* pre, int nb, UmmaFam
   return cudaGetLastError();
 }
 
-// the merges' shared-memory limit, raised once, outside any stream capture
-int grp_weights_gsc_prepare() {
-  static const int ok = [] {
-    return cudaFuncSetAttribute(k_gsc_upgma_grp, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
-                   cudaSuccess ? 1 : 0;
-  }();
-  return ok;
-}
+// the merges' limits, raised outside any stream capture
+int grp_weights_gsc_prepare() { return gsc_attrs() == cudaSuccess ? 1 : 0; }
 
 }  // namespace covgpu

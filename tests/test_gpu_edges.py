@@ -68,3 +68,35 @@ def test_reconstruction_with_ambiguity_codes(covgpu, oracle, N, L):
     for got, ref in zip(e.substitutions(0, seed=9), oracle.substitutions(s.ax, T, 9, 0xFFFFFFFF)):
         assert np.array_equal(got, ref)
     e.close()
+
+
+@pytest.mark.parametrize("N,L", [(7, 20), (256, 40), (257, 40), (513, 60), (1025, 24)])
+def test_gsc_weights_at_cluster_edges(covgpu, oracle, N, L):
+    """GSC weights around the sizes where the merges' cluster (8 or 16 CTAs) and
+    the rows per lane change, with many equal distances (short, duplicated
+    rows), against the oracle."""
+    s = covgpu.Synth(N, L, 0.6, 2, 1, 1, 2, 0.1, seed=N, tree_kind=1)
+    rng = np.random.default_rng(N)
+    for k in range(N // 4):
+        i, j = rng.integers(0, N, size=2)
+        s.ax[j] = s.ax[i]
+    e = covgpu.Engine(N, L)
+    e.set_alignment(0, s.ax)
+    g = e.weights_gsc(0, set=False)
+    e.close()
+    assert np.allclose(g, oracle.weights_gsc(s.ax), rtol=1e-10, atol=1e-13)
+
+
+@pytest.mark.parametrize("N,L", [(3, 31), (31, 33), (9000, 40)])
+def test_position_weights_and_gap_filter_by_slices(covgpu, oracle, N, L):
+    """Column counts in packed bytes (emptied every 255 rows of a slice) and
+    the gap filter's sums by slices of the sequences."""
+    s = covgpu.Synth(N, L, 1.0, 2, 1, 1, 2, 0.3, seed=N)
+    e = covgpu.Engine(N, L)
+    e.set_alignment(0, s.ax)
+    w = e.weights_pb(0, set=False)
+    assert np.allclose(w, oracle.weights_pb(s.ax), rtol=1e-12, atol=1e-15)
+    for thr in (0.5, 0.7, 0.75):
+        for wgt in (None, w):
+            assert np.array_equal(e.gapfilter(0, wgt, thr), oracle.gapfilter(s.ax, wgt, thr) == 1)
+    e.close()
