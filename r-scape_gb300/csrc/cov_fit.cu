@@ -23,17 +23,47 @@
 
 namespace covgpu {
 
+// x / b for positive x and b within FP32's range: FP32's reciprocal, two
+// Newton steps, and two residual corrections of the quotient (Newton-Raphson
+// reciprocal and Markstein's correction, IBM J. Res. Dev. 34, 1990), equal to
+// the IEEE quotient; without a branch, so several run side by side
+__device__ __forceinline__ double div_pos(double x, double b) {
+  double r = (double)__frcp_rn((float)b);
+  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+  double q = __dmul_rn(x, r);
+  q = __fma_rn(__fma_rn(-q, b, x), r, q);
+  return __fma_rn(__fma_rn(-q, b, x), r, q);
+}
+
 // regularised upper incomplete gamma Q(a, x): series for x < a + 1, Lentz's
-// continued fraction otherwise (Abramowitz & Stegun 6.5.29, 6.5.31)
-__device__ double gamma_q_dev(double a, double x, double lga) {
-  if (x <= 0.0) return 1.0;
+// continued fraction otherwise (Abramowitz & Stegun 6.5.29, 6.5.31), as the
+// part that is summed and the prefactor
+//   Q = 1 - sum pre  (x < a + 1),  Q = pre h  (else),  pre = x^a e^-x / Gamma(a)
+__device__ double gamma_q_sum(double a, double x) {
   if (x < a + 1.0) {
     double sum = 1.0 / a, del = sum, ap = a;
-    for (int n = 0; n < 10000; n++) {
-      ap += 1.0; del *= x / ap; sum += del;
-      if (fabs(del) < fabs(sum) * 1e-16) break;
+    // four quotients at a time: they do not depend on the terms, which do on
+    // one another (a dependent FP64 operation takes ~64 cycles here, a
+    // division ~800)
+    if (!(x < 1e30 && a < 1e30)) {   // outside div_pos's range
+      for (int n = 0; n < 10000; n++) {
+        ap += 1.0; del *= x / ap; sum += del;
+        if (fabs(del) < fabs(sum) * 1e-16) break;
+      }
+      return sum;
     }
-    return 1.0 - sum * exp(-x + a * log(x) - lga);
+    for (int n = 0; n < 10000; n += 4) {
+      double q[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) { ap += 1.0; q[k] = div_pos(x, ap); }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        del = __dmul_rn(del, q[k]); sum = __dadd_rn(sum, del);
+        if (fabs(del) < fabs(sum) * 1e-16) return sum;
+      }
+    }
+    return sum;
   }
   double b = x + 1.0 - a, c = 1.0 / 1e-300, d = 1.0 / b, h = d;
   for (int i = 1; i < 10000; i++) {
@@ -46,7 +76,15 @@ __device__ double gamma_q_dev(double a, double x, double lga) {
     h *= del;
     if (fabs(del - 1.0) < 1e-16) break;
   }
-  return exp(-x + a * log(x) - lga) * h;
+  return h;
+}
+__device__ __forceinline__ double gamma_q_pre(double a, double x, double lga) { return exp(-x + a * log(x) - lga); }
+__device__ __forceinline__ double gamma_q_join(double a, double x, double sum, double pre) {
+  return x < a + 1.0 ? __fma_rn(-sum, pre, 1.0) : __dmul_rn(pre, sum);
+}
+__device__ double gamma_q_dev(double a, double x, double lga) {
+  if (x <= 0.0) return 1.0;
+  return gamma_q_join(a, x, gamma_q_sum(a, x), gamma_q_pre(a, x, lga));
 }
 
 struct FitPoint { double lambda, tau, lga, lconst; };   // lconst = tau log lambda - lgamma(tau)
@@ -62,24 +100,37 @@ struct FitPoint { double lambda, tau, lga, lconst; };   // lconst = tau log lamb
 // of Q(lo) - Q(hi); closer to mu the difference of Q is used.
 __constant__ double c_inv[64];   // c_inv[k] = 1 / (k + 1)
 
-__device__ double gam_logp_bin(double lo, double h, double mu, double logx, const FitPoint& P) {
-  const double x = lo - mu;
-  if (x > 0.0 && h <= 0.0625 * x && P.lambda * h <= 0.5) {
-    const double r = h / x, s = P.lambda * h;
-    double dkm1 = 0.0, dk = 1.0, sum = 1.0;
-    for (int k = 0; k < 60; k++) {
-      const double dk1 = (((P.tau - 1.0 - k) * r - s) * dk - s * r * dkm1) * c_inv[k];
-      const double term = dk1 * c_inv[k + 1];
-      sum += term;
-      dkm1 = dk; dk = dk1;
-      if (fabs(term) <= 1e-17 * fabs(sum)) break;
-    }
-    return P.lconst + (P.tau - 1.0) * logx - P.lambda * x + log(h * sum);
+__device__ __forceinline__ bool gam_bin_far(double x, double h, const FitPoint& P) {
+  return x > 0.0 && h <= 0.0625 * x && P.lambda * h <= 0.5;
+}
+__device__ __forceinline__ double gam_logp_far(double x, double h, double logx, const FitPoint& P) {
+  const double r = h / x, s = P.lambda * h;
+  double dkm1 = 0.0, dk = 1.0, sum = 1.0;
+  for (int k = 0; k < 60; k++) {
+    const double dk1 = (((P.tau - 1.0 - k) * r - s) * dk - s * r * dkm1) * c_inv[k];
+    const double term = dk1 * c_inv[k + 1];
+    sum += term;
+    dkm1 = dk; dk = dk1;
+    if (fabs(term) <= 1e-17 * fabs(sum)) break;
   }
-  const double l = (lo < mu) ? mu : lo, hi = lo + h;
-  const double slo = (l <= mu) ? 1.0 : gamma_q_dev(P.tau, P.lambda * (l - mu), P.lga);
-  const double shi = (hi <= mu) ? 1.0 : gamma_q_dev(P.tau, P.lambda * (hi - mu), P.lga);
-  const double p = slo - shi;
+  return P.lconst + (P.tau - 1.0) * logx - P.lambda * x + log(h * sum);
+}
+// a bin near mu in four independent parts: k & 1 the prefactor or the sum of
+// Q, k >> 1 at the bin's lower or upper bound; then the four joined
+__device__ __forceinline__ double gam_near_part(int k, double lo, double h, double mu, const FitPoint& P) {
+  const double l = (k & 2) ? lo + h : ((lo < mu) ? mu : lo);
+  if (l <= mu) return 0.0;
+  const double x = P.lambda * (l - mu);
+  if (x <= 0.0) return 0.0;
+  return (k & 1) ? gamma_q_pre(P.tau, x, P.lga) : gamma_q_sum(P.tau, x);
+}
+__device__ __forceinline__ double gam_near_q(double l, double mu, const FitPoint& P, double sum, double pre) {
+  if (l <= mu) return 1.0;
+  const double x = P.lambda * (l - mu);
+  return x <= 0.0 ? 1.0 : gamma_q_join(P.tau, x, sum, pre);
+}
+__device__ __forceinline__ double gam_near_join(double lo, double h, double mu, const FitPoint& P, const double (&r)[4]) {
+  const double p = gam_near_q((lo < mu) ? mu : lo, mu, P, r[0], r[1]) - gam_near_q(lo + h, mu, P, r[2], r[3]);
   return log(p > 0.0 ? p : 1e-300);
 }
 
@@ -111,44 +162,106 @@ struct FitGrid {
   FitOut* out;
 };
 
-// evaluates the npts points in pts (shared) over the tail.  The work items
-// (point q, bin k), point-major, are spread over all threads of the grid:
-// FP64 throughput is per SM, so the grid is sized to use every SM's FP64
-// unit before it stacks warps on one.  Each block sums its items per point,
-// arrives at the grid barrier, then adds all block sums in block order into
-// F (shared).  False when the barrier timed out.
-__device__ bool fit_eval(const FitGrid& g, const FitPoint* pts, int npts, unsigned& phase, double* F, double* red,
-                         int* flag, int G, int bid) {
-  const int T = G * blockDim.x, nw = blockDim.x >> 5;
-  const int nitems = npts * g.nnz;
+constexpr int kFitNear = 192;   // bins near mu whose parts a block shares out
+constexpr int kFitOwn = 8;      // of which one thread owns at most these
+
+struct FitShared {
+  FitPoint pts[kFitMaxPts];
+  double F[kFitMaxPts], red[8 * kFitMaxPts], pc[kFitMaxPts][2], tmp[16];
+  int flag, ctl, nnear;
+  int near_it[kFitNear];
+  double near_r[4][kFitNear];
+};
+
+// evaluates the npts points in sh.pts over the tail.  The work items (point q,
+// bin k), point-major, are spread over the first `own` threads of each block
+// of the grid: FP64 throughput is per SM, so the grid is sized to use every
+// SM's FP64 unit before it stacks warps on one.  Each block sums its items
+// per point, arrives at the grid barrier, then adds all block sums in block
+// order into sh.F.  False when the barrier timed out.
+//
+// A bin near mu takes two incomplete gammas, each a series of divisions and a
+// prefactor: ~48,000 cycles one after the other, and the whole search waits
+// for them in every round.  The block's warps share their four parts out (one
+// part to a warp, so no warp diverges), the quotients of a series come four at
+// a time and the point sums are folded side by side: a search of three tails
+// of a 30 x 61 family (200 nulls) takes 156 us, 209 us with a thread's parts one
+// after the other.
+//
+// The list's size: the bins within 17 widths of mu make up to 102 items in a
+// round; more only when lambda w > 0.5, and those past the list are computed
+// where they are.
+__device__ bool fit_eval(const FitGrid& g, FitShared& sh, int npts, unsigned& phase, int own, int G, int bid) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int T = G * own, nw = own >> 5, ngrp = blockDim.x >> 7;   // the block is a multiple of 128 threads
+  const int nitems = npts * g.nnz, first = bid * own + tid;
   double* part = g.part + (size_t)(phase & 1u) * kFitMaxPts * G;
+  if (tid == 0) sh.nnear = 0;
+  __syncthreads();
+  int slot[kFitOwn], nslot = 0;
+  if (tid < own) {
+    for (int it = first; it < nitems; it += T) {
+      const int q = it / g.nnz, b = g.bins[it - q * g.nnz];
+      const double lo = g.w * b + g.bmin, hi = g.w * (b + 1) + g.bmin;
+      if (gam_bin_far(lo - g.mu, hi - lo, sh.pts[q]) || nslot == kFitOwn) continue;
+      const int s = atomicAdd(&sh.nnear, 1);
+      slot[nslot++] = s;
+      if (s < kFitNear) sh.near_it[s] = it;
+    }
+  }
+  __syncthreads();
+  const int nnear = min(sh.nnear, kFitNear);
+  for (int e = (warp >> 2) * 32 + lane; e < nnear; e += 32 * ngrp) {
+    const int it = sh.near_it[e], q = it / g.nnz, b = g.bins[it - q * g.nnz];
+    const double lo = g.w * b + g.bmin, hi = g.w * (b + 1) + g.bmin;
+    sh.near_r[warp & 3][e] = gam_near_part(warp & 3, lo, hi - lo, g.mu, sh.pts[q]);
+  }
+  __syncthreads();
   double acc[kFitMaxPts];
 #pragma unroll
   for (int q = 0; q < kFitMaxPts; q++) acc[q] = 0.0;
-  for (int it = bid * blockDim.x + threadIdx.x; it < nitems; it += T) {
-    const int q = it / g.nnz, k = it - q * g.nnz;
-    const int b = g.bins[k];
-    const double lo = g.w * b + g.bmin, hi = g.w * (b + 1) + g.bmin;
-    const double v = g.cnts[k] * gam_logp_bin(lo, hi - lo, g.mu, g.logx[k], pts[q]);
+  if (tid < own) {
+    int ns = 0;
+    for (int it = first; it < nitems; it += T) {
+      const int q = it / g.nnz, k = it - q * g.nnz;
+      const int b = g.bins[k];
+      const double lo = g.w * b + g.bmin, hi = g.w * (b + 1) + g.bmin, h = hi - lo;
+      double lp;
+      if (gam_bin_far(lo - g.mu, h, sh.pts[q])) {
+        lp = gam_logp_far(lo - g.mu, h, g.logx[k], sh.pts[q]);
+      } else {
+        double r[4];
+        const int s = ns < nslot ? slot[ns] : kFitNear;
+        ns++;
+        if (s < kFitNear) {
 #pragma unroll
-    for (int r = 0; r < kFitMaxPts; r++)
-      if (q == r) acc[r] -= v;
-  }
-  const int warp = threadIdx.x >> 5;
+          for (int j = 0; j < 4; j++) r[j] = sh.near_r[j][s];
+        } else {   // no room in the block's list
+#pragma unroll 1
+          for (int j = 0; j < 4; j++) r[j] = gam_near_part(j, lo, h, g.mu, sh.pts[q]);
+        }
+        lp = gam_near_join(lo, h, g.mu, sh.pts[q], r);
+      }
+      const double v = g.cnts[k] * lp;
 #pragma unroll
-  for (int q = 0; q < kFitMaxPts; q++) {
-    double a = acc[q];
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if ((threadIdx.x & 31) == 0) red[warp * kFitMaxPts + q] = a;
+      for (int r = 0; r < kFitMaxPts; r++)
+        if (q == r) acc[r] -= v;
+    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < kFitMaxPts; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < kFitMaxPts; q++) sh.red[warp * kFitMaxPts + q] = acc[q];
   }
   __syncthreads();
-  if (threadIdx.x < npts) {
+  if (tid < npts) {
     double t = 0.0;
-    for (int i = 0; i < nw; i++) t += red[i * kFitMaxPts + threadIdx.x];
-    part[threadIdx.x * G + bid] = t;
+    for (int i = 0; i < nw; i++) t += sh.red[i * kFitMaxPts + tid];
+    part[tid * G + bid] = t;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     __threadfence();
     atomicAdd(g.bar, 1u);
     const unsigned target = (phase + 1u) * (unsigned)G;
@@ -159,35 +272,49 @@ __device__ bool fit_eval(const FitGrid& g, const FitPoint* pts, int npts, unsign
       if (t0 == 0) t0 = now;
       else if (now - t0 > kFitWaitNs) { ok = 0; break; }
     }
-    *flag = ok;
+    sh.flag = ok;
   }
   __syncthreads();
-  if (!*flag) return false;
-  if (threadIdx.x < 32) {
-    for (int q = 0; q < npts; q++) {
-      double t = 0.0;
-      for (int i = threadIdx.x; i < G; i += 32) t += __ldcg(part + q * G + i);
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (threadIdx.x == 0) F[q] = t;
-    }
+  if (!sh.flag) return false;
+  if (tid < 32) {
+    double t[kFitMaxPts];   // the points' sums side by side
+#pragma unroll
+    for (int q = 0; q < kFitMaxPts; q++) t[q] = 0.0;
+    for (int i = tid; i < G; i += 32)
+#pragma unroll
+      for (int q = 0; q < kFitMaxPts; q++) t[q] += q < npts ? __ldcg(part + q * G + i) : 0.0;
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < kFitMaxPts; q++) t[q] += __shfl_xor_sync(0xffffffffu, t[q], o);
+    if (tid == 0)
+#pragma unroll
+      for (int q = 0; q < kFitMaxPts; q++)
+        if (q < npts) sh.F[q] = t[q];
   }
   __syncthreads();
   phase++;
   return true;
 }
 
-__device__ void fit_set_point(FitPoint* P, double l0, double l1) {
-  P->lambda = exp(l0);
-  P->tau = exp(l1);
-  P->lga = lgamma(P->tau);
-  P->lconst = P->tau * log(P->lambda) - P->lga;
-}
-
-// thread 0 has written the n simplex coordinates pc; lanes 0..n-1 turn them
-// into likelihood points in parallel
-__device__ __forceinline__ void fit_set_points(FitPoint* pts, const double (*pc)[2], int n) {
+// thread 0 has written the n simplex coordinates sh.pc; they become likelihood
+// points, the rate's and the shape's parts in two warps
+__device__ __forceinline__ void fit_set_points(FitShared& sh, int n) {
   __syncthreads();
-  if ((int)threadIdx.x < n) fit_set_point(&pts[threadIdx.x], pc[threadIdx.x][0], pc[threadIdx.x][1]);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane < n && warp == 0) {
+    const double tau = exp(sh.pc[lane][1]);
+    sh.pts[lane].tau = tau;
+    sh.pts[lane].lga = lgamma(tau);
+  } else if (lane < n && warp == 1) {
+    const double lambda = exp(sh.pc[lane][0]);
+    sh.pts[lane].lambda = lambda;
+    sh.tmp[lane] = log(lambda);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < n) {
+    FitPoint& P = sh.pts[threadIdx.x];
+    P.lconst = P.tau * sh.tmp[threadIdx.x] - P.lga;
+  }
   __syncthreads();
 }
 
@@ -202,10 +329,12 @@ __device__ __forceinline__ void fit_set_points(FitPoint* pts, const double (*pc)
 // visits, to 1e-12 in F and 1e-9 in theta.
 // (G, bid): the blocks of the search and this block's index; a grouped
 // launch runs one search per block (G = 1)
-__device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, double s01, int G, int bid) {
-  __shared__ FitPoint pts[kFitMaxPts];
-  __shared__ double F[kFitMaxPts], red[8 * kFitMaxPts], pc[kFitMaxPts][2];
-  __shared__ int flag, ctl;
+// own: the threads of a block that own items (the others help)
+__device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, double s01, int own, int G, int bid) {
+  __shared__ FitShared sh;
+  double (&F)[kFitMaxPts] = sh.F;
+  double (&pc)[kFitMaxPts][2] = sh.pc;
+  int &flag = sh.flag, &ctl = sh.ctl;
   {
     const int T = G * blockDim.x;
     for (int k = bid * blockDim.x + threadIdx.x; k < g.nnz; k += T) {
@@ -217,7 +346,7 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
   // no points publishes them grid-wide
   unsigned phase = 0;
   int evals = 0, status = 0;
-  if (!fit_eval(g, pts, 0, phase, F, red, &flag, G, bid)) status = 2;
+  if (!fit_eval(g, sh, 0, phase, own, G, bid)) status = 2;
 
   // ---- phase 1: Newton ----
   // Steps below kNewtonTol in (log lambda, log tau) end the search: the
@@ -238,9 +367,30 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
       pc[4][0] = th0;     pc[4][1] = th1 - H;
       pc[5][0] = th0 + H; pc[5][1] = th1 + H;
     }
-    fit_set_points(pts, pc, 6);
-    if (!fit_eval(g, pts, 6, phase, F, red, &flag, G, bid)) { status = 2; break; }
+    fit_set_points(sh, 6);
+    if (!fit_eval(g, sh, 6, phase, own, G, bid)) { status = 2; break; }
     evals += 6;
+    if (threadIdx.x < 32) {   // the five difference quotients, a lane each
+      const int k = threadIdx.x;
+      double num, den = H * H;
+      if (k == 0)      { num = F[1] - F[2]; den = 2.0 * H; }
+      else if (k == 1) { num = F[3] - F[4]; den = 2.0 * H; }
+      else if (k == 2) num = F[1] - 2.0 * F[0] + F[2];
+      else if (k == 3) num = F[3] - 2.0 * F[0] + F[4];
+      else             num = F[5] - F[1] - F[3] + F[0];
+      const double qt = num / den;
+      if (k < 5) sh.tmp[k] = qt;
+      __syncwarp();
+      // -H^-1 g, a lane per component
+      const double h00 = sh.tmp[2], h11 = sh.tmp[3], h01 = sh.tmp[4];
+      const double det = h00 * h11 - h01 * h01;
+      const double ga = sh.tmp[k == 0 ? 0 : 1], gb = sh.tmp[k == 0 ? 1 : 0], hh = k == 0 ? h11 : h00;
+      const double nd = -(hh * ga - h01 * gb);
+      const double dd = nd / det;
+      if (k < 2) sh.tmp[5 + k] = dd;
+      if (k == 0) sh.tmp[7] = det;
+      __syncwarp();
+    }
     if (threadIdx.x == 0) {
       ctl = 1;
       const double F0 = F[0];
@@ -251,13 +401,10 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
         if (fabs(d0) < kNewtonTol && fabs(d1) < kNewtonTol) { th0 = bth0; th1 = bth1; converged = 1; ctl = 0; }
       } else {
         bth0 = th0; bth1 = th1; bF = F0;
-        const double g0 = (F[1] - F[2]) / (2.0 * H), g1 = (F[3] - F[4]) / (2.0 * H);
-        const double h00 = (F[1] - 2.0 * F0 + F[2]) / (H * H), h11 = (F[3] - 2.0 * F0 + F[4]) / (H * H);
-        const double h01 = (F[5] - F[1] - F[3] + F0) / (H * H);
-        const double det = h00 * h11 - h01 * h01;
+        const double g0 = sh.tmp[0], g1 = sh.tmp[1], h00 = sh.tmp[2], h11 = sh.tmp[3], det = sh.tmp[7];
         if (h00 > 0.0 && h11 > 0.0 && det > 0.0) {
-          d0 = -(h11 * g0 - h01 * g1) / det;
-          d1 = -(h00 * g1 - h01 * g0) / det;
+          d0 = sh.tmp[5];
+          d1 = sh.tmp[6];
         } else {
           const double sc = fmax(fmax(fabs(h00), fabs(h11)), 1.0);
           d0 = -g0 / sc; d1 = -g1 / sc;
@@ -287,8 +434,8 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
   const bool need_nm = !flag;
   __syncthreads();
   if (need_nm && !status) {
-    fit_set_points(pts, pc, 3);
-    if (!fit_eval(g, pts, 3, phase, F, red, &flag, G, bid)) status = 2;
+    fit_set_points(sh, 3);
+    if (!fit_eval(g, sh, 3, phase, own, G, bid)) status = 2;
     evals += 3;
     if (threadIdx.x == 0) for (int k = 0; k < 3; k++) SF[k] = F[k];
     for (int it = 0; it < 4000 && !status; it++) {
@@ -311,8 +458,8 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
       }
       __syncthreads();
       if (!ctl) break;
-      fit_set_points(pts, pc, 3);
-      if (!fit_eval(g, pts, 3, phase, F, red, &flag, G, bid)) { status = 2; break; }
+      fit_set_points(sh, 3);
+      if (!fit_eval(g, sh, 3, phase, own, G, bid)) { status = 2; break; }
       evals += 3;
       if (threadIdx.x == 0) {
         const double fr = F[0];
@@ -337,8 +484,8 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
       }
       __syncthreads();
       if (ctl == 2) {
-        fit_set_points(pts, pc, 2);
-        if (!fit_eval(g, pts, 2, phase, F, red, &flag, G, bid)) { status = 2; break; }
+        fit_set_points(sh, 2);
+        if (!fit_eval(g, sh, 2, phase, own, G, bid)) { status = 2; break; }
         evals += 2;
         if (threadIdx.x == 0) {
           int nq = 0;
@@ -364,8 +511,8 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
 }
 
 __global__ void __launch_bounds__(256)
-k_gam_fit(FitGrid g, double s00, double s01) {
-  gam_fit_body(g, s00, s01, (int)gridDim.x, (int)blockIdx.x);
+k_gam_fit(FitGrid g, double s00, double s01, int own) {
+  gam_fit_body(g, s00, s01, own, (int)gridDim.x, (int)blockIdx.x);
 }
 
 // one search per block: fit e of the batch's fits
@@ -373,7 +520,7 @@ __global__ void __launch_bounds__(256)
 k_gam_fit_grp(const FitGrid* __restrict__ gs, const double2* __restrict__ start) {
   const FitGrid g = gs[blockIdx.x];
   const double2 s0 = start[blockIdx.x];
-  gam_fit_body(g, s0.x, s0.y, 1, 0);
+  gam_fit_body(g, s0.x, s0.y, 256, 1, 0);
 }
 
 struct FitWork {
@@ -422,7 +569,13 @@ __global__ void k_survfit(int cmin, int nb, double bmin, double w, double mass, 
 cudaError_t launch_survfit(int cmin, int nb, double bmin, double w, double mass, int doexp, double mu, double lambda,
                            double tau, double* d_sf, cudaStream_t st) {
   const int n = 2 * nb;
-  k_survfit<<<std::max(1, std::min(1024, (n + 255) / 256)), 256, 0, st>>>(cmin, nb, bmin, w, mass, doexp, mu, lambda,
+  // FP64 throughput is per SM: one warp per block until every SM has one (a
+  // table of ~3,000 bins in 12 blocks of 256 took 73-95 us)
+  int dev = 0, nsm = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int thr = 32 * std::max(1, std::min(8, (n + 32 * nsm - 1) / (32 * nsm)));
+  k_survfit<<<std::max(1, std::min(1024, (n + thr - 1) / thr)), thr, 0, st>>>(cmin, nb, bmin, w, mass, doexp, mu, lambda,
                                                                           tau, doexp ? 0.0 : std::lgamma(tau), d_sf);
   return cudaGetLastError();
 }
@@ -498,12 +651,16 @@ int gamma_fit_launch(FitWork* fwp, const uint64_t* h_obs, int cmin, int imax, do
   g.bins = fw.d_bins; g.cnts = fw.d_cnts; g.logx = fw.d_logx; g.nnz = nnz;
   g.bmin = bmin; g.w = w; g.mu = mu;
   g.part = fw.d_part; g.bar = fw.d_bar; g.out = fw.d_out;
-  void* args[] = {&g, &s00, &s01};
+  int own = 0;
+  void* args[] = {&g, &s00, &s01, &own};
   // one warp per SM until every SM has one, then up to 8 warps per block
   const int nitems = kFitMaxPts * nnz;
   const int W = std::max(1, std::min(8, (nitems + 32 * fw.max_grid - 1) / (32 * fw.max_grid)));
   const int G = std::max(1, std::min(fw.max_grid, (nitems + 32 * W - 1) / (32 * W)));
-  if (cudaLaunchCooperativeKernel((const void*)k_gam_fit, dim3(G), dim3(32 * W), args, 0, st) != cudaSuccess)
+  own = 32 * W;
+  // at least four warps, a multiple of four, for the parts of the bins near mu
+  if (cudaLaunchCooperativeKernel((const void*)k_gam_fit, dim3(G), dim3((own + 127) / 128 * 128), args, 0, st) !=
+      cudaSuccess)
     return 90;
   if (cudaMemcpyAsync(fw.h_out, fw.d_out, sizeof(FitOut), cudaMemcpyDeviceToHost, st) != cudaSuccess) return 90;
   return 0;

@@ -100,3 +100,43 @@ def test_position_weights_and_gap_filter_by_slices(covgpu, oracle, N, L):
         for wgt in (None, w):
             assert np.array_equal(e.gapfilter(0, wgt, thr), oracle.gapfilter(s.ax, wgt, thr) == 1)
     e.close()
+
+
+@pytest.mark.parametrize("N,L,ns,pmass,w0,want", [
+    # ~300 bins: one warp per block, 17 bins near mu at each of six points
+    (8, 40, 1, 0.05, 0.05, [(0.830686218287233, 0.5717117980558083), (10.803158200648957, 0.2815148742465867)]),
+    # coarse bins, half of the histogram in the tail
+    (8, 40, 1, 0.5, 0.5, [(1.822823517103002, 0.7979367241135228), (16.611265927604805, 0.8372782766560288)]),
+    # ~10^4 bins: more than one item per thread, every SM in the grid
+    (60, 100, 8, 0.3, 0.001, [(0.1162342608351604, 0.9960794172969336), (7.804012852676134, 1.2917766699223328)]),
+    # a tail of a few dozen bins, a third or more of them near mu
+    (60, 100, 8, 0.0005, 0.05, [(0.3792700169111325, 0.8599124467420373), (36.04358169921398, 1.492509473769629)]),
+])
+def test_tail_fit_at_list_edges(covgpu, oracle, N, L, ns, pmass, w0, want):
+    """The tail fit on the grid and on one block (in a batch): the histogram of
+    the oracle; lambda and tau of the serial evaluation of the same search (a
+    thread per bin, its incomplete gammas one after the other), which only the
+    order of operations could change (1e-9); both forms within 1e-6 of one
+    another (the search's convergence)."""
+    s = covgpu.Synth(N, L, 1.5, 8, 1, 8, 14, 0.08, seed=5)
+    w = np.ones(N)
+    kw = dict(pmass=pmass, w0=w0, nshuffle=ns, thresh=10.0)
+    T = oracle.TreeArrays(s.parent, s.left, s.right, s.ld, s.rd)
+    e = covgpu.Engine(N, L, maxslots=ns + 1, maxnull=ns)
+    e.set_tree(s.parent, s.left, s.right)
+    types = ["GTp", "MI"]
+    one = e.rscape(s.ax, w, types, counter=covgpu.TENSOR, **kw)
+    e.close()
+    b = covgpu.Batch()
+    fam = dict(ax=s.ax, parent=s.parent, left=s.left, right=s.right, wgt=w)
+    grp = b.rscape([fam, fam], types, counter=covgpu.TENSOR, **kw)
+    b.close()
+    for q, t in enumerate(types):
+        ref = oracle.rscape(s.ax, w, T, covtype=t, **kw)
+        lam, tau = want[q]
+        assert abs(one[q]["lambda_"] - lam) <= 1e-9 * lam, (t, one[q]["lambda_"], lam)
+        assert abs(one[q]["tau"] - tau) <= 1e-9 * tau, (t, one[q]["tau"], tau)
+        for g in (one[q], grp[0][q], grp[1][q]):
+            for k in ("h_nb", "h_imin", "h_imax", "h_cmin", "h_n", "h_Nc", "h_No"):
+                assert g[k] == ref[k], (t, k)
+            assert abs(g["lambda_"] - lam) <= 1e-6 * lam
