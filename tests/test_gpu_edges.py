@@ -140,3 +140,21 @@ def test_tail_fit_at_list_edges(covgpu, oracle, N, L, ns, pmass, w0, want):
             for k in ("h_nb", "h_imin", "h_imax", "h_cmin", "h_n", "h_Nc", "h_No"):
                 assert g[k] == ref[k], (t, k)
             assert abs(g["lambda_"] - lam) <= 1e-6 * lam
+
+
+@pytest.mark.parametrize("N,L", [(9, 40), (8, 64), (2, 65), (33, 97)])
+@pytest.mark.parametrize("rate,mean", [(0.3, 3.0), (1.0, 1.0), (0.02, 400.0), (1e-12, 2.0)])
+def test_simulated_gap_runs_by_words(covgpu, oracle, N, L, rate, mean):
+    """Rows that end inside, at and after a word of 32 columns; every column
+    open, runs across many words, hardly any: the oracle's alignment."""
+    s = covgpu.Synth(N, L, 1.5, max(1, L // 6), 1, 1, L // 6, 0.0, seed=3)
+    e = covgpu.Engine(N, L, maxslots=3, maxnull=0)
+    e.set_tree(s.parent, s.left, s.right)
+    Q4, pi4, Q16, pi16 = covgpu.synth_model()
+    e.simulate(s.ld, s.rd, Q4, pi4, Q16, pi16, s.ct, gap_rate=rate, gap_mean=mean, seed=9, rep0=1, nrep=3)
+    P4, P16 = e.sim_tables()
+    T = oracle.TreeArrays(s.parent, s.left, s.right, s.ld, s.rd)
+    for r in range(3):
+        ref = oracle.simulate(T, L, s.ct, P4, P16, pi4, pi16, None, rate, mean, 9, 1 + r)
+        assert np.array_equal(e.get_alignment(r), ref)
+    e.close()
