@@ -2,12 +2,15 @@
 // its C-ABI (include/covgpu.h).  One context = one device stream and the
 // device buffers for up to `maxslots` alignments of N x L.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <climits>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -103,6 +106,10 @@ struct covgpu_ctx {
   void* d_gsc = nullptr;       // GSC scratch, kept across calls
   size_t gsc_cap = 0;
   double* d_pbscr = nullptr;   // position-based weights scratch
+  // workspace of the calls that finish before they return (substitutions,
+  // power, gap filter, aggregation); grown when a call needs more
+  unsigned char* d_wrk = nullptr;
+  size_t wrk_cap = 0;
   bool want_qsum = false;     // covgpu_rscape keeps the null-score summary of type 0
   double qsum[17] = {0};
   bool have_qsum = false;
@@ -235,7 +242,7 @@ extern "C" void covgpu_destroy(covgpu_ctx* ctx) {
   for (FitWork* f : ctx->fitw) if (f) fitwork_destroy(f);
   void* sims[] = {ctx->d_simQ, ctx->d_simT, ctx->d_P4, ctx->d_P16, ctx->d_C4, ctx->d_C16, ctx->d_R, ctx->d_units,
                   ctx->d_simroot, ctx->d_simstate, ctx->d_nsubs, ctx->d_ndouble, ctx->d_njoin, ctx->d_featscr,
-                  ctx->d_feat, ctx->d_gsc, ctx->d_pbscr};
+                  ctx->d_feat, ctx->d_gsc, ctx->d_pbscr, ctx->d_wrk};
   for (void* p : sims) if (p) cudaFree(p);
   for (auto& e : ctx->ev) if (e) cudaEventDestroy(e);
   for (auto& e : ctx->fev) if (e) cudaEventDestroy(e);
@@ -254,6 +261,32 @@ static int build_tiles(covgpu_ctx* ctx) {
   CK(cudaMemcpy(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(TileRC), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ctx->d_tile_index, tindex.data(), tindex.size() * sizeof(int), cudaMemcpyHostToDevice));
   return 0;
+}
+
+// the workspace holds at least n bytes (a cudaMalloc and a cudaFree per call
+// took ~100 us each time and synchronised the device)
+static cudaError_t work_reserve(covgpu_ctx* ctx, size_t n) {
+  if (ctx->wrk_cap >= n) return cudaSuccess;
+  if (ctx->d_wrk) cudaFree(ctx->d_wrk);
+  ctx->d_wrk = nullptr;
+  ctx->wrk_cap = 0;
+  const cudaError_t e = cudaMalloc(&ctx->d_wrk, n);
+  if (e == cudaSuccess) ctx->wrk_cap = n;
+  return e;
+}
+
+// A caller's result array is often fresh memory whose pages do not exist yet.
+// A copy from the device into such pages raises a fault on each (64 KB) from
+// the device's side, ~90 us apiece: 8 alignments of 1000 x 1201 took 12.9 ms
+// to read, 0.73 ms with the pages made first.  Errors (an old kernel, memory
+// that is not the caller's) are left to the copy.
+static void result_pages(void* p, size_t n) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  if (!p || n < 4096) return;
+  const uintptr_t pg = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p & ~(pg - 1);
+  (void)madvise((void*)a, ((uintptr_t)p + n - a + pg - 1) & ~(pg - 1), MADV_POPULATE_WRITE);
 }
 
 extern "C" int covgpu_resize(covgpu_ctx* ctx, int N, int L) {
@@ -335,6 +368,7 @@ extern "C" int covgpu_get_alignment(covgpu_ctx* ctx, int slot, uint8_t* ax) {
   if (slot < 0 || slot >= ctx->maxslots) return fail(ctx, 11, "slot %d out of range", slot);
   CK(cudaSetDevice(ctx->dev));
   const uint8_t* src = ctx->d_ax + (size_t)slot * ctx->N * ctx->Lp;
+  result_pages(ax, (size_t)ctx->N * ctx->L);
   CK(cudaMemcpy2DAsync(ax, ctx->L, src, ctx->Lp, ctx->L, ctx->N, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   return 0;
@@ -462,15 +496,15 @@ extern "C" int covgpu_substitutions(covgpu_ctx* ctx, int slot, uint64_t seed, in
   if (!ctx->have_tree) return fail(ctx, 11, "no tree set");
   if (N < 2) return fail(ctx, 11, "substitutions need a tree of at least two leaves");
   if (slot < 0 || slot >= ctx->maxslots) return fail(ctx, 11, "bad slot");
-  const size_t rows = (size_t)(N - 1) * Lp;
-  uint8_t *F = ctx->d_fitch, *S = ctx->d_scratch, *tmp = nullptr;
-  if (!F || !S) {
-    CK(cudaMalloc(&tmp, 2 * rows));
-    F = tmp; S = tmp + rows;
-  }
+  const size_t rows = (size_t)(N - 1) * Lp; 
+  uint8_t *F = ctx->d_fitch, *S = ctx->d_scratch;
+  const bool own = F && S;
   const int Wb = (2 * (N - 1) + 31) / 32;
-  uint32_t* bits = nullptr;
-  cudaError_t e = cudaMalloc(&bits, 2 * (size_t)L * Wb * sizeof(uint32_t));
+  const size_t nbits = 2 * (size_t)L * Wb * sizeof(uint32_t);
+  cudaError_t e = work_reserve(ctx, nbits + (own ? 0 : 256 + 2 * rows));
+  if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
+  uint32_t* bits = (uint32_t*)ctx->d_wrk;
+  if (!own) { F = ctx->d_wrk + ((nbits + 255) & ~(size_t)255); S = F + rows; }
   if (e == cudaSuccess && !ctx->d_nsubs) {
     e = dalloc(&ctx->d_nsubs, (size_t)ctx->capL);
     if (e == cudaSuccess) e = dalloc(&ctx->d_ndouble, (size_t)ctx->capL * ctx->capL);
@@ -484,14 +518,14 @@ extern "C" int covgpu_substitutions(covgpu_ctx* ctx, int slot, uint64_t seed, in
   if (e == cudaSuccess)
     e = launch_substitutions(ax, F, ctx->d_left, ctx->d_right, N, L, Lp, includegaps ? 1 : 0, bits,
                              bits + (size_t)L * Wb, ctx->d_nsubs, ctx->d_ndouble, ctx->d_njoin, ctx->st);
+  result_pages(ndouble, (size_t)L * L * sizeof(int));
+  result_pages(njoin, (size_t)L * L * sizeof(int));
   if (e == cudaSuccess && nsubs) e = cudaMemcpyAsync(nsubs, ctx->d_nsubs, L * sizeof(int), cudaMemcpyDeviceToHost, ctx->st);
   if (e == cudaSuccess && ndouble)
     e = cudaMemcpyAsync(ndouble, ctx->d_ndouble, (size_t)L * L * sizeof(int), cudaMemcpyDeviceToHost, ctx->st);
   if (e == cudaSuccess && njoin)
     e = cudaMemcpyAsync(njoin, ctx->d_njoin, (size_t)L * L * sizeof(int), cudaMemcpyDeviceToHost, ctx->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
-  if (bits) cudaFree(bits);
-  if (tmp) cudaFree(tmp);
   if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
   ctx->nlaunch += 4;
   return 0;
@@ -510,20 +544,19 @@ extern "C" int covgpu_power(covgpu_ctx* ctx, int ns, const double* subs, const d
   for (int k = 0; k < 6; k++)
     if (src[k]) for (int s = 0; s < ns; s++) tab[(size_t)k * ns + s] = src[k][s];
   const int64_t P = (int64_t)L * (L - 1) / 2;
-  double *d_tab = nullptr, *d_out = nullptr;
-  CK(dalloc(&d_tab, tab.size()));
-  cudaError_t e = dalloc(&d_out, (size_t)3 * std::max<int64_t>(P, 1));
+  CK(work_reserve(ctx, (tab.size() + 3 * (size_t)P) * sizeof(double)));
+  double *d_tab = (double*)ctx->d_wrk, *d_out = d_tab + tab.size();
+  cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->st);
   if (e == cudaSuccess)
     e = launch_power(ctx->d_nsubs, ctx->d_ndouble, ctx->d_njoin, L, ns, d_tab, subs && prob, subs_join && prob_join,
                      subs_double && prob_double, d_out, d_out + P, d_out + 2 * P, ctx->st);
   double* outs[3] = {power, power_join, power_double};
+  for (double* o : outs) result_pages(o, P * sizeof(double));
   for (int k = 0; k < 3 && e == cudaSuccess; k++)
     if (outs[k] && P > 0)
       e = cudaMemcpyAsync(outs[k], d_out + k * P, P * sizeof(double), cudaMemcpyDeviceToHost, ctx->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
-  cudaFree(d_tab);
-  if (d_out) cudaFree(d_out);
   if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
   return 0;
 }
@@ -533,19 +566,14 @@ extern "C" int covgpu_gapfilter_dev(covgpu_ctx* ctx, int slot, const double* wgt
   CK(cudaSetDevice(ctx->dev));
   const int N = ctx->N, L = ctx->L, Lp = ctx->Lp;
   if (slot < 0 || slot >= ctx->maxslots || !useme) return fail(ctx, 11, "bad slot or output");
-  double* d_w = nullptr;
-  int* d_use = nullptr;
-  CK(dalloc(&d_use, (size_t)L));
+  CK(work_reserve(ctx, (wgt ? (size_t)N * sizeof(double) : 0) + (size_t)L * sizeof(int)));
+  double* d_w = wgt ? (double*)ctx->d_wrk : nullptr;
+  int* d_use = (int*)(ctx->d_wrk + (wgt ? (size_t)N * sizeof(double) : 0));
   cudaError_t e = cudaSuccess;
-  if (wgt) {
-    e = dalloc(&d_w, (size_t)N);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_w, wgt, N * sizeof(double), cudaMemcpyHostToDevice, ctx->st);
-  }
+  if (wgt) e = cudaMemcpyAsync(d_w, wgt, N * sizeof(double), cudaMemcpyHostToDevice, ctx->st);
   if (e == cudaSuccess) e = launch_gapfilter(ctx->d_ax + (size_t)slot * N * Lp, d_w, N, L, Lp, gapthresh, d_use, ctx->st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(useme, d_use, L * sizeof(int), cudaMemcpyDeviceToHost, ctx->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
-  cudaFree(d_use);
-  if (d_w) cudaFree(d_w);
   if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
   return 0;
 }
@@ -850,6 +878,7 @@ extern "C" int covgpu_get_cov(covgpu_ctx* ctx, int slot, int which, double* COV)
   const int64_t plane = (int64_t)ctx->ntiles * TPP;
   CK(launch_untile(ctx->d_cov + ((int64_t)rel * ctx->last_nout + which) * plane, ctx->d_tiles, ctx->ntiles, ctx->L,
                    -INFINITY, ctx->d_full, ctx->st));
+  result_pages(COV, (size_t)ctx->L * ctx->L * sizeof(double));
   CK(cudaMemcpyAsync(COV, ctx->d_full, (size_t)ctx->L * ctx->L * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   return 0;
@@ -891,6 +920,9 @@ extern "C" int covgpu_get_probs(covgpu_ctx* ctx, int slot, const double* wgt, do
     CK(cudaMemsetAsync(dpp, 0, LL * 18 * sizeof(double), ctx->st));
     CK(launch_probs_host_layout(ctx->d_cnt + (size_t)rel * ctx->ntiles * 32 * TPP, ctx->d_tiles, ctx->ntiles, L, wt,
                                 pp ? dpp : nullptr, nseff ? dns : nullptr, ngap ? dng : nullptr, ctx->st));
+    result_pages(pp, LL * 16 * sizeof(double));
+    result_pages(nseff, LL * sizeof(double));
+    result_pages(ngap, LL * sizeof(double));
     if (pp) CK(cudaMemcpyAsync(pp, dpp, LL * 16 * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
     if (nseff) CK(cudaMemcpyAsync(nseff, dns, LL * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
     if (ngap) CK(cudaMemcpyAsync(ngap, dng, LL * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
@@ -1592,10 +1624,10 @@ extern "C" int covgpu_aggregate(covgpu_ctx* ctx, int method, int nh, const int* 
     if (need_aux && !(aux[k] >= 0.0 && std::isfinite(aux[k]))) return fail(ctx, 11, "weight %d is negative", k);
   }
   const size_t nd = (size_t)nbp * 4 + nh + 1;   // pval, aux, term[2], pagg
-  double* d = nullptr;
-  int* d_off = nullptr;
-  CK(dalloc(&d, nd));
-  cudaError_t e = dalloc(&d_off, (size_t)nh + 1);
+  CK(work_reserve(ctx, nd * sizeof(double) + ((size_t)nh + 1) * sizeof(int)));
+  double* d = (double*)ctx->d_wrk;
+  int* d_off = (int*)(d + nd);
+  cudaError_t e = cudaSuccess;
   double *d_pval = d, *d_aux = d + nbp, *d_term = d + 2 * (size_t)nbp, *d_pagg = d + 4 * (size_t)nbp;
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_off, helix_off, ((size_t)nh + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->st);
   if (e == cudaSuccess && nbp)
@@ -1605,8 +1637,6 @@ extern "C" int covgpu_aggregate(covgpu_ctx* ctx, int method, int nh, const int* 
   if (e == cudaSuccess) e = launch_aggregate(method, nh, d_off, d_pval, d_aux, d_term, d_pagg, ctx->st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(pagg, d_pagg, (size_t)nh * sizeof(double), cudaMemcpyDeviceToHost, ctx->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
-  cudaFree(d);
-  if (d_off) cudaFree(d_off);
   if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
   // E-value: times the number of helices tested (rm->Eval, src/aggregate.c:114)
   if (Eagg)
@@ -1690,6 +1720,7 @@ extern "C" int covgpu_pair_classes(covgpu_ctx* ctx, int slot, double* wcf, doubl
   double* d = ctx->d_pcls;
   const float* cnt = ctx->d_cnt + (size_t)(slot - ctx->cnt_first) * ctx->ntiles * 32 * TPP;
   CK(launch_pair_classes(cnt, ctx->d_tiles, ctx->ntiles, L, d, d + P, d + 2 * P, ctx->st));
+  for (double* o : {wcf, wobble, noncan}) result_pages(o, P * sizeof(double));
   if (wcf) CK(cudaMemcpyAsync(wcf, d, P * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   if (wobble) CK(cudaMemcpyAsync(wobble, d + P, P * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   if (noncan) CK(cudaMemcpyAsync(noncan, d + 2 * P, P * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
@@ -1880,6 +1911,7 @@ extern "C" int covgpu_evalue_sets(covgpu_ctx* ctx, const double* COV, const void
   if (Eval) {
     if (!ctx->d_full) CK(dalloc(&ctx->d_full, (size_t)ctx->capL * ctx->capL));
     CK(launch_untile(evt, ctx->d_tiles, ctx->ntiles, L, INFINITY, ctx->d_full, ctx->st));
+    result_pages(Eval, (size_t)L * L * sizeof(double));
     CK(cudaMemcpyAsync(Eval, ctx->d_full, (size_t)L * L * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
   }
