@@ -867,4 +867,40 @@ cudaError_t grp_weights_limbs(FamDev* F, int nf, const int* pre, int nb, UmmaFam
 // the merges' limits, raised outside any stream capture
 int grp_weights_gsc_prepare() { return gsc_attrs() == cudaSuccess ? 1 : 0; }
 
+// rows of L bytes, one after the other, to a pitch of Lp: 16 bytes of a row
+// per thread, from the aligned words around them (src: aligned, readable for
+// 20 bytes past the last row); columns L .. Lp - 1 are left alone.  Bound by
+// memory: 60 MB moved at 20000 x 1500.
+__global__ void __launch_bounds__(256)
+k_spread_rows(const uint8_t* __restrict__ src, int64_t N, int L, int Lp, uint8_t* __restrict__ dst) {
+  const int per = Lp >> 4;
+  const int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (it >= N * per) return;
+  const int64_t r = it / per;
+  const int c = (int)(it - r * per) << 4;
+  if (c >= L) return;
+  const int64_t o = r * L + c;
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(src + (o & ~(int64_t)3));
+  const int sh = (int)(o & 3) * 8;
+  uint32_t v[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) v[k] = __ldg(w + k);
+#pragma unroll
+  for (int k = 0; k < 4; k++) v[k] = __funnelshift_r(v[k], v[k + 1], sh);
+  uint8_t* d = dst + r * Lp + c;
+  if (c + 16 <= L) {
+    *reinterpret_cast<uint4*>(d) = make_uint4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+      if (c + k < L) d[k] = (uint8_t)(v[k >> 2] >> (8 * (k & 3)));
+  }
+}
+
+cudaError_t launch_spread_rows(const uint8_t* src, int N, int L, int Lp, uint8_t* dst, cudaStream_t st) {
+  const int64_t items = (int64_t)N * (Lp >> 4);
+  k_spread_rows<<<(unsigned)((items + 255) / 256), 256, 0, st>>>(src, N, L, Lp, dst);
+  return cudaGetLastError();
+}
+
 }  // namespace covgpu

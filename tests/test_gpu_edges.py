@@ -158,3 +158,17 @@ def test_simulated_gap_runs_by_words(covgpu, oracle, N, L, rate, mean):
         ref = oracle.simulate(T, L, s.ct, P4, P16, pi4, pi16, None, rate, mean, 9, 1 + r)
         assert np.array_equal(e.get_alignment(r), ref)
     e.close()
+
+
+@pytest.mark.parametrize("L", [1, 15, 16, 17, 31, 32, 33, 47, 63, 95, 97, 130])
+def test_alignment_rows_round_trip(covgpu, L):
+    """Rows of every offset in a word, lengths around 16 and 32, two slots of
+    different content: what was set is what is read."""
+    rng = np.random.default_rng(L)
+    e = covgpu.Engine(37, L, maxslots=2, maxnull=0)
+    ax = [rng.integers(0, 18, (37, L)).astype(np.uint8) for _ in range(2)]
+    for k in (0, 1):
+        e.set_alignment(k, ax[k])
+    for k in (1, 0):
+        assert np.array_equal(e.get_alignment(k), ax[k])
+    e.close()
