@@ -48,128 +48,158 @@ __host__ __device__ __forceinline__ int exact_bin(double x, double bmin, double 
 }
 
 // ------------------------------------------------------------------------
-// Counting (plain SIMT path): one CTA per (tile, alignment); 256 threads,
-// each owning a 2x2 block of pairs and 4x16 fp32 accumulators.  Sequences
-// are staged 32 at a time in shared memory as float4 one-hot (i side) and
-// value-scaled one-hot (j side) vectors; every pair then takes 16 FMAs per
-// sequence.  The j-side values are integers (1, or one weight limb of at
-// most 2^b - 1 with N (2^b - 1) < 2^24), so every accumulator holds an exact
-// integer.
+// Counting (plain SIMT path): a CTA counts half a tile (16 rows by 32
+// columns) of one alignment; a thread owns four pairs of one column, 4x16
+// FP32 accumulators.  Sequences are staged 16 at a time in shared memory as
+// float4 one-hot (i side) and value-scaled one-hot (j side) vectors, two
+// buffers, the next codes loaded while the present ones are counted; every
+// pair then takes 16 FMAs per sequence.  The j-side values are integers (1,
+// or one weight limb of at most 2^b - 1 with N (2^b - 1) < 2^24), so every
+// accumulator holds an exact integer.
 //   MODE_UNIT   unit weights (RAF): FP32 counts, one plane
 //   MODE_EQUAL  all weights equal to w: the unit count times w as a
 //               double-float (unit_count)
-//   MODE_LIMBS  three weight limbs, counted one after the other (limb 2,
-//               then 1, then 0) and combined exactly as limb_count does: the
-//               partial result of the previous limb is kept in the output
-//               planes, which only this thread touches
+//   MODE_LIMBS  three weight limbs, 128 threads each, side by side (limb_count
+//               of the three through shared memory)
 // Double-float counts go to two planes per cell, [slot][tile][16][hi|lo][TPP].
+//
+// Bound by the FMA pipe where the grid fills the device, by its latency
+// below.  With one CTA of 256 threads per tile and the limbs one after the
+// other: 166 us at 400 x 351 (66 CTAs on 152 SMs), 76 us at 100 x 120 x 21,
+// 21 us at 30 x 61 x 201; so 68, 58 and 10 us.  Packed FMAs took 117 us at
+// 400 x 351 (twice the shared-memory reads on the i side), two pairs a thread
+// 99 us, 2x2 pairs a thread 69 us.
 // ------------------------------------------------------------------------
 enum CountMode { MODE_UNIT = 0, MODE_EQUAL = 1, MODE_LIMBS = 3 };
 
+constexpr int CS_ROWS = 16;   // rows of a tile that a CTA counts
+
+template <int NG>   // limbs counted side by side, 128 threads each
+union CountSmem {
+  struct {
+    float4 ohi[2][16][CS_ROWS];
+    float4 whj[NG][2][16][TP];
+  } st;
+  float ex[NG == 1 ? 1 : NG][64][128];   // the limbs' counts, to be combined
+};
+
 template <int MODE>
 __device__ __forceinline__ void count_simt_body(
-    const GridIdx g, const uint8_t* __restrict__ ax, int64_t slot_stride, const float* __restrict__ limbs, int N,
-    int Lp,
-             const TileRC* __restrict__ tiles, int ntiles, float* __restrict__ cnt, float B, float s_hi, float s_lo) {
-  __shared__ float4 ohi[32][TP];
-  __shared__ float4 whj[32][TP];
-  const int t = g.x, slot = g.y, tid = threadIdx.x;
+    CountSmem<MODE == MODE_LIMBS ? 3 : 1>& sm, const GridIdx g, int part, const uint8_t* __restrict__ ax,
+    int64_t slot_stride, const float* __restrict__ limbs, int N, int Lp, const TileRC* __restrict__ tiles, int ntiles,
+    float* __restrict__ cnt, float B, float s_hi, float s_lo) {
+  constexpr int NG = (MODE == MODE_LIMBS) ? 3 : 1;
+  const int t = g.x, slot = g.y, limb = threadIdx.x >> 7, tid = threadIdx.x & 127;
+  if (limb >= NG) return;
   const TileRC tr = tiles[t];
   const uint8_t* A = ax + (int64_t)slot * slot_stride;
-  const int ty = tid >> 4, tx = tid & 15;
-  constexpr int NPASS = (MODE == MODE_LIMBS) ? 3 : 1;
+  const int ty = tid >> 5, tx = tid & 31, i0 = part * CS_ROWS;   // rows 4 ty .. 4 ty + 3, column tx
   const int64_t tbase = (int64_t)slot * ntiles + t;
+  auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(128 * NG) : "memory"); };
+  float acc[4][16];
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+#pragma unroll
+    for (int c = 0; c < 16; c++) acc[p][c] = 0.f;
+  // a word of four codes of the j side per thread, of the i side for 64 threads
+  const int js = tid >> 3, jw = tid & 7, is = tid >> 2, iw = tid & 3;
+  const bool iside = limb == 0 && tid < 64;
+  uint32_t jc, ic;
+  float val;
+  auto load = [&](int s0) {
+    jc = ic = 0x04040404u;   // past N: gaps
+    val = 1.f;
+    if (s0 + js < N) {
+      jc = *reinterpret_cast<const uint32_t*>(A + (int64_t)(s0 + js) * Lp + tr.J * TP + 4 * jw);
+      if (MODE == MODE_LIMBS) val = limbs[(int64_t)limb * N + s0 + js];
+    }
+    if (iside && s0 + is < N)
+      ic = *reinterpret_cast<const uint32_t*>(A + (int64_t)(s0 + is) * Lp + tr.I * TP + i0 + 4 * iw);
+  };
+  auto onehot = [](float4* d, uint32_t codes, int w, float v) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int qq = (q + (w >> 1)) & 3;   // eight lanes write to eight groups of banks
+      const int code = (codes >> (8 * qq)) & 0xff;
+      d[4 * w + qq] = make_float4((code == 0) ? v : 0.f, (code == 1) ? v : 0.f, (code == 2) ? v : 0.f,
+                                  (code == 3) ? v : 0.f);
+    }
+  };
+  auto store = [&](int buf) {
+    onehot(sm.st.whj[limb][buf][js], jc, jw, val);
+    if (iside) onehot(sm.st.ohi[buf][is], ic, iw, 1.f);
+  };
+  load(0);
+  store(0);
+  sync();
+  int buf = 0;
+  for (int s0 = 0; s0 < N; s0 += 16, buf ^= 1) {
+    const bool more = s0 + 16 < N;
+    if (more) load(s0 + 16);
+    const int smax = min(16, N - s0);
+    const float4 *oi = &sm.st.ohi[buf][0][4 * ty], *wj = &sm.st.whj[limb][buf][0][tx];
 #pragma unroll 1
-  for (int pass = 0; pass < NPASS; pass++) {
-    const int limb = NPASS - 1 - pass;     // limbs 2, 1, 0
-    float acc[4][16];
+    for (int s4 = 0; s4 < smax; s4 += 4) {
 #pragma unroll
-    for (int p = 0; p < 4; p++)
+      for (int s = 0; s < 4; s++) {
+        float iv[4][4], jv[4];
 #pragma unroll
-      for (int c = 0; c < 16; c++) acc[p][c] = 0.f;
-    for (int s0 = 0; s0 < N; s0 += 32) {
+        for (int a = 0; a < 4; a++) *reinterpret_cast<float4*>(iv[a]) = oi[(s4 + s) * CS_ROWS + a];
+        *reinterpret_cast<float4*>(jv) = wj[(s4 + s) * TP];
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int e = tid + 256 * k;          // 0..2047
-        const int half = e >> 10, s = (e >> 5) & 31, c = e & 31;
-        const int seq = s0 + s;
-        int code = 4;
-        float val = 0.f;
-        if (seq < N) {
-          code = A[(int64_t)seq * Lp + (half ? tr.J : tr.I) * TP + c];
-          val = (half && MODE == MODE_LIMBS) ? limbs[(int64_t)limb * N + seq] : 1.f;
-        }
-        float4 v;
-        v.x = (code == 0) ? val : 0.f;
-        v.y = (code == 1) ? val : 0.f;
-        v.z = (code == 2) ? val : 0.f;
-        v.w = (code == 3) ? val : 0.f;
-        if (half) whj[s][c] = v; else ohi[s][c] = v;
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+          for (int x = 0; x < 4; x++)
+#pragma unroll
+            for (int y = 0; y < 4; y++) acc[a][x * 4 + y] = fmaf(iv[a][x], jv[y], acc[a][x * 4 + y]);
       }
-      __syncthreads();
-      const int smax = min(32, N - s0);
-      for (int s = 0; s < smax; s++) {
-        const float4 i0 = ohi[s][2 * ty], i1 = ohi[s][2 * ty + 1];
-        const float4 j0 = whj[s][2 * tx], j1 = whj[s][2 * tx + 1];
-        const float iv[2][4] = {{i0.x, i0.y, i0.z, i0.w}, {i1.x, i1.y, i1.z, i1.w}};
-        const float jv[2][4] = {{j0.x, j0.y, j0.z, j0.w}, {j1.x, j1.y, j1.z, j1.w}};
-#pragma unroll
-        for (int a = 0; a < 2; a++)
-#pragma unroll
-          for (int b = 0; b < 2; b++)
-#pragma unroll
-            for (int x = 0; x < 4; x++)
-#pragma unroll
-              for (int y = 0; y < 4; y++)
-                acc[a * 2 + b][x * 4 + y] = fmaf(iv[a][x], jv[b][y], acc[a * 2 + b][x * 4 + y]);
-      }
-      __syncthreads();
     }
-    if (MODE == MODE_UNIT) {
-      float* out = cnt + tbase * 16 * TPP;
+    if (more) store(buf ^ 1);
+    sync();
+  }
+  const int px = (i0 + 4 * ty) * TP + tx;   // the thread's first pair in the tile
+  if (MODE != MODE_LIMBS) {
+    float* out = cnt + tbase * (MODE == MODE_UNIT ? 16 : 32) * TPP + px;
 #pragma unroll
-      for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int c = 0; c < 16; c++)
-          *reinterpret_cast<float2*>(out + c * TPP + (2 * ty + a) * TP + 2 * tx) =
-              make_float2(acc[a * 2 + 0][c], acc[a * 2 + 1][c]);
-      continue;
-    }
-    float* out = cnt + tbase * 32 * TPP;
-#pragma unroll
-    for (int a = 0; a < 2; a++)
+    for (int a = 0; a < 4; a++)
 #pragma unroll
       for (int c = 0; c < 16; c++) {
-        float2* hp = reinterpret_cast<float2*>(out + (2 * c) * TPP + (2 * ty + a) * TP + 2 * tx);
-        float2* lp = reinterpret_cast<float2*>(out + (2 * c + 1) * TPP + (2 * ty + a) * TP + 2 * tx);
-        df r[2];
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          const float d = acc[a * 2 + b][c];
-          if (MODE == MODE_EQUAL) {
-            r[b] = unit_count(d, s_hi, s_lo);
-          } else if (limb == 2) {
-            r[b] = {d * (B * B), 0.f};                       // c2
-          } else if (limb == 1) {
-            const float2 h = *hp;
-            r[b] = two_sum(b ? h.y : h.x, d * B);           // s1 = c2 + c1
-          } else {
-            const float2 h = *hp, l = *lp;
-            const df s2 = two_sum(b ? h.y : h.x, d);        // s1.hi + c0
-            const df q = fast_two_sum(s2.hi, (b ? l.y : l.x) + s2.lo);
-            r[b] = {q.hi * s_hi, q.lo * s_hi};               // times 2^-E
-          }
+        if (MODE == MODE_UNIT) {
+          out[c * TPP + a * TP] = acc[a][c];
+        } else {
+          const df r = unit_count(acc[a][c], s_hi, s_lo);
+          out[(2 * c) * TPP + a * TP] = r.hi;
+          out[(2 * c + 1) * TPP + a * TP] = r.lo;
         }
-        *hp = make_float2(r[0].hi, r[1].hi);
-        *lp = make_float2(r[0].lo, r[1].lo);
       }
+    return;
+  }
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int c = 0; c < 16; c++) sm.ex[limb][c * 4 + a][tid] = acc[a][c];
+  sync();
+  float* out = cnt + tbase * 32 * TPP + px;
+#pragma unroll 4
+  for (int k = limb; k < 64; k += NG) {   // (cell, row): the three groups share the combination
+    const int c = k >> 2, a = k & 3;
+    const df r = limb_count(sm.ex[0][k][tid], sm.ex[1][k][tid], sm.ex[2][k][tid], B, s_hi);
+    out[(2 * c) * TPP + a * TP] = r.hi;
+    out[(2 * c + 1) * TPP + a * TP] = r.lo;
   }
 }
+
+constexpr int count_threads(int mode) { return mode == MODE_LIMBS ? 384 : 128; }
 template <int MODE>
-__global__ void __launch_bounds__(256, 2)
+constexpr int count_smem() { return (int)sizeof(CountSmem<MODE == MODE_LIMBS ? 3 : 1>); }
+
+template <int MODE>
+__global__ void __launch_bounds__(count_threads(MODE))
 k_count_simt(const uint8_t* __restrict__ ax, int64_t slot_stride, const float* __restrict__ limbs, int N, int Lp,
              const TileRC* __restrict__ tiles, int ntiles, float* __restrict__ cnt, float B, float s_hi, float s_lo) {
-  count_simt_body<MODE>(native_grid(), ax, slot_stride, limbs, N, Lp, tiles, ntiles, cnt, B, s_hi, s_lo);
+  extern __shared__ __align__(16) unsigned char count_sm[];
+  count_simt_body<MODE>(*reinterpret_cast<CountSmem<MODE == MODE_LIMBS ? 3 : 1>*>(count_sm), native_grid(),
+                        (int)blockIdx.z, ax, slot_stride, limbs, N, Lp, tiles, ntiles, cnt, B, s_hi, s_lo);
 }
 
 // constants of the bin function, split on the host
@@ -452,20 +482,42 @@ __global__ void k_meanp(const double* __restrict__ mpc, int L, int Lp, double* _
   meanp_body(native_grid(), mpc, L, Lp, meanp);
 }
 
-// ps[c][x], x over the five codes 0..4 (gap included), prior 1e-5.
-__global__ void k_ps(const uint8_t* __restrict__ ax, int64_t slot_stride, const double* __restrict__ w, int N, int L,
-                     int Lp, double* __restrict__ ps) {
-  const int slot = blockIdx.y;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= L) return;
-  const uint8_t* A = ax + (int64_t)slot * slot_stride;
-  double q[5] = {1e-5, 1e-5, 1e-5, 1e-5, 1e-5};
-  for (int s = 0; s < N; s++) {
-    const int r = A[(int64_t)s * Lp + c];
-    if (r < 5) q[r] += w[s];
+// ps[c][x], x over the five codes 0..4 (gap included), prior 1e-5.  The sum
+// of a code's weights runs over the sequences in their order, so a chain of
+// FP64 additions (~64 cycles each) bounds it: a lane per (column, code), six
+// columns to a warp, and the weights and codes staged 128 sequences at a time.
+// 400 x 351: 139 us with a thread per column (its five sums indexed by the
+// code, so in local memory), 31 us so.
+constexpr int kPsCols = 6;
+__global__ void __launch_bounds__(32)
+k_ps(const uint8_t* __restrict__ ax, int64_t slot_stride, const double* __restrict__ w, int N, int L, int Lp,
+     double* __restrict__ ps) {
+  __shared__ double sw[128];
+  __shared__ uint8_t sc[128][8];
+  const int slot = blockIdx.y, lane = threadIdx.x, c0 = blockIdx.x * kPsCols;
+  const uint8_t* A = ax + (int64_t)slot * slot_stride + c0;
+  const int cl = lane / 5, x = lane - 5 * cl;   // lanes 30 and 31: no column
+  const int nc = min(kPsCols, L - c0);
+  double q = 1e-5;
+  for (int s0 = 0; s0 < N; s0 += 128) {
+    const int n = min(128, N - s0);
+    for (int s = lane; s < n; s += 32) {
+      sw[s] = w[s0 + s];
+      for (int k = 0; k < nc; k++) sc[s][k] = A[(int64_t)(s0 + s) * Lp + k];
+    }
+    __syncwarp();
+    if (cl < nc) {
+#pragma unroll 8
+      for (int s = 0; s < n; s++)
+        if (sc[s][cl] == x) q += sw[s];
+    }
+    __syncwarp();
   }
-  double sum = q[0] + q[1] + q[2] + q[3] + q[4];
-  for (int x = 0; x < 5; x++) ps[((int64_t)slot * Lp + c) * 5 + x] = q[x] / sum;
+  double v[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) v[k] = __shfl_sync(0xffffffffu, q, min(5 * cl + k, 31));
+  const double sum = v[0] + v[1] + v[2] + v[3] + v[4];
+  if (cl < nc) ps[((int64_t)slot * Lp + c0 + cl) * 5 + x] = q / sum;
 }
 
 // ------------------------------------------------------------------------
@@ -1537,16 +1589,25 @@ k_evalue(const float2* __restrict__ cov, const TileRC* __restrict__ tiles, int n
 // C_q = hi + lo, nseff = sum_q C_q, pp = (1e-10 + C_xy) / sum_q (1e-10 + C_q)
 // at [i][j][4x + y] and [j][i][4y + x] (src/correlators.c:1300-1317,
 // 1695-1780), ngap[i][j] = wt - nseff, all in FP64 in that order
+//
+// A CTA takes 256 pairs of a tile (four CTAs to a tile: few tiles leave SMs
+// idle), a warp 32 pairs of one row.  The 16 quotients have one divisor: its
+// reciprocal once, then a product and two residual corrections each (equal to
+// the IEEE quotient: Markstein, IBM J. Res. Dev. 34, 1990).  The values go
+// through shared memory, so that 16 lanes write the 128 bytes of a pair.
+// Bound by the FP64 pipe; 400 x 351: 70 us with a thread per pair of a whole
+// tile writing its own 16 values, 33 us so.
 __global__ void __launch_bounds__(256)
 k_probs_host_layout(const float* __restrict__ cnt, const TileRC* __restrict__ tiles, int L, double wt,
                     double* __restrict__ pp, double* __restrict__ nseff, double* __restrict__ ngap) {
-  const int t = blockIdx.x, tid = threadIdx.x;
+  __shared__ double sv[8][32 * 17];
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const TileRC tr = tiles[t];
   const float* Cb = cnt + (int64_t)t * 32 * TPP;
-  for (int k = 0; k < 4; k++) {
-    const int p = tid + 256 * k;
-    const int i = tr.I * TP + (p >> 5), j = tr.J * TP + (p & 31);
-    if (!(i < j && j < L)) continue;
+  const int p = threadIdx.x + 256 * blockIdx.y;
+  const int i = tr.I * TP + (p >> 5), j = tr.J * TP + lane;
+  const bool ok = i < j && j < L;
+  if (ok) {
     double C[16], ne = 0.0, sum = 0.0;
 #pragma unroll
     for (int q = 0; q < 16; q++) {
@@ -1558,22 +1619,32 @@ k_probs_host_layout(const float* __restrict__ cnt, const TileRC* __restrict__ ti
     if (ngap) ngap[ij] = __dsub_rn(wt, ne);
     if (pp) {
 #pragma unroll
-      for (int q = 0; q < 16; q++) sum = __dadd_rn(sum, __dadd_rn(1e-10, C[q]));
+      for (int q = 0; q < 16; q++) { C[q] = __dadd_rn(1e-10, C[q]); sum = __dadd_rn(sum, C[q]); }
+      const double r = __drcp_rn(sum);
 #pragma unroll
-      for (int x = 0; x < 4; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) {
-          const double v = __ddiv_rn(__dadd_rn(1e-10, C[x * 4 + y]), sum);
-          pp[ij * 16 + x * 4 + y] = v;
-          pp[ji * 16 + y * 4 + x] = v;
-        }
+      for (int q = 0; q < 16; q++) {
+        double v = __dmul_rn(C[q], r);
+        v = __fma_rn(__fma_rn(-v, sum, C[q]), r, v);
+        sv[warp][lane * 17 + q] = __fma_rn(__fma_rn(-v, sum, C[q]), r, v);
+      }
     }
+  }
+  if (!pp) return;
+  __syncwarp();
+  const unsigned m = __ballot_sync(0xffffffffu, ok);
+  const int q = lane & 15, qt = 4 * (q & 3) + (q >> 2);
+  for (int k = 0; k < 32; k += 2) {
+    const int e = k + (lane >> 4);
+    if (!((m >> e) & 1u)) continue;
+    const int64_t je = tr.J * TP + e;
+    pp[((int64_t)i * L + je) * 16 + q] = sv[warp][e * 17 + q];
+    pp[(je * L + i) * 16 + q] = sv[warp][e * 17 + qt];
   }
 }
 
 cudaError_t launch_probs_host_layout(const float* cnt, const TileRC* tiles, int ntiles, int L, double wt, double* pp,
                                      double* nseff, double* ngap, cudaStream_t st) {
-  if (ntiles > 0) k_probs_host_layout<<<ntiles, 256, 0, st>>>(cnt, tiles, L, wt, pp, nseff, ngap);
+  if (ntiles > 0) k_probs_host_layout<<<dim3(ntiles, 4), 256, 0, st>>>(cnt, tiles, L, wt, pp, nseff, ngap);
   return cudaGetLastError();
 }
 
@@ -1638,18 +1709,29 @@ k_tile_rowsums(const float2* __restrict__ tilev, const TileRC* __restrict__ tile
 // ------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------
+template <int MODE>
+static cudaError_t count_simt_mode(const uint8_t* ax, int64_t slot_stride, const float* limbs, int N, int Lp,
+                                   const TileRC* tiles, int ntiles, int nslots, float* cnt, float B, float s_hi,
+                                   float s_lo, cudaStream_t st) {
+  constexpr int smem = count_smem<MODE>();
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k_count_simt<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_count_simt<MODE><<<dim3(ntiles, nslots, TP / CS_ROWS), count_threads(MODE), smem, st>>>(
+      ax, slot_stride, limbs, N, Lp, tiles, ntiles, cnt, B, s_hi, s_lo);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_count_simt(const uint8_t* ax, int64_t slot_stride, const CountWeights& W, bool unit, int N, int Lp,
                               const TileRC* tiles, int ntiles, int nslots, float* cnt, cudaStream_t st) {
-  dim3 grid(ntiles, nslots);
   if (unit)
-    k_count_simt<MODE_UNIT><<<grid, 256, 0, st>>>(ax, slot_stride, nullptr, N, Lp, tiles, ntiles, cnt, 1.f, 1.f, 0.f);
-  else if (W.nl == 1)
-    k_count_simt<MODE_EQUAL><<<grid, 256, 0, st>>>(ax, slot_stride, nullptr, N, Lp, tiles, ntiles, cnt, 1.f, W.s_hi,
-                                                    W.s_lo);
-  else
-    k_count_simt<MODE_LIMBS><<<grid, 256, 0, st>>>(ax, slot_stride, W.d_limbf, N, Lp, tiles, ntiles, cnt, W.B, W.s_hi,
-                                                    0.f);
-  return cudaGetLastError();
+    return count_simt_mode<MODE_UNIT>(ax, slot_stride, nullptr, N, Lp, tiles, ntiles, nslots, cnt, 1.f, 1.f, 0.f, st);
+  if (W.nl == 1)
+    return count_simt_mode<MODE_EQUAL>(ax, slot_stride, nullptr, N, Lp, tiles, ntiles, nslots, cnt, 1.f, W.s_hi,
+                                       W.s_lo, st);
+  return count_simt_mode<MODE_LIMBS>(ax, slot_stride, W.d_limbf, N, Lp, tiles, ntiles, nslots, cnt, W.B, W.s_hi, 0.f,
+                                     st);
 }
 
 cudaError_t launch_pair_marg(const float* cnt, int L, const TileRC* tiles, int ntiles, int nT, int nslots,
@@ -1667,7 +1749,7 @@ cudaError_t launch_pm_final(const double* part4, const double* partR, int L, int
 
 cudaError_t launch_ps(const uint8_t* ax, int64_t slot_stride, const double* w, int N, int L, int Lp, int nslots,
                       double* ps, cudaStream_t st) {
-  k_ps<<<dim3((L + 127) / 128, nslots), 128, 0, st>>>(ax, slot_stride, w, N, L, Lp, ps);
+  k_ps<<<dim3((L + kPsCols - 1) / kPsCols, nslots), 32, 0, st>>>(ax, slot_stride, w, N, L, Lp, ps);
   return cudaGetLastError();
 }
 
@@ -1886,18 +1968,25 @@ __device__ __forceinline__ int gx_cols256(const FamDev& d) { return (d.L + 255) 
 __device__ __forceinline__ int gx_one(const FamDev&) { return 1; }
 __device__ __forceinline__ int gx_apc(const FamDev& d) { return (d.ntiles + APC_TILES - 1) / APC_TILES; }
 
+// blockIdx.y: the tile's rows; MODE_LIMBS's shape also serves the families of
+// equal weights in its launch (their two idle groups of warps leave)
 template <bool UNIT>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(count_threads(UNIT ? MODE_UNIT : MODE_LIMBS))
 k_count_simt_grp(const FamDev* __restrict__ F, const int* __restrict__ pre, int nf) {
+  extern __shared__ __align__(16) unsigned char count_sm[];
+  auto& s1 = *reinterpret_cast<CountSmem<1>*>(count_sm);
   const GrpLoc l = grp_loc(pre, nf, gx_tiles, F);
   const FamDev& d = F[l.f];
   const int64_t ss = (int64_t)d.N * d.Lp;
+  const int part = (int)blockIdx.y;
   if (UNIT)
-    count_simt_body<MODE_UNIT>(l.g, d.ax, ss, nullptr, d.N, d.Lp, d.tiles, d.ntiles, d.ucnt, 1.f, 1.f, 0.f);
+    count_simt_body<MODE_UNIT>(s1, l.g, part, d.ax, ss, nullptr, d.N, d.Lp, d.tiles, d.ntiles, d.ucnt, 1.f, 1.f, 0.f);
   else if (d.nl == 1)
-    count_simt_body<MODE_EQUAL>(l.g, d.ax, ss, nullptr, d.N, d.Lp, d.tiles, d.ntiles, d.cnt, 1.f, d.s_hi, d.s_lo);
+    count_simt_body<MODE_EQUAL>(s1, l.g, part, d.ax, ss, nullptr, d.N, d.Lp, d.tiles, d.ntiles, d.cnt, 1.f, d.s_hi,
+                                d.s_lo);
   else
-    count_simt_body<MODE_LIMBS>(l.g, d.ax, ss, d.limbf, d.N, d.Lp, d.tiles, d.ntiles, d.cnt, d.B, d.s_hi, 0.f);
+    count_simt_body<MODE_LIMBS>(*reinterpret_cast<CountSmem<3>*>(count_sm), l.g, part, d.ax, ss, d.limbf, d.N, d.Lp,
+                                d.tiles, d.ntiles, d.cnt, d.B, d.s_hi, 0.f);
 }
 
 __global__ void __launch_bounds__(256)
@@ -2029,8 +2118,16 @@ BinC binc_host(double bmin, double w) { return make_binc(bmin, w); }
 cudaError_t grp_count_simt(const FamDev* F, int nf, const int* pre, int nb, bool unit, bool limbs, cudaStream_t st) {
   (void)limbs;
   if (nb <= 0) return cudaSuccess;
-  if (unit) k_count_simt_grp<true><<<nb, 256, 0, st>>>(F, pre, nf);
-  else      k_count_simt_grp<false><<<nb, 256, 0, st>>>(F, pre, nf);
+  const dim3 grid(nb, TP / CS_ROWS);
+  if (unit) {
+    k_count_simt_grp<true><<<grid, count_threads(MODE_UNIT), count_smem<MODE_UNIT>(), st>>>(F, pre, nf);
+  } else {
+    constexpr int smem = count_smem<MODE_LIMBS>();
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_count_simt_grp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_count_simt_grp<false><<<grid, count_threads(MODE_LIMBS), smem, st>>>(F, pre, nf);
+  }
   return cudaGetLastError();
 }
 

@@ -172,3 +172,28 @@ def test_alignment_rows_round_trip(covgpu, L):
     for k in (1, 0):
         assert np.array_equal(e.get_alignment(k), ax[k])
     e.close()
+
+
+@pytest.mark.parametrize("N", [2, 15, 16, 17, 33, 129])
+@pytest.mark.parametrize("L", [17, 32, 65, 97])
+@pytest.mark.parametrize("weights", ["limbs", "equal"])
+def test_plain_counts_at_chunk_edges(covgpu, oracle, N, L, weights):
+    """The plain counting path at the edges of its chunks of 16 sequences, its
+    half tiles and the single-column frequencies' chunks of 128: the counts
+    are exact, so the probabilities equal the tensor path's in every bit; the
+    frequencies (of the weights as given) within 1e-12 of the oracle's."""
+    rng = np.random.default_rng(N * 100 + L)
+    ax = rng.integers(0, 6, (N, L)).astype(np.uint8)
+    ax[ax == 5] = 15   # N: neither residue nor gap
+    w = rng.uniform(0.2, 3.0, N) if weights == "limbs" else np.full(N, 0.7)
+    got = []
+    for counter in (covgpu.SIMT, covgpu.TENSOR):
+        e = covgpu.Engine(N, L)
+        e.set_weights(w)
+        e.set_alignment(0, ax)
+        e.score(["GTp", "RAF"], counter=counter)
+        got.append(e.get_probs(0, w) + (e.get_cov(0, 1),))
+        e.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    assert np.allclose(got[0][4], oracle.probs(ax, w)[4], rtol=1e-12, atol=1e-12)
