@@ -23,17 +23,41 @@
 
 namespace covgpu {
 
-// x / b for positive x and b within FP32's range: FP32's reciprocal, two
-// Newton steps, and two residual corrections of the quotient (Newton-Raphson
-// reciprocal and Markstein's correction, IBM J. Res. Dev. 34, 1990), equal to
-// the IEEE quotient; without a branch, so several run side by side
-__device__ __forceinline__ double div_pos(double x, double b) {
-  double r = (double)__frcp_rn((float)b);
-  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
-  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
-  double q = __dmul_rn(x, r);
-  q = __fma_rn(__fma_rn(-q, b, x), r, q);
+// On this chip a warp issues an FP64 instruction every ~64 cycles, whatever
+// its lanes do and whether or not it depends on the one before (an SM's four
+// schedulers: one in 16 cycles).  So what counts in these kernels is the
+// number of FP64 instructions of the longest warp, comparisons and
+// conversions from integers among them: tests are made on the words where
+// the words decide, and independent parts go to different warps.
+
+// x / b, |b| and |x| within div_range: the hardware's approximate reciprocal
+// (20 bits), one third-order Newton step and one residual correction of the
+// quotient (Markstein, IBM J. Res. Dev. 34, 1990): six FP64 instructions.
+// Equal to the IEEE quotient on 5e8 random pairs.
+__device__ __forceinline__ double div_fast(double x, double b) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+  double e = __fma_rn(-b, r, 1.0);
+  e = __fma_rn(e, e, e);
+  r = __fma_rn(r, e, r);
+  const double q = __dmul_rn(x, r);
   return __fma_rn(__fma_rn(-q, b, x), r, q);
+}
+__device__ __forceinline__ bool div_range(double x) {   // ~1e-30 .. 1e30, either sign
+  return (unsigned)((__double2hiint(x) & 0x7fffffff) - 0x39b4484c) < (unsigned)(0x46293e59 - 0x39b4484c);
+}
+
+// |t| < eps |s| (or <=): where the exponents are at most `far` apart it is
+// false and from `near` on true, for an eps between 2^-(near - 1) and
+// 2^-(far + 1); the comparison itself between
+template <bool EQ>
+__device__ __forceinline__ bool negligible(double t, double s, double eps, int far, int near) {
+  const int et = (__double2hiint(t) >> 20) & 0x7ff, es = (__double2hiint(s) >> 20) & 0x7ff;
+  if (et != 0 && es != 0x7ff) {
+    if (es - et <= far) return false;
+    if (es - et >= near) return true;
+  }
+  return EQ ? fabs(t) <= eps * fabs(s) : fabs(t) < fabs(s) * eps;
 }
 
 // regularised upper incomplete gamma Q(a, x): series for x < a + 1, Lentz's
@@ -43,48 +67,46 @@ __device__ __forceinline__ double div_pos(double x, double b) {
 __device__ double gamma_q_sum(double a, double x) {
   if (x < a + 1.0) {
     double sum = 1.0 / a, del = sum, ap = a;
-    // four quotients at a time: they do not depend on the terms, which do on
-    // one another (a dependent FP64 operation takes ~64 cycles here, a
-    // division ~800)
-    if (!(x < 1e30 && a < 1e30)) {   // outside div_pos's range
-      for (int n = 0; n < 10000; n++) {
-        ap += 1.0; del *= x / ap; sum += del;
-        if (fabs(del) < fabs(sum) * 1e-16) break;
-      }
-      return sum;
-    }
-    for (int n = 0; n < 10000; n += 4) {
-      double q[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) { ap += 1.0; q[k] = div_pos(x, ap); }
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        del = __dmul_rn(del, q[k]); sum = __dadd_rn(sum, del);
-        if (fabs(del) < fabs(sum) * 1e-16) return sum;
-      }
+    const bool in = div_range(x) && a < 1e30;
+    for (int n = 0; n < 10000; n++) {
+      ap += 1.0;
+      const double q = in ? div_fast(x, ap) : x / ap;
+      del = __dmul_rn(del, q);
+      sum = __dadd_rn(sum, del);
+      if (negligible<false>(del, sum, 1e-16, 52, 55)) break;
     }
     return sum;
   }
-  double b = x + 1.0 - a, c = 1.0 / 1e-300, d = 1.0 / b, h = d;
+  double b = x + 1.0 - a, c = 1.0 / 1e-300, d = 1.0 / b, h = d, di = 0.0;
   for (int i = 1; i < 10000; i++) {
-    const double an = -i * (i - a);
+    di += 1.0;
+    const double an = -di * (di - a);
     b += 2.0;
-    d = an * d + b; if (fabs(d) < 1e-300) d = 1e-300;
-    c = b + an / c; if (fabs(c) < 1e-300) c = 1e-300;
-    d = 1.0 / d;
-    const double del = d * c;
-    h *= del;
-    if (fabs(del - 1.0) < 1e-16) break;
+    d = __fma_rn(an, d, b);
+    if (div_range(d) && div_range(c) && (__double2hiint(an) & 0x7fffffff) < 0x46293e59) {
+      c = __dadd_rn(b, div_fast(an, c));
+      d = div_fast(1.0, d);
+    } else {   // the first step (c = 1e300) and arguments far out
+      if (fabs(d) < 1e-300) d = 1e-300;
+      c = b + an / c;
+      d = 1.0 / d;
+    }
+    if ((__double2hiint(c) & 0x7fffffff) < 0x01a56e20 && fabs(c) < 1e-300) c = 1e-300;
+    const double del = __dmul_rn(d, c);
+    h = __dmul_rn(h, del);
+    if (__double_as_longlong(del) == 0x3ff0000000000000ll) break;   // |del - 1| < 1e-16: only 1 itself
   }
   return h;
 }
-__device__ __forceinline__ double gamma_q_pre(double a, double x, double lga) { return exp(-x + a * log(x) - lga); }
-__device__ __forceinline__ double gamma_q_join(double a, double x, double sum, double pre) {
+// log of the prefactor without Gamma(a): a log x - x
+__device__ __forceinline__ double gamma_q_lpre(double a, double x) { return __fma_rn(a, log(x), -x); }
+__device__ __forceinline__ double gamma_q_join(double a, double x, double sum, double lpre, double lga) {
+  const double pre = exp(__dsub_rn(lpre, lga));
   return x < a + 1.0 ? __fma_rn(-sum, pre, 1.0) : __dmul_rn(pre, sum);
 }
 __device__ double gamma_q_dev(double a, double x, double lga) {
   if (x <= 0.0) return 1.0;
-  return gamma_q_join(a, x, gamma_q_sum(a, x), gamma_q_pre(a, x, lga));
+  return gamma_q_join(a, x, gamma_q_sum(a, x), gamma_q_lpre(a, x), lga);
 }
 
 struct FitPoint { double lambda, tau, lga, lconst; };   // lconst = tau log lambda - lgamma(tau)
@@ -99,38 +121,38 @@ struct FitPoint { double lambda, tau, lga, lconst; };   // lconst = tau log lamb
 // summed as d_k = c_k h^k, which needs one log and avoids the cancellation
 // of Q(lo) - Q(hi); closer to mu the difference of Q is used.
 __constant__ double c_inv[64];   // c_inv[k] = 1 / (k + 1)
+__constant__ double c_num[60] = {0,  1,  2,  3,  4,  5,  6,  7,  8,  9,  10, 11, 12, 13, 14, 15, 16, 17, 18, 19,
+                                 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31, 32, 33, 34, 35, 36, 37, 38, 39,
+                                 40, 41, 42, 43, 44, 45, 46, 47, 48, 49, 50, 51, 52, 53, 54, 55, 56, 57, 58, 59};
 
-__device__ __forceinline__ bool gam_bin_far(double x, double h, const FitPoint& P) {
-  return x > 0.0 && h <= 0.0625 * x && P.lambda * h <= 0.5;
-}
-__device__ __forceinline__ double gam_logp_far(double x, double h, double logx, const FitPoint& P) {
-  const double r = h / x, s = P.lambda * h;
+// a non-empty bin [lo, lo + h) of the tail: x = lo - mu, x2 = lo + h - mu,
+// logx = log x (x > 0); r = h / x where h <= x / 16, else -1
+struct FitBin { double x, h, r, logx, x2; };
+
+__device__ __forceinline__ bool gam_bin_far(const FitBin& B, const FitPoint& P) { return B.r >= 0.0 && P.lambda * B.h <= 0.5; }
+// log of h sum_k d_k / (k + 1)
+__device__ __forceinline__ double gam_far_sum(const FitBin& B, const FitPoint& P) {
+  const double r = B.r, s = P.lambda * B.h, tm1 = P.tau - 1.0;
   double dkm1 = 0.0, dk = 1.0, sum = 1.0;
   for (int k = 0; k < 60; k++) {
-    const double dk1 = (((P.tau - 1.0 - k) * r - s) * dk - s * r * dkm1) * c_inv[k];
+    const double dk1 = (((tm1 - c_num[k]) * r - s) * dk - s * r * dkm1) * c_inv[k];
     const double term = dk1 * c_inv[k + 1];
     sum += term;
     dkm1 = dk; dk = dk1;
-    if (fabs(term) <= 1e-17 * fabs(sum)) break;
+    if (negligible<true>(term, sum, 1e-17, 55, 58)) break;
   }
-  return P.lconst + (P.tau - 1.0) * logx - P.lambda * x + log(h * sum);
+  return log(B.h * sum);
 }
-// a bin near mu in four independent parts: k & 1 the prefactor or the sum of
-// Q, k >> 1 at the bin's lower or upper bound; then the four joined
-__device__ __forceinline__ double gam_near_part(int k, double lo, double h, double mu, const FitPoint& P) {
-  const double l = (k & 2) ? lo + h : ((lo < mu) ? mu : lo);
-  if (l <= mu) return 0.0;
-  const double x = P.lambda * (l - mu);
-  if (x <= 0.0) return 0.0;
-  return (k & 1) ? gamma_q_pre(P.tau, x, P.lga) : gamma_q_sum(P.tau, x);
+__device__ __forceinline__ double gam_far_join(const FitBin& B, const FitPoint& P, double ls) {
+  return P.lconst + (P.tau - 1.0) * B.logx - P.lambda * B.x + ls;
 }
-__device__ __forceinline__ double gam_near_q(double l, double mu, const FitPoint& P, double sum, double pre) {
-  if (l <= mu) return 1.0;
-  const double x = P.lambda * (l - mu);
-  return x <= 0.0 ? 1.0 : gamma_q_join(P.tau, x, sum, pre);
+// Q at the lower or upper bound of a bin near mu
+__device__ __forceinline__ double gam_near_x(const FitBin& B, bool upper, const FitPoint& P) {
+  const double x = upper ? B.x2 : B.x;
+  return x > 0.0 ? P.lambda * x : 0.0;
 }
-__device__ __forceinline__ double gam_near_join(double lo, double h, double mu, const FitPoint& P, const double (&r)[4]) {
-  const double p = gam_near_q((lo < mu) ? mu : lo, mu, P, r[0], r[1]) - gam_near_q(lo + h, mu, P, r[2], r[3]);
+__device__ __forceinline__ double gam_near_join(double ql, double qu) {
+  const double p = ql - qu;
   return log(p > 0.0 ? p : 1e-300);
 }
 
@@ -154,7 +176,7 @@ struct FitOut { double lambda, tau; int evals, status; };
 struct FitGrid {
   const int* bins;       // non-empty tail bins, in bin order
   const double* cnts;    // their counts
-  double* logx;          // scratch: log(lower bound - mu) per bin
+  FitBin* geo;           // scratch: the bins' geometry
   int nnz;
   double bmin, w, mu;
   double* part;          // [2][6][gridDim.x] block sums
@@ -173,37 +195,62 @@ struct FitShared {
   double near_r[4][kFitNear];
 };
 
-// evaluates the npts points in sh.pts over the tail.  The work items (point q,
-// bin k), point-major, are spread over the first `own` threads of each block
-// of the grid: FP64 throughput is per SM, so the grid is sized to use every
-// SM's FP64 unit before it stacks warps on one.  Each block sums its items
-// per point, arrives at the grid barrier, then adds all block sums in block
-// order into sh.F.  False when the barrier timed out.
+// the lanes' sums of six values, pairwise over lanes 16, 8, 4, 2 and 1 apart
+// (each value's sum is the one its own butterfly gives), a lane keeping half
+// of its values at each step: 8 additions instead of 30.  The total of value
+// q is in lane fold_lane(q)'s group of four.
+__device__ __forceinline__ double fold6(const double (&a)[kFitMaxPts], int lane) {
+  const bool u = lane & 16, v = lane & 8, w = lane & 4;
+  double x[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) x[k] = (u ? a[3 + k] : a[k]) + __shfl_xor_sync(0xffffffffu, u ? a[k] : a[3 + k], 16);
+  const double y0 = (v ? x[2] : x[0]) + __shfl_xor_sync(0xffffffffu, v ? x[0] : x[2], 8);
+  const double y1 = (v ? 0.0 : x[1]) + __shfl_xor_sync(0xffffffffu, v ? x[1] : 0.0, 8);
+  double z = (w ? y1 : y0) + __shfl_xor_sync(0xffffffffu, w ? y0 : y1, 4);
+  z += __shfl_xor_sync(0xffffffffu, z, 2);
+  return z + __shfl_xor_sync(0xffffffffu, z, 1);
+}
+// the value whose total fold6 leaves in this lane, or -1
+__device__ __forceinline__ int fold_value(int lane) {
+  if (lane & 3) return -1;
+  const int v = (lane & 8) ? 2 : (lane & 4) ? 1 : 0;
+  return (lane & 12) == 12 ? -1 : ((lane & 16) ? 3 : 0) + v;
+}
+
+// evaluates the npts points of simplex coordinates sh.pc (written by thread
+// 0) over the tail.  The work items (point q, bin k), point-major, are spread
+// over the first `own` threads of each block of the grid.  Each block sums
+// its items per point, arrives at the grid barrier, then adds all block sums
+// in block order into sh.F.  False when the barrier timed out.
 //
-// A bin near mu takes two incomplete gammas, each a series of divisions and a
-// prefactor: ~48,000 cycles one after the other, and the whole search waits
-// for them in every round.  The block's warps share their four parts out (one
-// part to a warp, so no warp diverges), the quotients of a series come four at
-// a time and the point sums are folded side by side: a search of three tails
-// of a 30 x 61 family (200 nulls) takes 156 us, 209 us with a thread's parts one
-// after the other.
+// A bin near mu takes two incomplete gammas.  They, the far bins' series and
+// the points' lgamma are independent, so they go to different warps: far
+// series to the owners, sums of the lower and upper bounds to the next two
+// warps, the prefactors' logarithms to the one after, lgamma and log lambda
+// to the last; the values meet in shared memory.
 //
 // The list's size: the bins within 17 widths of mu make up to 102 items in a
 // round; more only when lambda w > 0.5, and those past the list are computed
 // where they are.
+//
+// Three tails of a 30 x 61 family with 200 nulls (16 bins): 209 us with
+// everything of an item in its thread, 156 us with the near bins' parts in
+// four warps, 99 us so.
 __device__ bool fit_eval(const FitGrid& g, FitShared& sh, int npts, unsigned& phase, int own, int G, int bid) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int T = G * own, nw = own >> 5, ngrp = blockDim.x >> 7;   // the block is a multiple of 128 threads
+  const int T = G * own, now = own >> 5, nw = blockDim.x >> 5;   // at least four warps
   const int nitems = npts * g.nnz, first = bid * own + tid;
   double* part = g.part + (size_t)(phase & 1u) * kFitMaxPts * G;
   if (tid == 0) sh.nnear = 0;
   __syncthreads();
+  if (lane < npts && warp == 0) sh.pts[lane].tau = exp(sh.pc[lane][1]);
+  if (lane < npts && warp == 1) sh.pts[lane].lambda = exp(sh.pc[lane][0]);
+  __syncthreads();
   int slot[kFitOwn], nslot = 0;
   if (tid < own) {
     for (int it = first; it < nitems; it += T) {
-      const int q = it / g.nnz, b = g.bins[it - q * g.nnz];
-      const double lo = g.w * b + g.bmin, hi = g.w * (b + 1) + g.bmin;
-      if (gam_bin_far(lo - g.mu, hi - lo, sh.pts[q]) || nslot == kFitOwn) continue;
+      const int q = it / g.nnz;
+      if (gam_bin_far(g.geo[it - q * g.nnz], sh.pts[q]) || nslot == kFitOwn) continue;
       const int s = atomicAdd(&sh.nnear, 1);
       slot[nslot++] = s;
       if (s < kFitNear) sh.near_it[s] = it;
@@ -211,53 +258,88 @@ __device__ bool fit_eval(const FitGrid& g, FitShared& sh, int npts, unsigned& ph
   }
   __syncthreads();
   const int nnear = min(sh.nnear, kFitNear);
-  for (int e = (warp >> 2) * 32 + lane; e < nnear; e += 32 * ngrp) {
-    const int it = sh.near_it[e], q = it / g.nnz, b = g.bins[it - q * g.nnz];
-    const double lo = g.w * b + g.bmin, hi = g.w * (b + 1) + g.bmin;
-    sh.near_r[warp & 3][e] = gam_near_part(warp & 3, lo, hi - lo, g.mu, sh.pts[q]);
+  double fls = 0.0;   // the far series of the thread's first item
+  if (tid < own && first < nitems) {
+    const int q = first / g.nnz;
+    const FitBin B = g.geo[first - q * g.nnz];
+    if (gam_bin_far(B, sh.pts[q])) fls = gam_far_sum(B, sh.pts[q]);
+  }
+  if (warp == nw - 1 && lane < npts) {
+    FitPoint& P = sh.pts[lane];
+    const double lga = lgamma(P.tau);
+    P.lga = lga;
+    P.lconst = P.tau * log(P.lambda) - lga;
+  }
+  for (int c = 0; c * 32 < nnear; c++) {
+    const int role = (warp - 4 * c) & (nw - 1), e = c * 32 + lane;   // nw is 4 or 8
+    if (role < 1 || role > 3 || e >= nnear) continue;
+    const int it = sh.near_it[e], q = it / g.nnz;
+    const FitBin B = g.geo[it - q * g.nnz];
+    const FitPoint& P = sh.pts[q];
+    const double tau = P.tau;
+    if (role < 3) {
+      const double x = gam_near_x(B, role == 2, P);
+      sh.near_r[role - 1][e] = x > 0.0 ? gamma_q_sum(tau, x) : 0.0;
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < 2; k++) {
+        const double x = gam_near_x(B, k, P);
+        sh.near_r[2 + k][e] = x > 0.0 ? gamma_q_lpre(tau, x) : 0.0;
+      }
+    }
   }
   __syncthreads();
-  double acc[kFitMaxPts];
-#pragma unroll
-  for (int q = 0; q < kFitMaxPts; q++) acc[q] = 0.0;
+  if (nnear > 0) {   // Q at the bounds, in the warps that made the sums
+    for (int c = 0; c * 32 < nnear; c++) {
+      const int role = (warp - 4 * c) & (nw - 1), e = c * 32 + lane;
+      if (role < 1 || role > 2 || e >= nnear) continue;
+      const int it = sh.near_it[e], q = it / g.nnz;
+      const FitBin B = g.geo[it - q * g.nnz];
+      const FitPoint& P = sh.pts[q];
+      const double x = gam_near_x(B, role == 2, P);
+      sh.near_r[role - 1][e] =
+          x > 0.0 ? gamma_q_join(P.tau, x, sh.near_r[role - 1][e], sh.near_r[role + 1][e], P.lga) : 1.0;
+    }
+    __syncthreads();
+  }
   if (tid < own) {
+    double acc[kFitMaxPts];
+#pragma unroll
+    for (int q = 0; q < kFitMaxPts; q++) acc[q] = 0.0;
     int ns = 0;
     for (int it = first; it < nitems; it += T) {
       const int q = it / g.nnz, k = it - q * g.nnz;
-      const int b = g.bins[k];
-      const double lo = g.w * b + g.bmin, hi = g.w * (b + 1) + g.bmin, h = hi - lo;
+      const FitBin B = g.geo[k];
+      const FitPoint& P = sh.pts[q];
       double lp;
-      if (gam_bin_far(lo - g.mu, h, sh.pts[q])) {
-        lp = gam_logp_far(lo - g.mu, h, g.logx[k], sh.pts[q]);
+      if (gam_bin_far(B, P)) {
+        lp = gam_far_join(B, P, it == first ? fls : gam_far_sum(B, P));
       } else {
-        double r[4];
+        double ql, qu;
         const int s = ns < nslot ? slot[ns] : kFitNear;
         ns++;
         if (s < kFitNear) {
-#pragma unroll
-          for (int j = 0; j < 4; j++) r[j] = sh.near_r[j][s];
+          ql = sh.near_r[0][s];
+          qu = sh.near_r[1][s];
         } else {   // no room in the block's list
-#pragma unroll 1
-          for (int j = 0; j < 4; j++) r[j] = gam_near_part(j, lo, h, g.mu, sh.pts[q]);
+          ql = gamma_q_dev(P.tau, gam_near_x(B, false, P), P.lga);
+          qu = gamma_q_dev(P.tau, gam_near_x(B, true, P), P.lga);
         }
-        lp = gam_near_join(lo, h, g.mu, sh.pts[q], r);
+        lp = gam_near_join(ql, qu);
       }
       const double v = g.cnts[k] * lp;
 #pragma unroll
       for (int r = 0; r < kFitMaxPts; r++)
         if (q == r) acc[r] -= v;
     }
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int q = 0; q < kFitMaxPts; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < kFitMaxPts; q++) sh.red[warp * kFitMaxPts + q] = acc[q];
+    const double z = fold6(acc, lane);
+    const int q = fold_value(lane);
+    if (q >= 0) sh.red[warp * kFitMaxPts + q] = z;
   }
   __syncthreads();
   if (tid < npts) {
-    double t = 0.0;
-    for (int i = 0; i < nw; i++) t += sh.red[i * kFitMaxPts + tid];
+    double t = sh.red[tid];
+    for (int i = 1; i < now; i++) t += sh.red[i * kFitMaxPts + tid];
     part[tid * G + bid] = t;
   }
   __syncthreads();
@@ -279,43 +361,17 @@ __device__ bool fit_eval(const FitGrid& g, FitShared& sh, int npts, unsigned& ph
   if (tid < 32) {
     double t[kFitMaxPts];   // the points' sums side by side
 #pragma unroll
-    for (int q = 0; q < kFitMaxPts; q++) t[q] = 0.0;
-    for (int i = tid; i < G; i += 32)
+    for (int q = 0; q < kFitMaxPts; q++) t[q] = (q < npts && tid < G) ? __ldcg(part + q * G + tid) : 0.0;
+    for (int i = tid + 32; i < G; i += 32)
 #pragma unroll
       for (int q = 0; q < kFitMaxPts; q++) t[q] += q < npts ? __ldcg(part + q * G + i) : 0.0;
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int q = 0; q < kFitMaxPts; q++) t[q] += __shfl_xor_sync(0xffffffffu, t[q], o);
-    if (tid == 0)
-#pragma unroll
-      for (int q = 0; q < kFitMaxPts; q++)
-        if (q < npts) sh.F[q] = t[q];
+    const double z = fold6(t, lane);
+    const int q = fold_value(lane);
+    if (q >= 0 && q < npts) sh.F[q] = z;
   }
   __syncthreads();
   phase++;
   return true;
-}
-
-// thread 0 has written the n simplex coordinates sh.pc; they become likelihood
-// points, the rate's and the shape's parts in two warps
-__device__ __forceinline__ void fit_set_points(FitShared& sh, int n) {
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane < n && warp == 0) {
-    const double tau = exp(sh.pc[lane][1]);
-    sh.pts[lane].tau = tau;
-    sh.pts[lane].lga = lgamma(tau);
-  } else if (lane < n && warp == 1) {
-    const double lambda = exp(sh.pc[lane][0]);
-    sh.pts[lane].lambda = lambda;
-    sh.tmp[lane] = log(lambda);
-  }
-  __syncthreads();
-  if ((int)threadIdx.x < n) {
-    FitPoint& P = sh.pts[threadIdx.x];
-    P.lconst = P.tau * sh.tmp[threadIdx.x] - P.lga;
-  }
-  __syncthreads();
 }
 
 // The search.  Phase 1, Newton on theta = (log lambda, log tau): every round
@@ -338,11 +394,17 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
   {
     const int T = G * blockDim.x;
     for (int k = bid * blockDim.x + threadIdx.x; k < g.nnz; k += T) {
-      const double x = (g.w * g.bins[k] + g.bmin) - g.mu;
-      g.logx[k] = (x > 0.0) ? log(x) : 0.0;
+      const double lo = g.w * g.bins[k] + g.bmin, hi = g.w * (g.bins[k] + 1) + g.bmin, h = hi - lo;
+      FitBin B;
+      B.x = lo - g.mu;
+      B.h = h;
+      B.r = (B.x > 0.0 && h <= 0.0625 * B.x) ? h / B.x : -1.0;
+      B.logx = (B.x > 0.0) ? log(B.x) : 0.0;
+      B.x2 = (lo + h) - g.mu;
+      g.geo[k] = B;
     }
   }
-  // the bins' log x are read by other blocks' threads: a barrier round with
+  // the bins' geometry is read by other blocks' threads: a barrier round with
   // no points publishes them grid-wide
   unsigned phase = 0;
   int evals = 0, status = 0;
@@ -367,7 +429,6 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
       pc[4][0] = th0;     pc[4][1] = th1 - H;
       pc[5][0] = th0 + H; pc[5][1] = th1 + H;
     }
-    fit_set_points(sh, 6);
     if (!fit_eval(g, sh, 6, phase, own, G, bid)) { status = 2; break; }
     evals += 6;
     if (threadIdx.x < 32) {   // the five difference quotients, a lane each
@@ -434,7 +495,6 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
   const bool need_nm = !flag;
   __syncthreads();
   if (need_nm && !status) {
-    fit_set_points(sh, 3);
     if (!fit_eval(g, sh, 3, phase, own, G, bid)) status = 2;
     evals += 3;
     if (threadIdx.x == 0) for (int k = 0; k < 3; k++) SF[k] = F[k];
@@ -458,7 +518,6 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
       }
       __syncthreads();
       if (!ctl) break;
-      fit_set_points(sh, 3);
       if (!fit_eval(g, sh, 3, phase, own, G, bid)) { status = 2; break; }
       evals += 3;
       if (threadIdx.x == 0) {
@@ -484,7 +543,6 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
       }
       __syncthreads();
       if (ctl == 2) {
-        fit_set_points(sh, 2);
         if (!fit_eval(g, sh, 2, phase, own, G, bid)) { status = 2; break; }
         evals += 2;
         if (threadIdx.x == 0) {
@@ -510,7 +568,7 @@ __device__ __forceinline__ void gam_fit_body(const FitGrid& g, double s00, doubl
   }
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 k_gam_fit(FitGrid g, double s00, double s01, int own) {
   gam_fit_body(g, s00, s01, own, (int)gridDim.x, (int)blockIdx.x);
 }
@@ -526,7 +584,7 @@ k_gam_fit_grp(const FitGrid* __restrict__ gs, const double2* __restrict__ start)
 struct FitWork {
   int* d_bins = nullptr;
   double* d_cnts = nullptr;
-  double* d_logx = nullptr;
+  FitBin* d_geo = nullptr;
   int cap_bins = 0;
   double* d_part = nullptr;
   unsigned* d_bar = nullptr;
@@ -540,7 +598,7 @@ void fitwork_destroy(FitWork* fw) {
   if (!fw) return;
   if (fw->d_bins) cudaFree(fw->d_bins);
   if (fw->d_cnts) cudaFree(fw->d_cnts);
-  if (fw->d_logx) cudaFree(fw->d_logx);
+  if (fw->d_geo) cudaFree(fw->d_geo);
   if (fw->d_part) cudaFree(fw->d_part);
   if (fw->d_bar) cudaFree(fw->d_bar);
   if (fw->d_out) cudaFree(fw->d_out);
@@ -550,33 +608,93 @@ void fitwork_destroy(FitWork* fw) {
 
 // survfit[b] = mass * S(upper bound of bin b) for b in [cmin, 2 nb), 0 below
 // (cov_histogram_SetSurvFitTail, src/covariation.c:1676-1699)
+__device__ __forceinline__ double surv_bin(int b, int cmin, double bmin, double w, double mass, int doexp, double mu,
+                                           double lambda, double tau, double lga) {
+  if (b < cmin) return 0.0;
+  const double x = w * (b + 1) + bmin;
+  double S;
+  if (x <= mu) S = 1.0;
+  else if (doexp) S = exp(-lambda * (x - mu));
+  else S = gamma_q_dev(tau, lambda * (x - mu), lga);
+  return mass * S;
+}
 __global__ void k_survfit(int cmin, int nb, double bmin, double w, double mass, int doexp, double mu, double lambda,
                           double tau, double lga, double* __restrict__ sf) {
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < 2 * nb; b += gridDim.x * blockDim.x) {
-    double v = 0.0;
-    if (b >= cmin) {
-      const double x = w * (b + 1) + bmin;
-      double S;
-      if (x <= mu) S = 1.0;
-      else if (doexp) S = exp(-lambda * (x - mu));
-      else S = gamma_q_dev(tau, lambda * (x - mu), lga);
-      v = mass * S;
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < 2 * nb; b += gridDim.x * blockDim.x)
+    sf[b] = surv_bin(b, cmin, bmin, w, mass, doexp, mu, lambda, tau, lga);
+}
+
+// the gamma survival with two lanes to a bin, a warp to a block: the even
+// lane carries the fraction's C, the odd lane its 1/D, so that a step is one
+// division of the warp instead of two; the steps' factors -i (i - a) are the
+// same for every bin and come from a table.
+constexpr int kFracTab = 96;
+__global__ void __launch_bounds__(32)
+k_survfit_pair(int cmin, int nb, double bmin, double w, double mass, double mu, double lambda, double tau, double lga,
+               double* __restrict__ sf) {
+  __shared__ double tab[kFracTab];
+  const int lane = threadIdx.x, odd = lane & 1, bin = blockIdx.x * 16 + (lane >> 1);
+  for (int i = lane; i < kFracTab; i += 32) tab[i] = -(double)(i + 1) * ((double)(i + 1) - tau);
+  __syncwarp();
+  const double xb = w * (bin + 1) + bmin;
+  const double x = xb <= mu ? 0.0 : lambda * (xb - mu);
+  const bool in = bin >= cmin && bin < 2 * nb && x > 0.0, frac = in && !(x < tau + 1.0);
+  double sum = 0.0;
+  if (in && !frac) sum = gamma_q_sum(tau, x);
+  __syncwarp();
+  if (__any_sync(0xffffffffu, frac)) {
+    double b = x + 1.0 - tau;
+    double v = 1.0 / b, h = v;
+    if (!odd) v = 1.0 / 1e-300;
+    bool done = !frac;
+    for (int i = 1; i < 10000 && !__all_sync(0xffffffffu, done); i++) {
+      const double an = i <= kFracTab ? tab[i - 1] : -(double)i * ((double)i - tau);
+      b += 2.0;
+      const double t = __fma_rn(an, v, b);
+      double den = odd ? t : v;
+      const double num = odd ? 1.0 : an;
+      double q;
+      if (div_range(den) && (__double2hiint(num) & 0x7fffffff) < 0x46293e59) {
+        q = div_fast(num, den);
+      } else {
+        if (odd && fabs(den) < 1e-300) den = 1e-300;
+        q = num / den;
+      }
+      const double s = __dadd_rn(b, q);
+      v = odd ? q : s;
+      if (!odd && (__double2hiint(v) & 0x7fffffff) < 0x01a56e20 && fabs(v) < 1e-300) v = 1e-300;
+      const double del = __dmul_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+      const double hn = __dmul_rn(h, del);
+      if (!done) h = hn;
+      done = done || __double_as_longlong(del) == 0x3ff0000000000000ll;
     }
-    sf[b] = v;
+    if (frac) sum = h;
   }
+  if (bin >= 2 * nb || odd) return;
+  double S = 0.0;
+  if (bin >= cmin) S = mass * (x > 0.0 ? gamma_q_join(tau, x, sum, gamma_q_lpre(tau, x), lga) : 1.0);
+  sf[bin] = S;
 }
 
 cudaError_t launch_survfit(int cmin, int nb, double bmin, double w, double mass, int doexp, double mu, double lambda,
                            double tau, double* d_sf, cudaStream_t st) {
   const int n = 2 * nb;
-  // FP64 throughput is per SM: one warp per block until every SM has one (a
-  // table of ~3,000 bins in 12 blocks of 256 took 73-95 us)
   int dev = 0, nsm = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int thr = 32 * std::max(1, std::min(8, (n + 32 * nsm - 1) / (32 * nsm)));
-  k_survfit<<<std::max(1, std::min(1024, (n + thr - 1) / thr)), thr, 0, st>>>(cmin, nb, bmin, w, mass, doexp, mu, lambda,
-                                                                          tau, doexp ? 0.0 : std::lgamma(tau), d_sf);
+  const double lga = doexp ? 0.0 : std::lgamma(tau);
+  // The time is that of the warp with the most FP64 instructions (the bins
+  // next to x = tau + 1 take ~60 steps of the fraction, the others ~10): two
+  // lanes to a bin until the short warps, several to a scheduler, take as long
+  // as that one, then a lane each.  1,440 bins (30 x 61): 69 us a lane per bin
+  // with IEEE divisions, 57 us with div_fast, 47 us in pairs.
+  if (!doexp && n <= 64 * 4 * nsm) {
+    k_survfit_pair<<<std::max(1, (n + 15) / 16), 32, 0, st>>>(cmin, nb, bmin, w, mass, mu, lambda, tau, lga, d_sf);
+  } else {
+    const int thr = 32 * std::max(1, std::min(8, (n + 32 * nsm - 1) / (32 * nsm)));
+    k_survfit<<<std::max(1, std::min(1024, (n + thr - 1) / thr)), thr, 0, st>>>(cmin, nb, bmin, w, mass, doexp, mu,
+                                                                            lambda, tau, lga, d_sf);
+  }
   return cudaGetLastError();
 }
 
@@ -636,11 +754,11 @@ int gamma_fit_launch(FitWork* fwp, const uint64_t* h_obs, int cmin, int imax, do
   if (fw.cap_bins < nnz) {
     if (fw.d_bins) cudaFree(fw.d_bins);
     if (fw.d_cnts) cudaFree(fw.d_cnts);
-    if (fw.d_logx) cudaFree(fw.d_logx);
-    fw.d_bins = nullptr; fw.d_cnts = nullptr; fw.d_logx = nullptr; fw.cap_bins = 0;
+    if (fw.d_geo) cudaFree(fw.d_geo);
+    fw.d_bins = nullptr; fw.d_cnts = nullptr; fw.d_geo = nullptr; fw.cap_bins = 0;
     if (cudaMalloc(&fw.d_bins, sizeof(int) * nnz) != cudaSuccess) return 90;
     if (cudaMalloc(&fw.d_cnts, sizeof(double) * nnz) != cudaSuccess) return 90;
-    if (cudaMalloc(&fw.d_logx, sizeof(double) * nnz) != cudaSuccess) return 90;
+    if (cudaMalloc(&fw.d_geo, sizeof(FitBin) * nnz) != cudaSuccess) return 90;
     fw.cap_bins = nnz;
   }
   if (cudaMemcpyAsync(fw.d_bins, bins.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, st) != cudaSuccess) return 90;
@@ -648,7 +766,7 @@ int gamma_fit_launch(FitWork* fwp, const uint64_t* h_obs, int cmin, int imax, do
   if (cudaMemsetAsync(fw.d_bar, 0, sizeof(unsigned), st) != cudaSuccess) return 90;
 
   FitGrid g;
-  g.bins = fw.d_bins; g.cnts = fw.d_cnts; g.logx = fw.d_logx; g.nnz = nnz;
+  g.bins = fw.d_bins; g.cnts = fw.d_cnts; g.geo = fw.d_geo; g.nnz = nnz;
   g.bmin = bmin; g.w = w; g.mu = mu;
   g.part = fw.d_part; g.bar = fw.d_bar; g.out = fw.d_out;
   int own = 0;
@@ -658,8 +776,8 @@ int gamma_fit_launch(FitWork* fwp, const uint64_t* h_obs, int cmin, int imax, do
   const int W = std::max(1, std::min(8, (nitems + 32 * fw.max_grid - 1) / (32 * fw.max_grid)));
   const int G = std::max(1, std::min(fw.max_grid, (nitems + 32 * W - 1) / (32 * W)));
   own = 32 * W;
-  // at least four warps, a multiple of four, for the parts of the bins near mu
-  if (cudaLaunchCooperativeKernel((const void*)k_gam_fit, dim3(G), dim3((own + 127) / 128 * 128), args, 0, st) !=
+  // four or eight warps, for the independent parts of an evaluation
+  if (cudaLaunchCooperativeKernel((const void*)k_gam_fit, dim3(G), dim3(own > 128 ? 256 : 128), args, 0, st) !=
       cudaSuccess)
     return 90;
   if (cudaMemcpyAsync(fw.h_out, fw.d_out, sizeof(FitOut), cudaMemcpyDeviceToHost, st) != cudaSuccess) return 90;
@@ -689,7 +807,7 @@ struct FitBatch {
   double2* d_start = nullptr;
   int* d_bins = nullptr;
   double* d_cnts = nullptr;
-  double* d_logx = nullptr;
+  FitBin* d_geo = nullptr;
   double* d_part = nullptr;
   unsigned* d_bar = nullptr;
   FitOut* d_out = nullptr;
@@ -702,7 +820,7 @@ struct FitBatch {
 FitBatch* fitbatch_create() { return new FitBatch(); }
 void fitbatch_destroy(FitBatch* fb) {
   if (!fb) return;
-  void* p[] = {fb->d_grid, fb->d_start, fb->d_bins, fb->d_cnts, fb->d_logx, fb->d_part, fb->d_bar, fb->d_out};
+  void* p[] = {fb->d_grid, fb->d_start, fb->d_bins, fb->d_cnts, fb->d_geo, fb->d_part, fb->d_bar, fb->d_out};
   for (void* x : p) if (x) cudaFree(x);
   if (fb->h_out) cudaFreeHost(fb->h_out);
   delete fb;
@@ -757,12 +875,12 @@ int gamma_fit_batch_launch(FitBatch* fb, int nfit, const FitReq* req, cudaStream
   if (fb->cap_bins < nb) {
     if (fb->d_bins) cudaFree(fb->d_bins);
     if (fb->d_cnts) cudaFree(fb->d_cnts);
-    if (fb->d_logx) cudaFree(fb->d_logx);
-    fb->d_bins = nullptr; fb->d_cnts = nullptr; fb->d_logx = nullptr; fb->cap_bins = 0;
+    if (fb->d_geo) cudaFree(fb->d_geo);
+    fb->d_bins = nullptr; fb->d_cnts = nullptr; fb->d_geo = nullptr; fb->cap_bins = 0;
     const int cap = std::max(nb, 4096);
     if (cudaMalloc(&fb->d_bins, sizeof(int) * cap) != cudaSuccess ||
         cudaMalloc(&fb->d_cnts, sizeof(double) * cap) != cudaSuccess ||
-        cudaMalloc(&fb->d_logx, sizeof(double) * cap) != cudaSuccess)
+        cudaMalloc(&fb->d_geo, sizeof(FitBin) * cap) != cudaSuccess)
       return 90;
     fb->cap_bins = cap;
   }
@@ -771,7 +889,7 @@ int gamma_fit_batch_launch(FitBatch* fb, int nfit, const FitReq* req, cudaStream
     const int e = fb->slot[k];
     if (e < 0) continue;
     FitGrid& g = grid[e];
-    g.bins = fb->d_bins + boff[e]; g.cnts = fb->d_cnts + boff[e]; g.logx = fb->d_logx + boff[e];
+    g.bins = fb->d_bins + boff[e]; g.cnts = fb->d_cnts + boff[e]; g.geo = fb->d_geo + boff[e];
     g.nnz = boff[e + 1] - boff[e];
     g.bmin = req[k].bmin; g.w = req[k].w; g.mu = req[k].phi;
     g.part = fb->d_part + (size_t)e * 2 * kFitMaxPts;
@@ -805,16 +923,7 @@ __global__ void k_survfit_grp(const SurvReq* __restrict__ r, const int* __restri
   const SurvReq& q = r[e];
   const int b = ((int)blockIdx.x - __ldg(pre + e)) * blockDim.x + threadIdx.x;
   if (b >= 2 * q.nb) return;
-  double v = 0.0;
-  if (b >= q.cmin) {
-    const double x = q.w * (b + 1) + q.bmin;
-    double S;
-    if (x <= q.mu) S = 1.0;
-    else if (q.doexp) S = exp(-q.lambda * (x - q.mu));
-    else S = gamma_q_dev(q.tau, q.lambda * (x - q.mu), q.lga);
-    v = q.mass * S;
-  }
-  q.sf[b] = v;
+  q.sf[b] = surv_bin(b, q.cmin, q.bmin, q.w, q.mass, q.doexp, q.mu, q.lambda, q.tau, q.lga);
 }
 
 cudaError_t grp_survfit(const SurvReq* d_req, const int* pre, int nr, int nb, cudaStream_t st) {

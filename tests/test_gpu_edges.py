@@ -197,3 +197,30 @@ def test_plain_counts_at_chunk_edges(covgpu, oracle, N, L, weights):
     for a, b in zip(*got):
         assert np.array_equal(a, b)
     assert np.allclose(got[0][4], oracle.probs(ax, w)[4], rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.parametrize("w0", [0.05, 0.002, 0.0004])
+@pytest.mark.parametrize("doexp", [0, 1])
+def test_survival_tables(covgpu, oracle, w0, doexp):
+    """E-values read from survival tables of hundreds to ~10^5 bins, two lanes
+    or one to a bin, on the grid and in a batch: the oracle's within 1e-4, as
+    in the pipeline's parity tests."""
+    s = covgpu.Synth(60, 100, 1.5, 16, 2, 4, 14, 0.08, seed=7)
+    w = covgpu.weights_pb(s.ax)
+    kw = dict(nshuffle=8, thresh=10.0, w0=w0, doexpfit=doexp)
+    e = covgpu.Engine(60, 100, maxslots=9, maxnull=8)
+    e.set_tree(s.parent, s.left, s.right)
+    one = e.rscape(s.ax, w, ["GTp"], counter=covgpu.TENSOR, **kw)[0]
+    e.close()
+    b = covgpu.Batch()
+    grp = b.rscape([dict(ax=s.ax, parent=s.parent, left=s.left, right=s.right, wgt=w)], ["GTp"],
+                   counter=covgpu.TENSOR, **kw)[0][0]
+    b.close()
+    ref = oracle.rscape(s.ax, w, oracle.TreeArrays(s.parent, s.left, s.right, s.ld, s.rd), covtype="GTp", **kw)
+    rh = {(i, j): E for (i, j, sc, E, p) in ref["hits"]}
+    assert len(rh) >= 5
+    for r in (one, grp):
+        gh = {(i, j): E for (i, j, sc, E, p) in r["hits"]}
+        assert set(gh) == set(rh)
+        for k in rh:
+            assert abs(gh[k] - rh[k]) <= 1e-4 * rh[k] + 1e-300, (k, gh[k], rh[k])
