@@ -71,11 +71,17 @@ __global__ void __launch_bounds__(256) k_feat_cols(const uint8_t* __restrict__ a
   const double wtot = *pwtot;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
+  // one FP64 addition a row, to the code's sum chosen by selects (29 us with
+  // the sums indexed in local memory, 20 us so at 400 x 300)
   double n[4] = {0.0, 0.0, 0.0, 0.0};
   if (c < L)
+#pragma unroll 4
     for (int s = wp; s < N; s += 8) {
       const int x = ax[(int64_t)s * Lp + c];
-      if (x < 4) n[x] += w[s];
+      const double a = ((x & 2) ? ((x & 1) ? n[3] : n[2]) : ((x & 1) ? n[1] : n[0])) + w[s];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (x == k) n[k] = a;
     }
   for (int x = 0; x < 4; x++) part[wp][x][lane] = n[x];
   __syncthreads();
@@ -163,69 +169,90 @@ __device__ double block_sum(double v, double* sh) {
   return r;
 }
 
+// K such sums side by side: sh[k][0] is the sum of v[k], in block_sum's order
+template <int K>
+__device__ void block_sums(const double (&v)[K], double (*sh)[1024]) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < K; k++) sh[k][t] = v[k];
+  __syncthreads();
+  for (int s = blockDim.x >> 1; s; s >>= 1) {
+    for (int e = t; e < K * s; e += blockDim.x) {
+      const int k = e / s, i = e - k * s;
+      sh[k][i] += sh[k][i + s];
+    }
+    __syncthreads();
+  }
+}
+
+// One block.  Its time is the FP64 instructions of its schedulers (a warp's
+// takes one ~64 cycles), so the sums fold side by side, and the quotients,
+// logarithms and roots are lanes of one instruction instead of every warp's
+// (the means) or one thread's (the rest): 73 us, 23 us so at 400 x 300.
 __global__ void __launch_bounds__(1024) k_feat_final(const double* __restrict__ col, const double* __restrict__ id,
                                                      const double* __restrict__ w, int N, int L, int M,
                                                      double tree_len, float* __restrict__ feat) {
-  __shared__ double sh[1024];
+  __shared__ double sh[5][1024];
+  __shared__ double tot[9], mean[4], var[4];   // means and variances of the weights, entropies, gaps, identities
   __shared__ int hist[2][16];
   const int t = threadIdx.x, nt = blockDim.x;
   if (t < 32) hist[t / 16][t % 16] = 0;
   __syncthreads();
-  // weights
-  double a = 0.0, b = 0.0;
-  for (int s = t; s < N; s += nt) { a += w[s]; b += w[s] * w[s]; }
-  const double sw = block_sum(a, sh), sw2 = block_sum(b, sh);
-  const double wmean = sw / N;
-  a = 0.0;
-  for (int s = t; s < N; s += nt) a += (w[s] - wmean) * (w[s] - wmean);
-  const double wvar = block_sum(a, sh) / N;
-  // columns
-  double sH = 0.0, sg = 0.0, sn[4] = {0.0, 0.0, 0.0, 0.0};
+  double v[4] = {0.0, 0.0, 0.0, 0.0}, u[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int s = t; s < N; s += nt) { v[0] += w[s]; v[1] += w[s] * w[s]; }
+  for (int k = t; k < M; k += nt) v[2] += id[k];
   for (int c = t; c < L; c += nt) {
     const double* o = col + (int64_t)c * kColStat;
-    sH += o[0]; sg += o[1];
-    for (int x = 0; x < 4; x++) sn[x] += o[2 + x];
+    v[3] += o[0]; u[4] += o[1];
+    for (int x = 0; x < 4; x++) u[x] += o[2 + x];
     atomicAdd(&hist[0][bin16(o[0], 8.0)], 1);
     atomicAdd(&hist[1][bin16(o[1], 16.0)], 1);
   }
-  const double mH = block_sum(sH, sh) / L, mg = block_sum(sg, sh) / L;
-  double comp[4];
-  for (int x = 0; x < 4; x++) comp[x] = block_sum(sn[x], sh);
-  a = 0.0; b = 0.0;
+  block_sums(v, sh);
+  if (t < 4) tot[t] = sh[t][0];   // weights, their squares, identities, entropies
+  __syncthreads();
+  block_sums(u, sh);
+  if (t < 5) tot[4 + t] = sh[t][0];   // four codes, gaps
+  __syncthreads();
+  const double den = (t == 0) ? (double)N : (t == 3) ? (double)M : (double)L;
+  if (t < 4) mean[t] = (t == 3 && !M) ? tot[2] : tot[t == 0 ? 0 : t == 1 ? 3 : t == 2 ? 8 : 2] / den;
+  __syncthreads();
+  for (int k = 0; k < 4; k++) v[k] = 0.0;
+  for (int s = t; s < N; s += nt) v[0] += (w[s] - mean[0]) * (w[s] - mean[0]);
   for (int c = t; c < L; c += nt) {
     const double* o = col + (int64_t)c * kColStat;
-    a += (o[0] - mH) * (o[0] - mH);
-    b += (o[1] - mg) * (o[1] - mg);
+    v[1] += (o[0] - mean[1]) * (o[0] - mean[1]);
+    v[2] += (o[1] - mean[2]) * (o[1] - mean[2]);
   }
-  const double vH = block_sum(a, sh) / L, vg = block_sum(b, sh) / L;
-  // identities
-  a = 0.0;
-  for (int k = t; k < M; k += nt) a += id[k];
-  const double mid = M ? block_sum(a, sh) / M : block_sum(0.0, sh);
-  a = 0.0;
-  for (int k = t; k < M; k += nt) a += (id[k] - mid) * (id[k] - mid);
-  const double vid = M ? block_sum(a, sh) / M : block_sum(0.0, sh);
+  for (int k = t; k < M; k += nt) v[3] += (id[k] - mean[3]) * (id[k] - mean[3]);
+  block_sums(v, sh);
+  if (t < 4) var[t] = (t == 3 && !M) ? sh[3][0] : sh[t][0] / den;
   __syncthreads();
-  if (t == 0) {
-    const double rtot = (comp[0] + comp[1]) + (comp[2] + comp[3]);
-    double f[5], g[10];
-    f[0] = log((double)N);
-    f[1] = log((double)L);
-    f[2] = sw2 > 0.0 ? log(sw * sw / sw2) : 0.0;
-    f[3] = mid;
-    f[4] = tree_len;
-    g[0] = sqrt(vid);
-    g[1] = mH;
-    g[2] = sqrt(vH);
-    g[3] = mg;
-    g[4] = sqrt(vg);
-    g[5] = wmean > 0.0 ? sqrt(wvar) / wmean : 0.0;
-    for (int x = 0; x < 4; x++) g[6 + x] = rtot > 0.0 ? comp[x] / rtot : 0.0;
-    for (int k = 0; k < 5; k++) feat[k] = (float)f[k];
-    for (int k = 0; k < 10; k++) feat[37 + k] = (float)g[k];
+  if (t < 32) {
+    const double sw = tot[0], sw2 = tot[1], rtot = (tot[4] + tot[5]) + (tot[6] + tot[7]);
+    // a quotient: lane 2 the effective number of sequences, lanes 8..11 the composition
+    const bool comp = t >= 8 && t < 12;
+    const double num = comp ? tot[t - 4] : sw * sw, dn = comp ? rtot : sw2;
+    const double q = dn > 0.0 ? num / dn : 0.0;
+    // logarithms (lanes 0..2), roots (lanes 4..7), the weights' root over their mean
+    double f = 0.0;
+    if (t < 3) f = log(t == 0 ? (double)N : t == 1 ? (double)L : q);
+    else if (t >= 4 && t < 8) f = sqrt(var[t - 4]);
+    if (t == 4) f = mean[0] > 0.0 ? f / mean[0] : 0.0;
+    if (t < 2) feat[t] = (float)f;
+    if (t == 2) feat[2] = sw2 > 0.0 ? (float)f : 0.f;
+    if (t == 3) { feat[3] = (float)mean[3]; feat[4] = (float)tree_len; feat[38] = (float)mean[1]; feat[40] = (float)mean[2]; }
+    if (t == 4) feat[42] = (float)f;
+    if (t == 5) feat[39] = (float)f;
+    if (t == 6) feat[41] = (float)f;
+    if (t == 7) feat[37] = (float)f;
+    if (comp) feat[43 + t - 8] = (float)q;
+  } else if (t < 64) {
+    const int e = t - 32;
+    feat[5 + e] = (float)((double)hist[e / 16][e % 16] / (double)L);
+  } else if (t < 128 && t - 64 + 47 < kNFeat) {
+    feat[t - 64 + 47] = 0.f;
   }
-  if (t < 32) feat[5 + t] = (float)((double)hist[t / 16][t % 16] / (double)L);
-  if (t >= 47 && t < kNFeat) feat[t] = 0.f;
 }
 
 __global__ void __launch_bounds__(1024) k_feat_wtot(const double* __restrict__ w, int N, double* __restrict__ out) {
@@ -262,6 +289,10 @@ constexpr int kHid = 256, kOut = 3;
 constexpr int oW1 = 0, ob1 = oW1 + kHid * kNFeat, oW2 = ob1 + kHid, ob2 = oW2 + kHid * kHid, oW3 = ob2 + kHid,
               ob3 = oW3 + kHid * kHid, oW4 = ob3 + kHid, ob4 = oW4 + kOut * kHid, kNParam = ob4 + kOut;
 static_assert(kNParam == COVGPU_MLP_NPARAM, "parameter layout");
+// a member's BF16 parameters start on a 16-byte boundary, and so does each of
+// its layers' weights
+constexpr int kPBStride = (kNParam + 7) / 8 * 8;
+static_assert(oW1 % 8 == 0 && oW2 % 8 == 0 && oW3 % 8 == 0 && oW4 % 8 == 0, "16-byte loads of the weights");
 
 __device__ __forceinline__ float ld_f(const float* p) { return *p; }
 __device__ __forceinline__ float ld_f(const __nv_bfloat16* p) { return __bfloat162float(*p); }
@@ -332,6 +363,84 @@ static void gemm(cudaStream_t st, const TA* A, int sam, int sak, const TB* B, in
                  const float* bias, const float* aux, float* C, float* C2 = nullptr) {
   const dim3 grid((Nc + 63) / 64, (M + 63) / 64);
   k_gemm<TA, TB, EPI><<<grid, 256, 0, st>>>(A, sam, sak, B, sbk, sbn, M, Nc, K, bias, aux, C, C2);
+}
+
+// One row through one member's whole network, a CTA each, a thread per hidden
+// unit: the unit's weights come to registers a layer ahead (they do not wait
+// for the activations), the activations are read from shared memory, and the
+// sums run over k in k_gemm's order, so the outputs have its bits.  A row of a
+// member through the four k_gemm launches took 94 us, nearly all of it the
+// latency of 64 small steps; 15 us so for one row of four members in one launch.
+//   Ym[member][row][kOut], not standardised back
+__device__ __forceinline__ float mlp_fma8(const uint4& w, const float* __restrict__ h, float acc) {
+  const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int e = 0; e < 4; e++) {   // two BF16 weights a word, the lower first
+    acc = fmaf(h[2 * e], __uint_as_float(v[e] << 16), acc);
+    acc = fmaf(h[2 * e + 1], __uint_as_float(v[e] & 0xffff0000u), acc);
+  }
+  return acc;
+}
+__device__ __forceinline__ float mlp_silu(float acc, float bias) {
+  const float z = acc + bias;
+  return z * sigm(z);
+}
+__global__ void __launch_bounds__(kHid) k_mlp_rows(const float* __restrict__ X, const float* __restrict__ nrm,
+                                                   const float* __restrict__ P, const __nv_bfloat16* __restrict__ PB,
+                                                   int nrow, float* __restrict__ Ym) {
+  constexpr int W1 = kNFeat / 8, W2 = kHid / 8;
+  __shared__ __align__(16) float x[kNFeat], ha[kHid], hb[kHid], w4[kOut][kHid];
+  const int row = blockIdx.x, mem = blockIdx.y, n = threadIdx.x;
+  const float* p = P + (size_t)mem * kNParam;
+  const __nv_bfloat16* pb = PB + (size_t)mem * kPBStride;
+  auto row8 = [&](int off, int K, int j) {
+    return __ldg(reinterpret_cast<const uint4*>(pb + off + (size_t)n * K + 8 * j));
+  };
+  uint4 w1[W1], w[W2];
+#pragma unroll
+  for (int j = 0; j < W1; j++) w1[j] = row8(oW1, kNFeat, j);
+#pragma unroll
+  for (int j = 0; j < W2; j++) w[j] = row8(oW2, kHid, j);
+  const float b1 = p[ob1 + n], b2 = p[ob2 + n], b3 = p[ob3 + n];
+#pragma unroll
+  for (int o = 0; o < kOut; o++) w4[o][n] = __bfloat162float(pb[oW4 + o * kHid + n]);
+  if (n < kNFeat) x[n] = (X[(int64_t)row * kNFeat + n] - nrm[n]) / nrm[kNFeat + n];
+  __syncthreads();
+  float acc = 0.f;
+#pragma unroll
+  for (int j = 0; j < W1; j++) acc = mlp_fma8(w1[j], x + 8 * j, acc);
+  ha[n] = mlp_silu(acc, b1);
+  __syncthreads();
+  acc = 0.f;
+#pragma unroll
+  for (int j = 0; j < W2; j++) {
+    acc = mlp_fma8(w[j], ha + 8 * j, acc);
+    w[j] = row8(oW3, kHid, j);
+  }
+  hb[n] = mlp_silu(acc, b2);
+  __syncthreads();
+  acc = 0.f;
+#pragma unroll
+  for (int j = 0; j < W2; j++) acc = mlp_fma8(w[j], hb + 8 * j, acc);
+  ha[n] = mlp_silu(acc, b3);
+  __syncthreads();
+  if (n < kOut) {
+    acc = 0.f;
+#pragma unroll 16
+    for (int k = 0; k < kHid; k++) acc = fmaf(ha[k], w4[n][k], acc);
+    Ym[((size_t)mem * nrow + row) * kOut + n] = acc + p[ob4 + n];
+  }
+}
+
+// the members' outputs summed in member order, averaged and standardised back
+__global__ void k_mlp_mean(const float* __restrict__ Ym, int n, int nmem, const float* __restrict__ nrm, float scale,
+                           float* __restrict__ Y) {
+  const float *ym = nrm + 2 * kNFeat, *ys = ym + kOut;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n * kOut) return;
+  float y = Ym[e];
+  for (int k = 1; k < nmem; k++) y = y + Ym[(size_t)k * n * kOut + e];
+  Y[e] = (y * scale) * ys[e % kOut] + ym[e % kOut];
 }
 
 // out[o] = sum_b G[b][o], b in order
@@ -433,6 +542,11 @@ __global__ void k_to_bf16(const float* __restrict__ p, __nv_bfloat16* __restrict
 
 using namespace covgpu;
 
+// up to so many rows a CTA per row and member (k_mlp_rows), above them the
+// layers as products: with four members 39 against 379 us for one row, 216
+// against 526 for 512, 379 against 529 for 1024, 543 against 528 for 1536
+constexpr int kMlpRows = 1024;
+
 struct covgpu_mlp {
   int dev = 0;
   cudaStream_t st = nullptr;
@@ -451,7 +565,7 @@ struct covgpu_mlp {
   int nmem = 0;
   float* mp = nullptr;
   __nv_bfloat16* mpb = nullptr;
-  float* Yacc = nullptr;
+  float* Yacc = nullptr;  // their outputs [members][rows][kOut]
 };
 
 static int mfail(covgpu_mlp* net, int code, const char* fmt, ...) {
@@ -590,9 +704,12 @@ extern "C" int covgpu_mlp_set_members(covgpu_mlp* net, const float* params, int 
   net->mp = nullptr; net->mpb = nullptr; net->Yacc = nullptr; net->nmem = 0;
   if (nmem == 0) return 0;
   const size_t n = (size_t)nmem * kNParam;
-  MCK(malloc_n(&net->mp, n)); MCK(malloc_n(&net->mpb, n)); MCK(malloc_n(&net->Yacc, (size_t)net->cap * kOut));
+  MCK(malloc_n(&net->mp, n)); MCK(malloc_n(&net->mpb, (size_t)nmem * kPBStride));
+  MCK(malloc_n(&net->Yacc, (size_t)std::max(net->cap, nmem * std::min(net->cap, kMlpRows)) * kOut));
   MCK(cudaMemcpyAsync(net->mp, params, n * sizeof(float), cudaMemcpyHostToDevice, net->st));
-  k_to_bf16<<<(int)((n + 255) / 256), 256, 0, net->st>>>(net->mp, net->mpb, (int)n);
+  for (int k = 0; k < nmem; k++)
+    k_to_bf16<<<(kNParam + 255) / 256, 256, 0, net->st>>>(net->mp + (size_t)k * kNParam,
+                                                          net->mpb + (size_t)k * kPBStride, kNParam);
   MCK(cudaGetLastError());
   MCK(cudaStreamSynchronize(net->st));
   net->nmem = nmem;
@@ -658,14 +775,23 @@ extern "C" int covgpu_mlp_forward(covgpu_mlp* net, const float* X, int n, float*
     const int B = std::min(net->cap, n - r0);
     MCK(cudaMemcpyAsync(net->Xin, X + (size_t)r0 * kNFeat, (size_t)B * kNFeat * sizeof(float),
                         cudaMemcpyHostToDevice, net->st));
-    k_gather<<<std::min(1024, (B * kNFeat + 255) / 256), 256, 0, net->st>>>(net->Xin, nullptr, nullptr, nullptr, 1,
-                                                                            B, net->nrm, net->Xb, nullptr);
-    if (net->nmem == 0) {
+    const bool rows = B <= kMlpRows;
+    if (!rows)
+      k_gather<<<std::min(1024, (B * kNFeat + 255) / 256), 256, 0, net->st>>>(net->Xin, nullptr, nullptr, nullptr, 1,
+                                                                              B, net->nrm, net->Xb, nullptr);
+    if (rows) {
+      const bool ens = net->nmem > 0;
+      const int nm = ens ? net->nmem : 1;
+      float* ym = ens ? net->Yacc : net->Yp;
+      k_mlp_rows<<<dim3(B, nm), kHid, 0, net->st>>>(net->Xin, net->nrm, ens ? net->mp : net->p,
+                                                    ens ? net->mpb : net->pb, B, ym);
+      k_mlp_mean<<<(B * kOut + 255) / 256, 256, 0, net->st>>>(ym, B, nm, net->nrm, 1.f / (float)nm, net->Yout);
+    } else if (net->nmem == 0) {
       enqueue_forward(net, B);
       k_denorm<<<(B * kOut + 255) / 256, 256, 0, net->st>>>(net->Yp, B, net->nrm, 1.f, net->Yout);
     } else {
       for (int k = 0; k < net->nmem; k++) {
-        enqueue_forward(net, B, net->mp + (size_t)k * kNParam, net->mpb + (size_t)k * kNParam);
+        enqueue_forward(net, B, net->mp + (size_t)k * kNParam, net->mpb + (size_t)k * kPBStride);
         k_accum<<<(B * kOut + 255) / 256, 256, 0, net->st>>>(net->Yp, B * kOut, k == 0, net->Yacc);
       }
       k_denorm<<<(B * kOut + 255) / 256, 256, 0, net->st>>>(net->Yacc, B, net->nrm, 1.f / (float)net->nmem,

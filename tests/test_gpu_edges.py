@@ -224,3 +224,19 @@ def test_survival_tables(covgpu, oracle, w0, doexp):
         assert set(gh) == set(rh)
         for k in rh:
             assert abs(gh[k] - rh[k]) <= 1e-4 * rh[k] + 1e-300, (k, gh[k], rh[k])
+
+
+@pytest.mark.parametrize("members", [0, 1, 3])
+def test_network_rows_equal_products(covgpu, members):
+    """The forward pass by rows (up to 1024 rows) gives the bits of the layers'
+    products (more rows)."""
+    rng = np.random.default_rng(members)
+    net = covgpu.MLP(batch_cap=2048)
+    p = net.params()
+    if members:
+        net.set_members(np.stack([p + 0.02 * rng.normal(size=p.shape).astype(np.float32) for _ in range(members)]))
+    X = rng.normal(size=(1025, 64)).astype(np.float32)
+    Y = net.forward(X)
+    for n in (1, 2, 1024):
+        assert np.array_equal(net.forward(X[:n]), Y[:n]), n
+    net.close()
