@@ -240,3 +240,17 @@ def test_network_rows_equal_products(covgpu, members):
     for n in (1, 2, 1024):
         assert np.array_equal(net.forward(X[:n]), Y[:n]), n
     net.close()
+
+
+@pytest.mark.parametrize("copies", [1, 3, 25, 70, 160])
+def test_batch_fit_does_not_depend_on_its_cluster(covgpu, copies):
+    """One family many times in a batch: clusters of eight, eight, six and two
+    blocks per fit and one block; lambda and tau keep their bits."""
+    s = covgpu.Synth(40, 60, 1.5, 9, 1, 4, 14, 0.08, seed=3)
+    fam = dict(ax=s.ax, parent=s.parent, left=s.left, right=s.right)
+    b = covgpu.Batch()
+    want = b.rscape([fam, fam], ["GTp"], counter=covgpu.TENSOR, nshuffle=20)[0][0]
+    for rows in b.rscape([fam] * copies, ["GTp"], counter=covgpu.TENSOR, nshuffle=20):
+        for k in ("lambda_", "tau", "sc_thresh", "nhit"):
+            assert rows[0][k] == want[k], k
+    b.close()
