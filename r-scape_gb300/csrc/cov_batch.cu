@@ -630,7 +630,7 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
   Pre pt3 = prefix(nf, [&](int k) { return (fams[k].tens && Lo.F[k].nl == 3) ? fams[k].ntiles * fams[k].nslots : 0; });
   Pre pt1 = prefix(nf, [&](int k) { return (fams[k].tens && Lo.F[k].nl == 1) ? fams[k].ntiles * fams[k].nslots : 0; });
   Pre psimt = prefix(nf, [&](int k) { return fams[k].tens ? 0 : fams[k].ntiles * fams[k].nslots; });
-  Pre ppm = prefix(nf, [&](int k) { return (fams[k].L + 127) / 128 * fams[k].nslots; });
+  Pre ppm = prefix(nf, [&](int k) { return (fams[k].L + 31) / 32 * fams[k].nslots; });
   Pre pmp = prefix(nf, [&](int k) { return fams[k].nslots; });
   Pre pcx = prefix(nf, [&](int k) { return (fams[k].L + 255) / 256 * fams[k].nslots * nout; });
   Pre psq = prefix(nf, [&](int k) { return fams[k].nslots * nout; });

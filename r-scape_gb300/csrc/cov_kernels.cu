@@ -415,40 +415,52 @@ k_pair_marg(const float* __restrict__ cnt, int L, const TileRC* __restrict__ til
 }
 
 // pm[c][x] = normalise(sum over every tile touching column c); one thread
-// per column.  pmdf is pm as a double-float; lpi[c][x] = {ln pm, 1/pm} as
-// double-floats (FP64 log and division, 0 where pm = 0) for the pair
-// statistics.  mpc[c][x] = pm[c][x] * (sum_{j>c} nseff[c][j]) feeds the CCF
-// column means (src/correlators.c:1030-1036).
+// per (column, state), 32 columns to a block, and one more warp for the
+// columns' sums of nseff.  pmdf is pm as a double-float;
+// lpi[c][x] = {ln pm, 1/pm} as double-floats (FP64 log and division, 0 where
+// pm = 0) for the pair statistics.  mpc[c][x] = pm[c][x] * (sum_{j>c}
+// nseff[c][j]) feeds the CCF column means (src/correlators.c:1030-1036).
+// Bound by FP64 instructions (a warp's takes one ~64 cycles): a thread per
+// column that made all four states' quotients and logarithms took 11.3 us at
+// 30 x 61 x 201 and 69 us at 500 x 400 x 201, now 6.3 and 56 us.
 __device__ __forceinline__ void pm_final_body(
     const GridIdx g, const double* __restrict__ part4, const double* __restrict__ partR, int L, int Lp, int nT,
                            double* __restrict__ pm, float2* __restrict__ pmdf, float4* __restrict__ lpi,
                            double* __restrict__ mpc, int* __restrict__ status) {
-  const int slot = g.y;
-  const int c = g.x * blockDim.x + threadIdx.x;
-  if (c >= L) return;
+  __shared__ double rsum[32];
+  const bool rows = threadIdx.x >= 128;   // the fifth warp
+  const int slot = g.y, x = threadIdx.x & 3, cl = rows ? (int)threadIdx.x - 128 : (int)threadIdx.x >> 2;
+  const int c = g.x * 32 + cl;
+  const bool in = c < L;
   const double* P = part4 + (int64_t)slot * nT * nT * TP * 4;
   const double* R = partR + (int64_t)slot * nT * nT * TP;
   const int I = c / TP, a = c % TP;
-  double m[4] = {0, 0, 0, 0}, rs = 0.0;
-  for (int K = 0; K < nT; K++) {
-    const double2* v = reinterpret_cast<const double2*>(P + (((int64_t)I * nT + K) * TP + a) * 4);
-    const double2 v0 = v[0], v1 = v[1];
-    m[0] += v0.x; m[1] += v0.y; m[2] += v1.x; m[3] += v1.y;
-    rs += R[((int64_t)I * nT + K) * TP + a];
+  double m = 0.0;
+  if (in) {
+    const double* v = rows ? R : P + x;
+    const int step = rows ? 1 : 4;
+#pragma unroll 4
+    for (int K = 0; K < nT; K++) m += v[(((int64_t)I * nT + K) * TP + a) * step];
   }
-  const double sum = m[0] + m[1] + m[2] + m[3];
-#pragma unroll
-  for (int x = 0; x < 4; x++) m[x] = (sum != 0.0) ? m[x] / sum : 0.25;
-  if (fabs(m[0] + m[1] + m[2] + m[3] - 1.0) > 1e-6) atomicExch(status, 2);
-#pragma unroll
-  for (int x = 0; x < 4; x++) {
-    const int64_t o = ((int64_t)slot * Lp + c) * 4 + x;
-    pm[o] = m[x];
-    st_df(pmdf + o, df_of(m[x]));
-    const df l = df_of(m[x] > 0.0 ? log(m[x]) : 0.0), r = df_of(m[x] > 0.0 ? 1.0 / m[x] : 0.0);
-    lpi[o] = make_float4(l.hi, l.lo, r.hi, r.lo);
-    mpc[o] = rs * m[x];
-  }
+  if (rows) rsum[cl] = m;
+  __syncthreads();
+  if (rows) return;
+  const int l0 = threadIdx.x & 28;
+  auto sum4 = [l0](double v) {
+    return __shfl_sync(0xffffffffu, v, l0) + __shfl_sync(0xffffffffu, v, l0 + 1) +
+           __shfl_sync(0xffffffffu, v, l0 + 2) + __shfl_sync(0xffffffffu, v, l0 + 3);
+  };
+  const double sum = sum4(m);
+  m = (sum != 0.0) ? m / sum : 0.25;
+  const double one = sum4(m);
+  if (!in) return;
+  if (x == 0 && fabs(one - 1.0) > 1e-6) atomicExch(status, 2);
+  const int64_t o = ((int64_t)slot * Lp + c) * 4 + x;
+  pm[o] = m;
+  st_df(pmdf + o, df_of(m));
+  const df l = df_of(m > 0.0 ? log(m) : 0.0), r = df_of(m > 0.0 ? 1.0 / m : 0.0);
+  lpi[o] = make_float4(l.hi, l.lo, r.hi, r.lo);
+  mpc[o] = rsum[cl] * m;
 }
 __global__ void k_pm_final(const double* __restrict__ part4, const double* __restrict__ partR, int L, int Lp, int nT,
                            double* __restrict__ pm, float2* __restrict__ pmdf, float4* __restrict__ lpi,
@@ -467,15 +479,17 @@ __device__ __forceinline__ void meanp_body(
 #pragma unroll
   for (int x = 0; x < 4; x++) buf[x][threadIdx.x] = acc[x];
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o)
-#pragma unroll
-      for (int x = 0; x < 4; x++) buf[x][threadIdx.x] += buf[x][threadIdx.x + o];
+  for (int lg = 7; lg >= 0; lg--) {   // the four sums side by side (256 threads)
+    const int o = 1 << lg;
+    for (int e = threadIdx.x; e < 4 * o; e += 256) {
+      const int x = e >> lg, i = e & (o - 1);
+      buf[x][i] += buf[x][i + o];
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 4) {
     const double s = buf[0][0] + buf[1][0] + buf[2][0] + buf[3][0];
-    for (int x = 0; x < 4; x++) meanp[slot * 4 + x] = (s != 0.0) ? buf[x][0] / s : 0.25;
+    meanp[slot * 4 + threadIdx.x] = (s != 0.0) ? buf[threadIdx.x][0] / s : 0.25;
   }
 }
 __global__ void k_meanp(const double* __restrict__ mpc, int L, int Lp, double* __restrict__ meanp) {
@@ -1742,7 +1756,7 @@ cudaError_t launch_pair_marg(const float* cnt, int L, const TileRC* tiles, int n
 
 cudaError_t launch_pm_final(const double* part4, const double* partR, int L, int Lp, int nT, int nslots, double* pm,
                             float2* pmdf, float4* lpi, double* mpc, double* meanp, int* status, cudaStream_t st) {
-  k_pm_final<<<dim3((L + 127) / 128, nslots), 128, 0, st>>>(part4, partR, L, Lp, nT, pm, pmdf, lpi, mpc, status);
+  k_pm_final<<<dim3((L + 31) / 32, nslots), 160, 0, st>>>(part4, partR, L, Lp, nT, pm, pmdf, lpi, mpc, status);
   k_meanp<<<nslots, 256, 0, st>>>(mpc, L, Lp, meanp);
   return cudaGetLastError();
 }
@@ -1963,7 +1977,7 @@ __device__ __forceinline__ GrpLoc grp_loc(const int* __restrict__ pre, int nf, i
   return GrpLoc{f, GridIdx{loc % gx, loc / gx, gx}};
 }
 __device__ __forceinline__ int gx_tiles(const FamDev& d) { return d.ntiles; }
-__device__ __forceinline__ int gx_cols128(const FamDev& d) { return (d.L + 127) / 128; }
+__device__ __forceinline__ int gx_cols32(const FamDev& d) { return (d.L + 31) / 32; }
 __device__ __forceinline__ int gx_cols256(const FamDev& d) { return (d.L + 255) / 256; }
 __device__ __forceinline__ int gx_one(const FamDev&) { return 1; }
 __device__ __forceinline__ int gx_apc(const FamDev& d) { return (d.ntiles + APC_TILES - 1) / APC_TILES; }
@@ -1997,7 +2011,7 @@ k_pair_marg_grp(const FamDev* __restrict__ F, const int* __restrict__ pre, int n
 }
 
 __global__ void k_pm_final_grp(const FamDev* __restrict__ F, const int* __restrict__ pre, int nf) {
-  const GrpLoc l = grp_loc(pre, nf, gx_cols128, F);
+  const GrpLoc l = grp_loc(pre, nf, gx_cols32, F);
   const FamDev& d = F[l.f];
   pm_final_body(l.g, d.part4, d.partR, d.L, d.Lp, d.nT, d.pm, d.pmdf, d.lpi, d.mpc, d.status);
 }
@@ -2134,7 +2148,7 @@ cudaError_t grp_count_simt(const FamDev* F, int nf, const int* pre, int nb, bool
 cudaError_t grp_marginals(const FamDev* F, int nf, const int* pre_marg, int nb_marg, const int* pre_pm, int nb_pm,
                           const int* pre_mp, int nb_mp, cudaStream_t st) {
   if (nb_marg > 0) k_pair_marg_grp<<<nb_marg, 256, 0, st>>>(F, pre_marg, nf);
-  if (nb_pm > 0) k_pm_final_grp<<<nb_pm, 128, 0, st>>>(F, pre_pm, nf);
+  if (nb_pm > 0) k_pm_final_grp<<<nb_pm, 160, 0, st>>>(F, pre_pm, nf);
   if (nb_mp > 0) k_meanp_grp<<<nb_mp, 256, 0, st>>>(F, pre_mp, nf);
   return cudaGetLastError();
 }
