@@ -195,7 +195,7 @@ int  covgpu_rscape(covgpu_ctx *ctx, const covgpu_params *p, const uint8_t *ax, c
  * (R-scape's rule, src/R-scape.c:1545-1562, where wgt is NULL), the nulls
  * (one launch per tree depth over every family), the counts (one persistent
  * tensor-core launch over every family's tiles), the statistics and APC/ASC,
- * the null histograms, the tail fits (one block per fit), the survival
+ * the null histograms, the tail fits (a cluster of blocks per fit), the survival
  * tables and the E-values; the host steps run once per phase for all
  * families.  Families are processed in chunks that fit the batch's device
  * budget (mem_gb; 0: a quarter of the free memory); the device passes of a

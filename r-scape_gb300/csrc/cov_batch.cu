@@ -14,7 +14,7 @@
 // one CTA per family for the merges, or position-based), the nulls (one
 // launch per tree depth over every family), the tensor count (one
 // persistent launch over every (family, alignment, tile) task), marginals,
-// statistics, APC/ASC, histograms, the tail fits (one block per fit),
+// statistics, APC/ASC, histograms, the tail fits (a cluster per fit),
 // survival tables and E-values.  The host steps between the passes
 // (cov_rscape_host.h) run for every family and statistic, with one host
 // round trip per phase for the whole chunk.  The device passes from the

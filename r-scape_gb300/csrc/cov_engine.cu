@@ -553,12 +553,13 @@ extern "C" int covgpu_power(covgpu_ctx* ctx, int ns, const double* subs, const d
   for (int k = 0; k < 6; k++)
     if (src[k]) for (int s = 0; s < ns; s++) tab[(size_t)k * ns + s] = src[k][s];
   const int64_t P = (int64_t)L * (L - 1) / 2;
-  CK(work_reserve(ctx, (tab.size() + 3 * (size_t)P) * sizeof(double)));
-  double *d_tab = (double*)ctx->d_wrk, *d_out = d_tab + tab.size();
+  const int T = power_table_size(ctx->N, L);
+  CK(work_reserve(ctx, (tab.size() + 3 * ((size_t)P + T)) * sizeof(double)));
+  double *d_tab = (double*)ctx->d_wrk, *d_out = d_tab + tab.size(), *d_F = d_out + 3 * P;
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->st);
   if (e == cudaSuccess)
-    e = launch_power(ctx->d_nsubs, ctx->d_ndouble, ctx->d_njoin, L, ns, d_tab, subs && prob, subs_join && prob_join,
+    e = launch_power(ctx->d_nsubs, ctx->d_ndouble, ctx->d_njoin, L, ns, d_tab, T, d_F, subs && prob, subs_join && prob_join,
                      subs_double && prob_double, d_out, d_out + P, d_out + 2 * P, ctx->st);
   double* outs[3] = {power, power_join, power_double};
   for (double* o : outs) result_pages(o, P * sizeof(double));

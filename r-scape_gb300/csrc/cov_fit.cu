@@ -238,7 +238,7 @@ __device__ __forceinline__ int fold_value(int lane) {
 // round; more only when lambda w > 0.5, and those past the list are computed
 // where they are.
 //
-// Three tails of a 30 x 61 family with 200 nulls (16 bins): 209 us with
+// The tail of a 30 x 61 family with 20 nulls (16 bins): 209 us with
 // everything of an item in its thread, 156 us with the near bins' parts in
 // four warps, 99 us so.
 //
@@ -850,7 +850,7 @@ int gamma_fit_collect(FitWork* fwp, double* ret_lambda, double* ret_tau, int* re
 
 
 // ------------------------------------------------------------------------
-// a batch of gamma fits (one block per fit, every search launched at once)
+// a batch of gamma fits (a cluster of blocks per fit, every search launched at once)
 // and the survival tables of a batch of tails
 // ------------------------------------------------------------------------
 struct FitBatch {

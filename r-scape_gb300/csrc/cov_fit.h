@@ -19,8 +19,8 @@ int gamma_fit_launch(FitWork* fw, const uint64_t* h_obs, int cmin, int imax, dou
                      cudaStream_t st);
 int gamma_fit_collect(FitWork* fw, double* ret_lambda, double* ret_tau, int* ret_evals);
 
-// a batch of gamma fits, one block each, launched together (the same search
-// as gamma_fit_launch on a grid of one block): launch, then, once the
+// a batch of gamma fits, a cluster of blocks each, launched together (the same search
+// as gamma_fit_launch summed in the order of one block): launch, then, once the
 // caller has synchronised the stream, collect fit k (0, 1 empty tail, 2
 // barrier timeout, or the search's status)
 struct FitReq { const uint64_t* obs; int cmin, imax; double bmin, w, phi; };

@@ -66,7 +66,7 @@ __host__ __device__ __forceinline__ int exact_bin(double x, double bmin, double 
 // Bound by the FMA pipe where the grid fills the device, by its latency
 // below.  With one CTA of 256 threads per tile and the limbs one after the
 // other: 166 us at 400 x 351 (66 CTAs on 152 SMs), 76 us at 100 x 120 x 21,
-// 21 us at 30 x 61 x 201; so 68, 58 and 10 us.  Packed FMAs took 117 us at
+// 21 us at 30 x 61 x 21; so 68, 58 and 10 us.  Packed FMAs took 117 us at
 // 400 x 351 (twice the shared-memory reads on the i side), two pairs a thread
 // 99 us, 2x2 pairs a thread 69 us.
 // ------------------------------------------------------------------------
@@ -422,7 +422,7 @@ k_pair_marg(const float* __restrict__ cnt, int L, const TileRC* __restrict__ til
 // nseff[c][j]) feeds the CCF column means (src/correlators.c:1030-1036).
 // Bound by FP64 instructions (a warp's takes one ~64 cycles): a thread per
 // column that made all four states' quotients and logarithms took 11.3 us at
-// 30 x 61 x 201 and 69 us at 500 x 400 x 201, now 6.3 and 56 us.
+// 30 x 61 x 21 and 69 us at 500 x 400 x 201, now 6.3 and 56 us.
 __device__ __forceinline__ void pm_final_body(
     const GridIdx g, const double* __restrict__ part4, const double* __restrict__ partR, int L, int Lp, int nT,
                            double* __restrict__ pm, float2* __restrict__ pmdf, float4* __restrict__ lpi,

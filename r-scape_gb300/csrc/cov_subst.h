@@ -13,8 +13,10 @@ cudaError_t launch_substitutions(const uint8_t* ax, const uint8_t* F, const int*
                                  int* njoin, cudaStream_t st);
 // per pair i < j (row-major upper triangle): tab = [subs, prob] x (single,
 // join, double), ns points each
+// entries per curve of launch_power's table F [3][T], 0 for none
+int power_table_size(int N, int L);
 cudaError_t launch_power(const int* nsubs, const int* ndouble, const int* njoin, int L, int ns, const double* tab,
-                         int have_single, int have_join, int have_double, double* power, double* power_join,
-                         double* power_double, cudaStream_t st);
+                         int T, double* F, int have_single, int have_join, int have_double, double* power,
+                         double* power_join, double* power_double, cudaStream_t st);
 
 }  // namespace covgpu

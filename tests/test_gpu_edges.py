@@ -254,3 +254,24 @@ def test_batch_fit_does_not_depend_on_its_cluster(covgpu, copies):
         for k in ("lambda_", "tau", "sc_thresh", "nhit"):
             assert rows[0][k] == want[k], k
     b.close()
+
+
+@pytest.mark.parametrize("N,L", [(200, 12), (5, 40), (60, 70)])
+@pytest.mark.parametrize("curve", ["rising", "unsorted", "one"])
+def test_power_tabled_and_scanned(covgpu, oracle, N, L, curve):
+    """Few pairs (each scans its curve) and many (the curves are tabled): the
+    oracle's step at every pair's counts, also for a curve whose points do not
+    rise and for a single point."""
+    s = covgpu.Synth(N, L, 1.5, max(1, L // 6), 1, 1, L // 6, 0.1, seed=4)
+    e = covgpu.Engine(N, L, maxslots=1, maxnull=0)
+    e.set_tree(s.parent, s.left, s.right)
+    e.set_alignment(0, s.ax)
+    ns, nd, nj = e.substitutions(0)
+    x = {"rising": np.arange(-1.0, 30.0, 1.5), "unsorted": np.array([0.0, 3.0, 2.0, 9.0, 1.0, 4.0]),
+         "one": np.array([1.0])}[curve]
+    y = np.linspace(0.05, 0.95, len(x))
+    got = e.power(single=(x, y), join=(x, y[::-1].copy()), double=(x, y))
+    e.close()
+    i, j = np.triu_indices(L, 1)
+    for g, n, p in zip(got, (ns[i] + ns[j], nj[i, j], nd[i, j]), (y, y[::-1], y)):
+        assert np.array_equal(g, [oracle.power_step(float(v), x, np.ascontiguousarray(p)) for v in n])
