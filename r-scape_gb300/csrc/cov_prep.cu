@@ -108,31 +108,52 @@ k_pb_rows(const uint8_t* __restrict__ ax, int L, int Lp, const double* __restric
   pb_rows_body(native_grid(), ax, L, Lp, inv, w);
 }
 
-// 32 columns by a CTA of 32 slices of the sequences, each summed in order, the
-// slices then in order.  One thread per column and all rows in turn: 286 us at
-// N=900 x L=700, 13 us now.
-__global__ void __launch_bounds__(1024)
+// A column's two sums (residues, residues and gaps) run over the sequences in
+// their order: where the fraction lies on the threshold, the rounding of the
+// sums decides, and any other order decides some columns differently.  So a
+// lane per (column, sum) of 16 columns, the first warp of a CTA, while the
+// other warps stage the next rows' codes and weights (GAP_ROWS, a row each).
+// Bound by the chain of FP64 additions (~64 cycles each); without weights the
+// sums are counts, in integers.  The whole call at N=20,000 x L=1,500: 3.84 ms
+// weighted and 3.34 without weights with a thread per column that read its rows
+// itself, 0.77 and 0.18 so (0.45 and 0.44 with 32 slices summed apart, which
+// gave the columns on the threshold another rounding).
+constexpr int GAP_COLS = 16, GAP_ROWS = 96;
+template <bool UNIT>
+__global__ void __launch_bounds__(32 + GAP_ROWS)
 k_gapfilter(const uint8_t* __restrict__ ax, const double* __restrict__ wgt, int N, int L, int Lp, double idthresh,
             int* __restrict__ useme) {
-  __shared__ double sr[32][33], st[32][33];
-  const int x0 = threadIdx.x & 31, slice = threadIdx.x >> 5, c = blockIdx.x * 32 + x0;
-  const int per = (N + 31) / 32, s1 = min(N, (slice + 1) * per);
-  double r = 0.0, tot = 0.0;
-#pragma unroll 4
-  for (int s = slice * per; s < s1; s++) {
-    const int x = ax[(int64_t)s * Lp + c];   // columns up to Lp, a multiple of 32, exist
-    const double w = wgt ? wgt[s] : 1.0;
-    if (x < 4 || (x > 4 && x <= 15)) { r += w; tot += w; }
-    else if (x == 4 || x == 16) tot += w;
-  }
-  sr[slice][x0] = r;
-  st[slice][x0] = tot;
+  __shared__ uint4 sc[2][GAP_ROWS];
+  __shared__ double sw[2][GAP_ROWS];
+  const int tid = threadIdx.x, c0 = blockIdx.x * GAP_COLS, row = tid - 32;
+  const int col = tid & 15, top = (tid & 16) ? 16 : 15;   // the first warp: residues up to 15, with gaps 16
+  auto stage = [&](int buf, int s) {
+    if (row < 0 || s + row >= N) return;
+    sc[buf][row] = *reinterpret_cast<const uint4*>(ax + (int64_t)(s + row) * Lp + c0);   // Lp is a multiple of 32
+    if (!UNIT) sw[buf][row] = wgt[s + row];
+  };
+  typename std::conditional<UNIT, int, double>::type q = 0;
+  stage(0, 0);
   __syncthreads();
-  if (slice == 0 && c < L) {
-    r = tot = 0.0;
-    for (int k = 0; k < 32; k++) { r += sr[k][x0]; tot += st[k][x0]; }
-    useme[c] = (r > 0.0 && r / tot >= idthresh) ? 1 : 0;
+  int buf = 0;
+  for (int s0 = 0; s0 < N; s0 += GAP_ROWS, buf ^= 1) {
+    stage(buf ^ 1, s0 + GAP_ROWS);
+    if (row < 0) {
+      const int n = min(GAP_ROWS, N - s0);
+      const uint8_t* code = reinterpret_cast<const uint8_t*>(sc[buf]) + col;
+#pragma unroll 8
+      for (int s = 0; s < n; s++) {
+        const int x = code[16 * s];
+        const bool in = x <= top && (x != 4 || top == 16);
+        if constexpr (UNIT) q += in;
+        else if (in) q += sw[buf][s];
+      }
+    }
+    __syncthreads();
   }
+  if (row >= 0) return;
+  const double v = (double)q, tot = __shfl_down_sync(0xffffffffu, v, 16);
+  if (top == 15 && c0 + col < L) useme[c0 + col] = (v > 0.0 && v / tot >= idthresh) ? 1 : 0;
 }
 
 __device__ __forceinline__ void gsc_codes_body(
@@ -692,7 +713,9 @@ cudaError_t launch_weights_pb(const uint8_t* ax, int N, int L, int Lp, double* i
 
 cudaError_t launch_gapfilter(const uint8_t* ax, const double* wgt, int N, int L, int Lp, double gapthresh, int* useme,
                              cudaStream_t st) {
-  k_gapfilter<<<(L + 31) / 32, 1024, 0, st>>>(ax, wgt, N, L, Lp, 1.0 - gapthresh, useme);
+  const int nb = (L + GAP_COLS - 1) / GAP_COLS, thr = 32 + GAP_ROWS;
+  if (wgt) k_gapfilter<false><<<nb, thr, 0, st>>>(ax, wgt, N, L, Lp, 1.0 - gapthresh, useme);
+  else     k_gapfilter<true><<<nb, thr, 0, st>>>(ax, wgt, N, L, Lp, 1.0 - gapthresh, useme);
   return cudaGetLastError();
 }
 

@@ -275,3 +275,28 @@ def test_power_tabled_and_scanned(covgpu, oracle, N, L, curve):
     i, j = np.triu_indices(L, 1)
     for g, n, p in zip(got, (ns[i] + ns[j], nj[i, j], nd[i, j]), (y, y[::-1], y)):
         assert np.array_equal(g, [oracle.power_step(float(v), x, np.ascontiguousarray(p)) for v in n])
+
+
+@pytest.mark.parametrize("N,L", [(64, 40), (96, 16), (97, 33), (200, 65), (1001, 48)])
+@pytest.mark.parametrize("thr", [0.5, 0.75, 0.25])
+def test_gap_filter_on_the_threshold(covgpu, oracle, N, L, thr):
+    """Columns whose weighted fraction lies exactly on the threshold: every
+    weight is held by four sequences, 1 - thr of them with a residue, so that
+    the rounding of the sums decides.  The sums run over the sequences in their
+    order, as the oracle's: the same columns."""
+    rng = np.random.default_rng(N + L)
+    n4 = N // 4
+    w = np.concatenate([np.repeat(rng.uniform(0.1, 3.0, n4), 4), rng.uniform(0.1, 3.0, N - 4 * n4)])
+    ax = np.full((N, L), 17, dtype=np.uint8)   # the sequences beyond 4 n4: missing, not counted
+    for c in range(L):
+        for k in range(n4):
+            res = rng.permutation(4) < 4 * (1 - thr)
+            ax[4 * k:4 * k + 4, c] = np.where(res, rng.choice([0, 1, 2, 3, 7, 15], 4), rng.choice([4, 16], 4))
+    p = rng.permutation(N)
+    ax, w = np.ascontiguousarray(ax[p]), np.ascontiguousarray(w[p])
+    ref = oracle.gapfilter(ax, w, thr) == 1
+    e = covgpu.Engine(N, L)
+    e.set_alignment(0, ax)
+    assert np.array_equal(e.gapfilter(0, w, thr), ref)
+    assert np.array_equal(e.gapfilter(0, None, thr), oracle.gapfilter(ax, None, thr) == 1)
+    e.close()
