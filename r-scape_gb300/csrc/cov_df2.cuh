@@ -85,11 +85,6 @@ __device__ __forceinline__ df2 df2_add_f(df2 a, f2 b) {
   const df2 s = two_sum2(a.hi, b);
   return fast_two_sum2(s.hi, add2(s.lo, a.lo));
 }
-// a + b, b no larger than a.hi (or a = 0)
-__device__ __forceinline__ df2 df2_add_f_fast(df2 a, f2 b) {
-  const df2 s = fast_two_sum2(a.hi, b);
-  return fast_two_sum2(s.hi, add2(s.lo, a.lo));
-}
 __device__ __forceinline__ df2 df2_add(df2 a, df2 b) {
   const df2 s = two_sum2(a.hi, b.hi);
   return fast_two_sum2(s.hi, add2(s.lo, add2(a.lo, b.lo)));

@@ -774,8 +774,8 @@ __device__ __forceinline__ void merged_stats(const StatsArgs& A, const df (&c)[1
 // Bound: the FMA pipe and the latency of its chains (58-63% of the pipe busy,
 // 16 warps of 122-128 registers per SM); HBM at 0.27 of its rate.  Against the
 // form before (one pair per thread, scalar operations, counts loaded where
-// they are used, one CTA per tile): 69 for 103 warp instructions per pair
-// for GT, MI, CHI and RAF; 8.53 for 9.53 ms on 21 alignments of
+// they are used, one CTA per tile): 70 for 103 warp instructions per pair
+// for GT, MI, CHI and RAF; 8.65 for 9.53 ms on 21 alignments of
 // 2,000 x 3,000; GT alone 1.16 for 1.44 ms on 201 alignments of 500 x 400.
 constexpr int STATS_UC = 6;   // allowed cells staged; with more, RAF reads its counts directly
 struct StatsSmem {
@@ -961,9 +961,9 @@ __device__ __forceinline__ void c16_tile(const StatsTask& task, const StatsTask*
           for (int y = 0; y < 4; y++) {
             const df2 c = cur[y];
             df2_acc(ne, c);
-            // counts are 0 or at least a weight's quantum, above the prior
-            // for weights that sum to N
-            const df2 cp = df2_add_f_fast(c, dup2(1e-10f));
+            // the full two_sum: a caller's weights may be of any scale, so a
+            // count may be smaller than the prior
+            const df2 cp = df2_add_f(c, dup2(1e-10f));
             const f2 ncp = neg2(cp.hi);
             if (y == 0) Rx = cp; else df2_acc(Rx, cp);
             df2_acc(K[y], cp);

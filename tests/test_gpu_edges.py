@@ -300,3 +300,32 @@ def test_gap_filter_on_the_threshold(covgpu, oracle, N, L, thr):
     assert np.array_equal(e.gapfilter(0, w, thr), ref)
     assert np.array_equal(e.gapfilter(0, None, thr), oracle.gapfilter(ax, None, thr) == 1)
     e.close()
+
+
+@pytest.mark.parametrize("shift", [0, 39, 41])
+@pytest.mark.parametrize("weights", ["limbs", "equal"])
+def test_statistics_at_the_weights_scale(covgpu, oracle, shift, weights):
+    """Weights of the size of one and 2^39 or 2^41 times smaller, where the pair
+    counts lie far below the prior of 1e-10, against the oracle to 1e-7 of the
+    largest score.  The prior is the FP32 number next to 1e-10, 1.34e-8 above
+    it, and MI goes as its inverse square there: 2.7e-8; the double-float terms
+    (2^-44 of p |ln p|, |ln p| up to 28) add less than 2e-8 of a largest MI of
+    9e-5.  Counts that lose their low word in the addition of the prior (a
+    two-sum for operands in the other order) put the scores off by 3e-7 and
+    1e-6."""
+    N, L = 40, 60
+    s = covgpu.Synth(N, L, 1.5, 8, 1, 4, 8, 0.15, seed=11, tree_kind=1)
+    w = np.random.default_rng(3).integers(1 << 29, 1 << 33, N) * 2.0 ** -32
+    w = (w if weights == "limbs" else np.full(N, 1.0 + 2.0 ** -20 + 2.0 ** -22)) * 2.0 ** -shift
+    e = covgpu.Engine(N, L)
+    e.set_weights(w)
+    e.set_alignment(0, s.ax)
+    iu = np.triu_indices(L, 1)
+    types = ["MI", "MIr", "CHI", "GT"]
+    for counter in (covgpu.SIMT, covgpu.TENSOR):
+        e.score(types, covclass=covgpu.C16, counter=counter)
+        for q, t in enumerate(types):
+            ref = oracle.cov_calculate(t, s.ax, w, covclass=covgpu.C16)[0][iu]
+            err = np.abs(e.get_cov(0, q)[iu] - ref).max()
+            assert err <= 1e-7 * np.abs(ref).max(), (t, err, np.abs(ref).max())
+    e.close()
