@@ -619,9 +619,13 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
   const size_t o_col = tb.put(pcol.v.data(), pcol.v.size() * 4), o_row = tb.put(prow.v.data(), prow.v.size() * 4);
   const size_t o_cod = tb.put(pcod.v.data(), pcod.v.size() * 4), o_id = tb.put(pid.v.data(), pid.v.size() * 4);
   const size_t o_up = tb.put(pup.v.data(), pup.v.size() * 4), o_lb = tb.put(plb.v.data(), plb.v.size() * 4);
-  Pre prs = prefix(nf, [&](int k) { return fams[k].ns > 0 ? fitch_blocks(fams[k].Lp) * fams[k].ns : 0; });
   int maxNnull = 1;
-  for (auto& f : fams) if (f.ns > 0) maxNnull = std::max(maxNnull, f.N);
+  int64_t null_cols = 0;
+  for (auto& f : fams)
+    if (f.ns > 0) { maxNnull = std::max(maxNnull, f.N); null_cols += (int64_t)f.Lp * f.ns; }
+  Pre prs = prefix(nf, [&](int k) {
+    return fams[k].ns > 0 ? fitch_blocks(fams[k].Lp, maxNnull, null_cols) * fams[k].ns : 0;
+  });
   Pre prr = prefix(nf, [&](int k) { return fams[k].ns > 0 ? (fams[k].Lp + 255) / 256 * fams[k].ns : 0; });
   Pre pprep = prefix(nf, [&](int k) {
     return fams[k].tens ? fams[k].Npad / 64 * (fams[k].Lp / 32) * fams[k].nslots : 0;
@@ -694,7 +698,7 @@ static int chunk_launch(covgpu_batch* b, Slot& S, const covgpu_params* p, const 
     // nulls: the reconstructions, the roots' rows, the replay down the tree
     if (prs.total()) {
       BK(cudaMemsetAsync(Lo.ns, 0, Lo.ns_bytes, S.st));
-      BK(grp_fitch(dF, nf, P(o_rs), prs.total(), maxNnull, P(o_rr), prr.total(), p->seed, S.st));
+      BK(grp_fitch(dF, nf, P(o_rs), prs.total(), maxNnull, null_cols, P(o_rr), prr.total(), p->seed, S.st));
       launches += 2;
     }
     for (int dd = 0; dd < maxdepth; dd++) {

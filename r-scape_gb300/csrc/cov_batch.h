@@ -108,10 +108,11 @@ int         grp_weights_gsc_prepare();
 // nulls (cov_null.cu): the reconstructions' substitution counts (zeroed
 // before) and the roots' rows; then one depth d of every family: lv[f] =
 // {offset of depth d in lnodes, nodes at depth d} (nn = 0: nothing at this
-// depth).  maxN: the largest N of the families with nulls.
-cudaError_t grp_fitch(const FamDev* F, int nf, const int* pre_cols, int nb_cols, int maxN, const int* pre_row,
-                      int nb_row, uint64_t seed, cudaStream_t st);
-int         fitch_blocks(int Lp);
+// depth).  maxN: the largest N of the families with nulls, cols: the columns
+// of all their nulls (padded).
+cudaError_t grp_fitch(const FamDev* F, int nf, const int* pre_cols, int nb_cols, int maxN, int64_t cols,
+                      const int* pre_row, int nb_row, uint64_t seed, cudaStream_t st);
+int         fitch_blocks(int Lp, int maxN, int64_t cols);   // blocks of a null of a family in pre_cols
 int         grp_null_prepare();
 cudaError_t grp_replay(const FamDev* F, int nf, const int2* lv, const int* pre, int nb, bool cta, bool srow,
                        int maxLp, uint64_t seed, cudaStream_t st);

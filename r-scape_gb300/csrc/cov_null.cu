@@ -38,6 +38,7 @@
 #include "cov_batch.h"
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 namespace covgpu {
 
@@ -81,12 +82,12 @@ __device__ __forceinline__ uint32_t state_codes(uint32_t w) {
 __device__ __forceinline__ uint32_t choose_word(uint32_t s, uint32_t pick, int L, uint64_t seed, uint32_t nid,
                                                 uint32_t node, int c0) {
   uint32_t multi = (s & (s - 0x01010101u)) & pick;   // sets are not empty: no borrow between bytes
-  if (multi == 0u) return s;
-  for (int b = 0; b < 4; b++)
-    if ((multi >> (8 * b)) & 0xFFu) {
-      const uint32_t st = (uint32_t)choose_member((s >> (8 * b)) & 0xFFu, seed, nid, node, (uint32_t)(c0 + b));
-      s = (s & ~(0xFFu << (8 * b))) | (1u << (8 * b + st));
-    }
+  while (multi) {   // each lane its next byte: as many draws as the lane with the most
+    const int sh = (__ffs(multi) - 1) & ~7;
+    const uint32_t st = (uint32_t)choose_member((s >> sh) & 0xFFu, seed, nid, node, (uint32_t)(c0 + (sh >> 3)));
+    s = (s & ~(0xFFu << sh)) | (1u << (sh + st));
+    multi &= ~(0xFFu << sh);
+  }
   return s;
 }
 
@@ -97,18 +98,28 @@ __device__ __forceinline__ uint32_t fitch_word(uint32_t a, uint32_t b) {
   return (I & ~z) | (U & z);
 }
 
-// The reconstruction of FW words of four columns by one CTA.  With SM the
-// leaves, the nodes' sets (then states) and the tree lie in shared memory, 38
-// bytes per sequence for 16 columns, so a depth costs a barrier and a few
-// shared accesses; alignments too deep for that take the rows from global
-// memory (the null's row buffer SR, each CTA its own columns).  Bound by
-// instructions on large alignments (64% of the issue slots; 457 us for 20
-// nulls of 2,000 x 3,000), by the barriers on small ones (13 us for 30 x 61).
+// The reconstruction of FW words of four columns by one CTA.  With KEEP_TREE
+// the leaves, the nodes' sets (then states) and the tree lie in shared memory,
+// 8 FW + 6 bytes per sequence, so a depth costs a barrier and a few shared
+// accesses; KEEP_WORDS leaves the tree in global memory; KEEP_NONE takes
+// everything from there (the rows from the null's buffer SR, each CTA its own
+// columns).  Bound by instructions on large alignments (64% of the issue slots;
+// 400 us for 20 nulls of 2,000 x 3,000), by the barriers on small ones (13 us
+// for 30 x 61).
 // With the reconstruction inside the replay, depth by depth, the null
-// generation took (now): 30 x 61, 20 nulls 134 us (50); 400 x 300, 20 nulls
-// 572 (236); 500 x 400, 200 nulls 895 (762); 2,000 x 3,000, 20 nulls 1,266
-// (1,076); the reconstruction alone, 701 x 650, 300 us in 42 launches (20).
-constexpr int FW = 4;
+// generation took (now): 30 x 61, 20 nulls 134 us (46); 400 x 300, 20 nulls
+// 572 (238); 500 x 400, 200 nulls 895 (740); 2,000 x 3,000, 20 nulls 1,266
+// (1,018); the reconstruction alone, 701 x 650, 300 us in 42 launches (20).
+//
+// The form by the number of sequences N and of columns of all nulls (us, the
+// whole null generation of 20 nulls unless said):
+//   {4, TREE}, {2, TREE}  while two CTAs of 512 threads fit an SM: 2,700 x
+//     2,000 1,218 and 1,233, 3,500 x 2,000 1,772 and 1,617
+//   {1, TREE}, {1, WORDS}  beyond, up to 4,096 columns: enough CTAs for the
+//     SMs where there are few columns (20,000 x 60, one null: 370; 849 with
+//     the rows in global memory)
+//   {8, NONE}  the rest: full sectors and 32 warps per SM (12,000 x 1,000:
+//     1,936; {1, TREE} 2,232, four words 2,191)
 struct FitchCols {
   const uint8_t* ax;
   int N, L, Lp;
@@ -121,37 +132,65 @@ struct FitchCols {
   bool all_rows;
   int* ns;         // [2N][25] branch counters, or nullptr
 };
-static size_t fitch_smem(int N) { return (size_t)N * (2 * FW * 4 + 3 * 2) + 16; }
-constexpr size_t FITCH_SMEM_MAX = 200 * 1024;
-static_assert(FITCH_SMEM_MAX / (2 * FW * 4 + 3 * 2) < 32768, "the tree's node numbers fit 16 bits");
+// the form of the kernel: words of a CTA and what it keeps in shared memory
+enum FitchKeep { KEEP_NONE = 0, KEEP_WORDS = 1, KEEP_TREE = 2 };
+static size_t fitch_smem(int N, int FW, int keep) {
+  return keep == KEEP_NONE ? 0 : (size_t)N * (2 * FW * 4 + (keep == KEEP_TREE ? 3 * 2 : 0)) + 16;
+}
+constexpr size_t FITCH_SMEM_MAX = 224 * 1024;
+static_assert(FITCH_SMEM_MAX / (2 * 4 + 3 * 2) < 32768, "the tree's node numbers fit 16 bits");
+constexpr size_t FITCH_SMEM_HALF = 113 * 1024;   // two CTAs per SM
+struct FitchForm { int fw, keep, threads; };
+static FitchForm fitch_form(int N, int64_t cols) {
+  // the widest depth of a tree of N leaves is about N / 10 nodes (coalescent)
+  const int thr = N >= 512 ? 512 : (N >= 128 ? 256 : 128);
+  for (int fw : {4, 2})
+    if (fitch_smem(N, fw, KEEP_TREE) <= FITCH_SMEM_HALF) return {fw, KEEP_TREE, thr};
+  for (int keep : {KEEP_TREE, KEEP_WORDS})
+    if (cols <= 4096 && fitch_smem(N, 1, keep) <= FITCH_SMEM_MAX) return {1, keep, 1024};
+  return {8, KEEP_NONE, 1024};
+}
+// f(FW, KEEP) of the form, as integral constants
+template <class FN>
+static cudaError_t with_fitch_form(FitchForm x, FN f) {
+  using std::integral_constant;
+  if (x.keep == KEEP_NONE) f(integral_constant<int, 8>(), integral_constant<int, KEEP_NONE>());
+  else if (x.fw == 4) f(integral_constant<int, 4>(), integral_constant<int, KEEP_TREE>());
+  else if (x.fw == 2) f(integral_constant<int, 2>(), integral_constant<int, KEEP_TREE>());
+  else if (x.keep == KEEP_TREE) f(integral_constant<int, 1>(), integral_constant<int, KEEP_TREE>());
+  else f(integral_constant<int, 1>(), integral_constant<int, KEEP_WORDS>());
+  return cudaGetLastError();
+}
 
-template <bool SM>
+template <int FW, int KEEP>
 __device__ __forceinline__ void fitch_cols(const FitchCols& a, int grp) {
   extern __shared__ __align__(16) uint32_t fsm[];
+  constexpr bool SM = KEEP != KEEP_NONE, TREE = KEEP == KEEP_TREE;
   const int N = a.N, tid = threadIdx.x, nthr = blockDim.x, c0 = grp * FW * 4;
   uint32_t* leaf = fsm;
   uint32_t* node = SM ? fsm + (size_t)N * FW : reinterpret_cast<uint32_t*>(a.SR + c0);
   const int stride = SM ? FW : a.Lp / 4;
-  int16_t* lr = reinterpret_cast<int16_t*>(fsm + (size_t)2 * N * FW);   // SM: left, right, lnodes
+  int16_t* lr = reinterpret_cast<int16_t*>(fsm + (size_t)2 * N * FW);   // TREE: left, right, lnodes
   if (SM) {
     for (int i = tid; i < N * FW; i += nthr) {
       const int s = i / FW, c = c0 + 4 * (i % FW);
       leaf[i] = leaf_word(*reinterpret_cast<const uint32_t*>(a.ax + (int64_t)s * a.Lp + c), s, c, a.seed, a.nid);
     }
-    for (int v = tid; v < N - 1; v += nthr) {
+    for (int v = tid; TREE && v < N - 1; v += nthr) {
       lr[v] = (int16_t)a.left[v]; lr[N + v] = (int16_t)a.right[v]; lr[2 * N + v] = (int16_t)a.lnodes[v];
     }
     __syncthreads();
   }
-  auto left = [&](int v) { return SM ? (int)lr[v] : a.left[v]; };
-  auto right = [&](int v) { return SM ? (int)lr[N + v] : a.right[v]; };
-  auto order = [&](int k) { return SM ? (int)lr[2 * N + k] : a.lnodes[k]; };
+  auto left = [&](int v) { return TREE ? (int)lr[v] : a.left[v]; };
+  auto right = [&](int v) { return TREE ? (int)lr[N + v] : a.right[v]; };
+  auto order = [&](int k) { return TREE ? (int)lr[2 * N + k] : a.lnodes[k]; };
   auto leafw = [&](int s, int w) -> uint32_t {
     if (SM) return leaf[s * FW + w];
     const int c = c0 + 4 * w;
     return leaf_word(*reinterpret_cast<const uint32_t*>(a.ax + (int64_t)s * a.Lp + c), s, c, a.seed, a.nid);
   };
   auto sets = [&](int ch, int w) -> uint32_t {
+    if (SM) return fsm[(ch > 0 ? N + ch : -ch) * FW + w] & ~(AMBIG * 0x01010101u);   // the nodes follow the leaves
     return ch > 0 ? node[(int64_t)ch * stride + w] : leafw(-ch, w) & ~(AMBIG * 0x01010101u);
   };
   for (int d = a.nlevels - 1; d >= 0; d--) {
@@ -185,29 +224,28 @@ __device__ __forceinline__ void fitch_cols(const FitchCols& a, int grp) {
       }
       // bytes that differ, not ambiguous (a leaf's bit 7); columns past L hold
       // gaps in every row and never differ
-      uint32_t diff = __vcmpne4(p, q) & ~__vcmpne4(q & (AMBIG * 0x01010101u), 0u);
+      const uint32_t diff = __vcmpne4(p, q) & ~__vcmpne4(q & (AMBIG * 0x01010101u), 0u);
       if (!a.ns || diff == 0u) continue;
       int* ns = a.ns + (int64_t)(ch > 0 ? N + ch : -ch) * 25;
-      do {
-        const int sh = (__ffs(diff) - 1) & ~7;
-        diff &= ~(0xFFu << sh);
-        const int x = __ffs((p >> sh) & 0xFFu) - 1, y = __ffs((q >> sh) & 0xFFu) - 1;
-        atomicAdd(ns + x * 5 + y, 1);
-      } while (diff);
+      const uint32_t kind = 5u * state_codes(p) + state_codes(q);   // four counters' places, below 25 where diff
+#pragma unroll
+      for (int b = 0; b < 4; b++)
+        if ((diff >> (8 * b)) & 1u) atomicAdd(ns + ((kind >> (8 * b)) & 0xFFu), 1);
     }
     __syncthreads();
   }
 }
-__device__ __forceinline__ int fitch_groups(int Lp) { return Lp / (FW * 4); }   // Lp is a multiple of 32
 
-template <bool SM>
-__global__ void __launch_bounds__(512)
+// the threads of FW words' forms (fitch_form)
+constexpr int fitch_max_threads(int FW) { return FW == 4 || FW == 2 ? 512 : 1024; }
+template <int FW, int KEEP>
+__global__ void __launch_bounds__(fitch_max_threads(FW))
 k_fitch_cols(FitchCols a, int64_t nstride, int64_t sstride) {
   a.nid += blockIdx.y;
   a.SR += blockIdx.y * sstride;
   a.F += blockIdx.y * sstride;
   if (a.ns) a.ns += blockIdx.y * nstride;
-  fitch_cols<SM>(a, blockIdx.x);
+  fitch_cols<FW, KEEP>(a, blockIdx.x);
 }
 
 // the root's row of the null: its states with the columns shuffled
@@ -540,16 +578,16 @@ static int replay_smem_limit() {
   return lim;
 }
 
-template <bool SM>
-__global__ void __launch_bounds__(512)
+template <int FW, int KEEP>
+__global__ void __launch_bounds__(fitch_max_threads(FW))
 k_fitch_cols_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre, uint64_t seed) {
   const int f = grp_find(pre, nf, (int)blockIdx.x);
   const FamDev& d = F[f];
-  const int gx = fitch_groups(d.Lp), loc = (int)blockIdx.x - __ldg(pre + f), q = loc / gx;
+  const int gx = d.Lp / (FW * 4), loc = (int)blockIdx.x - __ldg(pre + f), q = loc / gx;
   const FitchCols a{d.ax, d.N, d.L, d.Lp, d.left, d.right, d.lnodes, d.lnodes + (d.N - 1), d.nlevels, seed,
                     (uint32_t)q, d.scratch + (int64_t)q * (d.N - 1) * d.Lp, d.fitch + (int64_t)q * d.Lp, false,
                     d.ns + (int64_t)q * 2 * d.N * 25};
-  fitch_cols<SM>(a, loc % gx);
+  fitch_cols<FW, KEEP>(a, loc % gx);
 }
 
 // raises the shared-memory limits of this file's kernels on the current
@@ -561,7 +599,10 @@ static cudaError_t null_attrs() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < MAXDEV && done[dev].load()) return cudaSuccess;
-  const void* fit[] = {(const void*)k_fitch_cols<true>, (const void*)k_fitch_cols_grp<true>};
+  const void* fit[] = {(const void*)k_fitch_cols<4, KEEP_TREE>,     (const void*)k_fitch_cols<2, KEEP_TREE>,
+                       (const void*)k_fitch_cols<1, KEEP_TREE>,     (const void*)k_fitch_cols<1, KEEP_WORDS>,
+                       (const void*)k_fitch_cols_grp<4, KEEP_TREE>, (const void*)k_fitch_cols_grp<2, KEEP_TREE>,
+                       (const void*)k_fitch_cols_grp<1, KEEP_TREE>, (const void*)k_fitch_cols_grp<1, KEEP_WORDS>};
   for (const void* f : fit)
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FITCH_SMEM_MAX)) != cudaSuccess)
       return e;
@@ -572,18 +613,13 @@ static cudaError_t null_attrs() {
   return cudaSuccess;
 }
 
-// the widest depth of a tree of N leaves is about N / 10 nodes (coalescent): 4
-// words of each
-static int fitch_threads(int N) { return N >= 512 ? 512 : (N >= 128 ? 256 : 128); }
-
 static cudaError_t launch_fitch_cols(const FitchCols& a, int nnull, int64_t nstride, int64_t sstride,
                                      cudaStream_t st) {
-  const size_t sm = fitch_smem(a.N);
-  const dim3 g(a.Lp / (FW * 4), nnull);
-  const int thr = fitch_threads(a.N);
-  if (sm <= FITCH_SMEM_MAX) k_fitch_cols<true><<<g, thr, sm, st>>>(a, nstride, sstride);
-  else                      k_fitch_cols<false><<<g, thr, 0, st>>>(a, nstride, sstride);
-  return cudaGetLastError();
+  const FitchForm x = fitch_form(a.N, (int64_t)a.Lp * nnull);
+  return with_fitch_form(x, [&](auto fw, auto keep) {
+    k_fitch_cols<decltype(fw)::value, decltype(keep)::value>
+        <<<dim3(a.Lp / (x.fw * 4), nnull), x.threads, fitch_smem(a.N, x.fw, x.keep), st>>>(a, nstride, sstride);
+  });
 }
 
 cudaError_t launch_fitch_recon(const uint8_t* ax, int N, int L, int Lp, const NullTree& T, const int* level_nodes,
@@ -711,17 +747,21 @@ int replay_smem_max() {
   return lim;
 }
 
-cudaError_t grp_fitch(const FamDev* F, int nf, const int* pre_cols, int nb_cols, int maxN, const int* pre_row,
-                      int nb_row, uint64_t seed, cudaStream_t st) {
-  const size_t sm = fitch_smem(maxN);
+cudaError_t grp_fitch(const FamDev* F, int nf, const int* pre_cols, int nb_cols, int maxN, int64_t cols,
+                      const int* pre_row, int nb_row, uint64_t seed, cudaStream_t st) {
+  const FitchForm x = fitch_form(maxN, cols);
   if (nb_cols > 0) {
-    if (sm <= FITCH_SMEM_MAX) k_fitch_cols_grp<true><<<nb_cols, fitch_threads(maxN), sm, st>>>(F, nf, pre_cols, seed);
-    else                      k_fitch_cols_grp<false><<<nb_cols, 512, 0, st>>>(F, nf, pre_cols, seed);
+    const cudaError_t e = with_fitch_form(x, [&](auto fw, auto keep) {
+      k_fitch_cols_grp<decltype(fw)::value, decltype(keep)::value>
+          <<<nb_cols, x.threads, fitch_smem(maxN, x.fw, x.keep), st>>>(F, nf, pre_cols, seed);
+    });
+    if (e != cudaSuccess) return e;
   }
   if (nb_row > 0) k_root_row_grp<<<nb_row, 256, 0, st>>>(F, nf, pre_row, seed);
   return cudaGetLastError();
 }
-int fitch_blocks(int Lp) { return Lp / (FW * 4); }
+// Lp is a multiple of 32
+int fitch_blocks(int Lp, int maxN, int64_t cols) { return Lp / (fitch_form(maxN, cols).fw * 4); }
 int grp_null_prepare() { return null_attrs() == cudaSuccess ? 1 : 0; }
 
 // srow: every family of the launch has its rows staged in shared memory

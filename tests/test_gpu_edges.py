@@ -329,3 +329,47 @@ def test_statistics_at_the_weights_scale(covgpu, oracle, shift, weights):
             err = np.abs(e.get_cov(0, q)[iu] - ref).max()
             assert err <= 1e-7 * np.abs(ref).max(), (t, err, np.abs(ref).max())
     e.close()
+
+
+@pytest.mark.parametrize("N,L,ns", [(3100, 33, 3), (5400, 17, 2), (5400, 290, 15), (16400, 17, 2), (29000, 20, 1)])
+def test_nulls_of_deep_trees(covgpu, oracle, N, L, ns):
+    """Null alignments byte for byte in every form of the reconstruction beyond
+    the deepest tree that lies in shared memory with 16 columns: eight columns,
+    four columns, rows in global memory (many columns), four columns with the
+    tree in global memory, and everything in global memory; the reconstruction
+    itself in the same forms."""
+    s = covgpu.Synth(N, L, 1.5, 2, 1, 2, 2, 0.15, seed=N + L)
+    rng = np.random.default_rng(N)
+    for code in (5, 15, 17):
+        s.ax[rng.integers(0, N, N // 50), rng.integers(0, L, N // 50)] = code
+    e = covgpu.Engine(N, L, maxslots=ns + 1, maxnull=ns)
+    e.set_alignment(0, s.ax)
+    e.set_tree(s.parent, s.left, s.right)
+    e.make_nulls(7, 5, ns, 1)
+    T = oracle.TreeArrays(s.parent, s.left, s.right, s.ld, s.rd)
+    for q in sorted({0, ns - 1}):
+        assert np.array_equal(e.get_alignment(1 + q), oracle.null_msa(s.ax, T, 7, 5 + q)), q
+    for got, ref in zip(e.substitutions(0, seed=9), oracle.substitutions(s.ax, T, 9, 0xFFFFFFFF)):
+        assert np.array_equal(got, ref)
+    e.close()
+
+
+@pytest.mark.parametrize("deep", [(5400, 33), (3100, 60), (5400, 250)])
+def test_batch_with_a_deep_family(covgpu, deep):
+    """A deep family beside small ones: the batch's null scores (the forms of
+    the reconstruction by the deepest family of the chunk) are the single
+    calls'."""
+    fams = []
+    for k, (N, L) in enumerate([(30, 61), deep, (90, 64)]):
+        s = covgpu.Synth(N, L, 1.5, 4, 1, 4, 4, 0.1, seed=k + 2)
+        fams.append(dict(ax=s.ax, parent=s.parent, left=s.left, right=s.right, wgt=covgpu.weights_pb(s.ax)))
+    b = covgpu.Batch()
+    got = b.rscape(fams, ["GTp"], counter=covgpu.TENSOR, nshuffle=20)
+    b.close()
+    for f, rows in zip(fams, got):
+        e = covgpu.Engine(*f["ax"].shape, maxslots=21, maxnull=20)
+        e.set_tree(f["parent"], f["left"], f["right"])
+        one = e.rscape(f["ax"], f["wgt"], ["GTp"], counter=covgpu.TENSOR, nshuffle=20)[0]
+        e.close()
+        for k in ("null_minCOV", "null_maxCOV", "h_nb", "h_imin", "h_imax", "h_n", "nhit"):
+            assert rows[0][k] == one[k], k
