@@ -544,13 +544,17 @@ constexpr size_t NULL_SMEM_MAX = 100 * 1024;   // two CTAs per SM
 // CTAs of the cluster that replays one null in one launch, 0: a launch per
 // depth.  One launch wins where the depths are short: up to 13M columns x
 // sequences x nulls in all and rows of 1,024 columns (a warp's walk along a
-// longer row takes longer than the launches).  Measured against the launches
-// (us, the whole null generation): N=30 x L=61, 20 nulls 50 / 77 (C = 1);
-// 100 x 120 112 / 151; 400 x 300 236 / 375; 301 x 773 193 / 218; 2,000 x 300
-// 521 / 544; but 500 x 400 with 200 nulls 803 / 762, 100 x 3,000 263 / 205,
-// 2,000 x 3,000 1,338 / 1,076.
+// longer row takes longer than the launches), and while a null's cells are few
+// for the 128 warps of its cluster: the launches spread a depth over all SMs,
+// so the fewer the nulls, the sooner they win.  Measured against the launches
+// (us, the whole null generation): 30 x 61, 20 nulls 46 / 77 (C = 1); 100 x 120
+// 112 / 151; 400 x 300 238 / 375; 700 x 900 289 / 336; 2,000 x 300 530 / 545;
+// but 500 x 400 with 200 nulls 803 / 762, 100 x 3,000 263 / 205, 8,000 x 64
+// with 20 nulls 485 / 448, 4,000 x 300 with nine 710 / 636, 2,000 x 1,000 with
+// five 365 / 281; with one null 2,000 x 64 172 / 189 and 3,000 x 64 218 / 222,
+// 1,000 x 300 321 / 280 and 20,000 x 600 1,760 / 490.
 static int null_cluster(int N, int L, int nnull) {
-  if (L > 1024 || (double)N * L * nnull > 13e6) return 0;
+  if (L > 1024 || (double)N * L * nnull > 13e6 || (double)N * L > (nnull < 4 ? 0.2e6 : 0.7e6)) return 0;
   if ((int64_t)N * L < 8192) return 1;
   int dev = 0, nsm = 152, C = 8;
   cudaGetDevice(&dev);
