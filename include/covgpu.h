@@ -307,6 +307,13 @@ int  covgpu_autotune(covgpu_ctx *ctx, int first_slot, int nslots, int ncand, con
  * nT < 1, jcap too small). */
 int  covgpu_tile_order(int nT, int schedule, int *order, int *jpairs, int jcap, int *njpairs);
 
+/* host code (no device): the shape of covgpu_weights_gsc_dev's launch for N
+ * sequences on a device that places clusters of up to max_cluster CTAs: the
+ * cluster's CTAs and the rows per lane of its first warps (32 ctas rows >= N).
+ * Returns 0, or 11 where no shape holds N (more than 16,384, or 8,192 without
+ * clusters of 16). */
+int  covgpu_gsc_shape(int N, int max_cluster, int *ctas, int *rows);
+
 /* writes a 256 MB device buffer (larger than L2) on the context's stream */
 int  covgpu_flush_l2(covgpu_ctx *ctx);
 

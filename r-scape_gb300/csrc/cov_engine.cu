@@ -471,6 +471,8 @@ extern "C" int covgpu_weights_gsc_dev(covgpu_ctx* ctx, int slot, int set, double
   if (slot < 0 || slot >= ctx->maxslots || !wgt) return fail(ctx, 11, "bad slot or output");
   if (N > 16384) return fail(ctx, 11, "GSC weights are for up to 16384 sequences (N^2 distances)");
   if (N == 1) { wgt[0] = 1.0; return set ? covgpu_set_weights(ctx, wgt) : 0; }
+  if (N > gsc_max_sequences())
+    return fail(ctx, 90, "GSC weights: this device places clusters for up to %d sequences", gsc_max_sequences());
   // scratch kept across calls (families of a resized context reuse it)
   const size_t need = gsc_scratch_bytes(N, L) + ((size_t)N * sizeof(double) + 256);
   if (ctx->gsc_cap < need) {

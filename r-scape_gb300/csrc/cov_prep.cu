@@ -37,6 +37,7 @@
 #include "cov_dev.cuh"
 #include "cov_prep.h"
 #include "cov_batch.h"
+#include "covgpu.h"
 
 namespace covgpu {
 
@@ -641,40 +642,45 @@ k_gsc_upgma(double* __restrict__ D, int N, double* __restrict__ w, int G, double
   gsc_cluster_body<NR>(D, N, w, G, blockIdx.x % G, state);
 }
 
-// CTAs of the merges' cluster (N <= 16384)
-static int gsc_cluster(int N) { return N <= 256 ? 8 : 16; }
-// rows per lane: the smallest kernel that holds N
+constexpr int GSC_MAXR = 32;   // rows per lane at most
+// f(rows per lane) of the merges' kernel for N sequences
 template <class F>
-static cudaError_t gsc_with_nr(int N, int G, F f) {
-  const int nr = (N + 32 * G - 1) / (32 * G);
-  if (nr <= 1) return f(std::integral_constant<int, 1>());
-  if (nr <= 2) return f(std::integral_constant<int, 2>());
-  if (nr <= 4) return f(std::integral_constant<int, 4>());
-  if (nr <= 16) return f(std::integral_constant<int, 16>());
-  if (nr <= 32) return f(std::integral_constant<int, 32>());
+static cudaError_t gsc_with_nr(int nr, F f) {
+  switch (nr) {
+    case 1: return f(std::integral_constant<int, 1>());
+    case 2: return f(std::integral_constant<int, 2>());
+    case 4: return f(std::integral_constant<int, 4>());
+    case 16: return f(std::integral_constant<int, 16>());
+    case GSC_MAXR: return f(std::integral_constant<int, GSC_MAXR>());
+  }
   return cudaErrorInvalidValue;
 }
 
-template <class... A>
-static cudaError_t gsc_cluster_launch(const void* k, int grid, int G, size_t sm, cudaStream_t st, A... a) {
-  cudaLaunchConfig_t cfg = {};
+static void gsc_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* la, int grid, int G, size_t sm,
+                              cudaStream_t st) {
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(32 * (SCAN_WARPS + 1));
   cfg.dynamicSmemBytes = sm;
   cfg.stream = st;
-  cudaLaunchAttribute la[1];
   la[0].id = cudaLaunchAttributeClusterDimension;
   la[0].val.clusterDim.x = G;
   la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
   cfg.attrs = la;
   cfg.numAttrs = 1;
+}
+template <class... A>
+static cudaError_t gsc_cluster_launch(const void* k, int grid, int G, size_t sm, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute la[1];
+  gsc_launch_config(cfg, la, grid, G, sm, st);
   void* args[] = {(void*)&a...};
   return cudaLaunchKernelExC(&cfg, k, args);
 }
 
 // the merge kernels' limits (shared memory, clusters of 16) on the current
-// device, raised once (before any stream capture)
-static cudaError_t gsc_attrs();
+// device, raised once (before any stream capture), and the largest cluster
+// that the device places
+static cudaError_t gsc_attrs(int* max_cluster);
 
 size_t gsc_scratch_bytes(int N, int L) {
   const size_t Lw = ((size_t)L + 3) / 4;
@@ -691,16 +697,16 @@ cudaError_t launch_weights_gsc(const uint8_t* ax, int N, int L, int Lp, void* sc
   uint32_t* ra = (uint32_t*)p;            p += (size_t)N * Lw * sizeof(uint32_t);
   uint32_t* rb = (uint32_t*)p;            p += (size_t)N * Lw * sizeof(uint32_t);
   int* len = (int*)p;
-  if (N < 2) return cudaErrorInvalidValue;
-  const cudaError_t e = gsc_attrs();
+  int maxc = 0, G = 0, nr = 0;
+  const cudaError_t e = gsc_attrs(&maxc);
   if (e != cudaSuccess) return e;
+  if (N < 2 || covgpu_gsc_shape(N, maxc, &G, &nr)) return cudaErrorInvalidValue;
   k_gsc_codes<<<N, 256, 0, st>>>(ax, N, L, Lp, Lw, ra, rb, len);
   const int nt = (N + 31) / 32;
   k_gsc_ident<<<dim3(nt, nt), 256, 0, st>>>(ra, rb, len, N, Lw, D);
   // all merges in one launch of one cluster
-  const int G = gsc_cluster(N);
-  return gsc_with_nr(N, G, [&](auto nr) {
-    return gsc_cluster_launch((const void*)k_gsc_upgma<decltype(nr)::value>, G, G, gsc_cluster_smem(N), st, D, N, w, G,
+  return gsc_with_nr(nr, [&](auto rows) {
+    return gsc_cluster_launch((const void*)k_gsc_upgma<decltype(rows)::value>, G, G, gsc_cluster_smem(N), st, D, N, w, G,
                               state);
   });
 }
@@ -721,7 +727,7 @@ cudaError_t launch_gapfilter(const uint8_t* ax, const double* wgt, int N, int L,
 
 // ------------------------------------------------------------------------
 // grouped launches over a batch of families: position-based weights of the
-// families with pb set, GSC weights (one CTA per family for the merges) of
+// families with pb set, GSC weights (a cluster per family for the merges) of
 // those with gsc set
 // ------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
@@ -761,23 +767,34 @@ k_gsc_upgma_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pr
   gsc_cluster_body<NR>(d.gD, d.N, d.w, G, (int)blockIdx.x % G, nullptr);
 }
 
-static cudaError_t gsc_attrs() {
+static cudaError_t gsc_attrs(int* max_cluster) {
   constexpr int MAXDEV = 64;
-  static std::atomic<int> done[MAXDEV];
+  static std::atomic<int> known[MAXDEV];   // the largest cluster, 0: not asked yet
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < MAXDEV && done[dev].load()) return cudaSuccess;
+  if (dev < MAXDEV && (*max_cluster = known[dev].load()) > 0) return cudaSuccess;
   const void* k[] = {(const void*)k_gsc_upgma<1>, (const void*)k_gsc_upgma<2>, (const void*)k_gsc_upgma<4>,
-                     (const void*)k_gsc_upgma<16>, (const void*)k_gsc_upgma<32>, (const void*)k_gsc_upgma_grp<1>, (const void*)k_gsc_upgma_grp<2>,
-                     (const void*)k_gsc_upgma_grp<4>, (const void*)k_gsc_upgma_grp<16>,
-                     (const void*)k_gsc_upgma_grp<32>};
+                     (const void*)k_gsc_upgma<16>, (const void*)k_gsc_upgma<32>, (const void*)k_gsc_upgma_grp<1>,
+                     (const void*)k_gsc_upgma_grp<2>, (const void*)k_gsc_upgma_grp<4>,
+                     (const void*)k_gsc_upgma_grp<16>, (const void*)k_gsc_upgma_grp<32>};
+  int maxc = GSC_MAXG;
   for (const void* f : k) {
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GSC_SMEM_MAX)) != cudaSuccess)
       return e;
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+    // 16 CTAs with the most shared memory that they may take in one GPC?
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute la[1];
+    gsc_launch_config(cfg, la, GSC_MAXG, GSC_MAXG, GSC_SMEM_MAX, nullptr);
+    if (cudaOccupancyMaxActiveClusters(&n, f, &cfg) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      maxc = 8;
+    }
   }
-  if (dev < MAXDEV) done[dev].store(1);
+  if (dev < MAXDEV) known[dev].store(maxc);
+  *max_cluster = maxc;
   return cudaSuccess;
 }
 
@@ -794,12 +811,13 @@ cudaError_t grp_weights_pb(const FamDev* F, int nf, const int* pre_col, int nb_c
 cudaError_t grp_weights_gsc(const FamDev* F, int nf, const int* pre_codes, int nb_codes, const int* pre_ident,
                             int nb_ident, const int* pre_upgma, int nb_upgma, int maxN, cudaStream_t st) {
   if (nb_upgma <= 0) return cudaSuccess;
-  const int G = gsc_cluster(maxN);
-  if (gsc_state_global(maxN) || !grp_weights_gsc_prepare()) return cudaErrorInvalidValue;
+  int maxc = 0, G = 0, nr = 0;
+  if (gsc_state_global(maxN) || gsc_attrs(&maxc) != cudaSuccess || covgpu_gsc_shape(maxN, maxc, &G, &nr))
+    return cudaErrorInvalidValue;
   if (nb_codes > 0) k_gsc_codes_grp<<<nb_codes, 256, 0, st>>>(F, nf, pre_codes);
   if (nb_ident > 0) k_gsc_ident_grp<<<nb_ident, 256, 0, st>>>(F, nf, pre_ident);
-  return gsc_with_nr(maxN, G, [&](auto nr) {
-    return gsc_cluster_launch((const void*)k_gsc_upgma_grp<decltype(nr)::value>, nb_upgma * G, G,
+  return gsc_with_nr(nr, [&](auto rows) {
+    return gsc_cluster_launch((const void*)k_gsc_upgma_grp<decltype(rows)::value>, nb_upgma * G, G,
                               gsc_cluster_smem(maxN), st, F, nf, pre_upgma, G);
   });
 }
@@ -888,7 +906,15 @@ cudaError_t grp_weights_limbs(FamDev* F, int nf, const int* pre, int nb, UmmaFam
 }
 
 // the merges' limits, raised outside any stream capture
-int grp_weights_gsc_prepare() { return gsc_attrs() == cudaSuccess ? 1 : 0; }
+int grp_weights_gsc_prepare() {
+  int maxc;
+  return gsc_attrs(&maxc) == cudaSuccess ? 1 : 0;
+}
+
+int gsc_max_sequences() {
+  int maxc = 0;
+  return gsc_attrs(&maxc) == cudaSuccess ? 32 * GSC_MAXR * maxc : 0;
+}
 
 // rows of L bytes, one after the other, to a pitch of Lp: 16 bytes of a row
 // per thread, from the aligned words around them (src: aligned, readable for
@@ -927,3 +953,15 @@ cudaError_t launch_spread_rows(const uint8_t* src, int N, int L, int Lp, uint8_t
 }
 
 }  // namespace covgpu
+
+// CTAs of the merges' cluster: 16 for more than 256 sequences where the device
+// places such a cluster (16 is beyond the portable size), else 8; rows per
+// lane: the smallest kernel that holds N
+extern "C" int covgpu_gsc_shape(int N, int max_cluster, int* ctas, int* rows) {
+  if (N < 1 || max_cluster < 8 || !ctas || !rows) return 11;
+  *ctas = (N <= 256 || max_cluster < covgpu::GSC_MAXG) ? 8 : covgpu::GSC_MAXG;
+  const int need = (N + 32 * *ctas - 1) / (32 * *ctas);
+  for (int r : {1, 2, 4, 16, covgpu::GSC_MAXR})
+    if (need <= r) { *rows = r; return 0; }
+  return 11;
+}

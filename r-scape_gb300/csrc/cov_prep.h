@@ -11,6 +11,7 @@ cudaError_t launch_weights_pb(const uint8_t* ax, int N, int L, int Lp, double* i
 // unnormalised GSC weights w[N] (scratch of gsc_scratch_bytes(N, L) bytes,
 // 16-byte aligned)
 size_t      gsc_scratch_bytes(int N, int L);
+int         gsc_max_sequences();   // of the current device: 16384, 8192 without clusters of 16 CTAs (0: error)
 cudaError_t launch_weights_gsc(const uint8_t* ax, int N, int L, int Lp, void* scratch, double* w, cudaStream_t st);
 // useme[L]: 1 where the weighted residue fraction is at least 1 - gapthresh
 // (wgt null: unit weights)

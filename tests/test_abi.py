@@ -437,3 +437,21 @@ def test_covgpu_and_oracle_ctypes_mirrors_match(covgpu, oracle, tmp_path):
     _c_layouts_match(tmp_path, os.path.join(ROOT, "oracle"), "rscape_oracle.h",
                      [("orc_tree_t", oracle.Tree), ("orc_params_t", oracle.Params), ("orc_result_t", oracle.Result)],
                      {("orc_result_t", "lambda_"): "lambda"})
+
+
+@pytest.mark.parametrize("max_cluster", [8, 16])
+def test_gsc_launch_shapes_hold_every_size(covgpu, max_cluster):
+    """The cluster of the GSC merges and its rows per lane hold N sequences,
+    with no more CTAs than the device places, for every N up to the limit."""
+    lib = ctypes.CDLL(covgpu.LIBPATH)
+    g, r = ctypes.c_int(), ctypes.c_int()
+    limit = 1024 * max_cluster
+    for N in list(range(1, 1100)) + [2048, 2049, 4096, 4097, 8192, 8193, 16384]:
+        st = lib.covgpu_gsc_shape(N, max_cluster, ctypes.byref(g), ctypes.byref(r))
+        if N > limit:
+            assert st == 11, N
+            continue
+        assert st == 0 and g.value <= max_cluster and 32 * g.value * r.value >= N, N
+        assert r.value in (1, 2, 4, 16, 32)
+    assert lib.covgpu_gsc_shape(limit + 1, max_cluster, ctypes.byref(g), ctypes.byref(r)) == 11
+    assert lib.covgpu_gsc_shape(100, 4, ctypes.byref(g), ctypes.byref(r)) == 11
