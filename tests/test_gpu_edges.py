@@ -373,3 +373,69 @@ def test_batch_with_a_deep_family(covgpu, deep):
         e.close()
         for k in ("null_minCOV", "null_maxCOV", "h_nb", "h_imin", "h_imax", "h_n", "nhit"):
             assert rows[0][k] == one[k], k
+
+
+def _gsc_merge_by_merge(ax):
+    """GSC weights on UPGMA in numpy, a merge at a time in FP64: the closest
+    pair, ties to the first in row-major order; the operations of the oracle,
+    whose search over all pairs takes too long beyond a thousand sequences."""
+    N, L = ax.shape
+    X = np.stack([(ax == k) for k in range(4)], 2).reshape(N, -1).astype(np.float32)
+    n = (ax < 4).sum(1).astype(np.float64)
+    mn = np.minimum(n[:, None], n[None, :])
+    D = np.where(mn > 0, 1.0 - (X @ X.T).astype(np.float64) / np.maximum(mn, 1.0), 1.0)
+    np.fill_diagonal(D, np.inf)
+    up = np.array([(D[a, a + 1:].min(), a + 1 + D[a, a + 1:].argmin()) if a + 1 < N else (np.inf, 0)
+                   for a in range(N)])
+    rmin, rarg = up[:, 0].copy(), up[:, 1].astype(int)
+    w, cl = np.zeros(N), np.arange(N)
+    size, height, cw, alive = np.ones(N), np.zeros(N), np.zeros(N), np.ones(N, dtype=bool)
+
+    def rescan(r):
+        k = D[r, r + 1:].argmin() if r + 1 < N else 0
+        rmin[r], rarg[r] = (D[r, r + 1 + k], r + 1 + k) if r + 1 < N else (np.inf, 0)
+
+    for _ in range(N - 1):
+        a = int(rmin.argmin())
+        b = int(rarg[a])
+        h = D[a, b] / 2.0
+        bl = [max(h - height[k], 0.0) for k in (a, b)]
+        for k, x in ((a, bl[0]), (b, bl[1])):
+            m = cl == k
+            w[m] += x * w[m] / cw[k] if cw[k] > 0 else x / size[k]
+        cl[cl == b] = a
+        x = (D[a] * size[a] + D[b] * size[b]) / (size[a] + size[b])
+        alive[b] = False
+        x[~alive] = np.inf
+        x[a] = np.inf
+        D[a], D[:, a] = x, x
+        D[b], D[:, b] = np.inf, np.inf
+        cw[a] = (cw[a] + bl[0]) + (cw[b] + bl[1])
+        size[a], height[a], rmin[b] = size[a] + size[b], h, np.inf
+        lost = alive & ((rarg == a) | (rarg == b))
+        lost[a] = True
+        below = np.flatnonzero(alive[:a] & ~lost[:a])
+        better = below[(x[below] < rmin[below]) | ((x[below] == rmin[below]) & (a < rarg[below]))]
+        rmin[better], rarg[better] = x[better], a
+        for r in np.flatnonzero(lost):
+            rescan(r)
+    return w * N / w.sum()
+
+
+@pytest.mark.parametrize("N,L", [(300, 40), (2100, 60), (4097, 30), (8200, 48)])
+def test_gsc_weights_of_deep_alignments(covgpu, oracle, N, L):
+    """16 and 32 rows per lane, and the weights' state in global memory (8,200
+    sequences), against a merge at a time on the host; the smallest size also
+    against the oracle."""
+    s = covgpu.Synth(N, L, 1.0, 2, 1, 1, 2, 0.1, seed=N, tree_kind=1)
+    rng = np.random.default_rng(N)
+    dup = rng.integers(0, N, size=(N // 20, 2))
+    s.ax[dup[:, 1]] = s.ax[dup[:, 0]]
+    ref = _gsc_merge_by_merge(s.ax)
+    if N <= 1000:
+        assert np.allclose(ref, oracle.weights_gsc(s.ax), rtol=1e-10, atol=1e-13)
+    e = covgpu.Engine(N, L)
+    e.set_alignment(0, s.ax)
+    g = e.weights_gsc(0, set=False)
+    e.close()
+    assert np.allclose(g, ref, rtol=1e-10, atol=1e-13)
