@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "cov_dev.cuh"
+#include "cov_div.cuh"
 #include "cov_fit.h"
 
 namespace covgpu {
@@ -29,23 +30,6 @@ namespace covgpu {
 // number of FP64 instructions of the longest warp, comparisons and
 // conversions from integers among them: tests are made on the words where
 // the words decide, and independent parts go to different warps.
-
-// x / b, |b| and |x| within div_range: the hardware's approximate reciprocal
-// (20 bits), one third-order Newton step and one residual correction of the
-// quotient (Markstein, IBM J. Res. Dev. 34, 1990): six FP64 instructions.
-// Equal to the IEEE quotient on 5e8 random pairs.
-__device__ __forceinline__ double div_fast(double x, double b) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-  double e = __fma_rn(-b, r, 1.0);
-  e = __fma_rn(e, e, e);
-  r = __fma_rn(r, e, r);
-  const double q = __dmul_rn(x, r);
-  return __fma_rn(__fma_rn(-q, b, x), r, q);
-}
-__device__ __forceinline__ bool div_range(double x) {   // ~1e-30 .. 1e30, either sign
-  return (unsigned)((__double2hiint(x) & 0x7fffffff) - 0x39b4484c) < (unsigned)(0x46293e59 - 0x39b4484c);
-}
 
 // |t| < eps |s| (or <=): where the exponents are at most `far` apart it is
 // false and from `near` on true, for an eps between 2^-(near - 1) and
@@ -739,7 +723,7 @@ cudaError_t launch_survfit(int cmin, int nb, double bmin, double w, double mass,
   // next to x = tau + 1 take ~60 steps of the fraction, the others ~10): two
   // lanes to a bin until the short warps, several to a scheduler, take as long
   // as that one, then a lane each.  1,440 bins (30 x 61): 69 us a lane per bin
-  // with IEEE divisions, 57 us with div_fast, 47 us in pairs.
+  // with IEEE divisions, 57 us with div_fast, 48 us in pairs.
   if (!doexp && n <= 64 * 4 * nsm) {
     k_survfit_pair<<<std::max(1, (n + 15) / 16), 32, 0, st>>>(cmin, nb, bmin, w, mass, mu, lambda, tau, lga, d_sf);
   } else {

@@ -21,6 +21,7 @@
 // the E-value tables.
 #include "cov_dev.cuh"
 #include "cov_df2.cuh"
+#include "cov_div.cuh"
 #include "cov_kernels.h"
 #include "cov_batch.h"
 
@@ -1606,8 +1607,8 @@ k_evalue(const float2* __restrict__ cov, const TileRC* __restrict__ tiles, int n
 //
 // A CTA takes 256 pairs of a tile (four CTAs to a tile: few tiles leave SMs
 // idle), a warp 32 pairs of one row.  The 16 quotients have one divisor: its
-// reciprocal once, then a product and two residual corrections each (equal to
-// the IEEE quotient: Markstein, IBM J. Res. Dev. 34, 1990).  The values go
+// reciprocal once, then a product and two residual corrections each (div_by, the
+// IEEE quotient).  The values go
 // through shared memory, so that 16 lanes write the 128 bytes of a pair.
 // Bound by the FP64 pipe; 400 x 351: 70 us with a thread per pair of a whole
 // tile writing its own 16 values, 33 us so.
@@ -1636,11 +1637,8 @@ k_probs_host_layout(const float* __restrict__ cnt, const TileRC* __restrict__ ti
       for (int q = 0; q < 16; q++) { C[q] = __dadd_rn(1e-10, C[q]); sum = __dadd_rn(sum, C[q]); }
       const double r = __drcp_rn(sum);
 #pragma unroll
-      for (int q = 0; q < 16; q++) {
-        double v = __dmul_rn(C[q], r);
-        v = __fma_rn(__fma_rn(-v, sum, C[q]), r, v);
-        sv[warp][lane * 17 + q] = __fma_rn(__fma_rn(-v, sum, C[q]), r, v);
-      }
+      for (int q = 0; q < 16; q++)
+        sv[warp][lane * 17 + q] = div_by(C[q], sum, r);
     }
   }
   if (!pp) return;

@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "cov_dev.cuh"
+#include "cov_div.cuh"
 #include "cov_prep.h"
 #include "cov_batch.h"
 #include "covgpu.h"
@@ -242,19 +243,10 @@ __device__ __forceinline__ unsigned long long dkey(double d) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(d);
   return (u <= 0x7FF0000000000000ull) ? u : ~0ull;
 }
-// x / b correctly rounded from y = 1 / b correctly rounded: a quotient within
-// two ulps and two residual steps with exact FMA residuals (Markstein, IBM J.
-// Res. Dev. 34, 1990: a faithful quotient plus one such step is the correctly
-// rounded one).  Five FP64 operations where the reciprocal is shared by a whole
-// merge, against the general division's several dozen: this part issues two
-// FP64 operations per cycle and SM.  Finite x and b well inside the exponent
-// range.
-__device__ __forceinline__ double div_by(double x, double b, double y) {
-  double q = __dmul_rn(x, y);
-  q = __fma_rn(__fma_rn(-q, b, x), y, q);
-  return __fma_rn(__fma_rn(-q, b, x), y, q);
-}
-
+// A merge's distances have one divisor, so they are quotients by div_by: five
+// FP64 operations against the general division's several dozen, in a part that
+// issues two FP64 operations per cycle and SM.
+//
 // ------------------------------------------------------------------------
 // UPGMA by one cluster of G CTAs, one cluster barrier per merge.
 // Index i (row, column, leaf) belongs to CTA i % G.  Every CTA keeps a private

@@ -1,5 +1,9 @@
 """Kernel variants at the sizes where they can go wrong: tile edges, the
 smallest and largest of a variant's range, remainders (needs a GB300)."""
+import ctypes
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -439,3 +443,72 @@ def test_gsc_weights_of_deep_alignments(covgpu, oracle, N, L):
     g = e.weights_gsc(0, set=False)
     e.close()
     assert np.allclose(g, ref, rtol=1e-10, atol=1e-13)
+
+
+def _hard_quotients(rng, n, near):
+    """x, b whose quotient lies within 2^-105 of the middle of two numbers: b an
+    odd 53-bit integer, m the odd 54-bit middle with m b = -+1 mod 2^54, x = (m b
+    +- 1) / 2^54.  near: b near a power of two."""
+    xs, bs = [], []
+    while len(xs) < n:
+        b = int(rng.integers(1 << 52, 1 << 53)) | 1
+        if near:
+            k = int(rng.integers(0, 1 << 12)) | 1
+            b = (1 << 52) + k if len(xs) & 1 else (1 << 53) - k
+        for sgn in (1, -1):
+            m = (-sgn * pow(b, -1, 1 << 54)) % (1 << 54)
+            if m < 1 << 53:
+                continue
+            x = (m * b + sgn) >> 54
+            xs.append(float(x))
+            bs.append(float(b))
+    return np.array(xs[:n]), np.array(bs[:n])
+
+
+@pytest.mark.parametrize("kind", ["div_fast", "div_by"])
+def test_quotients_against_cuda_division(tmp_path, kind):
+    """The corrected quotients beside CUDA's division: random operands over
+    div_range and at its ends, operands next to powers of two, equal quotients
+    and small integers, and the hardest cases for rounding.  div_by is the
+    rounded quotient everywhere; div_fast too, but for the hardest cases, where
+    it may be the neighbour (its reciprocal may be an ulp off); outside
+    div_range nothing is claimed of div_fast."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    so = str(tmp_path / "quotients.so")
+    subprocess.run([os.environ.get("NVCC", "nvcc"), "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17",
+                    "-Xcompiler", "-fPIC", "-shared", "-I", os.path.join(here, "..", "r-scape_gb300", "csrc"),
+                    os.path.join(here, "quotients.cu"), "-o", so], check=True)
+    lib = ctypes.CDLL(so)
+    rng = np.random.default_rng(17)
+    n = 1 << 22
+
+    def run(x, b):
+        x, b = (np.ascontiguousarray(v, dtype=np.float64) for v in np.broadcast_arrays(x, b))
+        q, r, ok = np.zeros(len(x)), np.zeros(len(x)), np.zeros(len(x), dtype=np.int32)
+        assert lib.quotients(int(kind == "div_by"), *[ctypes.c_void_p(v.ctypes.data) for v in (x, b)], len(x),
+                             *[ctypes.c_void_p(v.ctypes.data) for v in (q, r, ok)]) == 0
+        return q, r, ok
+
+    def mantissa(size):
+        return rng.uniform(1.0, 2.0, size) * rng.choice([-1.0, 1.0], size)
+
+    sets = [(mantissa(n) * 2.0 ** rng.integers(-98, 99, n), mantissa(n) * 2.0 ** rng.integers(-98, 99, n)),
+            (mantissa(n) * 2.0 ** rng.choice([-98, 98], n), mantissa(n) * 2.0 ** rng.choice([-98, 98], n)),
+            (1.0 + 2.0 ** -52 * rng.integers(0, 64, n), 2.0 - 2.0 ** -52 * rng.integers(1, 64, n)),
+            (2.0 - 2.0 ** -52 * rng.integers(1, 64, n), 1.0 + 2.0 ** -52 * rng.integers(0, 64, n)),
+            (rng.integers(0, 5000, n).astype(float), rng.integers(1, 5000, n).astype(float))]
+    for x, b in sets:
+        q, r, ok = run(x, b)
+        assert np.array_equal(q, r)
+    for near in (False, True):
+        x, b = _hard_quotients(rng, 20000, near)
+        q, r, ok = run(x, b)
+        off = q != r
+        print("%s: %d of %d hard quotients the other neighbour" % (kind, off.sum(), len(x)))
+        assert np.all(np.abs(q - r) <= np.spacing(np.abs(r)))
+        if kind == "div_by":
+            assert not off.any()
+    # the ends of div_range
+    e = np.array([0.0, 0.99e-30, 1.01e-30, 0.99e30, 1.01e30, np.inf, np.nan])
+    ok = run(e, np.full(len(e), 1.0))[2]
+    assert ok.tolist() == [0, 0, 1, 1, 0, 0, 0]
