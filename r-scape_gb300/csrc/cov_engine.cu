@@ -218,7 +218,8 @@ extern "C" int covgpu_create(covgpu_ctx** ret, int device, int N, int L, int max
   CK(cudaMemset(ctx->d_status, 0, sizeof(int)));
   CK(dalloc(&ctx->d_nhits, MAXOUT + 1));   // per statistic, and the --structured pass's
   if (maxnull > 0 && N > 1) {
-    CK(dalloc(&ctx->d_fitch, (size_t)maxnull * (N - 1) * ctx->Lp));
+    // a root's row per null, or all states of one reconstruction (covgpu_substitutions)
+    CK(dalloc(&ctx->d_fitch, (size_t)std::max(maxnull, N - 1) * ctx->Lp));
     CK(dalloc(&ctx->d_scratch, (size_t)maxnull * (N - 1) * ctx->Lp));
     CK(dalloc(&ctx->d_bsub, (size_t)maxnull * 2 * N * 25));
   }

@@ -142,7 +142,7 @@ struct NullTree {
 // nid): F [N-1][Lp] states of the internal nodes, S [N-1][Lp] scratch sets
 cudaError_t launch_fitch_recon(const uint8_t* ax, int N, int L, int Lp, const NullTree& T, const int* level_nodes,
                                int nlevels, uint64_t seed, uint32_t nid, uint8_t* F, uint8_t* S, cudaStream_t st);
-// nulls first_null .. of the alignment ax into out_ax; fitch, rows
+// nulls first_null .. of the alignment ax into out_ax; fitch [nnull][Lp], rows
 // [nnull][N-1][Lp] and ns [nnull][2N][25] scratch; *nlaunch gains the launches
 cudaError_t launch_nullgen(const uint8_t* ax, int N, int L, int Lp, const NullTree& T, const int* level_nodes,
                            const int* level_off, int nlevels, uint64_t seed, uint32_t first_null, int nnull,

@@ -29,7 +29,7 @@
 // Random draws are counter-based (Philox keyed by the seed, the null index,
 // the node and the column), so the result does not depend on scheduling.
 //
-// Buffers (per null q): F[q] the root's states (row 0); ns[q][2N][25] the
+// Buffers (per null q): F[q][Lp] the root's states; ns[q][2N][25] the
 // substitutions from state a to state b on the branch above leaf s (entry s)
 // or internal node v (entry N + v), at 5 a + b; SR[q][v][Lp] node v's row of
 // the null alignment; leaf rows go straight to the output alignment slot.
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(fitch_max_threads(FW))
 k_fitch_cols(FitchCols a, int64_t nstride, int64_t sstride) {
   a.nid += blockIdx.y;
   a.SR += blockIdx.y * sstride;
-  a.F += blockIdx.y * sstride;
+  a.F += (int64_t)blockIdx.y * a.Lp;   // the root's rows of the nulls
   if (a.ns) a.ns += blockIdx.y * nstride;
   fitch_cols<FW, KEEP>(a, blockIdx.x);
 }
@@ -251,18 +251,18 @@ k_fitch_cols(FitchCols a, int64_t nstride, int64_t sstride) {
 // the root's row of the null: its states with the columns shuffled
 __device__ __forceinline__ void root_row_body(
     const GridIdx g, int L, int Lp, uint64_t seed, uint32_t first_null, int64_t stride, const uint8_t* __restrict__ F,
-    int64_t fstride, uint8_t* __restrict__ SR) {
+    uint8_t* __restrict__ SR) {
   const int c = g.x * blockDim.x + threadIdx.x, q = g.y;
   if (c >= Lp) return;
   uint32_t rk[6];
   round_keys(seed, TAG_COLPERM, first_null + q, 0, rk);
-  SR[q * stride + c] = (c < L) ? F[q * fstride + feistel_perm((uint32_t)c, feistel_hbits((uint32_t)L), (uint32_t)L, rk)]
-                               : (uint8_t)4;
+  const uint8_t* row = F + (int64_t)q * Lp;
+  SR[q * stride + c] = (c < L) ? row[feistel_perm((uint32_t)c, feistel_hbits((uint32_t)L), (uint32_t)L, rk)] : (uint8_t)4;
 }
 __global__ void __launch_bounds__(256)
 k_root_row(int L, int Lp, uint64_t seed, uint32_t first_null, int64_t stride, const uint8_t* __restrict__ F,
            uint8_t* __restrict__ SR) {
-  root_row_body(native_grid(), L, Lp, seed, first_null, stride, F, stride, SR);
+  root_row_body(native_grid(), L, Lp, seed, first_null, stride, F, SR);
 }
 
 // The replay of one (branch, null) item: the child's row starts as a copy of
@@ -526,7 +526,7 @@ k_null_replay(int N, int L, int Lp, const int* left, const int* right, const int
               uint8_t* out, int64_t out_stride, int csize, bool srow) {
   const int q = blockIdx.x / csize;
   const int64_t off = (int64_t)q * (N - 1) * Lp;
-  const NullOne a{N, L, Lp, left, right, lnodes, loff, nlevels, F + off, ns + (int64_t)q * 2 * N * 25, SR + off,
+  const NullOne a{N, L, Lp, left, right, lnodes, loff, nlevels, F + (int64_t)q * Lp, ns + (int64_t)q * 2 * N * 25, SR + off,
                   out + q * out_stride, seed, first_null + q};
   null_replay(a, blockIdx.x % csize, csize, srow);
 }
@@ -709,7 +709,7 @@ k_root_row_grp(const FamDev* __restrict__ F, int nf, const int* __restrict__ pre
   const int f = grp_find(pre, nf, (int)blockIdx.x);
   const FamDev& d = F[f];
   const int gx = (d.Lp + 255) / 256, loc = (int)blockIdx.x - __ldg(pre + f);
-  root_row_body(GridIdx{loc % gx, loc / gx, gx}, d.L, d.Lp, seed, 0u, (int64_t)(d.N - 1) * d.Lp, d.fitch, d.Lp,
+  root_row_body(GridIdx{loc % gx, loc / gx, gx}, d.L, d.Lp, seed, 0u, (int64_t)(d.N - 1) * d.Lp, d.fitch,
                 d.scratch);
 }
 

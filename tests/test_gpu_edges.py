@@ -512,3 +512,41 @@ def test_quotients_against_cuda_division(tmp_path, kind):
     e = np.array([0.0, 0.99e-30, 1.01e-30, 0.99e30, 1.01e30, np.inf, np.nan])
     ok = run(e, np.full(len(e), 1.0))[2]
     assert ok.tolist() == [0, 0, 1, 1, 0, 0, 0]
+
+
+def test_null_buffers_hold_what_the_generator_uses(covgpu):
+    """A context's device memory per null: the null's internal rows and its
+    branch counters (200 bytes per sequence); of the reconstruction only the
+    root's row is kept."""
+    import torch
+    N, L, Lp, ns = 4000, 500, 512, 200
+
+    def used(maxnull):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        e = covgpu.Engine(N, L, maxslots=1, maxnull=maxnull)
+        after = torch.cuda.mem_get_info()[0]
+        e.close()
+        return before - after
+
+    used(1)
+    per = (used(ns) - used(1)) / (ns - 1)
+    assert per <= 1.05 * N * (Lp + 200), per / N
+
+
+@pytest.mark.parametrize("N,L,ns", [(5, 40, 30), (60, 100, 3)])
+def test_reconstruction_and_nulls_share_a_buffer(covgpu, oracle, N, L, ns):
+    """More nulls than internal nodes and fewer: nulls, the reconstruction of
+    the same context, the nulls again."""
+    s = covgpu.Synth(N, L, 1.5, 4, 1, 4, 4, 0.1, seed=N)
+    e = covgpu.Engine(N, L, maxslots=ns + 1, maxnull=ns)
+    e.set_alignment(0, s.ax)
+    e.set_tree(s.parent, s.left, s.right)
+    T = oracle.TreeArrays(s.parent, s.left, s.right, s.ld, s.rd)
+    for _ in range(2):
+        e.make_nulls(7, 0, ns, 1)
+        for q in (0, ns - 1):
+            assert np.array_equal(e.get_alignment(1 + q), oracle.null_msa(s.ax, T, 7, q)), q
+        for got, ref in zip(e.substitutions(0, seed=9), oracle.substitutions(s.ax, T, 9, 0xFFFFFFFF)):
+            assert np.array_equal(got, ref)
+    e.close()
