@@ -106,8 +106,9 @@ struct covgpu_ctx {
   void* d_gsc = nullptr;       // GSC scratch, kept across calls
   size_t gsc_cap = 0;
   double* d_pbscr = nullptr;   // position-based weights scratch
-  // workspace of the calls that finish before they return (substitutions,
-  // power, gap filter, aggregation); grown when a call needs more
+  // workspace of the calls that finish before they return (alignment uploads,
+  // substitutions, power, gap filter, aggregation); grown when a call needs
+  // more, kept up to kWorkKeep bytes
   unsigned char* d_wrk = nullptr;
   size_t wrk_cap = 0;
   bool want_qsum = false;     // covgpu_rscape keeps the null-score summary of type 0
@@ -275,6 +276,21 @@ static cudaError_t work_reserve(covgpu_ctx* ctx, size_t n) {
   if (e == cudaSuccess) ctx->wrk_cap = n;
   return e;
 }
+// Gives a large workspace back when the call that took it ends (24 bytes per
+// pair of columns of covgpu_power: 108 MB at L = 3,000), so that a context does
+// not hold for its life what its largest call needed.
+constexpr size_t kWorkKeep = (size_t)64 << 20;
+struct WorkScope {
+  covgpu_ctx* ctx;
+  explicit WorkScope(covgpu_ctx* c) : ctx(c) {}
+  WorkScope(const WorkScope&) = delete;
+  ~WorkScope() {
+    if (ctx->wrk_cap <= kWorkKeep) return;
+    cudaFree(ctx->d_wrk);
+    ctx->d_wrk = nullptr;
+    ctx->wrk_cap = 0;
+  }
+};
 
 // A caller's result array is often fresh memory whose pages do not exist yet.
 // A copy from the device into such pages raises a fault on each (64 KB) from
@@ -362,6 +378,7 @@ extern "C" int covgpu_set_alignment(covgpu_ctx* ctx, int slot, const uint8_t* ax
   // one flat copy and a kernel that spreads the rows: the copy of rows to a
   // pitch runs row by row (20000 x 1500: 875 us, 181 + 11 us so; 30 x 61:
   // 16 us, 8 + 3 us).  Without room for the staging buffer, the pitched copy.
+  WorkScope scope(ctx);
   if (ctx->L != ctx->Lp && work_reserve(ctx, (size_t)n + 32) == cudaSuccess) {
     CK(cudaMemcpyAsync(ctx->d_wrk, ax, (size_t)n, cudaMemcpyHostToDevice, ctx->st));
     CK(launch_spread_rows(ctx->d_wrk, ctx->N, ctx->L, ctx->Lp, dst, ctx->st));
@@ -513,6 +530,7 @@ extern "C" int covgpu_substitutions(covgpu_ctx* ctx, int slot, uint64_t seed, in
   const bool own = F && S;
   const int Wb = (2 * (N - 1) + 31) / 32;
   const size_t nbits = 2 * (size_t)L * Wb * sizeof(uint32_t);
+  WorkScope scope(ctx);
   cudaError_t e = work_reserve(ctx, nbits + (own ? 0 : 256 + 2 * rows));
   if (e != cudaSuccess) return fail(ctx, 90, "CUDA error %s", cudaGetErrorString(e));
   uint32_t* bits = (uint32_t*)ctx->d_wrk;
@@ -557,6 +575,7 @@ extern "C" int covgpu_power(covgpu_ctx* ctx, int ns, const double* subs, const d
     if (src[k]) for (int s = 0; s < ns; s++) tab[(size_t)k * ns + s] = src[k][s];
   const int64_t P = (int64_t)L * (L - 1) / 2;
   const int T = power_table_size(ctx->N, L);
+  WorkScope scope(ctx);
   CK(work_reserve(ctx, (tab.size() + 3 * ((size_t)P + T)) * sizeof(double)));
   double *d_tab = (double*)ctx->d_wrk, *d_out = d_tab + tab.size(), *d_F = d_out + 3 * P;
   cudaError_t e = cudaSuccess;
@@ -579,6 +598,7 @@ extern "C" int covgpu_gapfilter_dev(covgpu_ctx* ctx, int slot, const double* wgt
   CK(cudaSetDevice(ctx->dev));
   const int N = ctx->N, L = ctx->L, Lp = ctx->Lp;
   if (slot < 0 || slot >= ctx->maxslots || !useme) return fail(ctx, 11, "bad slot or output");
+  WorkScope scope(ctx);
   CK(work_reserve(ctx, (wgt ? (size_t)N * sizeof(double) : 0) + (size_t)L * sizeof(int)));
   double* d_w = wgt ? (double*)ctx->d_wrk : nullptr;
   int* d_use = (int*)(ctx->d_wrk + (wgt ? (size_t)N * sizeof(double) : 0));
@@ -1637,6 +1657,7 @@ extern "C" int covgpu_aggregate(covgpu_ctx* ctx, int method, int nh, const int* 
     if (need_aux && !(aux[k] >= 0.0 && std::isfinite(aux[k]))) return fail(ctx, 11, "weight %d is negative", k);
   }
   const size_t nd = (size_t)nbp * 4 + nh + 1;   // pval, aux, term[2], pagg
+  WorkScope scope(ctx);
   CK(work_reserve(ctx, nd * sizeof(double) + ((size_t)nh + 1) * sizeof(int)));
   double* d = (double*)ctx->d_wrk;
   int* d_off = (int*)(d + nd);

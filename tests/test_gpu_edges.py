@@ -550,3 +550,27 @@ def test_reconstruction_and_nulls_share_a_buffer(covgpu, oracle, N, L, ns):
         for got, ref in zip(e.substitutions(0, seed=9), oracle.substitutions(s.ax, T, 9, 0xFFFFFFFF)):
             assert np.array_equal(got, ref)
     e.close()
+
+
+def test_a_large_workspace_is_given_back(covgpu):
+    """covgpu_power takes 24 bytes per pair of columns (108 MB here); the context
+    keeps no more than 64 MB of workspace after the call, and its results do not
+    depend on what it kept."""
+    import torch
+    N, L = 6, 3000
+    s = covgpu.Synth(N, L, 1.5, 8, 1, 4, 8, 0.1, seed=2)
+    e = covgpu.Engine(N, L)
+    e.set_tree(s.parent, s.left, s.right)
+    e.set_alignment(0, s.ax)
+    subs = e.substitutions(0)
+    x = np.arange(8.0)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    first = e.power(single=(x, x / 8), join=(x, x / 8), double=(x, x / 8))
+    assert before - torch.cuda.mem_get_info()[0] <= 66 << 20
+    e.set_alignment(0, s.ax)
+    for a, b in zip(subs, e.substitutions(0)):
+        assert np.array_equal(a, b)
+    for a, b in zip(first, e.power(single=(x, x / 8), join=(x, x / 8), double=(x, x / 8))):
+        assert np.array_equal(a, b)
+    e.close()
