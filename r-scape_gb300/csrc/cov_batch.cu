@@ -10,12 +10,12 @@
 // pitch close to each family's own).  A chunk's buffers sit in one arena,
 // buffer kind by buffer kind (every family's codes, then every family's
 // weights, ...), in the single-family layouts, and every device pass is one
-// grouped launch over the chunk's families (cov_batch.h): weights (GSC with
-// one CTA per family for the merges, or position-based), the nulls (one
-// launch per tree depth over every family), the tensor count (one
-// persistent launch over every (family, alignment, tile) task), marginals,
-// statistics, APC/ASC, histograms, the tail fits (a cluster per fit),
-// survival tables and E-values.  The host steps between the passes
+// grouped launch over the chunk's families (cov_batch.h): weights (GSC with a
+// cluster per family for the merges, or position-based), the nulls (the
+// reconstructions, then one launch per tree depth over every family), the
+// tensor count (one persistent launch over every (family, alignment, tile)
+// task), marginals, statistics, APC/ASC, histograms, the tail fits (a cluster
+// per fit), survival tables and E-values.  The host steps between the passes
 // (cov_rscape_host.h) run for every family and statistic, with one host
 // round trip per phase for the whole chunk.  The device passes from the
 // nulls to the corrected scores are captured once per chunk layout into a

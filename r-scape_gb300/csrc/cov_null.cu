@@ -79,7 +79,7 @@ __device__ __forceinline__ uint32_t state_codes(uint32_t w) {
 }
 // one state of every set of a word: the only member, or a random one; the
 // bytes of pick are considered, the others kept
-__device__ __forceinline__ uint32_t choose_word(uint32_t s, uint32_t pick, int L, uint64_t seed, uint32_t nid,
+__device__ __forceinline__ uint32_t choose_word(uint32_t s, uint32_t pick, uint64_t seed, uint32_t nid,
                                                 uint32_t node, int c0) {
   uint32_t multi = (s & (s - 0x01010101u)) & pick;   // sets are not empty: no borrow between bytes
   while (multi) {   // each lane its next byte: as many draws as the lane with the most
@@ -202,7 +202,7 @@ __device__ __forceinline__ void fitch_cols(const FitchCols& a, int grp) {
     __syncthreads();
   }
   for (int w = tid; w < FW; w += nthr) {   // the root's state
-    const uint32_t s = choose_word(node[w], 0xFFFFFFFFu, a.L, a.seed, a.nid, 0u, c0 + 4 * w);
+    const uint32_t s = choose_word(node[w], 0xFFFFFFFFu, a.seed, a.nid, 0u, c0 + 4 * w);
     node[w] = s;
     *reinterpret_cast<uint32_t*>(a.F + c0 + 4 * w) = state_codes(s);
   }
@@ -216,7 +216,7 @@ __device__ __forceinline__ void fitch_cols(const FitchCols& a, int grp) {
       if (ch > 0) {
         // the parent's state where the child's set holds it, else one of the set
         const uint32_t s = node[(int64_t)ch * stride + w], z = __vcmpeq4(s & p, 0u);
-        q = choose_word((p & ~z) | (s & z), z, a.L, a.seed, a.nid, (uint32_t)ch, c0 + 4 * w);
+        q = choose_word((p & ~z) | (s & z), z, a.seed, a.nid, (uint32_t)ch, c0 + 4 * w);
         node[(int64_t)ch * stride + w] = q;
         if (a.all_rows) *reinterpret_cast<uint32_t*>(a.F + (int64_t)ch * a.Lp + c0 + 4 * w) = state_codes(q);
       } else {
@@ -489,7 +489,7 @@ __device__ __forceinline__ void null_sync(int csize) {
   }
 }
 
-__device__ __forceinline__ void null_replay(const NullOne& a, int crank, int csize, bool srow) {
+__device__ __forceinline__ void null_replay(const NullOne& a, int crank, int csize) {
   extern __shared__ __align__(16) uint8_t rowbuf[];
   __shared__ int cum_s[NULL_WARPS][5][6];
   __shared__ int gcnt[NULL_WARPS][5], base[5];
@@ -507,12 +507,12 @@ __device__ __forceinline__ void null_replay(const NullOne& a, int crank, int csi
     if (n <= csize) {
       if (crank < n) {
         const ReplayItem it = replay_item(a.N, a.Lp, a.left, a.right, a.lnodes + o, crank, a.nid, a.SR, a.out, a.ns);
-        replay_item_cta<NULL_WARPS>(it, a.L, a.Lp, a.seed, cum_s[0], gcnt, base, srow ? rowbuf : nullptr);
+        replay_item_cta<NULL_WARPS>(it, a.L, a.Lp, a.seed, cum_s[0], gcnt, base, rowbuf);
       }
     } else {
       for (int item = warp * csize + crank; item < n; item += NULL_WARPS * csize) {
         const ReplayItem it = replay_item(a.N, a.Lp, a.left, a.right, a.lnodes + o, item, a.nid, a.SR, a.out, a.ns);
-        replay_item_warp(it, a.L, a.Lp, a.seed, lane, cum_s[warp], srow ? rowbuf + (size_t)warp * a.Lp : nullptr);
+        replay_item_warp(it, a.L, a.Lp, a.seed, lane, cum_s[warp], rowbuf + (size_t)warp * a.Lp);
         __syncwarp();
       }
     }
@@ -523,12 +523,12 @@ __device__ __forceinline__ void null_replay(const NullOne& a, int crank, int csi
 __global__ void __launch_bounds__(NULL_WARPS * 32, 2)
 k_null_replay(int N, int L, int Lp, const int* left, const int* right, const int* lnodes, const int* loff,
               int nlevels, uint64_t seed, uint32_t first_null, const uint8_t* F, const int* ns, uint8_t* SR,
-              uint8_t* out, int64_t out_stride, int csize, bool srow) {
+              uint8_t* out, int64_t out_stride, int csize) {
   const int q = blockIdx.x / csize;
   const int64_t off = (int64_t)q * (N - 1) * Lp;
   const NullOne a{N, L, Lp, left, right, lnodes, loff, nlevels, F + (int64_t)q * Lp, ns + (int64_t)q * 2 * N * 25, SR + off,
                   out + q * out_stride, seed, first_null + q};
-  null_replay(a, blockIdx.x % csize, csize, srow);
+  null_replay(a, blockIdx.x % csize, csize);
 }
 
 // items of a launch up to which the replay goes one CTA per item: measured on
@@ -540,7 +540,8 @@ constexpr int64_t kReplayCtaItems = 3000;
 
 bool replay_uses_cta(int64_t items) { return items <= kReplayCtaItems; }
 
-constexpr size_t NULL_SMEM_MAX = 100 * 1024;   // two CTAs per SM
+constexpr int NULL_MAXL = 1024;   // columns up to which one launch may replay a null
+static_assert(NULL_WARPS * NULL_MAXL <= 48 * 1024, "a row per warp within the shared memory that needs no opt-in");
 // CTAs of the cluster that replays one null in one launch, 0: a launch per
 // depth.  One launch wins where the depths are short: up to 13M columns x
 // sequences x nulls in all and rows of 1,024 columns (a warp's walk along a
@@ -554,7 +555,7 @@ constexpr size_t NULL_SMEM_MAX = 100 * 1024;   // two CTAs per SM
 // five 365 / 281; with one null 2,000 x 64 172 / 189 and 3,000 x 64 218 / 222,
 // 1,000 x 300 321 / 280 and 20,000 x 600 1,760 / 490.
 static int null_cluster(int N, int L, int nnull) {
-  if (L > 1024 || (double)N * L * nnull > 13e6 || (double)N * L > (nnull < 4 ? 0.2e6 : 0.7e6)) return 0;
+  if (L > NULL_MAXL || (double)N * L * nnull > 13e6 || (double)N * L > (nnull < 4 ? 0.2e6 : 0.7e6)) return 0;
   if ((int64_t)N * L < 8192) return 1;
   int dev = 0, nsm = 152, C = 8;
   cudaGetDevice(&dev);
@@ -610,9 +611,6 @@ static cudaError_t null_attrs() {
   for (const void* f : fit)
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FITCH_SMEM_MAX)) != cudaSuccess)
       return e;
-  if ((e = cudaFuncSetAttribute(k_null_replay, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NULL_SMEM_MAX)) !=
-      cudaSuccess)
-    return e;
   if (dev < MAXDEV) done[dev].store(1);
   return cudaSuccess;
 }
@@ -649,12 +647,10 @@ cudaError_t launch_nullgen(const uint8_t* ax, int N, int L, int Lp, const NullTr
   if ((e = launch_fitch_cols(a, nnull, nstride, stride, st)) != cudaSuccess) return e;
   const int C = null_cluster(N, L, nnull);
   if (C) {
-    const size_t sm = (size_t)NULL_WARPS * Lp;
-    const bool srow = sm <= NULL_SMEM_MAX;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C * nnull);
     cfg.blockDim = dim3(NULL_WARPS * 32);
-    cfg.dynamicSmemBytes = srow ? sm : 0;
+    cfg.dynamicSmemBytes = (size_t)NULL_WARPS * Lp;
     cfg.stream = st;
     cudaLaunchAttribute la[1];
     la[0].id = cudaLaunchAttributeClusterDimension;
@@ -664,8 +660,7 @@ cudaError_t launch_nullgen(const uint8_t* ax, int N, int L, int Lp, const NullTr
     cfg.numAttrs = 1;
     *nlaunch += 2;
     return cudaLaunchKernelEx(&cfg, k_null_replay, N, L, Lp, T.left, T.right, level_nodes, d_off, nlevels, seed,
-                              first_null, (const uint8_t*)fitch, (const int*)ns, rows, out_ax, out_slot_stride, C,
-                              srow);
+                              first_null, (const uint8_t*)fitch, (const int*)ns, rows, out_ax, out_slot_stride, C);
   }
   k_root_row<<<dim3((Lp + 255) / 256, nnull), 256, 0, st>>>(L, Lp, seed, first_null, stride, fitch, rows);
   *nlaunch += 2;
