@@ -777,7 +777,7 @@ __device__ __forceinline__ void merged_stats(const StatsArgs& A, const df (&c)[1
 // form before (one pair per thread, scalar operations, counts loaded where
 // they are used, one CTA per tile): 70 for 103 warp instructions per pair
 // for GT, MI, CHI and RAF; 8.65 for 9.53 ms on 21 alignments of
-// 2,000 x 3,000; GT alone 1.16 for 1.44 ms on 201 alignments of 500 x 400.
+// 2,000 x 3,000; GT alone 1.18 for 1.44 ms on 201 alignments of 500 x 400.
 constexpr int STATS_UC = 6;   // allowed cells staged; with more, RAF reads its counts directly
 struct StatsSmem {
   float2 ring[3][8][256];             // [row of cells][cell and word][thread]: a plane's two values

@@ -111,51 +111,119 @@ k_pb_rows(const uint8_t* __restrict__ ax, int L, int Lp, const double* __restric
 }
 
 // A column's two sums (residues, residues and gaps) run over the sequences in
-// their order: where the fraction lies on the threshold, the rounding of the
-// sums decides, and any other order decides some columns differently.  So a
-// lane per (column, sum) of 16 columns, the first warp of a CTA, while the
-// other warps stage the next rows' codes and weights (GAP_ROWS, a row each).
-// Bound by the chain of FP64 additions (~64 cycles each); without weights the
-// sums are counts, in integers.  The whole call at N=20,000 x L=1,500: 3.84 ms
-// weighted and 3.34 without weights with a thread per column that read its rows
-// itself, 0.77 and 0.18 so (0.45 and 0.44 with 32 slices summed apart, which
-// gave the columns on the threshold another rounding).
-constexpr int GAP_COLS = 16, GAP_ROWS = 96;
+// their order in FP64: where the fraction lies on the threshold, the rounding of
+// the sums decides, and any other order decides some columns differently.  But
+// that chain of additions (~64 cycles each) is needed only there.  So 32 columns
+// by a CTA of 8 words x 32 slices of the sequences sum the weights in FP32 first:
+// non-negative terms, so the fraction is off by less than (N / 16 + 70) 2^-24 of
+// itself, and a fraction further than twice that from the threshold is decided.
+// The first warp adds the other columns' weights in order, a lane per (column,
+// sum), while the others stage the next rows.  So are all columns where a weight is negative or not finite, the sums
+// leave FP32's range or the threshold is not positive.  Without weights the sums
+// are counts, in integers.
+// The whole call, weighted / without weights: 30 x 61 40 / 35 us with a thread per
+// column that read its rows itself, 23 / 21 so; 2,000 x 1,500 410 / 344, 45 / 29
+// so, 97 with every weighted sum in order; 194 with all columns on the threshold.
+constexpr int GAP_COLS = 32, GAP_SLICES = 32, GAP_ROWS = 96;
 template <bool UNIT>
-__global__ void __launch_bounds__(32 + GAP_ROWS)
+__global__ void __launch_bounds__(8 * GAP_SLICES)
 k_gapfilter(const uint8_t* __restrict__ ax, const double* __restrict__ wgt, int N, int L, int Lp, double idthresh,
             int* __restrict__ useme) {
-  __shared__ uint4 sc[2][GAP_ROWS];
-  __shared__ double sw[2][GAP_ROWS];
-  const int tid = threadIdx.x, c0 = blockIdx.x * GAP_COLS, row = tid - 32;
-  const int col = tid & 15, top = (tid & 16) ? 16 : 15;   // the first warp: residues up to 15, with gaps 16
-  auto stage = [&](int buf, int s) {
-    if (row < 0 || s + row >= N) return;
-    sc[buf][row] = *reinterpret_cast<const uint4*>(ax + (int64_t)(s + row) * Lp + c0);   // Lp is a multiple of 32
-    if (!UNIT) sw[buf][row] = wgt[s + row];
-  };
-  typename std::conditional<UNIT, int, double>::type q = 0;
-  stage(0, 0);
+  typedef typename std::conditional<UNIT, int, float>::type sum_t;
+  __shared__ union {
+    sum_t part[2][GAP_SLICES][GAP_COLS + 1];
+    struct { uint4 code[2][GAP_ROWS][GAP_COLS / 16]; double w[2][GAP_ROWS]; } row;
+  } sm;
+  __shared__ unsigned some, left;   // columns with a weight other than 0; columns to be summed in order
+  __shared__ int odd;               // a weight that is negative or not finite
+  const int tid = threadIdx.x, word = tid & 7, slice = tid >> 3, c0 = blockIdx.x * GAP_COLS;
+  if (tid == 0) { some = 0u; odd = 0; }
   __syncthreads();
-  int buf = 0;
-  for (int s0 = 0; s0 < N; s0 += GAP_ROWS, buf ^= 1) {
-    stage(buf ^ 1, s0 + GAP_ROWS);
-    if (row < 0) {
-      const int n = min(GAP_ROWS, N - s0);
-      const uint8_t* code = reinterpret_cast<const uint8_t*>(sc[buf]) + col;
-#pragma unroll 8
-      for (int s = 0; s < n; s++) {
-        const int x = code[16 * s];
-        const bool in = x <= top && (x != 4 || top == 16);
-        if constexpr (UNIT) q += in;
-        else if (in) q += sw[buf][s];
-      }
+  sum_t r[4] = {0, 0, 0, 0}, t[4] = {0, 0, 0, 0};
+  unsigned any = 0u;
+  bool bad = false;
+  const uint8_t* col = ax + c0 + 4 * word;   // Lp is a multiple of 32
+#pragma unroll 4
+  for (int s = slice; s < N; s += GAP_SLICES) {
+    const uint32_t v = *reinterpret_cast<const uint32_t*>(col + (int64_t)s * Lp);
+    sum_t w = 1;
+    bool nz = true;
+    if constexpr (!UNIT) {
+      const double wd = wgt[s];
+      const int hi = __double2hiint(wd);
+      bad |= (unsigned)hi >= 0x7ff00000u;
+      nz = ((hi << 1) | __double2loint(wd)) != 0;
+      w = (float)wd;
     }
-    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const uint32_t x = (v >> (8 * b)) & 0xFFu;
+      const bool in = x <= 16;
+      t[b] += in ? w : (sum_t)0;
+      r[b] += (x <= 15 && x != 4) ? w : (sum_t)0;
+      if constexpr (!UNIT) any |= (unsigned)(in && nz) << b;
+    }
   }
-  if (row >= 0) return;
-  const double v = (double)q, tot = __shfl_down_sync(0xffffffffu, v, 16);
-  if (top == 15 && c0 + col < L) useme[c0 + col] = (v > 0.0 && v / tot >= idthresh) ? 1 : 0;
+#pragma unroll
+  for (int b = 0; b < 4; b++) { sm.part[0][slice][4 * word + b] = r[b]; sm.part[1][slice][4 * word + b] = t[b]; }
+  if (any) atomicOr(&some, any << (4 * word));
+  if (bad) odd = 1;
+  __syncthreads();
+  if (tid < 32) {
+    sum_t rs = 0, ts = 0;
+    for (int k = 0; k < GAP_SLICES; k++) { rs += sm.part[0][k][tid]; ts += sm.part[1][k][tid]; }
+    const bool ok = c0 + tid < L;
+    if constexpr (UNIT) {
+      if (ok) useme[c0 + tid] = (rs > 0 && (double)rs / (double)ts >= idthresh) ? 1 : 0;
+    } else {
+      const float id = (float)idthresh, q = rs / ts;
+      const float margin = ((float)(N / GAP_SLICES) + 64.f) * 0x1p-22f * fmaxf(q, id);
+      const bool none = !odd && !((some >> tid) & 1u);   // no weight at all: neither sum is positive
+      const bool sure = none || (!odd && idthresh > 0.0 && ts > 1e-30f && ts < 1e30f && fabsf(q - id) > margin);
+      const unsigned hard = __ballot_sync(0xffffffffu, ok && !sure);
+      if (ok && sure) useme[c0 + tid] = !none && q > id;
+      if (tid == 0) left = hard;
+    }
+  }
+  if constexpr (!UNIT) {
+    __syncthreads();
+    unsigned hard = left;
+    const int row = tid - 32, k = tid & 15, top = (tid & 16) ? 16 : 15;   // residues up to 15, with gaps 16
+    auto stage = [&](int buf, int s) {
+      if (row < 0 || row >= GAP_ROWS || s + row >= N) return;
+      const uint4* a = reinterpret_cast<const uint4*>(ax + (int64_t)(s + row) * Lp + c0);
+      sm.row.code[buf][row][0] = a[0];
+      sm.row.code[buf][row][1] = a[1];
+      sm.row.w[buf][row] = wgt[s + row];
+    };
+    while (hard) {   // 16 columns at a time; the same in every thread
+      unsigned m = hard;
+      for (int j = 0; j < k; j++) m &= m - 1;
+      const int c = m ? __ffs(m) - 1 : 0;
+      double v = 0.0;
+      stage(0, 0);
+      __syncthreads();
+      int buf = 0;
+      for (int s0 = 0; s0 < N; s0 += GAP_ROWS, buf ^= 1) {
+        stage(buf ^ 1, s0 + GAP_ROWS);
+        if (row < 0) {
+          const int n = min(GAP_ROWS, N - s0);
+          const uint8_t* code = reinterpret_cast<const uint8_t*>(sm.row.code[buf]) + c;
+#pragma unroll 8
+          for (int s = 0; s < n; s++) {
+            const int x = code[GAP_COLS * s];
+            if (x <= top && (x != 4 || top == 16)) v += sm.row.w[buf][s];
+          }
+        }
+        __syncthreads();
+      }
+      if (row < 0) {
+        const double tot = __shfl_down_sync(0xffffffffu, v, 16);
+        if (m && top == 15) useme[c0 + c] = (v > 0.0 && v / tot >= idthresh) ? 1 : 0;
+      }
+      for (int j = 0; j < 16; j++) hard &= hard - 1;
+    }
+  }
 }
 
 __device__ __forceinline__ void gsc_codes_body(
@@ -711,7 +779,7 @@ cudaError_t launch_weights_pb(const uint8_t* ax, int N, int L, int Lp, double* i
 
 cudaError_t launch_gapfilter(const uint8_t* ax, const double* wgt, int N, int L, int Lp, double gapthresh, int* useme,
                              cudaStream_t st) {
-  const int nb = (L + GAP_COLS - 1) / GAP_COLS, thr = 32 + GAP_ROWS;
+  const int nb = (L + GAP_COLS - 1) / GAP_COLS, thr = 8 * GAP_SLICES;
   if (wgt) k_gapfilter<false><<<nb, thr, 0, st>>>(ax, wgt, N, L, Lp, 1.0 - gapthresh, useme);
   else     k_gapfilter<true><<<nb, thr, 0, st>>>(ax, wgt, N, L, Lp, 1.0 - gapthresh, useme);
   return cudaGetLastError();

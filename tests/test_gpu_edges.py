@@ -574,3 +574,41 @@ def test_a_large_workspace_is_given_back(covgpu):
     for a, b in zip(first, e.power(single=(x, x / 8), join=(x, x / 8), double=(x, x / 8))):
         assert np.array_equal(a, b)
     e.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -140, 2.0 ** -300, 2.0 ** 120, 2.0 ** 1000])
+@pytest.mark.parametrize("thr", [0.5, 0.25, 1.0, 1.5, 0.0, -0.5])
+def test_gap_filter_at_the_edges_of_its_sums(covgpu, oracle, scale, thr):
+    """Weights out of FP32's range and with zeros among them, columns without a
+    counted sequence or with weights of 0 alone, thresholds of 0 and below and
+    above 1, fractions from far to one part in 1e7 of the threshold: the
+    oracle's columns; so for a negative weight and one that is not finite."""
+    N, L = 333, 70
+    rng = np.random.default_rng(5)
+    w = rng.uniform(0.5, 2.0, N) * scale
+    w[rng.integers(0, N, 20)] = 0.0
+    ax = np.where(rng.random((N, L)) < rng.uniform(0, 1, L), 4, rng.choice([0, 1, 2, 3, 9, 16, 17], (N, L)))
+    ax[:, 0], ax[:, 1], ax[:, 2] = 17, np.where(w == 0.0, 2, 17), 4
+    half = rng.permutation(N)[:N // 2]
+    for k in range(8):   # residues and gaps of equal weight, then one residue's weight more by a little
+        ax[:, 10 + k] = 17
+        ax[half, 10 + k] = 1
+    w2 = w.copy()
+    other = np.setdiff1d(np.arange(N), half)[:len(half)]
+    w2[other] = w2[half]
+    for k in range(8):
+        ax[other, 10 + k] = 4
+    w2[half[np.flatnonzero(w2[half] > 0)[0]]] *= 1.0 + 1e-5
+    e = covgpu.Engine(N, L)
+    ax = np.ascontiguousarray(ax.astype(np.uint8))
+    e.set_alignment(0, ax)
+    cases = [w, w2]
+    for v in (-0.25 * scale, np.inf, np.nan):
+        w3 = w.copy()
+        w3[7] = v
+        cases.append(w3)
+    for x in cases:
+        with np.errstate(all="ignore"):
+            assert np.array_equal(e.gapfilter(0, x, thr), oracle.gapfilter(ax, x, thr) == 1)
+    assert np.array_equal(e.gapfilter(0, None, thr), oracle.gapfilter(ax, None, thr) == 1)
+    e.close()
