@@ -119,7 +119,7 @@ k_pb_rows(const uint8_t* __restrict__ ax, int L, int Lp, const double* __restric
 // itself, and a fraction further than twice that from the threshold is decided.
 // The first warp adds the other columns' weights in order, a lane per (column,
 // sum), while the others stage the next rows.  So are all columns where a weight is negative or not finite, the sums
-// leave FP32's range or the threshold is not positive.  Without weights the sums
+// come near the ends of FP32's range or the threshold is below 1e-6.  Without weights the sums
 // are counts, in integers.
 // The whole call, weighted / without weights: 30 x 61 40 / 35 us with a thread per
 // column that read its rows itself, 23 / 21 so; 2,000 x 1,500 410 / 344, 45 / 29
@@ -179,7 +179,7 @@ k_gapfilter(const uint8_t* __restrict__ ax, const double* __restrict__ wgt, int 
       const float id = (float)idthresh, q = rs / ts;
       const float margin = ((float)(N / GAP_SLICES) + 64.f) * 0x1p-22f * fmaxf(q, id);
       const bool none = !odd && !((some >> tid) & 1u);   // no weight at all: neither sum is positive
-      const bool sure = none || (!odd && idthresh > 0.0 && ts > 1e-30f && ts < 1e30f && fabsf(q - id) > margin);
+      const bool sure = none || (!odd && idthresh > 1e-6 && ts > 1e-20f && ts < 1e30f && fabsf(q - id) > margin);
       const unsigned hard = __ballot_sync(0xffffffffu, ok && !sure);
       if (ok && sure) useme[c0 + tid] = !none && q > id;
       if (tid == 0) left = hard;
@@ -702,7 +702,9 @@ k_gsc_upgma(double* __restrict__ D, int N, double* __restrict__ w, int G, double
   gsc_cluster_body<NR>(D, N, w, G, blockIdx.x % G, state);
 }
 
-constexpr int GSC_MAXR = 32;   // rows per lane at most
+// Rows per lane at most.  R-scape's rule takes these weights up to 1,000
+// sequences (two rows); 5 to 8 rows run in the kernel of 16.
+constexpr int GSC_MAXR = 32;
 // f(rows per lane) of the merges' kernel for N sequences
 template <class F>
 static cudaError_t gsc_with_nr(int nr, F f) {

@@ -577,7 +577,7 @@ def test_a_large_workspace_is_given_back(covgpu):
 
 
 @pytest.mark.parametrize("scale", [1.0, 2.0 ** -140, 2.0 ** -300, 2.0 ** 120, 2.0 ** 1000])
-@pytest.mark.parametrize("thr", [0.5, 0.25, 1.0, 1.5, 0.0, -0.5])
+@pytest.mark.parametrize("thr", [0.5, 0.25, 1.0, 1.0 - 1e-7, 1.5, 0.0, -0.5])
 def test_gap_filter_at_the_edges_of_its_sums(covgpu, oracle, scale, thr):
     """Weights out of FP32's range and with zeros among them, columns without a
     counted sequence or with weights of 0 alone, thresholds of 0 and below and
