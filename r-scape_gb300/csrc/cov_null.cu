@@ -4,15 +4,16 @@
 // The reconstruction depends on the columns only one by one, the replay only
 // on the branches' substitution counts and the parent's current row, so the
 // work goes in two parts:
-//   k_fitch_cols   a CTA per (16 columns, null), the whole tree in its shared
-//                  memory: the up pass of Tree_FitchAlgorithmAncenstral /
-//                  tree_fitch_column (src/msatree.c:173-227, 1700-1838):
-//                  intersection of the children's sets over the five states,
-//                  else the union of residues only (tree_fitch_upwards
-//                  :1877-1908), as byte-SIMD; the root's state; the down pass
-//                  (keep the parent's state when the child's set holds it);
-//                  and the substitutions of each kind on each branch, added
-//                  over the columns into the branch's 25 counters.
+//   k_fitch_cols   a CTA per (4 to 32 columns, null), the whole tree in its
+//                  shared memory where it fits: the up pass of
+//                  Tree_FitchAlgorithmAncenstral / tree_fitch_column
+//                  (src/msatree.c:173-227, 1700-1838): intersection of the
+//                  children's sets over the five states, else the union of
+//                  residues only (tree_fitch_upwards :1877-1908), as
+//                  byte-SIMD; the root's state; the down pass (keep the
+//                  parent's state when the child's set holds it); and the
+//                  substitutions of each kind on each branch, added over the
+//                  columns into the branch's 25 counters.
 //   the replay     the root's row with the columns shuffled
 //                  (msamanip_ShuffleColumns, src/msamanip.c:1164-1233; only
 //                  the root's shuffled row is ever read, every other row is
